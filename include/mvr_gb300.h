@@ -202,7 +202,9 @@ MVR_API int mvr_block_grid(const long long dims[3], const int kernel_size[3], co
 /* runIterations: `iterations` more iterations.  stats (or NULL) receives per iteration
  * and view-step {sumChange, maxChange} (Seq: num_views steps, Mul: 1 step).  With stats NULL
  * the block voxels outside the regions written back to psi (which the reference computes
- * and discards) are not computed; psi is bit-identical either way. */
+ * and discards) are not computed, and a view-step whose blocks all read psi before the step
+ * runs in FFT domains of the library's choice instead of the blocks' (odd kernel sizes, no
+ * dropped block, no forced schedule); psi is the same either way up to float rounding. */
 MVR_API int mvr_decon_run(mvr_decon *h, int iterations, double *stats);
 /* runIterations with the inputs on the host (no reference counterpart as one call: the
  * reference driver holds images, weights and psi in host memory and copies blocks per call):

@@ -487,20 +487,21 @@ int Engine<T>::set_schedule(Plan<T> &pl, int code)
 
 template <typename T>
 int Engine<T>::make_plan(Plan<T> &pl, const int b[3], const float *k1, const int kd1[3], const float *k2,
-                         const int kd2[3], bool k_on_device)
+                         const int kd2[3], bool k_on_device, int boundary)
 {
+    if (boundary < 0) boundary = boundary_;
     if (stream_ == nullptr) return fail(ERR_STATE, "engine not initialised");
     for (int d = 0; d < 3; ++d) {
         if (b[d] < 1 || kd1[d] < 1) return fail(ERR_ARG, "block and kernel sizes must be >= 1");
         if (k2 && kd2[d] != kd1[d]) return fail(ERR_ARG, "kernel1 and kernel2 must have the same size");
-        if (kd1[d] > b[d] && boundary_ == BOUNDARY_CIRCULAR)
+        if (kd1[d] > b[d] && boundary == BOUNDARY_CIRCULAR)
             return fail(ERR_ARG, "kernel larger than the block under circular boundary");
     }
     free_plan(pl);
     for (int d = 0; d < 3; ++d) {
         pl.b[d] = b[d];
         pl.kd[d] = kd1[d];
-        if (boundary_ == BOUNDARY_CIRCULAR) {
+        if (boundary == BOUNDARY_CIRCULAR) {
             pl.P[d] = b[d];
             pl.L[d] = 0;
             if (!fft_friendly(b[d]) || (d == 0 && (b[d] & 1)))
@@ -1169,6 +1170,298 @@ int Engine<T>::convolve(const Plan<T> &pl, const T *blk, int src_kind, float *ou
     ua.store = out;
     ua.partials = partials_;
     return launch_update(pl, bms, 1, S0_, ua, EPI_STORE, 0.0, nullptr);
+}
+
+// ---- separable transforms (sep.cuh) -------------------------------------------------------
+const std::vector<int> &sep_lengths(int axis)
+{
+    static const auto all = [](int (*up)(int)) {
+        std::vector<int> v;
+        for (int n = up(1); n; n = up(n + 1)) v.push_back(n);
+        return v;
+    };
+    static const std::vector<int> x = all(sep_len_x), yz = all(sep_len_yz);
+    return axis == 0 ? x : yz;
+}
+
+bool split_axis(int N, int k, const std::vector<int> &lens, bool even_lo, AxisTiles &out)
+{
+    const int r = k / 2, slack = even_lo ? 1 : 0;
+    if (r + (even_lo && (r & 1) ? 1 : 0) > N - 1) return false;
+    long long best = 0;
+    int P = 0, n = 0;
+    for (int len : lens) {
+        long long cnt;
+        if (len >= N + 2 * r + (even_lo ? (r & 1) : 0)) {
+            cnt = 1;
+        } else {
+            const long long edge = len - 3 * r - slack, inner = len - 4 * r - slack;
+            if (inner < 1) continue;
+            cnt = 2 + (2 * edge >= N ? 0 : (N - 2 * edge + inner - 1) / inner);
+        }
+        if (P == 0 || cnt * len < best) {
+            best = cnt * len;
+            P = len;
+            n = (int)cnt;
+        }
+        if (cnt == 1) break;
+    }
+    if (P == 0) return false;
+    out.P = P;
+    out.tiles.clear();
+    int e0 = 0;
+    for (int i = 0; i < n; ++i) {
+        const int cap = P - (i == 0 || i == n - 1 ? 3 : 4) * r - slack;
+        const int e1 = i == n - 1 ? N : std::min(N, e0 + cap);
+        SepAxis a;
+        a.lo = std::max(e0 - 2 * r, -r);
+        if (even_lo && (a.lo & 1)) --a.lo;
+        a.N = N;
+        a.v0 = std::max(a.lo, 0);
+        a.nv = std::min(N, a.lo + P) - a.v0;
+        a.q0 = std::max(e0 - r, 0);
+        a.nq = std::min(e1 + r, N) - a.q0;
+        a.w0 = e0;
+        a.nw = e1 - e0;
+        if (a.nw > 0) out.tiles.push_back(a);
+        e0 = e1;
+    }
+    return true;
+}
+
+namespace {
+// Tiles per launch: enough of the small ones to fill the device, at most 512 MB of spectrum.
+constexpr long long kSepBatchElems = 1LL << 26;
+
+inline SepTiles sep_tiles(const SepTile *t, int nt, int &planes)
+{
+    SepTiles tl{};
+    planes = 1;
+    for (int i = 0; i < nt; ++i) {
+        tl.t[i] = t[i];
+        planes = std::max(planes, t[i].a[2].nv);
+    }
+    return tl;
+}
+inline long long sep_elems(const int P[3]) { return ((long long)(P[0] / 32) * 16 + 1) * P[1] * P[2]; }
+inline UpdConst upd_const(double lambda, float minI, float maxI)
+{
+    UpdConst c;
+    c.minI = minI;
+    c.maxI = maxI;
+    c.inv_maxI = 1.0f / maxI;
+    c.two_lambda = (float)(2.0 * lambda);
+    c.tik = lambda > 0;
+    return c;
+}
+inline int max_rows(const SepTile *t, int nt)
+{
+    int m = 1;
+    for (int i = 0; i < nt; ++i) m = std::max(m, t[i].a[1].nw * t[i].a[2].nw);
+    return m;
+}
+}  // namespace
+
+template <typename T>
+int Engine<T>::sep_batch(const int P[3]) const
+{
+    return (int)std::max<long long>(1, std::min<long long>(kSepMaxTiles, kSepBatchElems / sep_elems(P)));
+}
+
+template <typename T>
+int Engine<T>::sep_reserve(const int P[3], int nt, bool mul, long long voxels, long long rows)
+{
+    MVR_TRY(reserve(sep_elems(P), 0, sep_row_ctas((int)rows), nt));
+    return mul ? reserve_prod(voxels) : (int)OK;
+}
+
+template <typename T>
+void Engine<T>::sep_free(SepPlan &pl)
+{
+    for (float2 **p : {&pl.twx, &pl.twy, &pl.twz, &pl.k1h, &pl.k2h}) {
+        cudaFree(*p);
+        *p = nullptr;
+    }
+}
+
+template <typename T>
+int Engine<T>::sep_make(SepPlan &pl, const int P[3], const float *k1, const float *k2, const int kd[3], bool on_device)
+{
+    if constexpr (sizeof(T) != sizeof(float)) {
+        return fail(ERR_STATE, "separable transforms are FP32 only");
+    } else {
+        if (stream_ == nullptr) return fail(ERR_STATE, "engine not initialised");
+        sep_free(pl);
+        for (int d = 0; d < 3; ++d) {
+            pl.P[d] = P[d];
+            pl.kd[d] = kd[d];
+        }
+        std::string e;
+        pl.twx = dev_twiddles_impl<float2>(P[0], stream_, e);
+        pl.twy = dev_twiddles_impl<float2>(P[1], stream_, e);
+        pl.twz = dev_twiddles_impl<float2>(P[2], stream_, e);
+        if (!pl.twx || !pl.twy || !pl.twz) return fail(ERR_CUDA, "twiddle upload: " + e);
+        const long long kn = (long long)kd[0] * kd[1] * kd[2];
+        if (!on_device && kn > kcap_) {
+            cudaFree(kbuf_);
+            kbuf_ = nullptr;
+            kcap_ = 0;
+            MVR_CUDA(cudaMalloc(&kbuf_, sizeof(float) * (size_t)kn));
+            kcap_ = kn;
+        }
+        MVR_TRY(reserve(sep_elems(P), 0, 1, 1));
+        MVR_CUDA(cudaMalloc(&pl.k1h, sizeof(float2) * (size_t)sep_elems(P)));
+        MVR_CUDA(cudaMalloc(&pl.k2h, sizeof(float2) * (size_t)sep_elems(P)));
+        const SepGeom g = sep_geom(P, kd[2]);
+        SepTiles tl{};
+        for (int d = 0; d < 3; ++d) tl.t[0].a[d].N = P[d];
+        for (int which = 0; which < 2; ++which) {
+            const float *k = which ? k2 : k1;
+            if (!on_device) {
+                MVR_CUDA(cudaMemcpyAsync(kbuf_, k, sizeof(float) * (size_t)kn, cudaMemcpyHostToDevice, stream_));
+                k = kbuf_;
+            }
+            SepSrc src{k, 1, {kd[0], kd[1], kd[2]}, 1.0 / ((double)P[0] * P[1] * P[2])};
+            launches_ += 3;
+            MVR_CUDA(sep_x_fwd(g, tl, 1, src, S0_, pl.twx, stream_));
+            MVR_CUDA(sep_y_fwd(g, tl, 1, SEP_KERNEL, kd, S0_, pl.twy, stream_));
+            MVR_CUDA(sep_z(g, tl, 1, SEP_KERNEL, 0, kd, S0_, which ? pl.k2h : pl.k1h, nullptr, pl.twz, stream_));
+        }
+        MVR_CUDA(cudaStreamSynchronize(stream_));
+        return OK;
+    }
+}
+
+// conv1 and the quotient's transform along x: psi to S0 (x, y; kept when another view needs it
+// again), times K1^ into S1, back to rows, quotient.  fresh: S0 does not hold psi's transform yet.
+template <typename T>
+int Engine<T>::sep_conv1(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, const float *psi,
+                         const float *img, float2 *S0, float2 *S1, bool fresh)
+{
+    double nv = 0.0, sv = 0.0, yv = 0.0, zq = 0.0, sq = 0.0, nq = 0.0;
+    for (int i = 0; i < nt; ++i) {
+        const SepAxis *a = tl.t[i].a;
+        nv += (double)a[0].nv * a[1].nv * a[2].nv;
+        sv += (double)g.nxb * 16 * a[1].nv * a[2].nv;
+        yv += (double)g.nxb * 16 * g.P[1] * a[2].nv;
+        zq += (double)g.nxb * 16 * g.P[1] * a[2].nq;
+        sq += (double)g.nxb * 16 * a[1].nq * a[2].nq;
+        nq += (double)a[0].nq * a[1].nq * a[2].nq;
+    }
+    const double kb = 8.0 * (double)sep_elems(g.P);
+    if (fresh) {
+        MVR_TRY(prof_begin(KK_ROWS_FWD, 4.0 * nv + 8.0 * sv));
+        MVR_CUDA(sep_x_fwd(g, tl, nt, SepSrc{psi, 0, {0, 0, 0}, 1.0}, S0, pl.twx, stream_));
+        MVR_TRY(prof_end());
+        MVR_TRY(prof_begin(KK_COLS_FWD, 8.0 * (sv + yv)));
+        MVR_CUDA(sep_y_fwd(g, tl, nt, SEP_MIRROR, nullptr, S0, pl.twy, stream_));
+        MVR_TRY(prof_end());
+    }
+    MVR_TRY(prof_begin(KK_COLS_ZMUL, 8.0 * (yv + zq) + kb));
+    MVR_CUDA(sep_z(g, tl, nt, SEP_MIRROR, 0, nullptr, S0, S1, pl.k1h, pl.twz, stream_));
+    MVR_TRY(prof_end());
+    MVR_TRY(prof_begin(KK_COLS_INV, 8.0 * (zq + sq)));
+    MVR_CUDA(sep_y_inv(g, tl, nt, 0, S1, pl.twy, stream_));
+    MVR_TRY(prof_end());
+    MVR_TRY(prof_begin(KK_ROWS_RATIO, 16.0 * sq + 4.0 * nq));
+    MVR_CUDA(sep_x_ratio(g, tl, nt, img, S1, pl.twx, stream_));
+    return prof_end();
+}
+
+// The second convolution of the quotient rows in S and the update.
+template <typename T>
+int Engine<T>::sep_finish(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, int epi, const SepUpd &u,
+                          float2 *S, double *stats_dev)
+{
+    double sq = 0.0, zq = 0.0, zw = 0.0, sw = 0.0, nw = 0.0;
+    for (int i = 0; i < nt; ++i) {
+        const SepAxis *a = tl.t[i].a;
+        sq += (double)g.nxb * 16 * a[1].nq * a[2].nq;
+        zq += (double)g.nxb * 16 * g.P[1] * a[2].nq;
+        zw += (double)g.nxb * 16 * g.P[1] * a[2].nw;
+        sw += (double)g.nxb * 16 * a[1].nw * a[2].nw;
+        nw += (double)a[0].nw * a[1].nw * a[2].nw;
+    }
+    MVR_TRY(prof_begin(KK_COLS_FWD, 8.0 * (sq + zq)));
+    MVR_CUDA(sep_y_fwd(g, tl, nt, SEP_FILL, nullptr, S, pl.twy, stream_));
+    MVR_TRY(prof_end());
+    MVR_TRY(prof_begin(KK_COLS_ZMUL, 8.0 * (zq + zw) + 8.0 * (double)sep_elems(g.P)));
+    MVR_CUDA(sep_z(g, tl, nt, SEP_FILL, 1, nullptr, S, S, pl.k2h, pl.twz, stream_));
+    MVR_TRY(prof_end());
+    MVR_TRY(prof_begin(KK_COLS_INV, 8.0 * (zw + sw)));
+    MVR_CUDA(sep_y_inv(g, tl, nt, 1, S, pl.twy, stream_));
+    MVR_TRY(prof_end());
+    const double per = epi == EPI_SEQ ? 12.0 : (epi == EPI_MUL_FIRST ? 8.0 : (epi == EPI_MUL_ACC ? 16.0 : 16.0 + 4.0 * u.nviews));
+    MVR_TRY(prof_begin(KK_ROWS_UPDATE, 8.0 * sw + per * nw));
+    MVR_CUDA(sep_x_update(g, tl, nt, epi, u, S, pl.twx, stream_));
+    MVR_TRY(prof_end());
+    if (stats_dev && (epi == EPI_SEQ || epi == EPI_MUL_FINAL)) {
+        const int slots = sep_row_ctas(max_rows(tl.t, nt));
+        MVR_TRY(prof_begin(KK_REDUCE, 16.0 * slots * nt));
+        k_reduce_stats<double><<<nt, 1024, 0, stream_>>>(u.partials, slots, stats_dev);
+        MVR_LAUNCHED("k_reduce_stats");
+        MVR_TRY(prof_end());
+    }
+    return OK;
+}
+
+template <typename T>
+int Engine<T>::sep_seq(const SepPlan &pl, const SepTile *tiles, int nt, const float *psi_src, float *psi_dst,
+                       const float *img, const float *w, float maxI, double *stats_dev)
+{
+    if constexpr (sizeof(T) != sizeof(float)) {
+        return fail(ERR_STATE, "separable transforms are FP32 only");
+    } else {
+        if (!pl.ready()) return fail(ERR_STATE, "kernels not set for this view");
+        if (nt < 1 || nt > kSepMaxTiles) return fail(ERR_ARG, "1..16 tiles per launch");
+        MVR_TRY(sep_reserve(pl.P, nt, false, 0, max_rows(tiles, nt)));
+        int planes;
+        const SepTiles tl = sep_tiles(tiles, nt, planes);
+        const SepGeom g = sep_geom(pl.P, planes);
+        MVR_TRY(sep_conv1(pl, g, tl, nt, psi_src, img, S0_, S0_, true));
+        SepUpd u{};
+        u.psi = psi_src;
+        u.dst = psi_dst;
+        u.weight[0] = w;
+        u.nviews = 1;
+        u.c = upd_const(lambda_, min_value_, maxI);
+        u.partials = stats_dev ? partials_ : nullptr;
+        return sep_finish(pl, g, tl, nt, EPI_SEQ, u, S0_, stats_dev);
+    }
+}
+
+template <typename T>
+int Engine<T>::sep_mul(const std::vector<const SepPlan *> &pls, const SepTile *tiles, int nt, const float *psi_src,
+                       float *psi_dst, const float *const *imgs, const float *const *ws, float maxI, double *stats_dev)
+{
+    if constexpr (sizeof(T) != sizeof(float)) {
+        return fail(ERR_STATE, "separable transforms are FP32 only");
+    } else {
+        const int nv = (int)pls.size();
+        if (nv < 1 || nv > kMaxViews) return fail(ERR_ARG, "number of views must be 1..16");
+        if (nt < 1 || nt > kSepMaxTiles) return fail(ERR_ARG, "1..16 tiles per launch");
+        for (const SepPlan *pl : pls)
+            if (!pl->ready()) return fail(ERR_STATE, "kernels not set for a view");
+        const SepAxis *a = tiles[0].a;
+        MVR_TRY(sep_reserve(pls[0]->P, nt, nv > 1, (long long)a[0].N * a[1].N * a[2].N, max_rows(tiles, nt)));
+        int planes;
+        const SepTiles tl = sep_tiles(tiles, nt, planes);
+        const SepGeom g = sep_geom(pls[0]->P, planes);
+        SepUpd u{};
+        u.psi = psi_src;
+        u.dst = psi_dst;
+        for (int v = 0; v < nv; ++v) u.weight[v] = ws[v];
+        u.nviews = nv;
+        u.prod = reinterpret_cast<float2 *>(prod_);
+        u.c = upd_const(lambda_, min_value_, maxI);
+        u.partials = stats_dev ? partials_ : nullptr;
+        for (int v = 0; v < nv; ++v) {
+            MVR_TRY(sep_conv1(*pls[v], g, tl, nt, psi_src, imgs[v], S0_, S1_, v == 0));
+            const int epi = v == nv - 1 ? EPI_MUL_FINAL : (v == 0 ? EPI_MUL_FIRST : EPI_MUL_ACC);
+            MVR_TRY(sep_finish(*pls[v], g, tl, nt, epi, u, S1_, stats_dev));
+        }
+        return OK;
+    }
 }
 
 template class Engine<float>;

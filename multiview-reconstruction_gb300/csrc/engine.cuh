@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "sep.cuh"
 
 namespace mvr {
 
@@ -78,6 +79,29 @@ struct Plan {
 //   path 3: the pair kernels (a cluster of two CTAs per plane, persistent).
 enum { SCHED_ROWS = 0, SCHED_PLANE = 1, SCHED_PLANE_PERSIST = 2, SCHED_PAIR = 3, SCHED_ZPIPE = 4 };
 
+// FFT domain of the separable transforms (sep.cuh) for one kernel pair, and its spectra.
+struct SepPlan {
+    int P[3] = {0, 0, 0};
+    int kd[3] = {0, 0, 0};
+    float2 *twx = nullptr, *twy = nullptr, *twz = nullptr;
+    float2 *k1h = nullptr, *k2h = nullptr;
+    bool ready() const { return k2h != nullptr; }
+};
+
+// One axis split into tiles: a region of N voxels, convolved with a kernel of k voxels twice, in
+// FFT domains of length P.  A tile that writes [w0, w0 + nw) needs psi on twice the kernel's
+// reach either side, and only once the reach beyond a face of the region.
+struct AxisTiles {
+    int P = 0;
+    std::vector<SepAxis> tiles;
+};
+// The split with the fewest transformed voxels (tiles x P) over the lengths `lens` (ascending);
+// false when there is none, or when the mirror extension would reflect twice (reach >= N).
+// even_lo: tiles start at even coordinates (8-byte loads of pairs along x).
+bool split_axis(int N, int k, const std::vector<int> &lens, bool even_lo, AxisTiles &out);
+// The lengths sep.cuh has passes for.
+const std::vector<int> &sep_lengths(int axis);
+
 // Where the block's output goes (volume driver) or the block itself (block API).
 struct BlockPlace {
     const void *psi_src = nullptr;  // T volume (mirror-single read)
@@ -103,8 +127,22 @@ public:
     // Plan for (block b, kernel kd); k1/k2 are host arrays (k2 may be null). Kernel
     // spectra are computed on the device.
     int make_plan(Plan<T> &pl, const int b[3], const float *k1, const int kd1[3], const float *k2,
-                  const int kd2[3], bool k_on_device = false);
+                  const int kd2[3], bool k_on_device = false, int boundary = -1);
     void free_plan(Plan<T> &pl);
+
+    // Separable transforms (FP32 engines): spectra of k1 / k2 (host or device) on the domain P,
+    // and one Seq step of view plan pl, or one Mul step of all views, over `nt` tiles of one
+    // region.  Only the tiles' written voxels are updated; stats_dev: 2 doubles per tile, over
+    // those voxels, or NULL.
+    int sep_make(SepPlan &pl, const int P[3], const float *k1, const float *k2, const int kd[3], bool on_device);
+    void sep_free(SepPlan &pl);
+    int sep_seq(const SepPlan &pl, const SepTile *tiles, int nt, const float *psi_src, float *psi_dst, const float *img,
+                const float *w, float maxI, double *stats_dev);
+    int sep_mul(const std::vector<const SepPlan *> &pls, const SepTile *tiles, int nt, const float *psi_src,
+                float *psi_dst, const float *const *imgs, const float *const *ws, float maxI, double *stats_dev);
+    // Tiles per launch for a domain, and the scratch a launch of nt tiles takes (allocated here).
+    int sep_batch(const int P[3]) const;
+    int sep_reserve(const int P[3], int nt, bool mul, long long voxels, long long rows);
     // The FFT schedules a plan admits (codes SCHED_*), and the one in use.
     int kernel_spectra(Plan<T> &pl, const float *k1, const float *k2, bool k_on_device);
     std::vector<int> schedule_candidates(const Plan<T> &pl) const;
@@ -169,6 +207,10 @@ private:
     int launch_update(const Plan<T> &pl, const BlockMaps &bms, int nb, V *S, const UpdateArgs &ua, int epi,
                       double bytes, double *stats_dev);
     BlockMaps block_maps(const Plan<T> &pl, const BlockPlace *bps, int nb) const;
+    int sep_conv1(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, const float *psi, const float *img,
+                  float2 *S0, float2 *S1, bool fresh);
+    int sep_finish(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, int epi, const SepUpd &u, float2 *S,
+                   double *stats_dev);
 
     int device_ = -1;
     int boundary_ = BOUNDARY_REFERENCE;

@@ -1,0 +1,126 @@
+"""Iterations without statistics run on the library's own tiles of the volume (separable
+transforms, csrc/sep.cuh): every transform length, volumes of more than one tile, odd and even
+rows, Seq and Mul, against the oracle driver on the caller's block grid.
+
+Tolerance: relative L2 1e-5 after one iteration (the FP32 bound of one iteration elsewhere), 1e-6
+against the same GPU iteration on the caller's blocks (float rounding of two transforms).
+"""
+import os
+
+import numpy as np
+import pytest
+
+import mvrgb300 as M
+import oracle as O
+import synthetic
+
+pytestmark = pytest.mark.gpu
+
+LEN_X = (64, 96, 128, 160, 192, 224, 256, 288, 320, 384, 448, 512, 576)
+LEN_YZ = (32, 48, 64, 80, 96, 112, 128, 144, 160, 192, 224, 256, 288, 320, 360, 400, 432, 480, 576)
+
+
+def rel(a, b):
+    a = np.asarray(a, dtype=np.float64)
+    b = np.asarray(b, dtype=np.float64)
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+def case(dims, kd, nv, seed):
+    rng = np.random.default_rng(seed)
+    shape = dims[::-1]
+    imgs = [rng.uniform(5, 200, shape).astype(np.float32) for _ in range(nv)]
+    for im in imgs:
+        im[rng.random(shape) < 0.02] = 0  # voxels without data
+    ws = [rng.uniform(0.2, 0.9, shape).astype(np.float32) for _ in range(nv)]
+    psfs = [synthetic.make_psf(kd, 1.0, 1.5, 40.0 * v) for v in range(nv)]
+    psi = rng.uniform(5, 150, shape).astype(np.float32)
+    return imgs, ws, psfs, psi
+
+
+def run(dims, kd, block, mul, blocks, seed, nv=2, its=1):
+    imgs, ws, psfs, psi = case(dims, kd, nv, seed)
+    old = os.environ.get("MVR_RATIO_BAND")
+    if blocks:
+        os.environ["MVR_RATIO_BAND"] = "0"  # keeps the steps on the caller's blocks
+    try:
+        with M.Deconvolution(dims, nv, block, mul=mul, psf_type=M.PSF_INDEPENDENT, lam=0.006) as d:
+            for v in range(nv):
+                d.set_view(v, imgs[v], ws[v], psfs[v])
+            d.prepare()
+            d.set_psi(psi)
+            ks = [d.kernels(v, psfs[v].shape) for v in range(nv)]
+            mx = d.max_intensities()
+            d.run_iterations(its)
+            out = d.get_psi()
+    finally:
+        if blocks:
+            if old is None:
+                del os.environ["MVR_RATIO_BAND"]
+            else:
+                os.environ["MVR_RATIO_BAND"] = old
+    return out, (psi, imgs, ws, [k[0] for k in ks], [k[1] for k in ks], mx)
+
+
+def check(dims, kd, block, mul, seed):
+    out, (psi, imgs, ws, k1s, k2s, mx) = run(dims, kd, block, mul, False, seed)
+    ref, _ = O.decon_run(psi, imgs, ws, k1s, k2s, block, 1, mul=mul, lam=0.006, max_intensities=mx)
+    assert np.isfinite(out).all()
+    assert rel(out, ref) <= 1e-5
+    assert rel(out, run(dims, kd, block, mul, True, seed)[0]) <= 1e-6
+
+
+@pytest.mark.parametrize("axis,n", [(0, n) for n in LEN_X] + [(a, n) for a in (1, 2) for n in LEN_YZ])
+def test_every_length_filled_to_the_last_voxel(axis, n):
+    # the volume and the kernel's reach (2 either side) fill the domain of n along one axis
+    dims = [37, 26, 22]
+    dims[axis] = n - 4
+    block = [48, 36, 36]
+    block[axis] = 96
+    check(tuple(dims), (5, 5, 5), tuple(block), bool((n // 16) % 2), n + axis)
+
+
+@pytest.mark.parametrize("dims,kd,block,mul", [
+    ((573, 26, 22), (5, 5, 5), (96, 36, 36), False),   # one voxel too long for one tile, each axis
+    ((38, 573, 22), (5, 7, 5), (48, 96, 36), True),
+    ((37, 26, 573), (7, 5, 5), (48, 36, 96), False),
+    ((590, 580, 9), (5, 5, 3), (160, 160, 20), False),  # four tiles
+    ((8, 9, 7), (3, 5, 7), (20, 20, 28), True),        # smaller than every length
+    ((64, 31, 47), (31, 15, 31), (128, 64, 128), False),  # the reach covers half of the volume
+    ((16, 8, 16), (31, 15, 31), (64, 32, 64), False),   # reach = size - 1: one reflection still suffices
+])
+def test_tiles_and_short_volumes(dims, kd, block, mul):
+    check(dims, kd, block, mul, sum(dims))
+
+
+def test_what_stays_on_the_blocks():
+    # even kernels, a kernel that reflects twice, a dropped block: the grid decides the result there
+    for dims, kd, block in (((36, 30, 44), (4, 6, 5), (40, 40, 40)), ((15, 30, 30), (31, 5, 5), (64, 32, 32))):
+        a, _ = run(dims, kd, block, False, False, 3)
+        b, _ = run(dims, kd, block, False, True, 3)
+        assert rel(a, b) <= 1e-6
+
+
+def test_unaligned_device_volumes():
+    # device images and weights on 4-byte boundaries (no 8-byte loads), even row length
+    torch = pytest.importorskip("torch")
+    dims, kd, block = (64, 30, 26), (5, 5, 5), (48, 36, 36)
+    imgs, ws, psfs, psi = case(dims, kd, 2, 11)
+    ref, _ = run(dims, kd, block, False, False, 11)
+    n = psi.size
+    keep = []
+    with M.Deconvolution(dims, 2, block, psf_type=M.PSF_INDEPENDENT, lam=0.006) as d:
+        for v in range(2):
+            p = []
+            for a in (imgs[v], ws[v]):
+                t = torch.empty(n + 1, dtype=torch.float32, device="cuda")
+                t[1:].copy_(torch.from_numpy(a.reshape(-1)))
+                keep.append(t)
+                p.append(t[1:].data_ptr())
+            torch.cuda.synchronize()
+            d.set_view_device(v, p[0], p[1], psfs[v])
+        d.prepare()
+        d.set_psi(psi)
+        d.run_iterations(1)
+        out = d.get_psi()
+    assert np.array_equal(out, ref)
