@@ -785,12 +785,6 @@ bool sched_env_forced()
         if (std::getenv(v)) return true;
     return false;
 }
-// any switch of the block kernels: the steps stay on the caller's blocks
-bool block_env_forced()
-{
-    const char *band = std::getenv("MVR_RATIO_BAND");
-    return sched_env_forced() || std::getenv("MVR_PAIR_KERNELS") || (band && band[0] == '0');
-}
 }  // namespace
 
 // DeconViewPSF.init 119-254 for all views in order.
@@ -1059,7 +1053,7 @@ int Decon<T>::make_tiles()
 {
     tiles_.assign(num_steps(), {});
     for (auto &vw : views_) free_tiles(vw);
-    if (force_sched_ >= 0 || block_env_forced()) return MVR_OK;
+    if (force_sched_ >= 0 || block_kernels_forced()) return MVR_OK;
     for (int st = 0; st < num_steps(); ++st) {
         if (!jacobi_[st]) continue;
         const int rc = make_step_tiles(st);
@@ -1094,7 +1088,7 @@ int Decon<T>::run_tiles(int st)
         for (size_t i = 0; i < tiles.size(); i += (size_t)per) {
             const int nt = (int)std::min<size_t>(per, tiles.size() - i);
             if (p_.mul)
-                D_TRY(eng(engine_.sep_mul(pls, &tiles[i], nt, psi_, stage_, imgs.data(), ws.data(), (float)miv, nullptr)));
+                D_TRY(eng(engine_.sep_mul(pls, std::vector<const SepTile *>(pls.size(), &tiles[i]).data(), nt, psi_, stage_, imgs.data(), ws.data(), (float)miv, nullptr)));
             else
                 D_TRY(eng(engine_.sep_seq(vw.sep, &tiles[i], nt, psi_, stage_, vw.img, vw.w, max_[st], nullptr)));
         }

@@ -1199,7 +1199,7 @@ bool split_axis(int N, int k, const std::vector<int> &lens, bool even_lo, AxisTi
             if (inner < 1) continue;
             cnt = 2 + (2 * edge >= N ? 0 : (N - 2 * edge + inner - 1) / inner);
         }
-        if (P == 0 || cnt * len < best) {
+        if (P == 0 || cnt * len <= best) {  // fewer tiles on a tie
             best = cnt * len;
             P = len;
             n = (int)cnt;
@@ -1227,6 +1227,33 @@ bool split_axis(int N, int k, const std::vector<int> &lens, bool even_lo, AxisTi
         e0 = e1;
     }
     return true;
+}
+
+bool block_tile(const int b[3], const int kd[3], int boundary, int P[3], SepTile &tile)
+{
+    for (int d = 0; d < 3; ++d) {
+        const std::vector<int> &lens = sep_lengths(d);
+        if (boundary == BOUNDARY_CIRCULAR) {
+            if (kd[d] > b[d] || !std::binary_search(lens.begin(), lens.end(), b[d])) return false;
+            P[d] = b[d];
+            tile.a[d] = SepAxis{0, b[d], 0, b[d], 0, b[d], 0, b[d]};
+        } else {
+            AxisTiles ax;  // the smallest length that holds the block and the reach either side
+            const int r = kd[d] / 2;
+            const auto fit = std::lower_bound(lens.begin(), lens.end(), b[d] + 2 * r + (d == 0 ? r & 1 : 0));
+            if (fit == lens.end() || !split_axis(b[d], kd[d], {*fit}, d == 0, ax)) return false;
+            P[d] = ax.P;
+            tile.a[d] = ax.tiles[0];
+        }
+    }
+    return true;
+}
+
+bool block_kernels_forced()
+{
+    for (const char *v : {"MVR_PLANE_KERNELS", "MVR_XY_PERSIST", "MVR_COLS_PIPE", "MVR_PAIR_KERNELS"})
+        if (std::getenv(v)) return true;
+    return ratio_band_off();
 }
 
 namespace {
@@ -1431,8 +1458,9 @@ int Engine<T>::sep_seq(const SepPlan &pl, const SepTile *tiles, int nt, const fl
 }
 
 template <typename T>
-int Engine<T>::sep_mul(const std::vector<const SepPlan *> &pls, const SepTile *tiles, int nt, const float *psi_src,
-                       float *psi_dst, const float *const *imgs, const float *const *ws, float maxI, double *stats_dev)
+int Engine<T>::sep_mul(const std::vector<const SepPlan *> &pls, const SepTile *const *tiles, int nt,
+                       const float *psi_src, float *psi_dst, const float *const *imgs, const float *const *ws,
+                       float maxI, double *stats_dev)
 {
     if constexpr (sizeof(T) != sizeof(float)) {
         return fail(ERR_STATE, "separable transforms are FP32 only");
@@ -1440,13 +1468,11 @@ int Engine<T>::sep_mul(const std::vector<const SepPlan *> &pls, const SepTile *t
         const int nv = (int)pls.size();
         if (nv < 1 || nv > kMaxViews) return fail(ERR_ARG, "number of views must be 1..16");
         if (nt < 1 || nt > kSepMaxTiles) return fail(ERR_ARG, "1..16 tiles per launch");
-        for (const SepPlan *pl : pls)
-            if (!pl->ready()) return fail(ERR_STATE, "kernels not set for a view");
-        const SepAxis *a = tiles[0].a;
-        MVR_TRY(sep_reserve(pls[0]->P, nt, nv > 1, (long long)a[0].N * a[1].N * a[2].N, max_rows(tiles, nt)));
-        int planes;
-        const SepTiles tl = sep_tiles(tiles, nt, planes);
-        const SepGeom g = sep_geom(pls[0]->P, planes);
+        const SepAxis *a = tiles[0][0].a;
+        for (int v = 0; v < nv; ++v) {
+            if (!pls[v]->ready()) return fail(ERR_STATE, "kernels not set for a view");
+            MVR_TRY(sep_reserve(pls[v]->P, nt, nv > 1, (long long)a[0].N * a[1].N * a[2].N, max_rows(tiles[v], nt)));
+        }
         SepUpd u{};
         u.psi = psi_src;
         u.dst = psi_dst;
@@ -1456,7 +1482,12 @@ int Engine<T>::sep_mul(const std::vector<const SepPlan *> &pls, const SepTile *t
         u.c = upd_const(lambda_, min_value_, maxI);
         u.partials = stats_dev ? partials_ : nullptr;
         for (int v = 0; v < nv; ++v) {
-            MVR_TRY(sep_conv1(*pls[v], g, tl, nt, psi_src, imgs[v], S0_, S1_, v == 0));
+            int planes;
+            const SepTiles tl = sep_tiles(tiles[v], nt, planes);
+            const SepGeom g = sep_geom(pls[v]->P, planes);
+            const bool same = v > 0 && std::memcmp(pls[v]->P, pls[v - 1]->P, sizeof(pls[v]->P)) == 0 &&
+                              std::memcmp(tiles[v], tiles[v - 1], sizeof(SepTile) * (size_t)nt) == 0;
+            MVR_TRY(sep_conv1(*pls[v], g, tl, nt, psi_src, imgs[v], S0_, S1_, !same));
             const int epi = v == nv - 1 ? EPI_MUL_FINAL : (v == 0 ? EPI_MUL_FIRST : EPI_MUL_ACC);
             MVR_TRY(sep_finish(*pls[v], g, tl, nt, epi, u, S1_, stats_dev));
         }

@@ -99,6 +99,12 @@ struct AxisTiles {
 // false when there is none, or when the mirror extension would reflect twice (reach >= N).
 // even_lo: tiles start at even coordinates (8-byte loads of pairs along x).
 bool split_axis(int N, int k, const std::vector<int> &lens, bool even_lo, AxisTiles &out);
+// The one tile of a block under the engine's boundary rule: the mirror-single / value-1 extension
+// around the block, or the block itself as a periodic domain.  false: no separable transforms.
+bool block_tile(const int b[3], const int kd[3], int boundary, int P[3], SepTile &tile);
+// One of the environment switches of the block kernels is set (MVR_PLANE_KERNELS, MVR_XY_PERSIST,
+// MVR_COLS_PIPE, MVR_PAIR_KERNELS, MVR_RATIO_BAND=0): no separable transforms.
+bool block_kernels_forced();
 // The lengths sep.cuh has passes for.
 const std::vector<int> &sep_lengths(int axis);
 
@@ -138,7 +144,8 @@ public:
     void sep_free(SepPlan &pl);
     int sep_seq(const SepPlan &pl, const SepTile *tiles, int nt, const float *psi_src, float *psi_dst, const float *img,
                 const float *w, float maxI, double *stats_dev);
-    int sep_mul(const std::vector<const SepPlan *> &pls, const SepTile *tiles, int nt, const float *psi_src,
+    // tiles: one array per view (views with one domain share psi's transform along x and y)
+    int sep_mul(const std::vector<const SepPlan *> &pls, const SepTile *const *tiles, int nt, const float *psi_src,
                 float *psi_dst, const float *const *imgs, const float *const *ws, float maxI, double *stats_dev);
     // Tiles per launch for a domain, and the scratch a launch of nt tiles takes (allocated here).
     int sep_batch(const int P[3]) const;
@@ -181,6 +188,7 @@ public:
     int prof_end();
     int profile_collect(KernelProfile &out);  // synchronises, then adds the pending times
     int device() const { return device_; }
+    int boundary() const { return boundary_; }
     const std::string &error() const { return err_; }
     int fail(int code, const std::string &msg);
     int cuda_check(cudaError_t e, const char *what);

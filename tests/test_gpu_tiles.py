@@ -124,3 +124,82 @@ def test_unaligned_device_volumes():
         d.run_iterations(1)
         out = d.get_psi()
     assert np.array_equal(out, ref)
+
+
+@pytest.mark.parametrize("b,kd,boundary", [
+    ((64, 32, 48), (5, 7, 9), M.BOUNDARY_CIRCULAR),
+    ((96, 112, 80), (9, 5, 15), M.BOUNDARY_CIRCULAR),
+    ((59, 43, 28), (5, 5, 5), M.BOUNDARY_REFERENCE),   # domain 64 x 48 x 32, filled
+    ((60, 45, 29), (5, 5, 5), M.BOUNDARY_REFERENCE),   # one voxel more on every axis
+    ((31, 30, 27), (6, 4, 8), M.BOUNDARY_REFERENCE),   # even kernels
+])
+def test_block_iteration_on_separable_transforms(b, kd, boundary):
+    # the whole block and its statistics (reference boundary), the effective region (circular)
+    rng = np.random.default_rng(sum(b))
+    shape = b[::-1]
+    k1 = synthetic.make_psf(kd, 1.0, 1.5, 30.0)
+    k2 = O.invert_kernel(k1)
+    img = rng.uniform(5, 300, shape).astype(np.float32)
+    img[rng.random(shape) < 0.05] = 0
+    w = rng.uniform(0, 1, shape).astype(np.float32)
+    psi = rng.uniform(5, 300, shape).astype(np.float32)
+    ref, ref_st = O.block_seq(psi, img, w, k1, k2, 0.006, 1e-4, 300.0)
+    with M.BlockWorker(b, 1e-4, 0.006, 1, boundary) as wk:
+        wk.set_kernels(0, k1, k2)
+        out = psi.copy()
+        st = wk.run_iteration(0, out, img, w, 300.0)
+    if boundary == M.BOUNDARY_CIRCULAR:
+        e = [k - 1 for k in kd]
+        sl = tuple(slice(e[d], b[d] - e[d]) for d in (2, 1, 0))
+        assert rel(out[sl], ref[sl]) <= 1e-5
+        ch = out.astype(np.float64) - psi
+        assert st.sum_change == pytest.approx(float(ch.sum()), rel=1e-4, abs=1e-2)
+        assert st.max_change == pytest.approx(float(ch.max()), rel=1e-5)
+    else:
+        assert rel(out, ref) <= 1e-5
+        scale = float(np.abs(out.astype(np.float64) - psi).sum()) + 1.0
+        assert abs(st.sum_change - ref_st[0]) <= 1e-4 * scale
+        assert abs(st.max_change - ref_st[1]) <= 1e-4 * max(1.0, abs(ref_st[1]))
+
+
+def test_mul_block_with_one_view_off_the_separable_path():
+    # a 21-voxel kernel reflects twice in a block of 8 rows: its view has no separable transforms,
+    # and the Mul step of both views runs on the block kernels
+    b = (40, 8, 24)
+    rng = np.random.default_rng(5)
+    shape = b[::-1]
+    psi = rng.uniform(5, 300, shape).astype(np.float32)
+    imgs = [rng.uniform(5, 300, shape).astype(np.float32) for _ in range(2)]
+    ws = [rng.uniform(0, 0.5, shape).astype(np.float32) for _ in range(2)]
+    k1s = [synthetic.make_psf(k, 1.0, 1.5, 20.0) for k in ((5, 5, 5), (5, 21, 5))]
+    k2s = [O.invert_kernel(k) for k in k1s]
+    ref, _ = O.block_mul(psi, imgs, ws, k1s, k2s, 0.006, 1e-4, [300.0, 280.0])
+    with M.BlockWorker(b, 1e-4, 0.006, 2, M.BOUNDARY_REFERENCE) as wk:
+        for v in range(2):
+            wk.set_kernels(v, k1s[v], k2s[v])
+        out = psi.copy()
+        wk.run_iteration_mul(out, imgs, ws, [300.0, 280.0])
+        assert rel(out, ref) <= 1e-5
+        one = psi.copy()  # the first view alone keeps its own path
+        wk.run_iteration(0, one, imgs[0], ws[0], 300.0)
+    r0, _ = O.block_seq(psi, imgs[0], ws[0], k1s[0], k2s[0], 0.006, 1e-4, 300.0)
+    assert rel(one, r0) <= 1e-5
+
+
+def test_mul_block_with_kernels_of_two_sizes():
+    b = (40, 36, 24)
+    rng = np.random.default_rng(6)
+    shape = b[::-1]
+    psi = rng.uniform(5, 300, shape).astype(np.float32)
+    imgs = [rng.uniform(5, 300, shape).astype(np.float32) for _ in range(3)]
+    ws = [rng.uniform(0, 0.4, shape).astype(np.float32) for _ in range(3)]
+    k1s = [synthetic.make_psf(k, 1.0, 1.5, 20.0) for k in ((5, 5, 5), (5, 5, 5), (9, 15, 7))]
+    k2s = [O.invert_kernel(k) for k in k1s]
+    mx = [300.0, 280.0, 260.0]
+    ref, _ = O.block_mul(psi, imgs, ws, k1s, k2s, 0.006, 1e-4, mx)
+    with M.BlockWorker(b, 1e-4, 0.006, 3, M.BOUNDARY_REFERENCE) as wk:
+        for v in range(3):
+            wk.set_kernels(v, k1s[v], k2s[v])
+        out = psi.copy()
+        wk.run_iteration_mul(out, imgs, ws, mx)
+    assert rel(out, ref) <= 1e-5
