@@ -1195,7 +1195,8 @@ bool split_axis(int N, int k, const std::vector<int> &lens, bool even_lo, AxisTi
         if (len >= N + 2 * r + (even_lo ? (r & 1) : 0)) {
             cnt = 1;
         } else {
-            const long long edge = len - 3 * r - slack, inner = len - 4 * r - slack;
+            // even splits with even starts: pairs stay whole
+            const long long edge = (len - 3 * r - slack) & ~slack, inner = (len - 4 * r - slack) & ~slack;
             if (inner < 1) continue;
             cnt = 2 + (2 * edge >= N ? 0 : (N - 2 * edge + inner - 1) / inner);
         }
@@ -1211,7 +1212,7 @@ bool split_axis(int N, int k, const std::vector<int> &lens, bool even_lo, AxisTi
     out.tiles.clear();
     int e0 = 0;
     for (int i = 0; i < n; ++i) {
-        const int cap = P - (i == 0 || i == n - 1 ? 3 : 4) * r - slack;
+        const int cap = (P - (i == 0 || i == n - 1 ? 3 : 4) * r - slack) & ~slack;
         const int e1 = i == n - 1 ? N : std::min(N, e0 + cap);
         SepAxis a;
         a.lo = std::max(e0 - 2 * r, -r);
@@ -1271,6 +1272,21 @@ inline SepTiles sep_tiles(const SepTile *t, int nt, int &planes)
     return tl;
 }
 inline long long sep_elems(const int P[3]) { return ((long long)(P[0] / 32) * 16 + 1) * P[1] * P[2]; }
+// The geometry of a batch, with the L2 priority rule: when the batch's spectra fit L2 but not
+// together with K1^, K2^ and the volumes of a view-step, those pass through evict-first (4-view
+// 256^3, 85 MB of spectrum: y and z passes 4 % faster; everything in L2, 2 views of 128 x 128 x 64,
+// or the spectrum far larger, 6 views of 512 x 512 x 256: the hint costs 6 % and 2 %).
+inline SepGeom sep_batch_geom(const int P[3], const SepTile *t, int nt, int planes, int device)
+{
+    SepGeom g = sep_geom(P, planes);
+    int l2 = 0;
+    if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device) != cudaSuccess) l2 = 0;
+    const double s = 8.0 * (double)g.stride * nt, k = 16.0 * (double)sep_elems(P);
+    double vol = 0.0;
+    for (int i = 0; i < nt; ++i) vol += 16.0 * t[i].a[0].nv * t[i].a[1].nv * t[i].a[2].nv;
+    g.stream = s <= l2 && s + k + vol > l2 ? 1 : 0;
+    return g;
+}
 inline UpdConst upd_const(double lambda, float minI, float maxI)
 {
     UpdConst c;
@@ -1298,7 +1314,7 @@ int Engine<T>::sep_batch(const int P[3]) const
 template <typename T>
 int Engine<T>::sep_reserve(const int P[3], int nt, bool mul, long long voxels, long long rows)
 {
-    MVR_TRY(reserve(sep_elems(P), 0, sep_row_ctas((int)rows), nt));
+    MVR_TRY(reserve(sep_elems(P), 0, sep_row_ctas(P[0], (int)rows), nt));
     return mul ? reserve_prod(voxels) : (int)OK;
 }
 
@@ -1423,7 +1439,7 @@ int Engine<T>::sep_finish(const SepPlan &pl, const SepGeom &g, const SepTiles &t
     MVR_CUDA(sep_x_update(g, tl, nt, epi, u, S, pl.twx, stream_));
     MVR_TRY(prof_end());
     if (stats_dev && (epi == EPI_SEQ || epi == EPI_MUL_FINAL)) {
-        const int slots = sep_row_ctas(max_rows(tl.t, nt));
+        const int slots = sep_row_ctas(g.P[0], max_rows(tl.t, nt));
         MVR_TRY(prof_begin(KK_REDUCE, 16.0 * slots * nt));
         k_reduce_stats<double><<<nt, 1024, 0, stream_>>>(u.partials, slots, stats_dev);
         MVR_LAUNCHED("k_reduce_stats");
@@ -1444,7 +1460,7 @@ int Engine<T>::sep_seq(const SepPlan &pl, const SepTile *tiles, int nt, const fl
         MVR_TRY(sep_reserve(pl.P, nt, false, 0, max_rows(tiles, nt)));
         int planes;
         const SepTiles tl = sep_tiles(tiles, nt, planes);
-        const SepGeom g = sep_geom(pl.P, planes);
+        const SepGeom g = sep_batch_geom(pl.P, tiles, nt, planes, device_);
         MVR_TRY(sep_conv1(pl, g, tl, nt, psi_src, img, S0_, S0_, true));
         SepUpd u{};
         u.psi = psi_src;
@@ -1484,7 +1500,7 @@ int Engine<T>::sep_mul(const std::vector<const SepPlan *> &pls, const SepTile *c
         for (int v = 0; v < nv; ++v) {
             int planes;
             const SepTiles tl = sep_tiles(tiles[v], nt, planes);
-            const SepGeom g = sep_geom(pls[v]->P, planes);
+            const SepGeom g = sep_batch_geom(pls[v]->P, tiles[v], nt, planes, device_);
             const bool same = v > 0 && std::memcmp(pls[v]->P, pls[v - 1]->P, sizeof(pls[v]->P)) == 0 &&
                               std::memcmp(tiles[v], tiles[v - 1], sizeof(SepTile) * (size_t)nt) == 0;
             MVR_TRY(sep_conv1(*pls[v], g, tl, nt, psi_src, imgs[v], S0_, S1_, !same));

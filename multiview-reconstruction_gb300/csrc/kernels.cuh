@@ -476,21 +476,37 @@ __global__ void __launch_bounds__(256) k_rows_ratio(typename Cx<T>::t *__restric
 // power-of-two exponent (stored as a float pair, 8 bytes per voxel; every factor is split
 // with frexpf first, so no partial product under- or overflows).  Zero, signed, Inf and NaN
 // factors propagate as in the double product.
+// frexpf from the bits of an ordinary number (the function handles zeros, subnormals, Inf and NaN).
+__device__ __forceinline__ float mulprod_split(float c, int &e)
+{
+    const unsigned b = __float_as_uint(c), ex = (b >> 23) & 255u;
+    if (ex - 1u < 254u) {
+        e = (int)ex - 126;
+        return __uint_as_float((b & 0x807fffffu) | 0x3f000000u);
+    }
+    return frexpf(c, &e);
+}
 __device__ __forceinline__ float2 mulprod_first(float c)
 {
     int e;
-    const float m = frexpf(c, &e);
+    const float m = mulprod_split(c, e);
     return make_float2(m, (float)e);
 }
 __device__ __forceinline__ float2 mulprod_acc(float2 p, float c)
 {
     int ec, e2;
-    const float mc = frexpf(c, &ec);
-    const float m = frexpf(__fmul_rn(p.x, mc), &e2);
+    const float mc = mulprod_split(c, ec);
+    const float m = mulprod_split(__fmul_rn(p.x, mc), e2);
     return make_float2(m, p.y + (float)(ec + e2));
 }
-// pow(prod, 1 / V) rounded to float: 2^(e / V) split into an integer power q and a
-// remainder r < V, so the float power function only sees m 2^r in [0.5, 2^(V-1)).
+__device__ __forceinline__ float mulprod_scale(float y, int q)
+{
+    return q >= -126 && q <= 126 ? y * __uint_as_float((unsigned)(q + 127) << 23) : ldexpf(y, q);
+}
+// pow(prod, 1 / V) rounded to float: 2^(e / V) split into an integer power q and a remainder
+// r < V, so that the root is taken of x = m 2^r in [0.5, 2^(V-1)): the approximate exponential of
+// the approximate logarithm (about 1e-6 off), then one Newton step on y^V = x, which squares
+// that error, so that the rounding of x / y^(V-1), divided by V, is what remains.
 // Math.pow of a negative base with the non-integer exponent 1 / V (V >= 2) is NaN.
 __device__ __forceinline__ float mulprod_root(float2 p, int V)
 {
@@ -500,11 +516,20 @@ __device__ __forceinline__ float mulprod_root(float2 p, int V)
     if (m == 0.0f) return 0.0f;
     if (!(m > 0.0f)) return __int_as_float(0x7fc00000);  // negative or NaN
     if (isinf(m)) return m;
-    const int q = e >= 0 ? e / V : -((V - 1 - e) / V);
-    const int r = e - q * V;
-    const float x = ldexpf(m, r);
-    const float y = V == 2 ? __fsqrt_rn(x) : powf(x, 1.0f / (float)V);
-    return ldexpf(y, q);
+    // floor(e / V): the half keeps the quotient 1 / (2 V) away from the integers
+    const float iv = __fdividef(1.0f, (float)V);
+    const int q = __float2int_rd(((float)e + 0.5f) * iv);
+    const float x = mulprod_scale(m, e - q * V);
+    float y;
+    if (V == 2) {
+        y = __fsqrt_rn(x);
+    } else {
+        y = exp2f(__log2f(x) * iv);
+        float t = y * y;
+        for (int k = 3; k < V; ++k) t *= y;
+        y = fmaf(__fdividef(x, t) - y, iv, y);
+    }
+    return mulprod_scale(y, q);
 }
 
 // ---- C2R -> update -------------------------------------------------------------------

@@ -58,7 +58,11 @@ int sep_len_yz(int n)
     return 0;
 }
 
-int sep_row_ctas(int rows) { return (rows + kSepRows - 1) / kSepRows; }
+int sep_row_ctas(int Px, int rows)
+{
+    const SxOps *o = sx_ops(Px);
+    return o ? (rows + o->rows - 1) / o->rows : 0;
+}
 
 cudaError_t sep_x_fwd(const SepGeom &g, const SepTiles &tl, int nt, const SepSrc &src, float2 *S, const float2 *twx,
                       cudaStream_t s)
@@ -67,7 +71,7 @@ cudaError_t sep_x_fwd(const SepGeom &g, const SepTiles &tl, int nt, const SepSrc
     if (!o) return cudaErrorInvalidValue;
     const int rows = src.kernel ? src.kd[1] * src.kd[2]
                                 : tile_max(tl, nt, [](const SepTile &t) { return t.a[1].nv * t.a[2].nv; });
-    return o->fwd(g, tl, nt, sep_row_ctas(rows), src, S, aligned8(src.vol), twx, s);
+    return o->fwd(g, tl, nt, sep_row_ctas(g.P[0], rows), src, S, aligned8(src.vol), twx, s);
 }
 
 cudaError_t sep_x_ratio(const SepGeom &g, const SepTiles &tl, int nt, const float *img, float2 *S, const float2 *twx,
@@ -76,7 +80,7 @@ cudaError_t sep_x_ratio(const SepGeom &g, const SepTiles &tl, int nt, const floa
     const SxOps *o = sx_ops(g.P[0]);
     if (!o) return cudaErrorInvalidValue;
     const int rows = tile_max(tl, nt, [](const SepTile &t) { return t.a[1].nq * t.a[2].nq; });
-    return o->ratio(g, tl, nt, sep_row_ctas(rows), img, S, aligned8(img), twx, s);
+    return o->ratio(g, tl, nt, sep_row_ctas(g.P[0], rows), img, S, aligned8(img), twx, s);
 }
 
 cudaError_t sep_x_update(const SepGeom &g, const SepTiles &tl, int nt, int epi, const SepUpd &u, const float2 *S,
@@ -86,7 +90,7 @@ cudaError_t sep_x_update(const SepGeom &g, const SepTiles &tl, int nt, int epi, 
     if (!o) return cudaErrorInvalidValue;
     const int rows = tile_max(tl, nt, [](const SepTile &t) { return t.a[1].nw * t.a[2].nw; });
     const bool vec = aligned8(u.psi) && aligned8(u.dst) && aligned8(u.weight[0]);
-    return o->update(g, tl, nt, sep_row_ctas(rows), epi, u, S, vec, twx, s);
+    return o->update(g, tl, nt, sep_row_ctas(g.P[0], rows), epi, u, S, vec, twx, s);
 }
 
 cudaError_t sep_y_fwd(const SepGeom &g, const SepTiles &tl, int nt, int map, const int kd[3], float2 *S,

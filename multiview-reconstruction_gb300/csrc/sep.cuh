@@ -44,6 +44,7 @@ struct SepGeom {
     int nxb;           // column blocks, Px / 32
     int Zs;            // planes a tile's spectrum buffer holds
     long long stride;  // complex values per tile: nxb Zs Py 16 + Zs Py
+    int stream;        // 1: volumes and K^ pass through L2 with the evict-first priority
 };
 inline SepGeom sep_geom(const int P[3], int planes)
 {
@@ -52,6 +53,7 @@ inline SepGeom sep_geom(const int P[3], int planes)
     g.nxb = P[0] / 32;
     g.Zs = planes;
     g.stride = ((long long)g.nxb * 16 + 1) * planes * P[1];
+    g.stream = 0;
     return g;
 }
 
@@ -76,8 +78,8 @@ struct SepUpd {
     double *partials;     // {sum, max} per CTA, or NULL: no statistics
 };
 
-// x passes.  Rows are taken 32 to a CTA; slots of the partials: sep_row_ctas per tile.
-int sep_row_ctas(int rows);
+// x passes.  CTAs per tile of a pass over `rows` rows, and slots of its partials.
+int sep_row_ctas(int Px, int rows);
 cudaError_t sep_x_fwd(const SepGeom &g, const SepTiles &tl, int nt, const SepSrc &src, float2 *S, const float2 *twx,
                       cudaStream_t s);
 cudaError_t sep_x_ratio(const SepGeom &g, const SepTiles &tl, int nt, const float *img, float2 *S, const float2 *twx,

@@ -6,6 +6,36 @@
 
 namespace mvr {
 
+// Global accesses with an L2 priority chosen at run time (SepGeom::stream): evict-first for what
+// a pass reads or writes once, so that the spectrum that the next pass reads stays in L2.
+__device__ __forceinline__ unsigned long long sep_policy(int stream)
+{
+    unsigned long long p;
+    if (stream) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    else asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ float sep_ld(const float *p, unsigned long long pol)
+{
+    float v;
+    asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ float2 sep_ld2(const void *p, unsigned long long pol)
+{
+    float2 v;
+    asm("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ void sep_st(float *p, float v, unsigned long long pol)
+{
+    asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(p), "f"(v), "l"(pol) : "memory");
+}
+__device__ __forceinline__ void sep_st2(void *p, float2 v, unsigned long long pol)
+{
+    asm volatile("st.global.L2::cache_hint.v2.f32 [%0], {%1, %2}, %3;" ::"l"(p), "f"(v.x), "f"(v.y), "l"(pol) : "memory");
+}
+
 // cos / sin of 2 pi j / n at compile time: the angle is reduced to the first octant by symmetry,
 // then the Taylor series (in double; the constants are rounded to float where they are used).
 struct SepCs {
@@ -58,6 +88,44 @@ __device__ __forceinline__ float2 sep_rot(float2 v, float c, float s)
     return INV ? make_float2(v.x * c - v.y * s, v.y * c + v.x * s) : make_float2(v.x * c + v.y * s, v.y * c - v.x * s);
 }
 
+// a + s b, both components with one fused paired instruction
+__device__ __forceinline__ float2 sep_fma(float2 a, float2 b, float s)
+{
+#if MVR_PAIRED_FP && defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+    return __ffma2_rn(b, make_float2(s, s), a);
+#else
+    return make_float2(fmaf(b.x, s, a.x), fmaf(b.y, s, a.y));
+#endif
+}
+// (m - i n, m + i n) forward, the reverse inverse
+template <bool INV>
+__device__ __forceinline__ void sep_pm(float2 m, float2 n, float2 &p, float2 &q)
+{
+    p = make_float2(m.x + n.y, m.y - n.x);
+    q = make_float2(m.x - n.y, m.y + n.x);
+    if (INV) {
+        const float2 t = p;
+        p = q;
+        q = t;
+    }
+}
+
+// 5 points with fused products: 14 paired instructions and 8 additions
+template <bool INV>
+__device__ __forceinline__ void sep_dft5(float2 *v)
+{
+    constexpr SepTab<5> t = sep_tab<5>();
+    const float2 a1 = cadd(v[1], v[4]), a2 = cadd(v[2], v[3]);
+    const float2 b1 = csub(v[1], v[4]), b2 = csub(v[2], v[3]);
+    const float2 m1 = sep_fma(sep_fma(v[0], a1, t.c[1]), a2, t.c[2]);
+    const float2 m2 = sep_fma(sep_fma(v[0], a1, t.c[2]), a2, t.c[1]);
+    const float2 n1 = sep_fma(cscale(b1, t.s[1]), b2, t.s[2]);
+    const float2 n2 = sep_fma(cscale(b1, t.s[2]), b2, -t.s[1]);
+    v[0] = cadd(v[0], cadd(a1, a2));
+    sep_pm<INV>(m1, n1, v[1], v[4]);
+    sep_pm<INV>(m2, n2, v[2], v[3]);
+}
+
 template <bool INV>
 __device__ __forceinline__ void dft7(float2 *v)
 {
@@ -72,21 +140,13 @@ __device__ __forceinline__ void dft7(float2 *v)
     v[0] = cadd(v0, cadd(a[0], cadd(a[1], a[2])));
 #pragma unroll
     for (int k = 1; k <= 3; ++k) {
-        float2 m = v0, n = make_float2(0.0f, 0.0f);
+        float2 m = v0, n = cscale(b[0], t.s[k]);
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            const float c = t.c[((q + 1) * k) % 7], s = t.s[((q + 1) * k) % 7];
-            m = make_float2(fmaf(a[q].x, c, m.x), fmaf(a[q].y, c, m.y));
-            n = make_float2(fmaf(b[q].x, s, n.x), fmaf(b[q].y, s, n.y));
+            m = sep_fma(m, a[q], t.c[((q + 1) * k) % 7]);
+            if (q) n = sep_fma(n, b[q], t.s[((q + 1) * k) % 7]);
         }
-        // forward m - i n, inverse m + i n
-        if (INV) {
-            v[k] = make_float2(m.x - n.y, m.y + n.x);
-            v[7 - k] = make_float2(m.x + n.y, m.y - n.x);
-        } else {
-            v[k] = make_float2(m.x + n.y, m.y - n.x);
-            v[7 - k] = make_float2(m.x - n.y, m.y + n.x);
-        }
+        sep_pm<INV>(m, n, v[k], v[7 - k]);
     }
 }
 
@@ -133,7 +193,7 @@ __device__ __forceinline__ void sep_dft(float2 *v)
     if constexpr (N == 2) dft2<INV>(v);
     else if constexpr (N == 3) dft3<INV>(v);
     else if constexpr (N == 4) dft4<INV>(v);
-    else if constexpr (N == 5) dft5<INV>(v);
+    else if constexpr (N == 5) sep_dft5<INV>(v);
     else if constexpr (N == 6) dft6<INV>(v);
     else if constexpr (N == 7) dft7<INV>(v);
     else if constexpr (N == 8) dft8<INV>(v);

@@ -1,7 +1,7 @@
 // x passes of the separable transforms (layout and tiles: sep.cuh): real rows of Px = 32 V, as
 // m = 16 V packed complex values.
 //
-// A CTA of V warps takes 32 rows (consecutive stored rows y, then z).  Phase 1, item (row, t < 16):
+// A CTA takes 32 or 16 rows (consecutive stored rows y, then z).  Phase 1, item (row, t < 16):
 // V-point DFT over the packed values t + 16 v, times W_m^(t k1); phase 2, item (row, k1): 16-point
 // DFT over t, frequency k1 + V k2 at k2, fused with the packed-real split (which pairs f with
 // m - f, held by item V - k1 of the same row: lanes 0-15 and 16-31 of one warp take the two, the
@@ -10,8 +10,9 @@
 // pieces of a row touch every bank once), and the lines move between shared and global memory
 // 16 bytes a thread, 4 rows (512 contiguous bytes) a warp.
 //
-// Three to seven CTAs per SM, so that one CTA's loads overlap another's transforms: the
-// passes are bound by instruction issue and HBM traffic together.
+// Three or more CTAs per SM, so that one CTA's loads overlap another's transforms: the passes are
+// bound by instruction issue and HBM traffic together.  65536 rows of 288 reals (one view of 256^3),
+// algorithmic bytes: forward 38 us (3.8 TB/s), quotient 54 us (4.1 TB/s), update 60 us (4.6 TB/s).
 #pragma once
 #include "pdl.cuh"
 #include "rows_warp.cuh"
@@ -21,37 +22,50 @@
 
 namespace mvr {
 
-constexpr int kSepRows = 32;  // rows per CTA
-constexpr int kSepRS = 18;    // complex values per row of a column block in shared memory
+constexpr int kSepRS = 18;  // complex values per row of a column block in shared memory
 
+// 32 rows and a warp per phase-2 unit up to V = 10; 16 rows above (half the shared memory and twice
+// the CTAs per SM for the same threads), with 256 threads for V = 12 ... 16 so that phase 1 is
+// one full round.
 template <int V>
 struct SxShape {
-    static constexpr int m = 16 * V, Px = 32 * V, NT = 32 * V;
-    static constexpr int BS = kSepRows * kSepRS;  // complex values per column block
-    static constexpr int MINB = NT > 512 ? 1 : (NT == 512 ? 2 : (896 / NT > 8 ? 8 : 896 / NT));
+    static constexpr int m = 16 * V, Px = 32 * V;
+    static constexpr int R = V >= 12 ? 16 : 32;  // rows per CTA
+    static constexpr int NT = V >= 12 && V <= 16 ? 256 : R * V;
+    static constexpr int BS = R * kSepRS;        // complex values per column block
+    static constexpr int UNITS = V * R / 32;     // phase-2 units of a warp each
+    // CTAs per SM for a register budget sized to `threads` threads per SM
+    static constexpr int minb(int threads) { return NT > threads ? 1 : (threads / NT > 8 ? 8 : threads / NT); }
+    // measured on 65536 rows of 288 (4-view 256^3) and of 576: forward 37.6 us at 1152 (40.7 at 896),
+    // quotient 53.7 us at 896 (56.2 at 1152), Seq update 60 us at 896 (75 at 1152); update of the
+    // lengths that load a chunk at a time, 285 us at 1152 (361 at 896)
+    static constexpr int MINB_FWD = minb(1152), MINB_RATIO = minb(896), MINB_UPD = minb(V < 12 ? 896 : 1152);
     static constexpr size_t smem = sizeof(float2) * (size_t)(V * BS + Px);
 };
 
 // Row tables of a CTA (static shared memory).
+template <int V>
 struct SxRows {
-    long long a[kSepRows], b[kSepRows];  // row bases in the volume (-1: no row) and in the spectrum
+    long long a[SxShape<V>::R], b[SxShape<V>::R];  // row bases in the volume (-1: no row) and in the spectrum
 };
 
-// x phase 2 with the packed-real split (forward) or merge (inverse), one unit per warp.
+// x phase 2 with the packed-real split (forward) or merge (inverse), one unit per warp and round.
 template <int V, bool INV>
 __device__ __forceinline__ void sx_p2(float2 *A, const float2 *twx)
 {
-    constexpr int T = 16;
-    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr int T = 16, RB = SxShape<V>::R / 16;
+    const int l = threadIdx.x & 31;
+    for (int w = threadIdx.x >> 5; w < SxShape<V>::UNITS; w += SxShape<V>::NT / 32) {
     int k1, row, h;
     bool self;
     if (V % 2 == 0) {  // pairs (1, V-1) ... and last (0, V/2), 16 rows each
-        const int jp = w >> 1;
+        const int jp = w / RB;
         h = l >> 4;
-        row = (w & 1) * 16 + (l & 15);
+        row = (w % RB) * 16 + (l & 15);
         self = jp == V / 2 - 1;
         k1 = self ? (h ? V / 2 : 0) : (h ? V - 1 - jp : 1 + jp);
     } else {  // pairs (1, V-1) ... on 16 rows, and k1 = 0 on 32 rows
+        static_assert(V % 2 == 0 || RB == 2, "odd V: 32 rows");
         self = w == V - 1;
         const int jp = w >> 1;
         h = self ? 0 : l >> 4;
@@ -101,73 +115,132 @@ __device__ __forceinline__ void sx_p2(float2 *A, const float2 *twx)
     if (INV) sep_dft<T, true>(b);
 #pragma unroll
     for (int t = 0; t < T / 2; ++t) p[t] = make_float4(b[2 * t].x, b[2 * t].y, b[2 * t + 1].x, b[2 * t + 1].y);
+    }
+}
+
+// Twiddles in shared memory: W_Px^f for the split (f < m), then W_m^(t k1) at m + 16 k1 + t, so that
+// the 16 lanes of a row read one line (W_Px^(2 t k1) from the plain table is up to a 16-way bank
+// conflict: forward 40.8 -> 37.6 us, quotient 55.6 -> 53.7 us on 65536 rows of 288, forward 135 -> 115 us
+// on the rows of 576 of a 512 x 512 x 256 view).
+template <int V>
+__device__ __forceinline__ void sx_twiddles(float2 *tw, const float2 *__restrict__ twg)
+{
+    typedef SxShape<V> SH;
+    for (int i = threadIdx.x; i < SH::m; i += SH::NT) {
+        tw[i] = __ldg(&twg[i]);
+        tw[SH::m + i] = __ldg(&twg[2 * (i & 15) * (i >> 4)]);
+    }
 }
 
 template <int V, bool INV>
 __device__ __forceinline__ void sx_p1(float2 (&a)[V], const float2 *twx, int t)
 {
+    const float2 *w = twx + SxShape<V>::m + t;
     if (!INV) {
         sep_dft<V, false>(a);
 #pragma unroll
-        for (int k1 = 1; k1 < V; ++k1) a[k1] = cmul(a[k1], twx[2 * t * k1]);
+        for (int k1 = 1; k1 < V; ++k1) a[k1] = cmul(a[k1], w[16 * k1]);
     } else {
 #pragma unroll
-        for (int k1 = 1; k1 < V; ++k1) a[k1] = cmul(a[k1], cconj(twx[2 * t * k1]));
+        for (int k1 = 1; k1 < V; ++k1) a[k1] = cmul(a[k1], cconj(w[16 * k1]));
         sep_dft<V, true>(a);
     }
 }
 
-// The CTA's lines from shared memory to the spectrum, and back (cp.async).
-template <int V>
-__device__ __forceinline__ void sx_store_lines(float2 *S, long long bstride, const float2 *A, const long long *rowb)
+// The CTA's lines between shared memory and the spectrum: a thread keeps its 16-byte piece q of a
+// row and walks the column blocks (one pointer step each).  f(shared piece, global piece, row
+// exists), the row's base checked once per row.
+template <int V, class F>
+__device__ __forceinline__ void sx_lines(float2 *A, float2 *S, long long bstride, const long long *rowb, F f)
 {
+    typedef SxShape<V> SH;
+    constexpr int per = 8 * SH::R;                            // pieces per column block
+    constexpr int G = SH::NT >= per ? SH::NT / per : 1;       // column blocks at a time
+    constexpr int step = SH::NT >= per ? SH::R : SH::NT / 8;  // rows at a time
+    const int tid = threadIdx.x;
+    if (G * per < SH::NT && tid >= G * per) return;
+    const int g = G > 1 ? tid / per : 0, q = tid & 7;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int i = threadIdx.x + k * SxShape<V>::NT;
-        const int q = i & 7, row = (i >> 3) & 31, k1 = i >> 8;
-        if (rowb[row] >= 0)
-            *reinterpret_cast<float4 *>(S + k1 * bstride + rowb[row] + 2 * q) =
-                *reinterpret_cast<const float4 *>(A + k1 * SxShape<V>::BS + row * kSepRS + 2 * q);
+    for (int r0 = 0; r0 < SH::R; r0 += step) {
+        const int row = r0 + ((tid - g * per) >> 3);
+        if (SH::R % step != 0 && row >= SH::R) break;
+        const long long rb = rowb[row];
+        float2 *a = A + g * SH::BS + row * kSepRS + 2 * q;
+        float2 *p = S + (rb >= 0 ? rb + 2 * q + g * bstride : 0);
+#pragma unroll
+        for (int k1 = 0; k1 < V; k1 += G) {
+            if (V % G == 0 || k1 + g < V) f(a + k1 * SH::BS, p, rb >= 0);
+            p += rb >= 0 ? G * bstride : 0;
+        }
     }
+}
+template <int V>
+__device__ __forceinline__ void sx_store_lines(float2 *S, long long bstride, float2 *A, const long long *rowb)
+{
+    sx_lines<V>(A, S, bstride, rowb, [](float2 *a, float2 *p, bool ok) {
+        if (ok) *reinterpret_cast<float4 *>(p) = *reinterpret_cast<const float4 *>(a);
+    });
 }
 template <int V>
 __device__ __forceinline__ void sx_load_lines(float2 *A, const float2 *S, long long bstride, const long long *rowb)
 {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int i = threadIdx.x + k * SxShape<V>::NT;
-        const int q = i & 7, row = (i >> 3) & 31, k1 = i >> 8;
-        const bool ok = rowb[row] >= 0;
-        const unsigned d = (unsigned)__cvta_generic_to_shared(A + k1 * SxShape<V>::BS + row * kSepRS + 2 * q);
-        const float2 *s = S + (ok ? k1 * bstride + rowb[row] + 2 * q : 0);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(s), "r"(ok ? 16 : 0) : "memory");
-    }
+    sx_lines<V>(A, const_cast<float2 *>(S), bstride, rowb, [](float2 *a, float2 *p, bool ok) {
+        const unsigned d = (unsigned)__cvta_generic_to_shared(a);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(p), "r"(ok ? 16 : 0) : "memory");
+    });
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
-// The two voxels at x = g, g + 1 of a volume row under the mirror-single extension.
-__device__ __forceinline__ float2 sx_pair(const float *__restrict__ row, int g, int N, bool vec)
+// Pairs of voxels (x, x + 1) of a volume row at x = g0 + 32 v, v < V, with zeros outside
+// [x0, x0 + n).  PAIRS: no pair is split by the range and every row starts on 8 bytes, so that a
+// pair is one predicated 8-byte load.
+template <int V, bool PAIRS>
+__device__ __forceinline__ void sx_load_zero(float2 (&a)[V], const float *row, int g0, int x0, int n,
+                                             unsigned long long pol)
 {
-    if (g >= 0 && g + 1 < N) {
-        if (vec) return __ldg(reinterpret_cast<const float2 *>(row + g));
-        return make_float2(__ldg(row + g), __ldg(row + g + 1));
+    const float *p = row + g0;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        const int r = g0 - x0 + 32 * v;
+        if (PAIRS) {
+            a[v] = (unsigned)r < (unsigned)n ? sep_ld2(p + 32 * v, pol) : make_float2(0.0f, 0.0f);
+        } else {
+            a[v].x = (unsigned)r < (unsigned)n ? sep_ld(p + 32 * v, pol) : 0.0f;
+            a[v].y = (unsigned)(r + 1) < (unsigned)n ? sep_ld(p + 32 * v + 1, pol) : 0.0f;
+        }
     }
-    const int a = abs(g), b = abs(g + 1), top = 2 * N - 2;
-    return make_float2(__ldg(row + min(max(min(a, top - a), 0), N - 1)), __ldg(row + min(max(min(b, top - b), 0), N - 1)));
 }
-// The same with zeros outside [x0, x0 + n).
-__device__ __forceinline__ float2 sx_pair_zero(const float *__restrict__ row, int g, int x0, int n, bool vec)
+// The same under the mirror-single extension of [0, N).
+template <int V, bool PAIRS>
+__device__ __forceinline__ void sx_load_mirror(float2 (&a)[V], const float *row, int g0, int N,
+                                               unsigned long long pol)
 {
-    const bool i0 = (unsigned)(g - x0) < (unsigned)n, i1 = (unsigned)(g + 1 - x0) < (unsigned)n;
-    if (i0 && i1 && vec) return __ldg(reinterpret_cast<const float2 *>(row + g));
-    return make_float2(i0 ? __ldg(row + g) : 0.0f, i1 ? __ldg(row + g + 1) : 0.0f);
+    const float *p = row + g0;
+    const int top = 2 * N - 2;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        const int g = g0 + 32 * v;
+        if (PAIRS && (unsigned)g < (unsigned)N) {
+            a[v] = sep_ld2(p + 32 * v, pol);
+        } else {
+            const int i = abs(g), j = abs(g + 1);
+            a[v].x = sep_ld(row + min(max(min(i, top - i), 0), N - 1), pol);
+            a[v].y = sep_ld(row + min(max(min(j, top - j), 0), N - 1), pol);
+        }
+    }
+}
+// Pairs start at even offsets from an even lo: whole in [x0, x0 + n) and 8-byte aligned in every row?
+__device__ __forceinline__ bool sx_pairs(int vec, const SepAxis &a, int x0, int n)
+{
+    return vec && !((a.N | a.lo | x0 | n) & 1);
 }
 
-// Rows r0 + [0, 32) of `ny` rows x `nz` planes from (y0, z0): their bases in the volume and in
+// Rows r0 + [0, R) of `ny` rows x `nz` planes from (y0, z0): their bases in the volume and in
 // the tile's spectrum.
-__device__ __forceinline__ void sx_rows(SxRows &sr, const SepTile &t, int r0, int y0, int ny, int z0, int nz, int Py)
+template <int V>
+__device__ __forceinline__ void sx_rows(SxRows<V> &sr, const SepTile &t, int r0, int y0, int ny, int z0, int nz, int Py)
 {
-    if (threadIdx.x < kSepRows) {
+    if (threadIdx.x < SxShape<V>::R) {
         const int r = r0 + threadIdx.x, z = r / ny, y = r - z * ny;
         const bool ok = z < nz;
         sr.a[threadIdx.x] = ok ? ((long long)(z0 + z) * t.a[1].N + y0 + y) * t.a[0].N : -1;
@@ -177,25 +250,27 @@ __device__ __forceinline__ void sx_rows(SxRows &sr, const SepTile &t, int r0, in
 
 // ---- forward ------------------------------------------------------------------------------
 template <int V>
-__global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB)
+__global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_FWD)
     k_sep_x_fwd(SepSrc src, float2 *__restrict__ S, const SepTiles tl, SepGeom g, int vec,
                 const float2 *__restrict__ twg)
 {
     typedef SxShape<V> SH;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ SxRows sr;
+    __shared__ SxRows<V> sr;
     float2 *A = reinterpret_cast<float2 *>(smem_raw);
     float2 *tw = A + V * SH::BS;
     const SepTile &t = tl.t[blockIdx.y];
     pdl_trigger();
     const int ny = src.kernel ? src.kd[1] : t.a[1].nv, nz = src.kernel ? src.kd[2] : t.a[2].nv;
-    const int r0 = blockIdx.x * kSepRows;
+    const int r0 = blockIdx.x * SH::R;
     if (r0 >= ny * nz) return;
-    for (int i = threadIdx.x; i < SH::Px; i += SH::NT) tw[i] = __ldg(&twg[i]);
-    sx_rows(sr, t, r0, src.kernel ? 0 : t.a[1].v0, ny, src.kernel ? 0 : t.a[2].v0, nz, g.P[1]);
+    sx_twiddles<V>(tw, twg);
+    sx_rows<V>(sr, t, r0, src.kernel ? 0 : t.a[1].v0, ny, src.kernel ? 0 : t.a[2].v0, nz, g.P[1]);
     __syncthreads();
+    const unsigned long long pol = sep_policy(g.stream);
+    const bool pairs = sx_pairs(vec, t.a[0], 0, t.a[0].N);
     pdl_wait();
-    for (int it = threadIdx.x; it < kSepRows * 16; it += SH::NT) {
+    for (int it = threadIdx.x; it < SH::R * 16; it += SH::NT) {
         const int q = it & 15, row = it >> 4;
         const long long base = sr.a[row];
         float2 a[V];
@@ -204,9 +279,8 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB)
             for (int v = 0; v < V; ++v) a[v] = make_float2(0.0f, 0.0f);
         } else if (!src.kernel) {
             const float *p = src.vol + base;
-            const bool pv = vec && !((base + t.a[0].lo) & 1);
-#pragma unroll
-            for (int v = 0; v < V; ++v) a[v] = sx_pair(p, t.a[0].lo + 2 * (q + 16 * v), t.a[0].N, pv);
+            if (pairs) sx_load_mirror<V, true>(a, p, t.a[0].lo + 2 * q, t.a[0].N, pol);
+            else sx_load_mirror<V, false>(a, p, t.a[0].lo + 2 * q, t.a[0].N, pol);
         } else {  // taps wrapped around the origin, scaled
             const int r = r0 + row, z = r / ny, y = r - z * ny;
             const float *p = src.vol + ((long long)z * src.kd[1] + y) * src.kd[0];
@@ -235,42 +309,49 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB)
 // ---- conv1 -> quotient -> forward ------------------------------------------------------------
 // DeconvolutionMethods.java:71-74: img > 0 ? img / conv1 : 1, img zero outside the volume.
 template <int V>
-__global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB)
+__global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_RATIO)
     k_sep_x_ratio(float2 *__restrict__ S, const float *__restrict__ img, const SepTiles tl, SepGeom g, int vec,
                   const float2 *__restrict__ twg)
 {
     typedef SxShape<V> SH;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ SxRows sr;
+    __shared__ SxRows<V> sr;
     float2 *A = reinterpret_cast<float2 *>(smem_raw);
     float2 *tw = A + V * SH::BS;
     const SepTile &t = tl.t[blockIdx.y];
     pdl_trigger();
-    const int r0 = blockIdx.x * kSepRows;
+    const int r0 = blockIdx.x * SH::R;
     if (r0 >= t.a[1].nq * t.a[2].nq) return;
-    for (int i = threadIdx.x; i < SH::Px; i += SH::NT) tw[i] = __ldg(&twg[i]);
-    sx_rows(sr, t, r0, t.a[1].q0, t.a[1].nq, t.a[2].q0, t.a[2].nq, g.P[1]);
+    sx_twiddles<V>(tw, twg);
+    sx_rows<V>(sr, t, r0, t.a[1].q0, t.a[1].nq, t.a[2].q0, t.a[2].nq, g.P[1]);
     __syncthreads();
     pdl_wait();
     float2 *base = S + (long long)blockIdx.y * g.stride;
     const long long bstride = (long long)g.Zs * g.P[1] * 16;
+    const unsigned long long pol = sep_policy(g.stream);
+    const bool pairs = sx_pairs(vec, t.a[0], 0, t.a[0].N);
     sx_load_lines<V>(A, base, bstride, sr.b);
     __syncthreads();
     sx_p2<V, true>(A, tw);
     __syncthreads();
-    for (int it = threadIdx.x; it < kSepRows * 16; it += SH::NT) {
+    for (int it = threadIdx.x; it < SH::R * 16; it += SH::NT) {
         const int q = it & 15, row = it >> 4;
         const long long ib = sr.a[row];
-        const bool pv = vec && !((ib + t.a[0].lo) & 1);
+        constexpr bool EARLY = V < 12;  // the image ahead of the transform, as the registers allow
         float2 im[V], a[V];
-#pragma unroll
-        for (int v = 0; v < V; ++v)
-            im[v] = ib < 0 ? make_float2(0.0f, 0.0f)
-                           : sx_pair_zero(img + ib, t.a[0].lo + 2 * (q + 16 * v), 0, t.a[0].N, pv);
+        const int n = ib < 0 ? 0 : t.a[0].N;  // no row: no voxel
+        if (EARLY) {
+            if (pairs) sx_load_zero<V, true>(im, img + ib, t.a[0].lo + 2 * q, 0, n, pol);
+            else sx_load_zero<V, false>(im, img + ib, t.a[0].lo + 2 * q, 0, n, pol);
+        }
         float2 *p = A + row * kSepRS + q;
 #pragma unroll
         for (int k1 = 0; k1 < V; ++k1) a[k1] = p[k1 * SH::BS];
         sx_p1<V, true>(a, tw, q);
+        if (!EARLY) {
+            if (pairs) sx_load_zero<V, true>(im, img + ib, t.a[0].lo + 2 * q, 0, n, pol);
+            else sx_load_zero<V, false>(im, img + ib, t.a[0].lo + 2 * q, 0, n, pol);
+        }
 #pragma unroll
         for (int v = 0; v < V; ++v) a[v] = make_float2(quotient_fast(im[v].x, a[v].x), quotient_fast(im[v].y, a[v].y));
         sx_p1<V, false>(a, tw, q);
@@ -284,22 +365,149 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB)
 }
 
 // ---- conv2 -> update ----------------------------------------------------------------------
+__device__ __forceinline__ void sx_change(float next, float last, float &ksum, float &kcomp, float &kmax)
+{
+    const float ch = next - last;  // signed change (DeconvolutionMethods.java:308)
+    const float ky = ch - kcomp;
+    const float kt = ksum + ky;
+    kcomp = (kt - ksum) - ky;
+    ksum = kt;
+    kmax = kmax > ch ? kmax : ch;
+}
+
+// One row item of the Seq update: conv2 at the voxels x = g0 + 32 v + {0, 1}, the new psi for those
+// in [x0, x0 + nx).
+template <int V, bool ST, bool PAIRS>
+__device__ __forceinline__ void sx_update_row(const float2 *p, const float2 *tw, int q, const SepUpd &u, long long vb,
+                                              int g0, int x0, int nx, float &ksum, float &kcomp, float &kmax,
+                                              unsigned long long pol)
+{
+    constexpr int BS = SxShape<V>::BS;
+    // psi and the weight ahead of the transform where the registers allow, else 6 pairs at a time, all
+    // loads of a chunk ahead of its stores (a load per store, in turn: 1.71 against 1.37 ms for the 6
+    // views of 512 x 512 x 256)
+    constexpr bool EARLY = V < 12;
+    constexpr int CH = EARLY ? V : 6;
+    float2 prev[CH], w[CH], a[V];
+    if (EARLY) {
+        sx_load_zero<CH, PAIRS>(prev, u.psi + vb, g0, x0, nx, pol);
+        sx_load_zero<CH, PAIRS>(w, u.weight[0] + vb, g0, x0, nx, pol);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < V; ++k1) a[k1] = p[k1 * BS];
+    sx_p1<V, true>(a, tw, q);
+#pragma unroll
+    for (int c0 = 0; c0 < V; c0 += CH) {
+        if (!EARLY) {  // (pairs past the last of a partial chunk lie past the tile, so past the range)
+            sx_load_zero<CH, PAIRS>(prev, u.psi + vb, g0 + 32 * c0, x0, nx, pol);
+            sx_load_zero<CH, PAIRS>(w, u.weight[0] + vb, g0 + 32 * c0, x0, nx, pol);
+        }
+#pragma unroll
+        for (int j = 0; j < CH; ++j) {
+            const int v = c0 + j;
+            if (v >= V) break;
+            const int r = g0 - x0 + 32 * v;
+            const bool i0 = (unsigned)r < (unsigned)nx, i1 = PAIRS ? i0 : (unsigned)(r + 1) < (unsigned)nx;
+            if (!i0 && !i1) continue;
+            const float2 next = make_float2(next_value_fast(prev[j].x, a[v].x, w[j].x, u.c),
+                                            next_value_fast(prev[j].y, a[v].y, w[j].y, u.c));
+            if (ST && i0) sx_change(next.x, prev[j].x, ksum, kcomp, kmax);
+            if (ST && i1) sx_change(next.y, prev[j].y, ksum, kcomp, kmax);
+            float *o = u.dst + vb + g0 + 32 * v;
+            if (PAIRS) {
+                sep_st2(o, next, pol);
+            } else {
+                if (i0) sep_st(o, next.x, pol);
+                if (i1) sep_st(o + 1, next.y, pol);
+            }
+        }
+    }
+}
+
+// The Mul pass over the CTA's rows of conv2 (natural order in shared memory): the running product
+// (EPI_MUL_FIRST, EPI_MUL_ACC) or the final value, U pairs of voxels a thread at a time with all
+// their loads in flight; lanes run along x.  (On the registers of the transform, as Seq does it, the
+// products spill or are loaded one by one: 82 us a view on 211 x 187 x 143, 49 us in this form.)
+template <int V, bool ST>
+__device__ __forceinline__ void sx_mul_rows(const float2 *A, const SepUpd &u, int epi, const SepTile &t,
+                                            const long long *rowa, float &ksum, float &kcomp, float &kmax,
+                                            unsigned long long pol)
+{
+    typedef SxShape<V> SH;
+    constexpr int U = 4, items = SH::R * SH::m;
+    const int lo = t.a[0].lo, x0 = t.a[0].w0, nx = t.a[0].nw;
+    const bool acc = epi != EPI_MUL_FIRST && u.nviews > 1, fin = epi == EPI_MUL_FINAL;
+    for (int i0 = threadIdx.x; i0 < items; i0 += U * SH::NT) {
+        float2 pr[U][2], last[U], w[U];
+        long long at[U];
+        bool in[U][2];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int i = i0 + k * SH::NT, row = i / SH::m, j = i - row * SH::m;
+            const long long vb = i < items ? rowa[row] : -1;
+            const int r = lo + 2 * j - x0;
+            in[k][0] = vb >= 0 && (unsigned)r < (unsigned)nx;
+            in[k][1] = vb >= 0 && (unsigned)(r + 1) < (unsigned)nx;
+            at[k] = vb + lo + 2 * j;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                pr[k][h] = acc && in[k][h] ? u.prod[at[k] + h] : make_float2(0.0f, 0.0f);
+            last[k] = w[k] = make_float2(0.0f, 0.0f);
+            if (fin) {
+                if (in[k][0]) last[k].x = sep_ld(u.psi + at[k], pol);
+                if (in[k][1]) last[k].y = sep_ld(u.psi + at[k] + 1, pol);
+            }
+        }
+        if (fin)
+            for (int v = 0; v < u.nviews; ++v) {
+                float2 wv[U];
+#pragma unroll
+                for (int k = 0; k < U; ++k)
+                    wv[k] = make_float2(in[k][0] ? sep_ld(u.weight[v] + at[k], pol) : 0.0f,
+                                        in[k][1] ? sep_ld(u.weight[v] + at[k] + 1, pol) : 0.0f);
+#pragma unroll
+                for (int k = 0; k < U; ++k) w[k] = cadd(w[k], wv[k]);
+            }
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int i = i0 + k * SH::NT, row = i / SH::m, j = i - row * SH::m;
+            if (i >= items) break;
+            const float2 c = A[(j >> 4) * SH::BS + row * kSepRS + (j & 15)];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (!in[k][h]) continue;
+                const float cv = h ? c.y : c.x;
+                const float2 q = acc ? mulprod_acc(pr[k][h], cv) : mulprod_first(cv);
+                if (!fin) {
+                    u.prod[at[k] + h] = q;
+                    continue;
+                }
+                const float wt = h ? w[k].y : w[k].x, prev = h ? last[k].y : last[k].x;
+                const float next = next_value(prev, mulprod_root(q, u.nviews), wt < 1.0f ? wt : 1.0f, u.c.two_lambda,
+                                              u.c.tik, u.c.minI, u.c.maxI);
+                if (ST) sx_change(next, prev, ksum, kcomp, kmax);
+                sep_st(u.dst + at[k] + h, next, pol);
+            }
+        }
+    }
+}
+
 // The written voxels alone: Seq (DeconvolutionMethods.java:103-182, 320-358) or the running product
 // and final value of Mul (:370-419); with ST the change statistics over them.
 template <int V, bool MUL, bool ST>
-__global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB)
+__global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_UPD)
     k_sep_x_update(const float2 *__restrict__ S, SepUpd u, int epi, const SepTiles tl, SepGeom g, int vec,
                    const float2 *__restrict__ twg)
 {
     typedef SxShape<V> SH;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ SxRows sr;
+    __shared__ SxRows<V> sr;
     __shared__ double red_s[32], red_m[32];
     float2 *A = reinterpret_cast<float2 *>(smem_raw);
     float2 *tw = A + V * SH::BS;
     const SepTile &t = tl.t[blockIdx.y];
     pdl_trigger();
-    const int r0 = blockIdx.x * kSepRows;
+    const int r0 = blockIdx.x * SH::R;
     const long long slot = (long long)blockIdx.y * gridDim.x + blockIdx.x;
     if (r0 >= t.a[1].nw * t.a[2].nw) {
         if (ST && threadIdx.x == 0) {
@@ -309,8 +517,8 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB)
         }
         return;
     }
-    for (int i = threadIdx.x; i < SH::Px; i += SH::NT) tw[i] = __ldg(&twg[i]);
-    sx_rows(sr, t, r0, t.a[1].w0, t.a[1].nw, t.a[2].w0, t.a[2].nw, g.P[1]);
+    sx_twiddles<V>(tw, twg);
+    sx_rows<V>(sr, t, r0, t.a[1].w0, t.a[1].nw, t.a[2].w0, t.a[2].nw, g.P[1]);
     __syncthreads();
     pdl_wait();
     sx_load_lines<V>(A, S + (long long)blockIdx.y * g.stride, (long long)g.Zs * g.P[1] * 16, sr.b);
@@ -319,80 +527,35 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB)
     __syncthreads();
     float ksum = 0.0f, kcomp = 0.0f, kmax = -1.0f;
     const int x0 = t.a[0].w0, nx = t.a[0].nw;
-    for (int it = threadIdx.x; it < kSepRows * 16; it += SH::NT) {
+    const unsigned long long pol = sep_policy(g.stream);
+    const bool pairs = sx_pairs(vec, t.a[0], x0, nx);
+    for (int it = threadIdx.x; it < SH::R * 16; it += SH::NT) {
         const int q = it & 15, row = it >> 4;
         const long long vb = sr.a[row];
-        if (vb < 0) continue;
-        const bool pv = vec && !((vb + t.a[0].lo) & 1);
-        const int g0 = t.a[0].lo + 2 * q;
-        float2 last[V], wv[V], a[V];
-        if (!MUL) {
+        float2 *p = A + row * kSepRS + q;
+        if constexpr (MUL) {
+            float2 a[V];
 #pragma unroll
-            for (int v = 0; v < V; ++v) {
-                last[v] = sx_pair_zero(u.psi + vb, g0 + 32 * v, x0, nx, pv);
-                wv[v] = sx_pair_zero(u.weight[0] + vb, g0 + 32 * v, x0, nx, pv);
-            }
+            for (int k1 = 0; k1 < V; ++k1) a[k1] = p[k1 * SH::BS];
+            sx_p1<V, true>(a, tw, q);
+#pragma unroll
+            for (int v = 0; v < V; ++v) p[v * SH::BS] = a[v];
+        } else {
+            if (vb < 0) continue;
+            const int g0 = t.a[0].lo + 2 * q;
+            if (pairs) sx_update_row<V, ST, true>(p, tw, q, u, vb, g0, x0, nx, ksum, kcomp, kmax, pol);
+            else sx_update_row<V, ST, false>(p, tw, q, u, vb, g0, x0, nx, ksum, kcomp, kmax, pol);
         }
-        const float2 *p = A + row * kSepRS + q;
-#pragma unroll
-        for (int k1 = 0; k1 < V; ++k1) a[k1] = p[k1 * SH::BS];
-        sx_p1<V, true>(a, tw, q);
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const int x = g0 + 32 * v;
-            const bool i0 = (unsigned)(x - x0) < (unsigned)nx, i1 = (unsigned)(x + 1 - x0) < (unsigned)nx;
-            if (!i0 && !i1) continue;
-            float next[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float cv = h ? a[v].y : a[v].x;
-                if (!(h ? i1 : i0)) continue;
-                float prev, w, f = cv;
-                if (!MUL) {
-                    prev = h ? last[v].y : last[v].x;
-                    w = h ? wv[v].y : wv[v].x;
-                } else {
-                    float2 *pp = u.prod + vb + x + h;
-                    if (epi == EPI_MUL_FIRST) {
-                        *pp = mulprod_first(cv);
-                        continue;
-                    }
-                    const float2 pr = u.nviews == 1 ? mulprod_first(cv) : mulprod_acc(*pp, cv);
-                    if (epi == EPI_MUL_ACC) {
-                        *pp = pr;
-                        continue;
-                    }
-                    f = mulprod_root(pr, u.nviews);
-                    w = 0.0f;
-                    for (int k = 0; k < u.nviews; ++k) w += __ldg(u.weight[k] + vb + x + h);
-                    w = w < 1.0f ? w : 1.0f;
-                    prev = __ldg(u.psi + vb + x + h);
-                }
-                next[h] = MUL ? next_value(prev, f, w, u.c.two_lambda, u.c.tik, u.c.minI, u.c.maxI)
-                              : next_value_fast(prev, f, w, u.c);
-                if (ST) {
-                    const float ch = next[h] - prev;  // signed change (DeconvolutionMethods.java:308)
-                    const float ky = ch - kcomp;
-                    const float kt = ksum + ky;
-                    kcomp = (kt - ksum) - ky;
-                    ksum = kt;
-                    kmax = kmax > ch ? kmax : ch;
-                }
-            }
-            if (MUL && epi != EPI_MUL_FINAL) continue;
-            float *o = u.dst + vb + x;
-            if (i0 && i1 && pv) {
-                *reinterpret_cast<float2 *>(o) = make_float2(next[0], next[1]);
-            } else {
-                if (i0) o[0] = next[0];
-                if (i1) o[1] = next[1];
-            }
-        }
+    }
+    if constexpr (MUL) {
+        __syncthreads();
+        sx_mul_rows<V, ST>(A, u, epi, t, sr.a, ksum, kcomp, kmax, pol);
     }
     if (ST) stats_to_partials(ksum, kcomp, kmax, red_s, red_m, u.partials, slot);
 }
 
 struct SxOps {
+    int rows;  // per CTA
     cudaError_t (*fwd)(const SepGeom &, const SepTiles &, int, int, const SepSrc &, float2 *, int, const float2 *,
                        cudaStream_t);
     cudaError_t (*ratio)(const SepGeom &, const SepTiles &, int, int, const float *, float2 *, int, const float2 *,
@@ -452,7 +615,7 @@ struct Sx {
     }
     static const SxOps *ops()
     {
-        static const SxOps o = {&fwd, &ratio, &update};
+        static const SxOps o = {SH::R, &fwd, &ratio, &update};
         return &o;
     }
 };

@@ -8,8 +8,10 @@
 //   phase 2, thread (column, k1): T-point DFT over t; position k2 + T k1 holds frequency
 //                                 k1 + V k2, straight back to global memory.
 // One exchange through shared memory per direction: a y pass has one, the z pass (forward,
-// spectral product, inverse) two.  Bound by HBM and L2 traffic; 16 max(T, V) threads, so that
-// one round covers either phase.
+// spectral product, inverse) two.  16 max(T, V) threads, so that one round covers either phase.
+// Where a column's rows or planes are stored (mirrored, or a constant) is tabulated once per CTA as
+// 32-bit byte offsets.  Bound by HBM and L2 traffic (y: 6.1 TB/s of algorithmic bytes on 288-long
+// columns) and, in the z pass, by the load latency of the data and K^ (4.9 TB/s on 320).
 #pragma once
 #include "pdl.cuh"
 #include "sep.cuh"
@@ -54,26 +56,69 @@ struct YzShape {
     static constexpr int W = T > V ? T : V;
     static constexpr int NT = 16 * W;
     // CTAs per SM the register budget is sized for
-    static constexpr int MINB = NT <= 128 ? 6 : (NT <= 192 ? 4 : (NT <= 256 ? 3 : 2));
-    static constexpr size_t smem = sizeof(float2) * (size_t)(16 * n + n);
+    static constexpr int TW = (n + NT - 1) / NT;  // twiddles a thread fetches
+    // CTAs per SM the register budget is sized for: 1152 threads for the y passes (56 registers; 4-view
+    // 256^3: 6.1 TB/s of algorithmic bytes, 5.0 at 640 threads), 960 for z (4.9 TB/s, 4.6 at 640); two
+    // CTAs where a thread holds 24 values (56 registers spill: 5.5 -> 4.7 TB/s on 576-long columns)
+    static constexpr int minb(int threads) { return W >= 24 ? 2 : (threads / NT > 8 ? 8 : threads / NT); }
+    static constexpr int MINB_Y = minb(1152), MINB_Z = minb(960);
+    // tile, twiddles, byte offsets of the input rows or planes
+    static constexpr size_t smem = sizeof(float2) * (size_t)(16 * n + n) + sizeof(unsigned) * (size_t)n;
 };
 
-// ---- y forward, in place ----------------------------------------------------------------
-// fill: value of the quotient's constant rows in column 0 (the x transform of ones: Px)
-template <int T, int V, int MAP>
-__device__ __forceinline__ void sep_y_load(float2 (&a)[V], const float2 *slot, const SepRows &rows, int u, int c,
-                                           float2 fill)
+// Byte offsets of the stored rows (planes) of the domain indices, kSepNone for constant ones.
+constexpr unsigned kSepNone = 0xffffffffu;
+template <int n, int NT>
+__device__ __forceinline__ void sep_offsets(unsigned *off, const SepRows &rows, int map, unsigned pitch)
 {
+    for (int j = threadIdx.x; j < n; j += NT) {
+        int i;
+        bool ok;
+        if (map == SEP_MIRROR) ok = rows.at<SEP_MIRROR>(j, i);
+        else if (map == SEP_FILL) ok = rows.at<SEP_FILL>(j, i);
+        else ok = rows.at<SEP_KERNEL>(j, i);
+        off[j] = ok ? (unsigned)i * pitch : kSepNone;
+    }
+}
+// Phase 1's values of thread u: elements u + T v of the column at `base` + `at` bytes.
+template <int T, int V>
+__device__ __forceinline__ void sep_load(float2 (&a)[V], const float2 *base, unsigned at, const unsigned *off, int u,
+                                         bool live, float2 fill)
+{
+    const char *p = reinterpret_cast<const char *>(base);
 #pragma unroll
     for (int v = 0; v < V; ++v) {
-        int i;
-        const bool ok = rows.at<MAP>(u + T * v, i);
-        a[v] = ok ? slot[i * 16 + c] : fill;
+        const unsigned o = off[u + T * v];
+        a[v] = live && o != kSepNone ? *reinterpret_cast<const float2 *>(p + (o + at)) : fill;
     }
 }
 
+// The twiddles: fetched ahead of the wait for the predecessor, put down behind the loads of the data.
 template <int T, int V>
-__global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB)
+__device__ __forceinline__ void sep_tw_fetch(float2 (&r)[YzShape<T, V>::TW], const float2 *__restrict__ twg)
+{
+    typedef YzShape<T, V> SH;
+#pragma unroll
+    for (int k = 0; k < SH::TW; ++k) {
+        const int i = threadIdx.x + k * SH::NT;
+        r[k] = i < SH::n ? __ldg(&twg[i]) : make_float2(0.0f, 0.0f);
+    }
+}
+template <int T, int V>
+__device__ __forceinline__ void sep_tw_put(float2 *tw, const float2 (&r)[YzShape<T, V>::TW])
+{
+    typedef YzShape<T, V> SH;
+#pragma unroll
+    for (int k = 0; k < SH::TW; ++k) {
+        const int i = threadIdx.x + k * SH::NT;
+        if (i < SH::n) tw[i] = r[k];
+    }
+}
+
+// ---- y forward, in place ----------------------------------------------------------------
+// fill: value of the quotient's constant rows in column 0 (the x transform of ones: Px)
+template <int T, int V>
+__global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Y)
     k_sep_y_fwd(float2 *S, const SepTiles tl, SepGeom g, int map, int kdy, int kdz, const float2 *__restrict__ twg)
 {
     typedef YzShape<T, V> SH;
@@ -83,8 +128,8 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB)
     float2 *tw = A + 16 * n;
     const int z = blockIdx.x, xb = blockIdx.y;
     const SepTile &tile = tl.t[blockIdx.z];
+    unsigned *off = reinterpret_cast<unsigned *>(tw + n);
     pdl_trigger();
-    for (int i = threadIdx.x; i < n; i += SH::NT) tw[i] = __ldg(&twg[i]);
     const int planes = map == SEP_MIRROR ? tile.a[2].nv : (map == SEP_FILL ? tile.a[2].nq : kdz);
     if (z >= planes) return;
     const SepRows rows(tile.a[1], map, n, kdy);
@@ -92,13 +137,14 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB)
     float2 *slot = base + ((long long)xb * g.Zs + z) * n * 16;
     const int c = threadIdx.x & 15, u = threadIdx.x >> 4;
     const float2 fill = make_float2(map == SEP_FILL && xb == 0 && c == 0 ? (float)g.P[0] : 0.0f, 0.0f);
+    float2 twr[SH::TW];
+    sep_tw_fetch<T, V>(twr, twg);
+    sep_offsets<n, SH::NT>(off, rows, map, 128);
+    __syncthreads();
     pdl_wait();
     float2 a[V];
-    if (u < T) {
-        if (map == SEP_MIRROR) sep_y_load<T, V, SEP_MIRROR>(a, slot, rows, u, c, fill);
-        else if (map == SEP_FILL) sep_y_load<T, V, SEP_FILL>(a, slot, rows, u, c, fill);
-        else sep_y_load<T, V, SEP_KERNEL>(a, slot, rows, u, c, fill);
-    }
+    if (u < T) sep_load<T, V>(a, slot, 8 * c, off, u, true, fill);
+    sep_tw_put<T, V>(tw, twr);
     __syncthreads();  // the twiddles; every row of the slot is read before phase 2 rewrites it
     if (u < T) {
         sep_dft<V, false>(a);
@@ -141,7 +187,7 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB)
 
 // ---- y inverse, in place ------------------------------------------------------------------
 template <int T, int V>
-__global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB)
+__global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Y)
     k_sep_y_inv(float2 *S, const SepTiles tl, SepGeom g, int out_w, const float2 *__restrict__ twg)
 {
     typedef YzShape<T, V> SH;
@@ -193,20 +239,8 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB)
 }
 
 // ---- z: forward, times K, inverse -----------------------------------------------------------
-template <int T, int V, int MAP>
-__device__ __forceinline__ void sep_z_load(float2 (&a)[V], const float2 *col, long long pitch, const SepRows &rows,
-                                           int u, bool live, float2 fill)
-{
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-        int i;
-        const bool ok = rows.at<MAP>(u + T * v, i);
-        a[v] = live && ok ? col[i * pitch] : fill;
-    }
-}
-
 template <int T, int V, bool MUL>
-__global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB)
+__global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Z)
     k_sep_z(const float2 *src, float2 *dst, const float2 *__restrict__ K, const SepTiles tl, SepGeom g, int map,
             int out_w, int kdz, const float2 *__restrict__ twg)
 {
@@ -215,31 +249,32 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *A = reinterpret_cast<float2 *>(smem_raw);
     float2 *tw = A + 16 * n;
+    unsigned *off = reinterpret_cast<unsigned *>(tw + n);
     const int Py = g.P[1];
     const SepTile &tile = tl.t[blockIdx.y];
     pdl_trigger();
-    for (int i = threadIdx.x; i < n; i += SH::NT) tw[i] = __ldg(&twg[i]);
     const int c = threadIdx.x & 15, u = threadIdx.x >> 4;
     // the 16 columns: one line of column block xb at y, or 16 y of the Nyquist plane
     const int xb = blockIdx.x / Py, y = blockIdx.x - xb * Py;
     const bool nyq = xb == g.nxb;
     const int cols = nyq ? min(16, Py - 16 * y) : 16;
     const bool live = c < cols;
-    const long long pitch = nyq ? Py : (long long)Py * 16;
+    const unsigned pitch = nyq ? Py : Py * 16;
     const long long block = (long long)xb * Py * 16;  // times the planes of the buffer
-    const long long at = (nyq ? 0 : (long long)y * 16) + (nyq ? 16 * y : 0) + c;
-    const float2 *sp = src + (long long)blockIdx.y * g.stride + block * g.Zs + at;
+    const unsigned at = 16 * y + c;
+    const float2 *sp = src + (long long)blockIdx.y * g.stride + block * g.Zs;
     const SepRows rows(tile.a[2], map, n, kdz);
     // a plane of the constant quotient: its y transform is one value, at frequency 0 of column 0
     const float2 fill = make_float2(map == SEP_FILL && xb == 0 && y == 0 && c == 0
                                         ? (float)g.P[0] * (float)Py : 0.0f, 0.0f);
+    float2 twr[SH::TW];
+    sep_tw_fetch<T, V>(twr, twg);
+    sep_offsets<n, SH::NT>(off, rows, map, 8 * pitch);
+    __syncthreads();
     pdl_wait();
     float2 a[V];
-    if (u < T) {
-        if (map == SEP_MIRROR) sep_z_load<T, V, SEP_MIRROR>(a, sp, pitch, rows, u, live, fill);
-        else if (map == SEP_FILL) sep_z_load<T, V, SEP_FILL>(a, sp, pitch, rows, u, live, fill);
-        else sep_z_load<T, V, SEP_KERNEL>(a, sp, pitch, rows, u, live, fill);
-    }
+    if (u < T) sep_load<T, V>(a, sp, 8 * at, off, u, live, fill);
+    sep_tw_put<T, V>(tw, twr);
     __syncthreads();  // the twiddles
     if (u < T) {
         sep_dft<V, false>(a);
@@ -250,9 +285,11 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB)
     }
     float2 b[T], kv[T];
     if (MUL && u < V) {  // K's values are on their way while the CTA meets at the barrier
-        const float2 *kp = K + block * n + at + (long long)(T * u) * pitch;
+        const float2 *kp = K + block * n;
+        const unsigned k0 = at + T * u * pitch;
+        const unsigned long long pol = sep_policy(g.stream);
 #pragma unroll
-        for (int k2 = 0; k2 < T; ++k2) kv[k2] = live ? __ldg(kp + k2 * pitch) : make_float2(0.0f, 0.0f);
+        for (int k2 = 0; k2 < T; ++k2) kv[k2] = live ? sep_ld2(kp + (k0 + k2 * pitch), pol) : make_float2(0.0f, 0.0f);
     }
     __syncthreads();
     if (u < V) {
@@ -262,9 +299,10 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB)
     }
     if constexpr (!MUL) {  // a kernel spectrum: every plane of dst
         if (u < V && live) {
-            float2 *dp = dst + block * n + at + (long long)(T * u) * pitch;
+            float2 *dp = dst + block * n;
+            const unsigned k0 = at + T * u * pitch;
 #pragma unroll
-            for (int k2 = 0; k2 < T; ++k2) dp[k2 * pitch] = b[k2];
+            for (int k2 = 0; k2 < T; ++k2) dp[k0 + k2 * pitch] = b[k2];
         }
         return;
     } else {
@@ -283,12 +321,12 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB)
             for (int k1 = 1; k1 < V; ++k1) a[k1] = cmul(a[k1], cconj(tw[u * k1]));
             sep_dft<V, true>(a);
             const int r0 = out_w ? tile.a[2].w0 : tile.a[2].q0, nr = out_w ? tile.a[2].nw : tile.a[2].nq;
-            const int off = tile.a[2].lo - r0;
-            float2 *dp = dst + (long long)blockIdx.y * g.stride + block * g.Zs + at;
+            const int i0 = tile.a[2].lo - r0 + u;
+            float2 *dp = dst + (long long)blockIdx.y * g.stride + block * g.Zs;
 #pragma unroll
             for (int v = 0; v < V; ++v) {
-                const int i = off + u + T * v;
-                if ((unsigned)i < (unsigned)nr) dp[i * pitch] = a[v];
+                const unsigned i = i0 + T * v;
+                if (i < (unsigned)nr) dp[at + i * pitch] = a[v];
             }
         }
     }
