@@ -28,20 +28,19 @@ inline bool invert_affine(const double *m, double *inv)
 
 // AffineTransform3D.apply: each coordinate s0 m0 + s1 m1 + s2 m2 + m3 summed left to right,
 // every operation rounded (no contraction into fused multiply-adds).
-__host__ __device__ __forceinline__ void apply_affine(const double *m, const double *s, double *t)
+__host__ __device__ __forceinline__ double apply_affine_row(const double *m, const double *s)
 {
 #ifdef __CUDA_ARCH__
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-        t[r] = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(s[0], m[4 * r]), __dmul_rn(s[1], m[4 * r + 1])),
-                                   __dmul_rn(s[2], m[4 * r + 2])),
-                         m[4 * r + 3]);
+    return __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(s[0], m[0]), __dmul_rn(s[1], m[1])), __dmul_rn(s[2], m[2])), m[3]);
 #else
-    for (int r = 0; r < 3; ++r) {
-        volatile double p0 = s[0] * m[4 * r], p1 = s[1] * m[4 * r + 1], p2 = s[2] * m[4 * r + 2];
-        t[r] = ((p0 + p1) + p2) + m[4 * r + 3];
-    }
+    volatile double p0 = s[0] * m[0], p1 = s[1] * m[1], p2 = s[2] * m[2];
+    return ((p0 + p1) + p2) + m[3];
 #endif
+}
+__host__ __device__ __forceinline__ void apply_affine(const double *m, const double *s, double *t)
+{
+#pragma unroll
+    for (int r = 0; r < 3; ++r) t[r] = apply_affine_row(m + 4 * r, s);
 }
 
 // Linear interpolation from the corner values at floor(t) + (dx, dy, dz): weights in double

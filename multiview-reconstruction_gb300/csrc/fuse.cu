@@ -17,6 +17,7 @@
 //   deconvolution weight = sum(wd_v) (CombineWeightsSumRandomAccess.get)
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -29,15 +30,64 @@ namespace mvr {
 namespace {
 
 constexpr int kFuseMaxViews = 16;
+constexpr int kFuseRows = 8;        // rows of one plane a CTA takes at a time
+constexpr int kFuseThreads = 256;
+
+// ---- pairs of floats (hi + lo, about 48 bits) ------------------------------------------------
+// The GPU's double rate is a small fraction of its float rate: one fused voxel in double (affine
+// map, eight corner weights, table products) took 13.1 ms for 3 views into a 256^3 box.  The sums
+// and products that decide a rounding or a branch run on pairs of floats instead; the products'
+// and sums' rounding errors come from fused multiply-adds and two-sums (Dekker, Knuth).
+struct FPair {
+    float h, l;
+};
+__host__ __device__ __forceinline__ FPair fp_from(double v)
+{
+    FPair p;
+    p.h = (float)v;
+    p.l = (float)(v - (double)p.h);
+    return p;
+}
+__device__ __forceinline__ FPair fp_quick(float a, float b)  // |a| >= |b|
+{
+    const float s = __fadd_rn(a, b);
+    return {s, __fsub_rn(b, __fsub_rn(s, a))};
+}
+__device__ __forceinline__ FPair fp_sum(float a, float b)
+{
+    const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+    return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
+}
+__device__ __forceinline__ FPair fp_add(FPair a, FPair b)
+{
+    const FPair s = fp_sum(a.h, b.h);
+    return fp_quick(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
+}
+__device__ __forceinline__ FPair fp_add(FPair a, float b)
+{
+    const FPair s = fp_sum(a.h, b);
+    return fp_quick(s.h, __fadd_rn(s.l, a.l));
+}
+__device__ __forceinline__ FPair fp_mul(FPair a, float b)
+{
+    const float p = __fmul_rn(a.h, b);
+    return fp_quick(p, __fmaf_rn(a.l, b, __fmaf_rn(a.h, b, -p)));
+}
+__device__ __forceinline__ FPair fp_prod(float a, float b)
+{
+    const float p = __fmul_rn(a, b);
+    return {p, __fmaf_rn(a, b, -p)};
+}
 
 struct FuseView {
     const float *img;
     int dims[3];
     double inv[12];  // world -> view pixel, row-packed 3 x 4
+    FPair step[3];   // inv[0], inv[4], inv[8]: t per voxel of x
     float fb[3], fr[3], db[3], dr[3];
     int fblend, dblend;
-    int adjust;        // intensity adjustment v -> v m00 + m01 (double, stored as float)
-    double m00, m01;
+    int adjust;        // intensity adjustment v -> v m00 + m01 (rounded once to float)
+    FPair m00, m01;
 };
 
 struct FuseViews {
@@ -45,10 +95,11 @@ struct FuseViews {
     int n;
 };
 
-// BlendingRealRandomAccess.computeWeight on an interval [0, dims - 1] at a float location
-// (float arithmetic as in the reference, the look-up table product in double).
+// BlendingRealRandomAccess.computeWeight on an interval [0, dims - 1] at a float location (float
+// arithmetic as in the reference).  The table product w lut[i] is rounded once, its entry index
+// (int)(rel 1000 + 0.5) taken from the exact product rel 1000.
 __device__ __forceinline__ float blend_weight(const float *loc, const int *dims, const float *border,
-                                              const float *range, const double *lut)
+                                              const float *range, const FPair *__restrict__ lut)
 {
     float tmp[3];
 #pragma unroll
@@ -62,58 +113,110 @@ __device__ __forceinline__ float blend_weight(const float *loc, const int *dims,
     float w = 1.0f;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
+        if (!(tmp[d] < range[d])) continue;  // exactly the quotients that round to 1 or more
         const float rel = __fdiv_rn(tmp[d], range[d]);
-        if (rel < 1.0f) w = (float)((double)w * lut[(int)((double)rel * 1000.0 + 0.5)]);
+        const FPair p = fp_prod(rel, 1000.0f);
+        float k = floorf(__fadd_rn(p.h, 0.5f));
+        const float r = __fadd_rn(__fsub_rn(p.h, k), p.l);  // rel 1000 - k: p.h - k is exact
+        if (r >= 0.5f) k += 1.0f;
+        else if (r < -0.5f) k -= 1.0f;
+        const FPair c = lut[(int)k];
+        const FPair q = fp_mul(c, w);
+        w = __fadd_rn(q.h, q.l);
     }
     return w;
 }
 
-// Linear interpolation of a float volume at t (all eight neighbours exist: t is strictly
-// inside), the interpolator of the reference's views (NLinearInterpolator3D order); with
-// `adjust` every neighbour goes through the intensity adjustment first
-// (IntensityAdjuster.apply, fusion/intensityadjust/IntensityAdjuster.java: v m00 + m01 in
-// double, stored as float).
-__device__ __forceinline__ float trilinear(const FuseView &v, const double *t)
+// Linear interpolation at floor(t) + f in [0, 1)^3 (all eight neighbours exist: t lies strictly
+// inside): differences and fused multiply-adds along x, y, z.  With `adjust` every neighbour goes
+// through the intensity adjustment first (IntensityAdjuster.apply,
+// fusion/intensityadjust/IntensityAdjuster.java: v m00 + m01, stored as float).
+__device__ __forceinline__ float fuse_value(const FuseView &v, float x)
 {
-    const double f[3] = {floor(t[0]), floor(t[1]), floor(t[2])};
-    const double w[3] = {__dsub_rn(t[0], f[0]), __dsub_rn(t[1], f[1]), __dsub_rn(t[2], f[2])};
+    if (!v.adjust) return x;
+    const FPair q = fp_add(fp_mul(v.m00, x), v.m01);
+    return __fadd_rn(q.h, q.l);
+}
+__device__ __forceinline__ float lerp(float a, float b, float f) { return __fmaf_rn(f, __fsub_rn(b, a), a); }
+__device__ __forceinline__ float trilinear(const FuseView &v, const int *i, const float *f)
+{
     const long long sy = v.dims[0], sz = (long long)v.dims[0] * v.dims[1];
-    const float *p = v.img + (long long)f[2] * sz + (long long)f[1] * sy + (long long)f[0];
-    return nlinear3(w, [&](int dx, int dy, int dz) {
-        const float x = __ldg(p + dz * sz + dy * sy + dx);
-        return v.adjust ? __double2float_rn(__dadd_rn(__dmul_rn((double)x, v.m00), v.m01)) : x;
-    });
+    const float *p = v.img + ((long long)i[2] * v.dims[1] + i[1]) * sy + i[0];
+    float c[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) c[k] = __ldg(p + (k & 1) + (k & 2 ? sy : 0) + (k & 4 ? sz : 0));
+#pragma unroll
+    for (int k = 0; k < 8; ++k) c[k] = fuse_value(v, c[k]);
+    return lerp(lerp(lerp(c[0], c[1], f[0]), lerp(c[2], c[3], f[0]), f[1]),
+                lerp(lerp(c[4], c[5], f[0]), lerp(c[6], c[7], f[0]), f[1]), f[2]);
 }
 
-__global__ void k_fuse_group(FuseViews fv, long long bx, long long by, long long bz, int nx, int ny, int nz,
-                             float *__restrict__ out_img, float *__restrict__ out_w, const double *__restrict__ lut)
+// A CTA takes kFuseRows rows of the box: the part of t that is constant along a row is formed in
+// double, once per row, view and axis (apply_affine at the row's first voxel), and t = base + x
+// step on pairs of floats per voxel.  Bound by instruction issue (about 200 float instructions
+// per voxel and view) and the corner loads.
+__global__ void __launch_bounds__(kFuseThreads)
+    k_fuse_group(const __grid_constant__ FuseViews fv, long long bx, long long by, long long bz, int nx, int ny, int nz,
+                 float *__restrict__ out_img, float *__restrict__ out_w, const FPair *__restrict__ lut)
 {
-    const long long n = (long long)nx * ny * nz;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % nx);
-        const int y = (int)((i / nx) % ny);
-        const int z = (int)(i / ((long long)nx * ny));
-        const double s0 = (double)(x + bx), s1 = (double)(y + by), s2 = (double)(z + bz);
-        double sumI = 0.0, sumW = 0.0, sumD = 0.0;
+    __shared__ FPair base[kFuseRows][kFuseMaxViews][3];
+    const int y0 = blockIdx.x * kFuseRows, z = blockIdx.y;
+    const int rows = min(kFuseRows, ny - y0);
+    for (int i = threadIdx.x; i < rows * fv.n; i += kFuseThreads) {
+        const int k = i / rows, r = i - k * rows;
+        const double s[3] = {(double)bx, (double)(y0 + r + by), (double)(z + bz)};
+        double t[3];
+        apply_affine(fv.v[k].inv, s, t);
+        for (int d = 0; d < 3; ++d) base[r][k][d] = fp_from(t[d]);
+    }
+    __syncthreads();
+    const int total = rows * nx;
+    for (int i = threadIdx.x; i < total; i += kFuseThreads) {
+        const int r = i / nx, x = i - r * nx;
+        FPair sumI = {0.0f, 0.0f}, sumW = {0.0f, 0.0f}, sumD = {0.0f, 0.0f};
         for (int k = 0; k < fv.n; ++k) {
             const FuseView &v = fv.v[k];
-            const double sp[3] = {s0, s1, s2};
-            double t[3];
-            apply_affine(v.inv, sp, t);
-            const float tf[3] = {(float)t[0], (float)t[1], (float)t[2]};
+            float tf[3], f[3];
+            int c[3];
+            bool in = true;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                FPair t = fp_add(fp_mul(v.step[d], (float)x), base[r][k][d]);
+                const float top = (float)(v.dims[d] - 1);
+                // next to a face of the view (a whole plane of samples, when the views are a quarter turn
+                // apart) the rounding of the double evaluation decides inside or outside: take that one
+                if (fabsf(t.h) < 1e-6f || fabsf(__fadd_rn(__fsub_rn(t.h, top), t.l)) < 1e-6f) {
+                    const double s[3] = {(double)(x + bx), (double)(y0 + r + by), (double)(z + bz)};
+                    t = fp_from(apply_affine_row(v.inv + 4 * d, s));
+                }
+                tf[d] = t.h;
+                in = in && (t.h > 0.0f || (t.h == 0.0f && t.l > 0.0f)) && (t.h < top || (t.h == top && t.l < 0.0f));
+                float fl = floorf(t.h);
+                f[d] = __fadd_rn(__fsub_rn(t.h, fl), t.l);
+                if (f[d] < 0.0f) {  // t just below an integer
+                    fl -= 1.0f;
+                    f[d] += 1.0f;
+                }
+                c[d] = (int)fl;
+            }
             const float wf = v.fblend ? blend_weight(tf, v.dims, v.fb, v.fr, lut) : 1.0f;
             const float wd = v.dblend ? blend_weight(tf, v.dims, v.db, v.dr, lut) : 1.0f;
-            sumD += (double)wd;
+            sumD = fp_add(sumD, wd);
             if (wf == 0.0f) continue;
-            float val = 0.0f;  // outsideValueImg
-            if (t[0] > 0.0 && t[1] > 0.0 && t[2] > 0.0 && t[0] < v.dims[0] - 1 && t[1] < v.dims[1] - 1 &&
-                t[2] < v.dims[2] - 1)
-                val = fmaxf(1.0f, trilinear(v, t));  // minValueImg
-            sumI += (double)val * (double)wf;
-            sumW += (double)wf;
+            const float val = in ? fmaxf(1.0f, trilinear(v, c, f)) : 0.0f;  // minValueImg, outsideValueImg
+            sumI = fp_add(sumI, fp_prod(val, wf));
+            sumW = fp_add(sumW, wf);
         }
-        out_img[i] = sumW > 0.0 ? (float)(sumI / sumW) : 0.0f;
-        out_w[i] = (float)sumD;
+        float im = 0.0f;
+        if (sumW.h > 0.0f) {
+            // sumI / sumW: the float quotient and the correction by its residual
+            const float q = __fdiv_rn(sumI.h, sumW.h);
+            const float e = __fadd_rn(__fmaf_rn(-q, sumW.h, sumI.h), __fmaf_rn(-q, sumW.l, sumI.l));
+            im = __fadd_rn(q, __fdividef(e, sumW.h));
+        }
+        const long long o = ((long long)z * ny + y0 + r) * nx + x;
+        out_img[o] = im;
+        out_w[o] = __fadd_rn(sumD.h, sumD.l);
     }
 }
 
@@ -157,27 +260,30 @@ extern "C" MVR_API int mvr_fuse_group(const mvr_fuse_view *views, int num_views,
         v.fblend = s.fusion_blend;
         v.dblend = s.decon_blend;
         v.adjust = s.intensity_adjust ? 1 : 0;
-        v.m00 = s.intensity[0];
-        v.m01 = s.intensity[1];
+        v.m00 = fp_from(s.intensity[0]);
+        v.m01 = fp_from(s.intensity[1]);
         v.img = s.img;
         if (!invert_affine(s.model, v.inv)) return fuse_fail(MVR_ERR_ARG, "mvr_fuse_group: a view model is singular");
+        for (int d = 0; d < 3; ++d) v.step[d] = fp_from(v.inv[4 * d]);
     }
     // the blending look-up table of BlendingRealRandomAccess: d runs from 0 in steps of 0.001
     // (accumulated in double, as there), entry (int)(d * 1000 + 0.5) = (cos((1 - d) pi) + 1) / 2
-    std::vector<double> lut(1001, 0.0);
-    for (double d = 0; d <= 1.0001; d = d + 0.001) lut[(int)(d * 1000.0 + 0.5)] = (std::cos((1 - d) * M_PI) + 1) / 2;
+    std::vector<FPair> lut(1001, FPair{0.0f, 0.0f});
+    for (double d = 0; d <= 1.0001; d = d + 0.001) lut[(int)(d * 1000.0 + 0.5)] = fp_from((std::cos((1 - d) * M_PI) + 1) / 2);
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) return fuse_fail(MVR_ERR_CUDA, cudaGetErrorString(e));
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    double *dlut = nullptr;
-    e = cudaMalloc(&dlut, sizeof(double) * lut.size());
+    FPair *dlut = nullptr;
+    e = cudaMalloc(&dlut, sizeof(FPair) * lut.size());
     if (e != cudaSuccess) return fuse_fail(e == cudaErrorMemoryAllocation ? MVR_ERR_OOM : MVR_ERR_CUDA, cudaGetErrorString(e));
-    e = cudaMemcpyAsync(dlut, lut.data(), sizeof(double) * lut.size(), cudaMemcpyHostToDevice, s);
-    const long long n = (long long)bb_dims[0] * bb_dims[1] * bb_dims[2];
-    if (e == cudaSuccess) {
-        const int grid = (int)std::min<long long>((n + 255) / 256, 152LL * 16);
-        k_fuse_group<<<grid, 256, 0, s>>>(fv, bb_min[0], bb_min[1], bb_min[2], bb_dims[0], bb_dims[1], bb_dims[2],
-                                          image_out, weight_out, dlut);
+    e = cudaMemcpyAsync(dlut, lut.data(), sizeof(FPair) * lut.size(), cudaMemcpyHostToDevice, s);
+    // planes beyond the grid's y limit go out in further launches
+    for (int z0 = 0; z0 < bb_dims[2] && e == cudaSuccess; z0 += 65535) {
+        const int nz = std::min(65535, bb_dims[2] - z0);
+        const long long at = (long long)z0 * bb_dims[0] * bb_dims[1];
+        const dim3 grid((unsigned)((bb_dims[1] + kFuseRows - 1) / kFuseRows), (unsigned)nz);
+        k_fuse_group<<<grid, kFuseThreads, 0, s>>>(fv, bb_min[0], bb_min[1], bb_min[2] + z0, bb_dims[0], bb_dims[1], nz,
+                                                   image_out + at, weight_out + at, dlut);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -63,3 +63,52 @@ def test_fuse_group_matches_oracle(blend):
     assert np.abs(img - ref_img)[safe].max() <= 1e-5 * max(1.0, float(np.abs(ref_img).max()))
     assert np.abs(w - ref_w)[safe].max() <= 1e-6
     assert (ref_img > 0).mean() > 0.3  # the views cover a good part of the box
+
+
+@pytest.mark.parametrize("bb_min,bb_dims,angle,scale,shift,nv,blend", [
+    ((0, 0, 0), (1, 1, 1), 10.0, 1.0, (-3.3, -2.7, -1.9), 1, False),       # one voxel
+    ((2, 1, 1), (7, 9, 3), 25.0, 1.5, (0.31, -0.47, 0.23), 2, True),       # a row group and one row more
+    ((-3, -2, -1), (33, 8, 5), 0.0, 1.0, (0.0, 0.0, 0.0), 1, True),        # samples on the voxels and borders
+    ((-3, -2, -9), (40, 17, 30), 90.0, 1.0, (0.0, 0.0, 8.0), 1, False),    # axes exchanged
+    ((1000000, -2000000, 500000), (31, 20, 9), 33.0, 2.0, (1000000.37, -2000000.61, 500000.43), 3, True),  # far away
+    ((0, 0, 0), (300, 3, 2), -20.0, 1.0, (0.7, 0.1, 0.9), 16, True),       # 16 views, rows longer than a CTA
+])
+def test_fuse_group_edges(bb_min, bb_dims, angle, scale, shift, nv, blend):
+    # the pair arithmetic against the oracle's doubles; voxels within 1e-6 of a border or of a step of the
+    # blending table (1 / 1000 of the range) may round to the other side and are left out
+    rng = np.random.default_rng(nv + bb_dims[0])
+    views = []
+    for k in range(nv):
+        img = rng.uniform(0, 300, (8, 24, 40)).astype(np.float32)
+        v = {"img": img, "model": model(angle + 3.0 * k, scale, np.asarray(shift) + 0.11 * k)}
+        if k % 3 == 1:
+            v["intensity"] = (0.731, 12.5)
+        if blend:
+            v["fusion"] = ((1.0, 2.0, 0.0), (10.0, 7.0, 3.0))
+            v["decon"] = ((0.5, 0.0, 0.5), (6.0, 6.0, 2.0))
+        views.append(v)
+    ref_img, ref_w = O.fuse_group(views, bb_min, bb_dims)
+    dev = [torch.from_numpy(v["img"]).cuda() for v in views]
+    out_i = torch.full((bb_dims[2], bb_dims[1], bb_dims[0]), -1.0, device="cuda")
+    out_w = torch.full_like(out_i, -1.0)
+    gv = [dict(v, img_ptr=d.data_ptr(), dims=(40, 24, 8)) for v, d in zip(views, dev)]
+    M.fuse_group(gv, bb_min, bb_dims, out_i.data_ptr(), out_w.data_ptr())
+    z, y, x = np.meshgrid(*[np.arange(n) for n in bb_dims[::-1]], indexing="ij")
+    s = np.stack([x + bb_min[0], y + bb_min[1], z + bb_min[2]], -1).astype(np.float64)
+    safe = np.ones(s.shape[:-1], bool)
+    dims = np.array((40, 24, 8), dtype=np.float64)
+    for v in views:
+        inv = O._invert_affine(v["model"])
+        t = s @ inv[:, :3].T + inv[:, 3]
+        whole = np.abs(t - np.round(t)) == 0  # exact samples take the same branch on both sides
+        near = (np.abs(t) <= 1e-6) | (np.abs(t - (dims - 1)) <= 1e-6)
+        safe &= ~np.any(near & ~whole, axis=-1)
+        for key in ("fusion", "decon"):
+            if v.get(key):
+                b, r = (np.asarray(a) for a in v[key])
+                e = np.minimum(t - b, dims - 1 - t - b) / r * 1000 + 0.5
+                safe &= ~np.any((np.abs(e - np.round(e)) < 1e-3) & (e > 0) & (e < 1001), axis=-1)
+    got_i, got_w = out_i.cpu().numpy(), out_w.cpu().numpy()
+    assert safe.mean() > (0.8 if nv < 16 else 0.3) or angle == 0.0
+    assert np.abs(got_i - ref_img)[safe].max(initial=0.0) <= 1e-5 * max(1.0, float(np.abs(ref_img).max()))
+    assert np.abs(got_w - ref_w)[safe].max(initial=0.0) <= 1e-6 * max(1, nv)
