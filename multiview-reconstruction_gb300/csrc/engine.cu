@@ -325,6 +325,9 @@ Engine<T>::~Engine()
         cudaEventDestroy(p.b);
     }
     for (auto e : event_pool_) cudaEventDestroy(e);
+    if (ev_fork_) cudaEventDestroy(ev_fork_);
+    if (ev_join_) cudaEventDestroy(ev_join_);
+    if (side_) cudaStreamDestroy(side_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -1367,12 +1370,69 @@ int Engine<T>::sep_make(SepPlan &pl, const int P[3], const float *k1, const floa
             SepSrc src{k, 1, {kd[0], kd[1], kd[2]}, 1.0 / ((double)P[0] * P[1] * P[2])};
             launches_ += 3;
             MVR_CUDA(sep_x_fwd(g, tl, 1, src, S0_, pl.twx, stream_));
-            MVR_CUDA(sep_y_fwd(g, tl, 1, SEP_KERNEL, kd, S0_, pl.twy, stream_));
-            MVR_CUDA(sep_z(g, tl, 1, SEP_KERNEL, 0, kd, S0_, which ? pl.k2h : pl.k1h, nullptr, pl.twz, stream_));
+            const SepSlab all{0, g.nxb, false};
+            MVR_CUDA(sep_y_fwd(g, all, tl, 1, SEP_KERNEL, kd, S0_, pl.twy, stream_));
+            MVR_CUDA(sep_z(g, all, tl, 1, SEP_KERNEL, 0, kd, S0_, which ? pl.k2h : pl.k1h, nullptr, pl.twz, stream_));
         }
         MVR_CUDA(cudaStreamSynchronize(stream_));
         return OK;
     }
+}
+
+// The three passes work on a column block alone, so where a batch's spectra outgrow L2 they run over
+// slabs of column blocks, each through all three while it is in L2, alternating between two
+// streams so that one slab's launches fill the other's tails: 4-view 256^3 (85 MB of spectrum) 1.255
+// -> 1.217 ms per iteration, 6 views of 512 x 512 x 256 (340 MB) 8.48 -> 8.08 ms; slabs of 12 MB lose
+// 12 % on the former to half-empty launches, 60 MB give nothing.  Below two slabs, and under
+// the profiler (which times launches on one stream), the passes run whole.
+constexpr double kSepSlab = 36e6;
+
+template <typename T>
+int Engine<T>::sep_yzy(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, int map, int out_w,
+                       const float2 *K, float2 *S0, float2 *S1, bool fwd, const double *bytes, bool &first)
+{
+    const double xb_bytes = 128.0 * g.Zs * g.P[1] * nt;  // one column block of the batch
+    const int per = (int)std::max(1.0, kSepSlab / xb_bytes);
+    const int slabs = prof_on_ || xb_bytes * g.nxb < 2.0 * kSepSlab ? 1 : (g.nxb + per - 1) / per;
+    first = false;
+    if (slabs == 1) {
+        const SepSlab all{0, g.nxb, false};
+        if (fwd) {
+            MVR_TRY(prof_begin(KK_COLS_FWD, bytes[0]));
+            MVR_CUDA(sep_y_fwd(g, all, tl, nt, map, nullptr, S0, pl.twy, stream_));
+            MVR_TRY(prof_end());
+        }
+        MVR_TRY(prof_begin(KK_COLS_ZMUL, bytes[1]));
+        MVR_CUDA(sep_z(g, all, tl, nt, map, out_w, nullptr, S0, S1, K, pl.twz, stream_));
+        MVR_TRY(prof_end());
+        MVR_TRY(prof_begin(KK_COLS_INV, bytes[2]));
+        MVR_CUDA(sep_y_inv(g, all, tl, nt, out_w, S1, pl.twy, stream_));
+        return prof_end();
+    }
+    if (!side_) {
+        MVR_CUDA(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
+        MVR_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
+        MVR_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
+    }
+    MVR_CUDA(cudaEventRecord(ev_fork_, stream_));
+    MVR_CUDA(cudaStreamWaitEvent(side_, ev_fork_, 0));
+    SepGeom gs = g;
+    gs.stream = 1;  // K^ past the slabs
+    for (int i = 0; i < slabs; ++i) {
+        cudaStream_t s = i & 1 ? side_ : stream_;
+        const int x0 = (int)((long long)g.nxb * i / slabs), x1 = (int)((long long)g.nxb * (i + 1) / slabs);
+        SepSlab sl{x0, x1 - x0, i == 1};
+        if (fwd) MVR_CUDA(sep_y_fwd(gs, sl, tl, nt, map, nullptr, S0, pl.twy, s));
+        if (fwd) sl.first = false;
+        MVR_CUDA(sep_z(gs, sl, tl, nt, map, out_w, nullptr, S0, S1, K, pl.twz, s));
+        sl.first = false;
+        MVR_CUDA(sep_y_inv(gs, sl, tl, nt, out_w, S1, pl.twy, s));
+        launches_ += 3;
+    }
+    MVR_CUDA(cudaEventRecord(ev_join_, side_));
+    MVR_CUDA(cudaStreamWaitEvent(stream_, ev_join_, 0));
+    first = true;
+    return OK;
 }
 
 // conv1 and the quotient's transform along x: psi to S0 (x, y; kept when another view needs it
@@ -1396,18 +1456,12 @@ int Engine<T>::sep_conv1(const SepPlan &pl, const SepGeom &g, const SepTiles &tl
         MVR_TRY(prof_begin(KK_ROWS_FWD, 4.0 * nv + 8.0 * sv));
         MVR_CUDA(sep_x_fwd(g, tl, nt, SepSrc{psi, 0, {0, 0, 0}, 1.0}, S0, pl.twx, stream_));
         MVR_TRY(prof_end());
-        MVR_TRY(prof_begin(KK_COLS_FWD, 8.0 * (sv + yv)));
-        MVR_CUDA(sep_y_fwd(g, tl, nt, SEP_MIRROR, nullptr, S0, pl.twy, stream_));
-        MVR_TRY(prof_end());
     }
-    MVR_TRY(prof_begin(KK_COLS_ZMUL, 8.0 * (yv + zq) + kb));
-    MVR_CUDA(sep_z(g, tl, nt, SEP_MIRROR, 0, nullptr, S0, S1, pl.k1h, pl.twz, stream_));
-    MVR_TRY(prof_end());
-    MVR_TRY(prof_begin(KK_COLS_INV, 8.0 * (zq + sq)));
-    MVR_CUDA(sep_y_inv(g, tl, nt, 0, S1, pl.twy, stream_));
-    MVR_TRY(prof_end());
+    const double by[3] = {8.0 * (sv + yv), 8.0 * (yv + zq) + kb, 8.0 * (zq + sq)};
+    bool first = false;
+    MVR_TRY(sep_yzy(pl, g, tl, nt, SEP_MIRROR, 0, pl.k1h, S0, S1, fresh, by, first));
     MVR_TRY(prof_begin(KK_ROWS_RATIO, 16.0 * sq + 4.0 * nq));
-    MVR_CUDA(sep_x_ratio(g, tl, nt, img, S1, pl.twx, stream_));
+    MVR_CUDA(sep_x_ratio(g, tl, nt, img, S1, pl.twx, stream_, first));
     return prof_end();
 }
 
@@ -1425,18 +1479,12 @@ int Engine<T>::sep_finish(const SepPlan &pl, const SepGeom &g, const SepTiles &t
         sw += (double)g.nxb * 16 * a[1].nw * a[2].nw;
         nw += (double)a[0].nw * a[1].nw * a[2].nw;
     }
-    MVR_TRY(prof_begin(KK_COLS_FWD, 8.0 * (sq + zq)));
-    MVR_CUDA(sep_y_fwd(g, tl, nt, SEP_FILL, nullptr, S, pl.twy, stream_));
-    MVR_TRY(prof_end());
-    MVR_TRY(prof_begin(KK_COLS_ZMUL, 8.0 * (zq + zw) + 8.0 * (double)sep_elems(g.P)));
-    MVR_CUDA(sep_z(g, tl, nt, SEP_FILL, 1, nullptr, S, S, pl.k2h, pl.twz, stream_));
-    MVR_TRY(prof_end());
-    MVR_TRY(prof_begin(KK_COLS_INV, 8.0 * (zw + sw)));
-    MVR_CUDA(sep_y_inv(g, tl, nt, 1, S, pl.twy, stream_));
-    MVR_TRY(prof_end());
+    const double by[3] = {8.0 * (sq + zq), 8.0 * (zq + zw) + 8.0 * (double)sep_elems(g.P), 8.0 * (zw + sw)};
+    bool first = false;
+    MVR_TRY(sep_yzy(pl, g, tl, nt, SEP_FILL, 1, pl.k2h, S, S, true, by, first));
     const double per = epi == EPI_SEQ ? 12.0 : (epi == EPI_MUL_FIRST ? 8.0 : (epi == EPI_MUL_ACC ? 16.0 : 16.0 + 4.0 * u.nviews));
     MVR_TRY(prof_begin(KK_ROWS_UPDATE, 8.0 * sw + per * nw));
-    MVR_CUDA(sep_x_update(g, tl, nt, epi, u, S, pl.twx, stream_));
+    MVR_CUDA(sep_x_update(g, tl, nt, epi, u, S, pl.twx, stream_, first));
     MVR_TRY(prof_end());
     if (stats_dev && (epi == EPI_SEQ || epi == EPI_MUL_FINAL)) {
         const int slots = sep_row_ctas(g.P[0], max_rows(tl.t, nt));

@@ -215,6 +215,10 @@ private:
     int launch_update(const Plan<T> &pl, const BlockMaps &bms, int nb, V *S, const UpdateArgs &ua, int epi,
                       double bytes, double *stats_dev);
     BlockMaps block_maps(const Plan<T> &pl, const BlockPlace *bps, int nb) const;
+    // y forward, z (times K), y inverse of a tile batch, the column blocks in slabs on two streams when
+    // the spectra outgrow L2; first: the passes ended in a join of the streams
+    int sep_yzy(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, int map, int out_w, const float2 *K,
+                float2 *S0, float2 *S1, bool fwd, const double *bytes, bool &first);
     int sep_conv1(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, const float *psi, const float *img,
                   float2 *S0, float2 *S1, bool fresh);
     int sep_finish(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, int epi, const SepUpd &u, float2 *S,
@@ -225,6 +229,8 @@ private:
     double lambda_ = 0.0;
     float min_value_ = 1e-4f;
     cudaStream_t stream_ = nullptr;
+    cudaStream_t side_ = nullptr;                       // every other slab of sep_yzy
+    cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
     V *S0_ = nullptr, *S1_ = nullptr;
     long long Scap_ = 0;
     double *prod_ = nullptr;

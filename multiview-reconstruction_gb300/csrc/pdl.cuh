@@ -41,4 +41,14 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
+// The same, or an ordinary launch (full: behind a join of two streams).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dep(bool full, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                       Args &&...args)
+{
+    if (!full) return launch_pdl(kernel, grid, block, smem, s, std::forward<Args>(args)...);
+    kernel<<<grid, block, smem, s>>>(std::forward<Args>(args)...);
+    return cudaGetLastError();
+}
+
 }  // namespace mvr

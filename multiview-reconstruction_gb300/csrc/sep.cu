@@ -75,25 +75,25 @@ cudaError_t sep_x_fwd(const SepGeom &g, const SepTiles &tl, int nt, const SepSrc
 }
 
 cudaError_t sep_x_ratio(const SepGeom &g, const SepTiles &tl, int nt, const float *img, float2 *S, const float2 *twx,
-                        cudaStream_t s)
+                        cudaStream_t s, bool first)
 {
     const SxOps *o = sx_ops(g.P[0]);
     if (!o) return cudaErrorInvalidValue;
     const int rows = tile_max(tl, nt, [](const SepTile &t) { return t.a[1].nq * t.a[2].nq; });
-    return o->ratio(g, tl, nt, sep_row_ctas(g.P[0], rows), img, S, aligned8(img), twx, s);
+    return o->ratio(g, tl, nt, sep_row_ctas(g.P[0], rows), img, S, aligned8(img), twx, s, first);
 }
 
 cudaError_t sep_x_update(const SepGeom &g, const SepTiles &tl, int nt, int epi, const SepUpd &u, const float2 *S,
-                         const float2 *twx, cudaStream_t s)
+                         const float2 *twx, cudaStream_t s, bool first)
 {
     const SxOps *o = sx_ops(g.P[0]);
     if (!o) return cudaErrorInvalidValue;
     const int rows = tile_max(tl, nt, [](const SepTile &t) { return t.a[1].nw * t.a[2].nw; });
     const bool vec = aligned8(u.psi) && aligned8(u.dst) && aligned8(u.weight[0]);
-    return o->update(g, tl, nt, sep_row_ctas(g.P[0], rows), epi, u, S, vec, twx, s);
+    return o->update(g, tl, nt, sep_row_ctas(g.P[0], rows), epi, u, S, vec, twx, s, first);
 }
 
-cudaError_t sep_y_fwd(const SepGeom &g, const SepTiles &tl, int nt, int map, const int kd[3], float2 *S,
+cudaError_t sep_y_fwd(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int map, const int kd[3], float2 *S,
                       const float2 *twy, cudaStream_t s)
 {
     const YzOps *o = yz_ops(g.P[1]);
@@ -101,24 +101,24 @@ cudaError_t sep_y_fwd(const SepGeom &g, const SepTiles &tl, int nt, int map, con
     const int planes = map == SEP_MIRROR ? tile_max(tl, nt, [](const SepTile &t) { return t.a[2].nv; })
                        : map == SEP_FILL ? tile_max(tl, nt, [](const SepTile &t) { return t.a[2].nq; })
                                          : kd[2];
-    return o->y_fwd(g, tl, nt, map, kd ? kd[1] : 0, kd ? kd[2] : 0, S, twy, s, planes);
+    return o->y_fwd(g, sl, tl, nt, map, kd ? kd[1] : 0, kd ? kd[2] : 0, S, twy, s, planes);
 }
 
-cudaError_t sep_y_inv(const SepGeom &g, const SepTiles &tl, int nt, int out_w, float2 *S, const float2 *twy,
+cudaError_t sep_y_inv(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int out_w, float2 *S, const float2 *twy,
                       cudaStream_t s)
 {
     const YzOps *o = yz_ops(g.P[1]);
     if (!o) return cudaErrorInvalidValue;
     const int planes = tile_max(tl, nt, [out_w](const SepTile &t) { return out_w ? t.a[2].nw : t.a[2].nq; });
-    return o->y_inv(g, tl, nt, out_w, S, twy, s, planes);
+    return o->y_inv(g, sl, tl, nt, out_w, S, twy, s, planes);
 }
 
-cudaError_t sep_z(const SepGeom &g, const SepTiles &tl, int nt, int map, int out_w, const int kd[3], const float2 *src,
+cudaError_t sep_z(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int map, int out_w, const int kd[3], const float2 *src,
                   float2 *dst, const float2 *K, const float2 *twz, cudaStream_t s)
 {
     const YzOps *o = yz_ops(g.P[2]);
     if (!o) return cudaErrorInvalidValue;
-    return o->z(g, tl, nt, map, out_w, kd ? kd[2] : 0, src, dst, K, twz, s);
+    return o->z(g, sl, tl, nt, map, out_w, kd ? kd[2] : 0, src, dst, K, twz, s);
 }
 
 }  // namespace mvr

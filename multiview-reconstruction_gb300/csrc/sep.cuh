@@ -57,6 +57,13 @@ inline SepGeom sep_geom(const int P[3], int planes)
     return g;
 }
 
+// The column blocks [x0, x0 + n) of a y or z pass (the Nyquist plane goes with block 0).  first: the
+// launch follows a join of streams (no programmatic dependence on its predecessor).
+struct SepSlab {
+    int x0, n;
+    bool first;
+};
+
 // The smallest supported transform length >= n along x, and along y and z (0: none).
 int sep_len_x(int n);
 int sep_len_yz(int n);
@@ -83,10 +90,10 @@ int sep_row_ctas(int Px, int rows);
 cudaError_t sep_x_fwd(const SepGeom &g, const SepTiles &tl, int nt, const SepSrc &src, float2 *S, const float2 *twx,
                       cudaStream_t s);
 cudaError_t sep_x_ratio(const SepGeom &g, const SepTiles &tl, int nt, const float *img, float2 *S, const float2 *twx,
-                        cudaStream_t s);
+                        cudaStream_t s, bool first = false);
 // epi: EPI_SEQ, EPI_MUL_FIRST, EPI_MUL_ACC or EPI_MUL_FINAL
 cudaError_t sep_x_update(const SepGeom &g, const SepTiles &tl, int nt, int epi, const SepUpd &u, const float2 *S,
-                         const float2 *twx, cudaStream_t s);
+                         const float2 *twx, cudaStream_t s, bool first = false);
 
 // Where a pass finds its input rows or planes along the transformed axis.
 enum SepMap {
@@ -97,14 +104,14 @@ enum SepMap {
 // y passes in place, over planes [0, planes) of each tile's buffer: forward from the stored rows,
 // inverse to the quotient's rows (out_w 0) or the written rows (out_w 1).
 // kd: the kernel's size (SEP_KERNEL; else NULL).
-cudaError_t sep_y_fwd(const SepGeom &g, const SepTiles &tl, int nt, int map, const int kd[3], float2 *S,
+cudaError_t sep_y_fwd(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int map, const int kd[3], float2 *S,
                       const float2 *twy, cudaStream_t s);
-cudaError_t sep_y_inv(const SepGeom &g, const SepTiles &tl, int nt, int out_w, float2 *S, const float2 *twy,
+cudaError_t sep_y_inv(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int out_w, float2 *S, const float2 *twy,
                       cudaStream_t s);
 // z pass: forward, times K, inverse; src planes by `map`, dst planes: the quotient's (out_w 0) or
 // the written ones (out_w 1).  K NULL: forward alone, every plane of a kernel spectrum (dst with
 // Zs = Pz) stored.
-cudaError_t sep_z(const SepGeom &g, const SepTiles &tl, int nt, int map, int out_w, const int kd[3], const float2 *src,
+cudaError_t sep_z(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int map, int out_w, const int kd[3], const float2 *src,
                   float2 *dst, const float2 *K, const float2 *twz, cudaStream_t s);
 
 }  // namespace mvr

@@ -559,9 +559,9 @@ struct SxOps {
     cudaError_t (*fwd)(const SepGeom &, const SepTiles &, int, int, const SepSrc &, float2 *, int, const float2 *,
                        cudaStream_t);
     cudaError_t (*ratio)(const SepGeom &, const SepTiles &, int, int, const float *, float2 *, int, const float2 *,
-                         cudaStream_t);
+                         cudaStream_t, bool);
     cudaError_t (*update)(const SepGeom &, const SepTiles &, int, int, int, const SepUpd &, const float2 *, int,
-                          const float2 *, cudaStream_t);
+                          const float2 *, cudaStream_t, bool);
 };
 
 template <int V>
@@ -595,20 +595,20 @@ struct Sx {
         return launch_pdl(k_sep_x_fwd<V>, dim3(ctas, nt), SH::NT, SH::smem, s, src, S, tl, g, vec, tw);
     }
     static cudaError_t ratio(const SepGeom &g, const SepTiles &tl, int nt, int ctas, const float *img, float2 *S,
-                             int vec, const float2 *tw, cudaStream_t s)
+                             int vec, const float2 *tw, cudaStream_t s, bool first)
     {
         const cudaError_t e = ready();
         if (e != cudaSuccess) return e;
-        return launch_pdl(k_sep_x_ratio<V>, dim3(ctas, nt), SH::NT, SH::smem, s, S, img, tl, g, vec, tw);
+        return launch_dep(first, k_sep_x_ratio<V>, dim3(ctas, nt), SH::NT, SH::smem, s, S, img, tl, g, vec, tw);
     }
     static cudaError_t update(const SepGeom &g, const SepTiles &tl, int nt, int ctas, int epi, const SepUpd &u,
-                              const float2 *S, int vec, const float2 *tw, cudaStream_t s)
+                              const float2 *S, int vec, const float2 *tw, cudaStream_t s, bool first)
     {
         const cudaError_t e = ready();
         if (e != cudaSuccess) return e;
         const dim3 grid(ctas, nt);
         const bool st = u.partials && (epi == EPI_SEQ || epi == EPI_MUL_FINAL);
-#define SX_UPD(M, ST) launch_pdl(k_sep_x_update<V, M, ST>, grid, SH::NT, SH::smem, s, S, u, epi, tl, g, vec, tw)
+#define SX_UPD(M, ST) launch_dep(first, k_sep_x_update<V, M, ST>, grid, SH::NT, SH::smem, s, S, u, epi, tl, g, vec, tw)
         if (epi == EPI_SEQ) return st ? SX_UPD(false, true) : SX_UPD(false, false);
         return st ? SX_UPD(true, true) : SX_UPD(true, false);
 #undef SX_UPD

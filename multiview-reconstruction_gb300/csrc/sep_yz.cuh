@@ -119,14 +119,17 @@ __device__ __forceinline__ void sep_tw_put(float2 *tw, const float2 (&r)[YzShape
 // fill: value of the quotient's constant rows in column 0 (the x transform of ones: Px)
 template <int T, int V>
 __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Y)
-    k_sep_y_fwd(float2 *S, const SepTiles tl, SepGeom g, int map, int kdy, int kdz, const float2 *__restrict__ twg)
+    k_sep_y_fwd(float2 *S, const SepTiles tl, SepGeom g, SepSlab sl, int map, int kdy, int kdz,
+                const float2 *__restrict__ twg)
 {
     typedef YzShape<T, V> SH;
     constexpr int n = SH::n;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *A = reinterpret_cast<float2 *>(smem_raw);
     float2 *tw = A + 16 * n;
-    const int z = blockIdx.x, xb = blockIdx.y;
+    // planes from the last to the first, all column blocks of a plane together: the rows pass before
+    // left the last planes in L2
+    const int z = gridDim.y - 1 - blockIdx.y, xb = sl.x0 + blockIdx.x;
     const SepTile &tile = tl.t[blockIdx.z];
     unsigned *off = reinterpret_cast<unsigned *>(tw + n);
     pdl_trigger();
@@ -188,14 +191,15 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Y)
 // ---- y inverse, in place ------------------------------------------------------------------
 template <int T, int V>
 __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Y)
-    k_sep_y_inv(float2 *S, const SepTiles tl, SepGeom g, int out_w, const float2 *__restrict__ twg)
+    k_sep_y_inv(float2 *S, const SepTiles tl, SepGeom g, SepSlab sl, int out_w, const float2 *__restrict__ twg)
 {
     typedef YzShape<T, V> SH;
     constexpr int n = SH::n;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *A = reinterpret_cast<float2 *>(smem_raw);
     float2 *tw = A + 16 * n;
-    const int z = blockIdx.x, xb = blockIdx.y;
+    // column blocks from the last to the first: the z pass before left the last ones in L2
+    const int z = blockIdx.x, xb = sl.x0 + gridDim.y - 1 - blockIdx.y;
     const SepTile &tile = tl.t[blockIdx.z];
     pdl_trigger();
     for (int i = threadIdx.x; i < n; i += SH::NT) tw[i] = __ldg(&twg[i]);
@@ -241,8 +245,8 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Y)
 // ---- z: forward, times K, inverse -----------------------------------------------------------
 template <int T, int V, bool MUL>
 __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Z)
-    k_sep_z(const float2 *src, float2 *dst, const float2 *__restrict__ K, const SepTiles tl, SepGeom g, int map,
-            int out_w, int kdz, const float2 *__restrict__ twg)
+    k_sep_z(const float2 *src, float2 *dst, const float2 *__restrict__ K, const SepTiles tl, SepGeom g,
+            SepSlab sl, int map, int out_w, int kdz, const float2 *__restrict__ twg)
 {
     typedef YzShape<T, V> SH;
     constexpr int n = SH::n;
@@ -254,9 +258,11 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Z)
     const SepTile &tile = tl.t[blockIdx.y];
     pdl_trigger();
     const int c = threadIdx.x & 15, u = threadIdx.x >> 4;
-    // the 16 columns: one line of column block xb at y, or 16 y of the Nyquist plane
-    const int xb = blockIdx.x / Py, y = blockIdx.x - xb * Py;
-    const bool nyq = xb == g.nxb;
+    // the 16 columns: one line of column block xb at y, or 16 y of the Nyquist plane (behind the
+    // slab of column block 0)
+    const int xq = blockIdx.x / Py, y = blockIdx.x - xq * Py;
+    const bool nyq = xq == sl.n;
+    const int xb = nyq ? g.nxb : sl.x0 + xq;
     const int cols = nyq ? min(16, Py - 16 * y) : 16;
     const bool live = c < cols;
     const unsigned pitch = nyq ? Py : Py * 16;
@@ -334,11 +340,12 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Z)
 
 // The launches of one length.
 struct YzOps {
-    cudaError_t (*y_fwd)(const SepGeom &, const SepTiles &, int, int, int, int, float2 *, const float2 *, cudaStream_t,
-                         int);
-    cudaError_t (*y_inv)(const SepGeom &, const SepTiles &, int, int, float2 *, const float2 *, cudaStream_t, int);
-    cudaError_t (*z)(const SepGeom &, const SepTiles &, int, int, int, int, const float2 *, float2 *, const float2 *,
-                     const float2 *, cudaStream_t);
+    cudaError_t (*y_fwd)(const SepGeom &, const SepSlab &, const SepTiles &, int, int, int, int, float2 *, const float2 *,
+                         cudaStream_t, int);
+    cudaError_t (*y_inv)(const SepGeom &, const SepSlab &, const SepTiles &, int, int, float2 *, const float2 *,
+                         cudaStream_t, int);
+    cudaError_t (*z)(const SepGeom &, const SepSlab &, const SepTiles &, int, int, int, int, const float2 *, float2 *,
+                     const float2 *, const float2 *, cudaStream_t);
 };
 
 template <int T, int V>
@@ -358,29 +365,29 @@ struct Yz {
         static const cudaError_t e = limits();
         return e;
     }
-    static cudaError_t y_fwd(const SepGeom &g, const SepTiles &tl, int nt, int map, int kdy, int kdz, float2 *S,
+    static cudaError_t y_fwd(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int map, int kdy, int kdz, float2 *S,
                              const float2 *tw, cudaStream_t s, int planes)
     {
         const cudaError_t e = ready();
         if (e != cudaSuccess) return e;
-        return launch_pdl(k_sep_y_fwd<T, V>, dim3(planes, g.nxb, nt), SH::NT, SH::smem, s, S, tl, g, map, kdy, kdz, tw);
+        return launch_dep(sl.first, k_sep_y_fwd<T, V>, dim3(sl.n, planes, nt), SH::NT, SH::smem, s, S, tl, g, sl, map, kdy, kdz, tw);
     }
-    static cudaError_t y_inv(const SepGeom &g, const SepTiles &tl, int nt, int out_w, float2 *S, const float2 *tw,
+    static cudaError_t y_inv(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int out_w, float2 *S, const float2 *tw,
                              cudaStream_t s, int planes)
     {
         const cudaError_t e = ready();
         if (e != cudaSuccess) return e;
-        return launch_pdl(k_sep_y_inv<T, V>, dim3(planes, g.nxb, nt), SH::NT, SH::smem, s, S, tl, g, out_w, tw);
+        return launch_dep(sl.first, k_sep_y_inv<T, V>, dim3(planes, sl.n, nt), SH::NT, SH::smem, s, S, tl, g, sl, out_w, tw);
     }
-    static cudaError_t z(const SepGeom &g, const SepTiles &tl, int nt, int map, int out_w, int kdz, const float2 *src,
+    static cudaError_t z(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int map, int out_w, int kdz, const float2 *src,
                          float2 *dst, const float2 *K, const float2 *tw, cudaStream_t s)
     {
         const cudaError_t e = ready();
         if (e != cudaSuccess) return e;
-        const dim3 grid(g.nxb * g.P[1] + (g.P[1] + 15) / 16, nt);
+        const dim3 grid(sl.n * g.P[1] + (sl.x0 == 0 ? (g.P[1] + 15) / 16 : 0), nt);
         if (K)
-            return launch_pdl(k_sep_z<T, V, true>, grid, SH::NT, SH::smem, s, src, dst, K, tl, g, map, out_w, kdz, tw);
-        return launch_pdl(k_sep_z<T, V, false>, grid, SH::NT, SH::smem, s, src, dst, K, tl, g, map, out_w, kdz, tw);
+            return launch_dep(sl.first, k_sep_z<T, V, true>, grid, SH::NT, SH::smem, s, src, dst, K, tl, g, sl, map, out_w, kdz, tw);
+        return launch_dep(sl.first, k_sep_z<T, V, false>, grid, SH::NT, SH::smem, s, src, dst, K, tl, g, sl, map, out_w, kdz, tw);
     }
     static const YzOps *ops()
     {
