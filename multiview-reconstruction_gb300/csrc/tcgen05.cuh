@@ -36,6 +36,14 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N)
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// The same with A and B M/N-major (both transposed): 8 consecutive rows (M or N) of one K form the 16
+// bytes of a core matrix row, 8 consecutive K its 128 bytes; the descriptor's leading offset
+// then steps 8 K, its stride offset 8 rows.
+__host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N)
+{
+    return idesc_bf16(M, N) | (1u << 15) | (1u << 16);
+}
+
 // Allocation by one full warp; the tensor-memory address is written to *dst.
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst, uint32_t ncols)
 {
