@@ -1439,7 +1439,7 @@ int Engine<T>::sep_yzy(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, 
 // again), times K1^ into S1, back to rows, quotient.  fresh: S0 does not hold psi's transform yet.
 template <typename T>
 int Engine<T>::sep_conv1(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, const float *psi,
-                         const float *img, float2 *S0, float2 *S1, bool fresh)
+                         const float *img, float2 *S0, float2 *S1, bool fresh, cudaEvent_t img_ready)
 {
     double nv = 0.0, sv = 0.0, yv = 0.0, zq = 0.0, sq = 0.0, nq = 0.0;
     for (int i = 0; i < nt; ++i) {
@@ -1460,6 +1460,10 @@ int Engine<T>::sep_conv1(const SepPlan &pl, const SepGeom &g, const SepTiles &tl
     const double by[3] = {8.0 * (sv + yv), 8.0 * (yv + zq) + kb, 8.0 * (zq + sq)};
     bool first = false;
     MVR_TRY(sep_yzy(pl, g, tl, nt, SEP_MIRROR, 0, pl.k1h, S0, S1, fresh, by, first));
+    if (img_ready) {
+        MVR_CUDA(cudaStreamWaitEvent(stream_, img_ready, 0));
+        first = true;
+    }
     MVR_TRY(prof_begin(KK_ROWS_RATIO, 16.0 * sq + 4.0 * nq));
     MVR_CUDA(sep_x_ratio(g, tl, nt, img, S1, pl.twx, stream_, first));
     return prof_end();
@@ -1468,7 +1472,7 @@ int Engine<T>::sep_conv1(const SepPlan &pl, const SepGeom &g, const SepTiles &tl
 // The second convolution of the quotient rows in S and the update.
 template <typename T>
 int Engine<T>::sep_finish(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, int epi, const SepUpd &u,
-                          float2 *S, double *stats_dev)
+                          float2 *S, double *stats_dev, cudaEvent_t w_ready)
 {
     double sq = 0.0, zq = 0.0, zw = 0.0, sw = 0.0, nw = 0.0;
     for (int i = 0; i < nt; ++i) {
@@ -1482,6 +1486,10 @@ int Engine<T>::sep_finish(const SepPlan &pl, const SepGeom &g, const SepTiles &t
     const double by[3] = {8.0 * (sq + zq), 8.0 * (zq + zw) + 8.0 * (double)sep_elems(g.P), 8.0 * (zw + sw)};
     bool first = false;
     MVR_TRY(sep_yzy(pl, g, tl, nt, SEP_FILL, 1, pl.k2h, S, S, true, by, first));
+    if (w_ready) {
+        MVR_CUDA(cudaStreamWaitEvent(stream_, w_ready, 0));
+        first = true;
+    }
     const double per = epi == EPI_SEQ ? 12.0 : (epi == EPI_MUL_FIRST ? 8.0 : (epi == EPI_MUL_ACC ? 16.0 : 16.0 + 4.0 * u.nviews));
     MVR_TRY(prof_begin(KK_ROWS_UPDATE, 8.0 * sw + per * nw));
     MVR_CUDA(sep_x_update(g, tl, nt, epi, u, S, pl.twx, stream_, first));
@@ -1498,7 +1506,8 @@ int Engine<T>::sep_finish(const SepPlan &pl, const SepGeom &g, const SepTiles &t
 
 template <typename T>
 int Engine<T>::sep_seq(const SepPlan &pl, const SepTile *tiles, int nt, const float *psi_src, float *psi_dst,
-                       const float *img, const float *w, float maxI, double *stats_dev)
+                       const float *img, const float *w, float maxI, double *stats_dev, cudaEvent_t img_ready,
+                       cudaEvent_t w_ready)
 {
     if constexpr (sizeof(T) != sizeof(float)) {
         return fail(ERR_STATE, "separable transforms are FP32 only");
@@ -1509,7 +1518,7 @@ int Engine<T>::sep_seq(const SepPlan &pl, const SepTile *tiles, int nt, const fl
         int planes;
         const SepTiles tl = sep_tiles(tiles, nt, planes);
         const SepGeom g = sep_batch_geom(pl.P, tiles, nt, planes, device_);
-        MVR_TRY(sep_conv1(pl, g, tl, nt, psi_src, img, S0_, S0_, true));
+        MVR_TRY(sep_conv1(pl, g, tl, nt, psi_src, img, S0_, S0_, true, img_ready));
         SepUpd u{};
         u.psi = psi_src;
         u.dst = psi_dst;
@@ -1517,7 +1526,7 @@ int Engine<T>::sep_seq(const SepPlan &pl, const SepTile *tiles, int nt, const fl
         u.nviews = 1;
         u.c = upd_const(lambda_, min_value_, maxI);
         u.partials = stats_dev ? partials_ : nullptr;
-        return sep_finish(pl, g, tl, nt, EPI_SEQ, u, S0_, stats_dev);
+        return sep_finish(pl, g, tl, nt, EPI_SEQ, u, S0_, stats_dev, w_ready);
     }
 }
 

@@ -142,8 +142,10 @@ public:
     // those voxels, or NULL.
     int sep_make(SepPlan &pl, const int P[3], const float *k1, const float *k2, const int kd[3], bool on_device);
     void sep_free(SepPlan &pl);
+    // img_ready, w_ready (or NULL): events behind the image's and the weight's arrival on the device
     int sep_seq(const SepPlan &pl, const SepTile *tiles, int nt, const float *psi_src, float *psi_dst, const float *img,
-                const float *w, float maxI, double *stats_dev);
+                const float *w, float maxI, double *stats_dev, cudaEvent_t img_ready = nullptr,
+                cudaEvent_t w_ready = nullptr);
     // tiles: one array per view (views with one domain share psi's transform along x and y)
     int sep_mul(const std::vector<const SepPlan *> &pls, const SepTile *const *tiles, int nt, const float *psi_src,
                 float *psi_dst, const float *const *imgs, const float *const *ws, float maxI, double *stats_dev);
@@ -220,9 +222,9 @@ private:
     int sep_yzy(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, int map, int out_w, const float2 *K,
                 float2 *S0, float2 *S1, bool fwd, const double *bytes, bool &first);
     int sep_conv1(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, const float *psi, const float *img,
-                  float2 *S0, float2 *S1, bool fresh);
+                  float2 *S0, float2 *S1, bool fresh, cudaEvent_t img_ready = nullptr);
     int sep_finish(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, int epi, const SepUpd &u, float2 *S,
-                   double *stats_dev);
+                   double *stats_dev, cudaEvent_t w_ready = nullptr);
 
     int device_ = -1;
     int boundary_ = BOUNDARY_REFERENCE;
