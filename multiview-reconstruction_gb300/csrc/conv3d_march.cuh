@@ -1,0 +1,285 @@
+// Forward and data-gradient 3x3x3 convolutions by columns of planes.
+//
+// A CTA walks a run of output planes, z fastest, of 8 x 16 columns of output voxels (x, y).  Every
+// input plane of a column (10 x 18 voxels with its halo, zero outside the volume) is copied into shared
+// memory once, through a ring of kMarchStages buffers, and multiplied once: the products of one offset
+// (dy, dx) with the weights of all three dz give the plane's share of three output planes, so the
+// three go into one product of 3 N columns whose accumulators are the tensor-memory columns of the
+// output planes z - 1, z and z + 1.  These columns are a ring of R planes: an output plane is
+// complete, and read back, once the input plane behind it has been multiplied.
+//
+// A K-group-major plane (the 16-byte chunk of channels 8j..8j+7 of halo voxel h = hx + 10 hy at byte
+// j * kMarchLbo + 16 h) needs no copies per offset: eight x-consecutive voxels are one core matrix, the
+// next line of the column is 10 rows further, and an offset is the same layout started
+// 16 ((1 + dx) + 10 (1 + dy)) bytes later.
+//
+// What bounds it: the operands' way out of shared memory.  A product of 128 rows reads 4 KB of A however
+// few columns it has, so 16 output channels at a time pay nine times for what 3 x 16 pay three times;
+// with B's 1.5 KB a product of 48 columns took 48 cycles.  Taking dz into the columns
+// divides the products by three (9 per 16 input channels and plane), loading a plane once divides
+// the copies by three against bricks with a halo of three planes, and the weights (27 N C) come once
+// per run instead of once per brick.  The products go out from one elected lane of a warp of its own:
+// issued behind `threadIdx.x == 0`, with descriptors formed per product, the first layer below took
+// 230 us, most of them one thread's chain of instructions.
+// One layer on 128^3 voxels (64^3 for 96 channels), bricks before and runs after: 48 -> 16 channels
+// 680 and 115 us, 16 -> 16 193 and 60, 96 -> 32 292 and 70; 16 -> 32 40 and 26, 32 -> 64 (32^3) 20 and 19.
+#pragma once
+#include "conv3d_tc.cuh"
+
+namespace mvr {
+
+constexpr int kMarchX = 8, kMarchY = 16;  // a column's lines: 128 rows of a product
+constexpr int kMarchHX = kMarchX + 2, kMarchHY = kMarchY + 2, kMarchPlane = kMarchHX * kMarchHY;
+constexpr int kMarchLbo = (kMarchPlane + 1) * 16;  // one padding row: distinct banks for the K groups
+constexpr int kMarchStages = 4;
+constexpr int kMarchThreads = 160;  // four warps copy planes and write results, one issues products
+
+// Output channels of one CTA: all of them while the weights leave room for two CTAs or, with many
+// input channels, for the ring of planes; the others are another CTA's, which reads the planes again.
+template <int N, int C>
+__host__ __device__ constexpr int march_ns()
+{
+    return N > 64 || 27 * N * C * 2 > 64 * 1024 ? N / 2 : N;
+}
+// tensor-memory columns of a CTA: a quarter of the SM's for the small channel counts, whose planes
+// are short and need more CTAs in flight, else half
+template <int NS, int C>
+__host__ __device__ constexpr int march_cols()
+{
+    return NS <= 32 && C <= 16 ? 128 : 256;
+}
+template <int NS, int C>
+__host__ __device__ constexpr size_t march_smem()
+{
+    return (size_t)kMarchStages * (C / 8) * kMarchLbo + 27 * (size_t)NS * C * 2 + 1024;
+}
+
+// A place in a CTA's run of output planes: the run goes through the planes of all columns, z fastest,
+// and falls into parts of one column each.  A part of nz output planes has nz + 2 steps, one per input
+// plane z = zs - 1 + p.
+struct MarchAt {
+    long long u;  // output plane of the run that the part starts at
+    int x0, y0, zs, b, nz, p;
+    __device__ __forceinline__ void start(const ConvGeom &g, long long u1)
+    {
+        const int nbx = (g.W + kMarchX - 1) / kMarchX, nby = (g.H + kMarchY - 1) / kMarchY;
+        const long long col = u / g.D;
+        zs = (int)(u - col * g.D);
+        nz = (int)min((long long)(g.D - zs), u1 - u);
+        x0 = (int)(col % nbx) * kMarchX;
+        y0 = (int)(col / nbx % nby) * kMarchY;
+        b = (int)(col / nbx / nby);
+        p = 0;
+    }
+    // the next step; true at the start of a part
+    __device__ __forceinline__ bool next(const ConvGeom &g, long long u1)
+    {
+        if (++p < nz + 2) return false;
+        u += nz;
+        if (u < u1) start(g, u1);
+        return u < u1;
+    }
+};
+
+// OUT_MODE 0: BF16 output with bias (+ReLU when relu != 0); 1: FP32 output, no bias.
+// CU > 0: the input is the concatenation [nearest x2 upsampling of `act` (CU channels, a volume of
+// half the size), act2 (C - CU channels)].
+template <int N, int C, int OUT_MODE, int CU = 0>
+__global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloat16 *__restrict__ act,
+                                                      const __nv_bfloat16 *__restrict__ wk,
+                                                      const float *__restrict__ bias, void *out, ConvGeom g, int sign,
+                                                      int relu, int *err,
+                                                      const __nv_bfloat16 *__restrict__ act2 = nullptr)
+{
+    constexpr int NS = march_ns<N, C>(), ST = kMarchStages, CH = C / 8;
+    constexpr uint32_t COLS = march_cols<NS, C>();
+    constexpr int R = (int)COLS / NS;  // ring of output planes: three being added to, one being read
+    constexpr int PB = CH * kMarchLbo, B_TAP = 3 * NS * C * 2;
+    constexpr int ITEMS = kMarchPlane * CH, LI = (ITEMS + 127) / 128;
+    static_assert(N % NS == 0 && NS % 16 == 0 && 3 * NS <= 256 && C % 16 == 0 && R >= 4, "tile shape");
+    static_assert(CU % 8 == 0 && (CU == 0 || CU < C), "concatenated channel split");
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t *sB = smem + ((ST * PB + 1023) / 1024) * 1024;
+    __shared__ __align__(8) uint64_t done[ST];
+    __shared__ uint32_t tbase;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    if (warp == 0) tc::tmem_alloc(&tbase, COLS);
+    if (tid == 0) {
+        for (int i = 0; i < ST; ++i) tc::mbar_init(&done[i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    const long long planes =
+        (long long)((g.W + kMarchX - 1) / kMarchX) * ((g.H + kMarchY - 1) / kMarchY) * g.B * g.D;
+    const long long u1 = planes * (blockIdx.x + 1) / gridDim.x;
+    const int co0 = blockIdx.y * NS;
+    // the copies run kMarchStages - 1 steps ahead of the products, past the ends of parts
+    MarchAt ld, at;
+    ld.u = at.u = planes * blockIdx.x / gridDim.x;
+    ld.start(g, u1);
+    at.start(g, u1);
+    int off[LI];
+    // this thread's 16-byte chunks of a plane, channel chunk fastest: offset in chunks from the
+    // halo's corner (x0 - 1, y0 - 1), of the low volume (x0 / 2 - 1, y0 / 2 - 1); -1 outside
+    auto chunks = [&]() {
+#pragma unroll
+        for (int i = 0; i < LI; ++i) {
+            const int k = tid + 128 * i, h = k / CH, j = k - h * CH;
+            const int xx = ld.x0 - 1 + h % kMarchHX, yy = ld.y0 - 1 + h / kMarchHX;
+            const bool in = k < ITEMS && xx >= 0 && yy >= 0 && xx < g.W && yy < g.H;
+            if constexpr (CU == 0) off[i] = in ? ((h / kMarchHX) * g.W + h % kMarchHX) * CH + j : -1;
+            else if (j < CU / 8)
+                off[i] = in ? ((h / kMarchHX + 1) / 2 * (g.W >> 1) + (h % kMarchHX + 1) / 2) * (CU / 8) + j : -1;
+            else off[i] = in ? ((h / kMarchHX) * g.W + h % kMarchHX) * (CH - CU / 8) + j - CU / 8 : -1;
+        }
+    };
+    chunks();
+    auto corner = [&](int z, int D, int H, int W, int y, int x) { return (((long long)ld.b * D + z) * H + y) * W + x; };
+    auto load = [&](int s) {  // the next input plane, of step s, into its buffer
+        uint8_t *dst = smem + (s % ST) * PB;
+        const int z = ld.zs - 1 + ld.p;
+        const bool zin = z >= 0 && z < g.D;
+        const int zz = zin ? z : 0;
+        const uint4 *lo, *hi = nullptr;
+        if constexpr (CU == 0) {
+            lo = reinterpret_cast<const uint4 *>(act) + corner(zz, g.D, g.H, g.W, ld.y0 - 1, ld.x0 - 1) * CH;
+        } else {
+            lo = reinterpret_cast<const uint4 *>(act) +
+                 corner(zz >> 1, g.D >> 1, g.H >> 1, g.W >> 1, ld.y0 / 2 - 1, ld.x0 / 2 - 1) * (CU / 8);
+            hi = reinterpret_cast<const uint4 *>(act2) + corner(zz, g.D, g.H, g.W, ld.y0 - 1, ld.x0 - 1) * (CH - CU / 8);
+        }
+#pragma unroll
+        for (int i = 0; i < LI; ++i) {
+            const int k = tid + 128 * i, h = k / CH, j = k - h * CH;
+            const bool in = zin && off[i] >= 0;
+            const uint4 *src = CU == 0 || j < CU / 8 ? lo : hi;
+            if ((i + 1) * 128 <= ITEMS || k < ITEMS)
+                cp_async16(dst + j * kMarchLbo + 16 * h, in ? src + off[i] : reinterpret_cast<const uint4 *>(act), in);
+        }
+        if (ld.next(g, u1)) chunks();
+    };
+    // the weights, per offset (dy, dx) 3 NS rows: output plane z - 1 (dz = 1), z, z + 1, each NS channels
+    // (every CTA reads the same ones at the same time: each starts at a place of its own)
+    constexpr int WN = 27 * NS * CH;
+    const int rot = (int)((blockIdx.x * 331u) % WN);
+    for (int s0 = tid; s0 < WN; s0 += kMarchThreads) {
+        const int s = s0 + rot < WN ? s0 + rot : s0 + rot - WN;
+        const int t = s / (3 * NS * CH), rem = s - t * (3 * NS * CH), r = rem / CH, j = rem - r * CH;
+        const int i = r / NS, tz = (1 - i) * sign + 1;
+        cp_async16(sB + t * B_TAP + tc::core_offset(r, 8 * j, C),
+                   reinterpret_cast<const uint4 *>(
+                       wk + ((long long)(co0 + r - i * NS) * 27 + 9 * tz + (sign > 0 ? t : 8 - t)) * C) + j, true);
+    }
+#pragma unroll 1
+    for (int s = 0; s < ST; ++s) {
+        if (ld.u < u1 && warp < 4) load(s);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tbase, 0);
+    const uint32_t hbase = tc::smem_u32(smem), bbase = tc::smem_u32(sB);
+    int ring = 0;  // output planes of the parts before: plane j of a part has the columns of slot (ring + j) % R
+    // the products of step s, issued by one lane; its share i goes to the part's output plane p - 2 + i
+    auto products = [&](int s) {
+        const int i0 = max(0, 2 - at.p), i1 = min(3, at.nz + 2 - at.p);  // the planes that the part has
+        const int s0 = (ring + at.p - 2 + i0) % R;                      // ring slot of the first
+        const int n0 = min(i1 - i0, R - s0), n1 = i1 - i0 - n0;          // columns up to the ring's end, and from its start
+        const uint64_t a0 = tc::smem_desc(hbase + (uint32_t)(s % ST) * PB, kMarchLbo, kMarchHX * 16);
+        const uint64_t b0 = tc::smem_desc(bbase, 128, C * 16);
+        // the newest output plane starts here, the others go on
+        for (int i = i0; i < i1; ++i)
+            tc::mma_bf16(tmem + (uint32_t)((ring + at.p - 2 + i) % R * NS), a0, b0 + (uint32_t)(i * NS * C * 2 / 16),
+                         tc::idesc_bf16(128, NS), i != 2);
+#pragma unroll 1
+        for (int seg = 0; seg < (n1 > 0 ? 2 : 1); ++seg) {
+            const int n = seg ? n1 : n0, i = seg ? i0 + n0 : i0;
+            const uint32_t d = tmem + (seg ? 0u : (uint32_t)(s0 * NS));
+            const uint32_t id = tc::idesc_bf16(128, NS) + ((uint32_t)((n - 1) * (NS >> 3)) << 17);
+            const uint64_t bs = b0 + (uint32_t)(i * NS * C * 2 / 16);
+#pragma unroll
+            for (int t = 0; t < 9; ++t)
+#pragma unroll
+                for (int k = 0; k < C / 16; ++k)
+                    if (t > 0 || k > 0)
+                        tc::mma_bf16_acc(d, a0 + (uint32_t)(2 * k * kMarchLbo / 16 + t % 3 + kMarchHX * (t / 3)),
+                                         bs + (uint32_t)(t * B_TAP / 16 + k * 16), id);
+        }
+        tc::mma_commit(&done[s % ST]);
+    };
+    bool ok = true;
+    int s = 0, slot = -1;  // slot of the output plane that step s - 1 completed, or -1
+    long long n = 0;       // this thread's voxel of it
+    bool rv = false;
+#pragma unroll 1
+    for (;; ++s) {
+        const bool more = at.u < u1;
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(ST - 2) : "memory");  // step s's plane has landed
+        tc::fence_proxy_async();
+        tc::fence_before_sync();
+        ok = __syncthreads_and(ok) != 0;
+        if (!ok) break;  // the whole CTA
+        if (more && warp == 4) {
+            tc::fence_after_sync();
+            if (tc::elect_one()) products(s);
+            __syncwarp();
+        }
+        if (s > 0 && warp < 4) {
+            // while step s is multiplied: step s - 1's buffer is free and its output plane complete
+            ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[(s - 1) % ST], ((s - 1) / ST) & 1, kTcWaitIter));
+            if (ok && ld.u < u1) load(s - 1 + ST);  // on a timeout this warp writes no more
+            tc::fence_after_sync();
+            if (ok && slot >= 0) {
+                const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(slot * NS);
+#pragma unroll
+                for (int c0 = 0; c0 < NS; c0 += 16) {
+                    float v[16];
+                    tc::tmem_ld16(trow + c0, v);
+                    if (!rv) continue;
+                    if (OUT_MODE == 0) {
+                        __align__(16) __nv_bfloat16 w[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            float a = v[j] + (bias ? bias[co0 + c0 + j] : 0.0f);
+                            if (relu) a = fmaxf(a, 0.0f);
+                            w[j] = __float2bfloat16(a);
+                        }
+                        uint4 *op = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(out) + n * N + co0 + c0);
+                        op[0] = reinterpret_cast<const uint4 *>(w)[0];
+                        op[1] = reinterpret_cast<const uint4 *>(w)[1];
+                    } else {
+                        float4 *op = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + n * N + co0 + c0);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            op[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    }
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        if (!more) break;
+        slot = -1;
+        if (at.p >= 2) {
+            const int x = at.x0 + (tid & 7), y = at.y0 + (tid >> 3 & 15);
+            slot = (ring + at.p - 2) % R;
+            n = (((long long)at.b * g.D + at.zs + at.p - 2) * g.H + y) * g.W + x;
+            rv = x < g.W && y < g.H;
+        }
+        const int nz = at.nz;
+        if (at.next(g, u1)) ring = (ring + nz) % R;
+    }
+    if (!__syncthreads_and(ok)) {
+        // a wait ran out: let every copy and product in flight finish (bounded) before the tensor
+        // memory goes back
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        if (tid == 0) {
+            atomicExch(err, 1);
+            for (int q = max(0, s - ST); q < s; ++q) tc::mbar_wait(&done[q % ST], (q / ST) & 1, kTcWaitIter);
+        }
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, COLS);
+}
+
+}  // namespace mvr

@@ -66,6 +66,24 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
+// The same, always added to D.
+__device__ __forceinline__ void mma_bf16_acc(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc));
+}
+
+// True in one lane of a converged warp.  A warp that issues products in such a branch forms their
+// descriptors in uniform registers; behind `threadIdx.x == 0` each is a chain of vector instructions.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
+    return e != 0;
+}
+
 // Arrive on *mbar once every tcgen05 operation this thread issued has completed.
 __device__ __forceinline__ void mma_commit(uint64_t *mbar)
 {

@@ -25,11 +25,9 @@
 #include <string>
 #include <vector>
 
-#include <cudaTypedefs.h>
-
 #include "../../include/mvr_gb300.h"
 #include "conv3d_tc.cuh"
-#include "conv3d_tma.cuh"
+#include "conv3d_march.cuh"
 #include "fsum.cuh"
 
 namespace mvr {
@@ -42,98 +40,40 @@ int rsize(long long n) { return (int)std::max<long long>(1, std::min<long long>(
 int gsize(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 152 * 32)); }
 
 // ---- tcgen05 convolution launchers --------------------------------------------------
-template <int N, int C>
-size_t conv_smem() { return 2 * (128 * C * 2 + N * C * 2); }
 template <int N>
 size_t wgrad_smem() { return (size_t)kWgStages * wgrad_stage_bytes<N>(); }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no libcuda link)
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
+// Forward and data-gradient convolutions (k_conv3d_march): one wave of CTAs, each a run of at least
+// kMarchMin output planes.  A run reads two input planes beyond its own and its weights, so runs of
+// 12 planes were better only on large levels, which have them anyway (32 -> 64 channels on 32^3: runs
+// of 3, 6 and 12 planes 14, 19 and 28 us; 16 -> 32 on 64^3 27, 24 and 28 us).
+constexpr int kMarchMin = 4;
+template <int N, int C, int OUT, int CU>
+cudaError_t launch_march(const bf16 *act, const bf16 *act2, const bf16 *w, const float *bias, void *out,
+                         const ConvGeom &g, int sign, int relu, int *err, cudaStream_t s)
 {
-    static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) !=
-                cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    }();
-    return fn;
-}
-
-// MVR_CONV_TMA=0 keeps every convolution on k_conv3d_shift
-bool conv_tma_enabled()
-{
-    const char *e = std::getenv("MVR_CONV_TMA");
-    return !(e && e[0] == '0');
-}
-
-// The persistent TMA convolution (k_conv3d_tma) of a shape that fits: the tensor map of the
-// [B][D][H][W][C] input with a box of 8 channels x 10 x 18 x 3 voxels, one CTA per SM slot.
-// cudaErrorNotSupported when no encoder is available (the caller falls back).
-template <int N, int C, int OUT>
-cudaError_t launch_conv_tma(const bf16 *act, const bf16 *w, const float *bias, void *out, const ConvGeom &g, int sign,
-                            int relu, int *err, cudaStream_t s)
-{
-    const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-    if (!enc) return cudaErrorNotSupported;
-    CUtensorMap map;
-    const cuuint64_t dims[5] = {(cuuint64_t)C, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)g.D, (cuuint64_t)g.B};
-    const cuuint64_t strides[4] = {(cuuint64_t)C * 2, (cuuint64_t)g.W * C * 2, (cuuint64_t)g.H * g.W * C * 2,
-                                   (cuuint64_t)g.D * g.H * g.W * C * 2};
-    const cuuint32_t box[5] = {8, (cuuint32_t)kShHX, (cuuint32_t)kShHY, (cuuint32_t)kShHZ, 1};
-    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16 *>(act), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    constexpr int NS = march_ns<N, C>();
+    if ((reinterpret_cast<uintptr_t>(act) | reinterpret_cast<uintptr_t>(act2) | reinterpret_cast<uintptr_t>(w) |
+         reinterpret_cast<uintptr_t>(out)) & 15)
         return cudaErrorInvalidValue;
-    const size_t sm = conv_tma_smem<N, C>();
+    const size_t sm = march_smem<NS, C>();
     cudaError_t e =
-        cudaFuncSetAttribute(k_conv3d_tma<N, C, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_conv3d_tma<N, C, OUT>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(k_conv3d_march<N, C, OUT, CU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    int per = 0, dev = 0, nsm = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_conv3d_tma<N, C, OUT>, 128, sm)) != cudaSuccess)
-        return e;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    const long long bricks =
-        (long long)((g.W + kShX - 1) / kShX) * ((g.H + kShY - 1) / kShY) * g.D * g.B;
-    const long long grid = std::min<long long>(bricks, (long long)nsm * std::max(1, per));
-    k_conv3d_tma<N, C, OUT><<<(unsigned)grid, 128, sm, s>>>(map, w, bias, out, g, sign, relu, err);
+    const long long res = std::max<long long>(1, std::min<long long>((227 * 1024) / (sm + 1024), 512 / march_cols<NS, C>()));
+    const long long planes =
+        (long long)((g.W + kMarchX - 1) / kMarchX) * ((g.H + kMarchY - 1) / kMarchY) * g.B * g.D;
+    const long long grid = std::min(std::max<long long>(152 * res / (N / NS), 1), (planes + kMarchMin - 1) / kMarchMin);
+    k_conv3d_march<N, C, OUT, CU><<<dim3((unsigned)grid, N / NS), kMarchThreads, sm, s>>>(act, w, bias, out, g, sign,
+                                                                                          relu, err, act2);
     return cudaGetLastError();
 }
 
-// Forward and data-gradient convolutions run on 8 x 16 x 1 output bricks with the input
-// halo staged once in shared memory and one descriptor per tap: the persistent TMA kernel
-// where its buffers fit and N + C >= 48 (k_conv3d_tma), else k_conv3d_shift; k_conv3d_brick
-// (halo, per-tap copies) and k_conv3d_tc (gathered per tap) are earlier forms of the same
-// product.  Measured on the 128^3 grid (ncu, serialised): 16 <- 48 channels 632 against
-// 680 us, 32 <- 16 (64^3) 40 against 49 us, 64 <- 32 (32^3) 20 against 28 us, but 16 <- 16
-// 251 against 193 us: the halo's tiles have a 16-byte inner extent (one K group of one voxel),
-// which the copy engine moves as that many small rows, and the threads' 16-byte
-// asynchronous copies of k_conv3d_shift keep up with it when the tile is small.
 template <int N, int C, int OUT>
 cudaError_t launch_conv(const bf16 *act, const bf16 *w, const float *bias, void *out, const ConvGeom &g, int sign,
                         int relu, int *err, cudaStream_t s)
 {
-    if constexpr (conv_tma_fits<N, C>() && N + C >= 48) {
-        if (conv_tma_enabled()) {
-            const cudaError_t e = launch_conv_tma<N, C, OUT>(act, w, bias, out, g, sign, relu, err, s);
-            if (e != cudaErrorNotSupported) return e;
-        }
-    }
-    const size_t sm = conv_shift_smem<N, C>();
-    cudaError_t e =
-        cudaFuncSetAttribute(k_conv3d_shift<N, C, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    const long long bricks =
-        (long long)((g.W + kShX - 1) / kShX) * ((g.H + kShY - 1) / kShY) * g.D * g.B;
-    k_conv3d_shift<N, C, OUT><<<(unsigned)bricks, 128, sm, s>>>(act, w, bias, out, g, sign, relu, err);
-    return cudaGetLastError();
+    return launch_march<N, C, OUT, 0>(act, nullptr, w, bias, out, g, sign, relu, err, s);
 }
 
 // Decoder convolution (bias, ReLU, BF16 out) on the concatenation [up(low) (CU channels),
@@ -142,14 +82,7 @@ template <int N, int C, int CU>
 cudaError_t launch_conv_concat(const bf16 *low, const bf16 *skip, const bf16 *w, const float *bias, void *out,
                                const ConvGeom &g, int *err, cudaStream_t s)
 {
-    const size_t sm = conv_shift_smem<N, C>();
-    cudaError_t e =
-        cudaFuncSetAttribute(k_conv3d_shift<N, C, 0, CU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    const long long bricks =
-        (long long)((g.W + kShX - 1) / kShX) * ((g.H + kShY - 1) / kShY) * g.D * g.B;
-    k_conv3d_shift<N, C, 0, CU><<<(unsigned)bricks, 128, sm, s>>>(low, w, bias, out, g, 1, 1, err, skip);
-    return cudaGetLastError();
+    return launch_march<N, C, 0, CU>(low, skip, w, bias, out, g, 1, 1, err, s);
 }
 
 template <int N, int C>
@@ -722,8 +655,6 @@ int UNet::forward(float *pred, bool fused)
     k_pool<<<gsize(g3_.nvox * 32), 256, 0, s_>>>(e2_, p2_, g3_, 32);
     C_(conv_any(64, 32, 0, p2_, wt_[2], params_ + boff_[2], b3_, g3_, 1, 1, err_dev_, s_))
     if (fused) {  // inference: the decoder convolutions read [up(low), skip] directly
-        // (materialising [up(d2), e1] for the TMA kernel costs more than that kernel saves:
-        // 82 + 632 against 680 us on the 128^3 grid)
         C_((launch_conv_concat<32, 96, 64>(b3_, e2_, wt_[3], params_ + boff_[3], d2_, g2_, err_dev_, s_)))
         C_((launch_conv_concat<16, 48, 32>(d2_, e1_, wt_[4], params_ + boff_[4], d1_, g1_, err_dev_, s_)))
     } else {  // training: the concatenations are kept for the backward pass

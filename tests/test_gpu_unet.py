@@ -124,3 +124,28 @@ def test_fused_decoder_inference_equals_materialised_concat():
         assert float(pred.abs().max()) > 0
     finally:
         net.close()
+
+
+# columns of 8 x 16 voxels, runs of planes: single planes and lines, ragged columns, parts of several
+# columns and samples in one run
+@pytest.mark.parametrize("ci,co", [(16, 16), (16, 32), (32, 64), (96, 32), (48, 16)])
+@pytest.mark.parametrize("dims", [(1, 1, 1, 1), (7, 5, 1, 2), (9, 17, 6, 1), (8, 16, 23, 1), (20, 33, 11, 3)])
+def test_conv_columns_and_runs(ci, co, dims):
+    X, Y, Z, B = dims
+    rng = np.random.default_rng(1000 * ci + 10 * co + X)
+    x = U.bf16(rng.standard_normal((B, Z, Y, X, ci)))
+    w = U.bf16(0.1 * rng.standard_normal((co, 27, ci)))
+    b = rng.standard_normal(co).astype(np.float32)
+    g = U.bf16(rng.standard_normal((B, Z, Y, X, co)))
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    xd, wd, bd = dev_bf16(x), dev_bf16(w), torch.from_numpy(b).cuda()
+    yd = torch.zeros((B, Z, Y, X, co), dtype=torch.int16, device="cuda")
+    M.conv3d_tc(xd.data_ptr(), ci, wd.data_ptr(), co, bd.data_ptr(), 0, 0, yd.data_ptr(), dims, err.data_ptr())
+    # rounding to 8 bits: at most 2^-8 of each value
+    assert rel(host_bf16(yd), U.conv_fwd(x, w, b, relu=False)) <= 4e-3
+    gd, wtd = dev_bf16(g), dev_bf16(np.ascontiguousarray(w.transpose(2, 1, 0)))
+    dxd = torch.zeros((B, Z, Y, X, ci), dtype=torch.float32, device="cuda")
+    M.conv3d_tc(gd.data_ptr(), co, wtd.data_ptr(), ci, 0, 0, 1, dxd.data_ptr(), dims, err.data_ptr())
+    # at most 27 * 64 FP32 additions of products that are exact: about sqrt(1728) 2^-24 of the sum's norm
+    assert rel(dxd.cpu().numpy(), U.conv_dgrad(g, w)) <= 1e-5
+    assert int(err.item()) == 0
