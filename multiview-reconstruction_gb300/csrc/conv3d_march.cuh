@@ -81,9 +81,61 @@ struct MarchAt {
     }
 };
 
+// The copies of input planes, by 128 threads.  CU > 0: the input is the concatenation [nearest x2
+// upsampling of `act` (CU channels, a volume of half the size), act2 (C - CU channels)].
+template <int C, int CU>
+struct MarchPlanes {
+    static constexpr int CH = C / 8, ITEMS = kMarchPlane * CH, LI = (ITEMS + 127) / 128;
+    static_assert(CU % 8 == 0 && (CU == 0 || CU < C), "concatenated channel split");
+    const ConvGeom &g;
+    const uint4 *act, *act2;
+    int tid;
+    // this thread's 16-byte chunks of a plane, channel chunk fastest: offset in chunks from the halo's
+    // corner (x0 - 1, y0 - 1), of the low volume (x0 / 2 - 1, y0 / 2 - 1); -1 outside
+    int off[LI];
+    __device__ __forceinline__ MarchPlanes(const ConvGeom &g_, const __nv_bfloat16 *a, const __nv_bfloat16 *a2, int t)
+        : g(g_), act(reinterpret_cast<const uint4 *>(a)), act2(reinterpret_cast<const uint4 *>(a2)), tid(t)
+    {
+    }
+    __device__ __forceinline__ void column(const MarchAt &at)
+    {
+#pragma unroll
+        for (int i = 0; i < LI; ++i) {
+            const int k = tid + 128 * i, h = k / CH, j = k - h * CH;
+            const int xx = at.x0 - 1 + h % kMarchHX, yy = at.y0 - 1 + h / kMarchHX;
+            const bool in = k < ITEMS && xx >= 0 && yy >= 0 && xx < g.W && yy < g.H;
+            if constexpr (CU == 0) off[i] = in ? ((h / kMarchHX) * g.W + h % kMarchHX) * CH + j : -1;
+            else if (j < CU / 8)
+                off[i] = in ? ((h / kMarchHX + 1) / 2 * (g.W >> 1) + (h % kMarchHX + 1) / 2) * (CU / 8) + j : -1;
+            else off[i] = in ? ((h / kMarchHX) * g.W + h % kMarchHX) * (CH - CU / 8) + j - CU / 8 : -1;
+        }
+    }
+    __device__ __forceinline__ void copy(const MarchAt &at, uint8_t *dst) const
+    {
+        auto corner = [&](int z, int D, int H, int W, int y, int x) {
+            return (((long long)at.b * D + z) * H + y) * W + x;
+        };
+        const int z = at.zs - 1 + at.p;
+        const bool zin = z >= 0 && z < g.D;
+        const int zz = zin ? z : 0;
+        const uint4 *lo, *hi = nullptr;
+        if constexpr (CU == 0) {
+            lo = act + corner(zz, g.D, g.H, g.W, at.y0 - 1, at.x0 - 1) * CH;
+        } else {
+            lo = act + corner(zz >> 1, g.D >> 1, g.H >> 1, g.W >> 1, at.y0 / 2 - 1, at.x0 / 2 - 1) * (CU / 8);
+            hi = act2 + corner(zz, g.D, g.H, g.W, at.y0 - 1, at.x0 - 1) * (CH - CU / 8);
+        }
+#pragma unroll
+        for (int i = 0; i < LI; ++i) {
+            const int k = tid + 128 * i, h = k / CH, j = k - h * CH;
+            const bool in = zin && off[i] >= 0;
+            const uint4 *src = CU == 0 || j < CU / 8 ? lo : hi;
+            if ((i + 1) * 128 <= ITEMS || k < ITEMS) cp_async16(dst + j * kMarchLbo + 16 * h, in ? src + off[i] : act, in);
+        }
+    }
+};
+
 // OUT_MODE 0: BF16 output with bias (+ReLU when relu != 0); 1: FP32 output, no bias.
-// CU > 0: the input is the concatenation [nearest x2 upsampling of `act` (CU channels, a volume of
-// half the size), act2 (C - CU channels)].
 template <int N, int C, int OUT_MODE, int CU = 0>
 __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloat16 *__restrict__ act,
                                                       const __nv_bfloat16 *__restrict__ wk,
@@ -95,9 +147,7 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
     constexpr uint32_t COLS = march_cols<NS, C>();
     constexpr int R = (int)COLS / NS;  // ring of output planes: three being added to, one being read
     constexpr int PB = CH * kMarchLbo, B_TAP = 3 * NS * C * 2;
-    constexpr int ITEMS = kMarchPlane * CH, LI = (ITEMS + 127) / 128;
     static_assert(N % NS == 0 && NS % 16 == 0 && 3 * NS <= 256 && C % 16 == 0 && R >= 4, "tile shape");
-    static_assert(CU % 8 == 0 && (CU == 0 || CU < C), "concatenated channel split");
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *sB = smem + ((ST * PB + 1023) / 1024) * 1024;
     __shared__ __align__(8) uint64_t done[ST];
@@ -117,45 +167,11 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
     ld.u = at.u = planes * blockIdx.x / gridDim.x;
     ld.start(g, u1);
     at.start(g, u1);
-    int off[LI];
-    // this thread's 16-byte chunks of a plane, channel chunk fastest: offset in chunks from the
-    // halo's corner (x0 - 1, y0 - 1), of the low volume (x0 / 2 - 1, y0 / 2 - 1); -1 outside
-    auto chunks = [&]() {
-#pragma unroll
-        for (int i = 0; i < LI; ++i) {
-            const int k = tid + 128 * i, h = k / CH, j = k - h * CH;
-            const int xx = ld.x0 - 1 + h % kMarchHX, yy = ld.y0 - 1 + h / kMarchHX;
-            const bool in = k < ITEMS && xx >= 0 && yy >= 0 && xx < g.W && yy < g.H;
-            if constexpr (CU == 0) off[i] = in ? ((h / kMarchHX) * g.W + h % kMarchHX) * CH + j : -1;
-            else if (j < CU / 8)
-                off[i] = in ? ((h / kMarchHX + 1) / 2 * (g.W >> 1) + (h % kMarchHX + 1) / 2) * (CU / 8) + j : -1;
-            else off[i] = in ? ((h / kMarchHX) * g.W + h % kMarchHX) * (CH - CU / 8) + j - CU / 8 : -1;
-        }
-    };
-    chunks();
-    auto corner = [&](int z, int D, int H, int W, int y, int x) { return (((long long)ld.b * D + z) * H + y) * W + x; };
+    MarchPlanes<C, CU> in(g, act, act2, tid);
+    in.column(ld);
     auto load = [&](int s) {  // the next input plane, of step s, into its buffer
-        uint8_t *dst = smem + (s % ST) * PB;
-        const int z = ld.zs - 1 + ld.p;
-        const bool zin = z >= 0 && z < g.D;
-        const int zz = zin ? z : 0;
-        const uint4 *lo, *hi = nullptr;
-        if constexpr (CU == 0) {
-            lo = reinterpret_cast<const uint4 *>(act) + corner(zz, g.D, g.H, g.W, ld.y0 - 1, ld.x0 - 1) * CH;
-        } else {
-            lo = reinterpret_cast<const uint4 *>(act) +
-                 corner(zz >> 1, g.D >> 1, g.H >> 1, g.W >> 1, ld.y0 / 2 - 1, ld.x0 / 2 - 1) * (CU / 8);
-            hi = reinterpret_cast<const uint4 *>(act2) + corner(zz, g.D, g.H, g.W, ld.y0 - 1, ld.x0 - 1) * (CH - CU / 8);
-        }
-#pragma unroll
-        for (int i = 0; i < LI; ++i) {
-            const int k = tid + 128 * i, h = k / CH, j = k - h * CH;
-            const bool in = zin && off[i] >= 0;
-            const uint4 *src = CU == 0 || j < CU / 8 ? lo : hi;
-            if ((i + 1) * 128 <= ITEMS || k < ITEMS)
-                cp_async16(dst + j * kMarchLbo + 16 * h, in ? src + off[i] : reinterpret_cast<const uint4 *>(act), in);
-        }
-        if (ld.next(g, u1)) chunks();
+        in.copy(ld, smem + (s % ST) * PB);
+        if (ld.next(g, u1)) in.column(ld);
     };
     // the weights, per offset (dy, dx) 3 NS rows: output plane z - 1 (dz = 1), z, z + 1, each NS channels
     // (every CTA reads the same ones at the same time: each starts at a place of its own)
@@ -280,6 +296,184 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, COLS);
+}
+
+// Weight gradient over the same runs: dW[co][t][ci] += sum_n G[n][co] X[n + off(t)][ci].
+//
+// The contraction runs over voxels: both operands are M/N-major, the 8 channels (16 bytes) of one voxel
+// one core matrix row and 8 x-consecutive voxels one core matrix, so a plane of X in shared memory is
+// the A operand of every offset (dy, dx) by its start address alone, and three consecutive planes
+// of G in their ring are B for the three dz: product columns (i, co) of the offset's accumulators, G
+// plane z - 1 + i against X plane z.  The accumulators of all offsets stay in tensor memory
+// through the run (3 N columns each; with more output channels a CTA takes part of the offsets) and
+// go into dW with FP32 atomics at its end.  Rows beyond C are read from whatever follows the
+// plane and dropped.
+//
+// What bounds it: the operands' way out of shared memory, 2 KB of A (64 rows; 4 KB for more than 64
+// channels) and 1.5 KB of B per product.  48 x 16 channels on
+// 4 x 64^3 voxels: 97 us (0.85 ms with 27 copies of X out of L2, one per offset), 16 x 16: 94 us (0.30),
+// 96 x 32 on 4 x 32^3: 42 us (0.25).  A column's ragged edge multiplies G's zeros with the X beside
+// it, so there a non-finite X reaches the gradient of the outward offsets as well.
+constexpr int kWgRing = 8;  // planes of G: three being multiplied, the others on their way
+constexpr int kWgGroup = 128 * 16 + 16;  // stride of G's channel groups (padding: distinct banks)
+template <int N>
+__host__ __device__ constexpr int wgrad_offsets()  // offsets (dy, dx) of one CTA
+{
+    return 512 / (3 * N) < 9 ? 512 / (3 * N) : 9;
+}
+template <int N>
+__host__ __device__ constexpr int wgrad_splits()
+{
+    return (9 + wgrad_offsets<N>() - 1) / wgrad_offsets<N>();
+}
+template <int N, int C>
+__host__ __device__ constexpr size_t wgrad_march_smem()
+{
+    return (size_t)kMarchStages * (C / 8) * kMarchLbo + (size_t)kWgRing * (N / 8) * kWgGroup;
+}
+
+template <int N, int C, int CU = 0>
+__global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat16 *__restrict__ X,
+                                                               const __nv_bfloat16 *__restrict__ G, float *dW,
+                                                               ConvGeom g, int *err,
+                                                               const __nv_bfloat16 *__restrict__ X2 = nullptr)
+{
+    constexpr int ST = kMarchStages, RG = kWgRing, CH = C / 8, PB = CH * kMarchLbo, GB = (N / 8) * kWgGroup;
+    constexpr int M = C <= 64 ? 64 : 128;
+    static_assert(C <= 128 && N % 16 == 0 && 3 * N <= 256, "tile shape");
+    // A's rows beyond C end inside the ring of G
+    static_assert((M / 8 - CH) * kMarchLbo <= RG * GB, "rows beyond C stay in shared memory");
+    static_assert(ST + 2 <= RG, "a plane of G is copied when its slot's last products are done");
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t *sG = smem + ST * PB;
+    __shared__ __align__(8) uint64_t done[ST];
+    __shared__ uint32_t tbase;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    if (warp == 0) tc::tmem_alloc(&tbase, 512);
+    if (tid == 0) {
+        for (int i = 0; i < ST; ++i) tc::mbar_init(&done[i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    const long long planes =
+        (long long)((g.W + kMarchX - 1) / kMarchX) * ((g.H + kMarchY - 1) / kMarchY) * g.B * g.D;
+    const long long u1 = planes * (blockIdx.x + 1) / gridDim.x;
+    const int t0 = 9 * blockIdx.y / gridDim.y, t1 = 9 * (blockIdx.y + 1) / gridDim.y;
+    MarchAt ld, at;
+    ld.u = at.u = planes * blockIdx.x / gridDim.x;
+    ld.start(g, u1);
+    at.start(g, u1);
+    MarchPlanes<C, CU> in(g, X, X2, tid);
+    in.column(ld);
+    int lring = 0;  // output planes of the parts before: plane j of a part is in slot (ring + j) % RG
+    auto load = [&](int s) {  // the next plane of X, of step s, and of G
+        in.copy(ld, smem + (s % ST) * PB);
+        if (ld.p < ld.nz) {
+            uint8_t *dst = sG + (lring + ld.p) % RG * GB;
+            const long long z = (long long)ld.b * g.D + ld.zs + ld.p;
+#pragma unroll
+            for (int i = 0; i < N / 8; ++i) {
+                const int k = tid + 128 * i, v = k / (N / 8), j = k - v * (N / 8);
+                const int x = ld.x0 + (v & 7), y = ld.y0 + (v >> 3);
+                const bool ok = x < g.W && y < g.H;
+                cp_async16(dst + j * kWgGroup + 16 * v, ok ? G + ((z * g.H + y) * g.W + x) * N + 8 * j : G, ok);
+            }
+        }
+        const int nz = ld.nz;
+        if (ld.next(g, u1)) {
+            lring = (lring + nz) % RG;
+            in.column(ld);
+        }
+    };
+#pragma unroll 1
+    for (int s = 0; s < ST; ++s) {
+        if (ld.u < u1 && warp < 4) load(s);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tbase, 0);
+    const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+    if (warp < 4)
+        for (int c = 0; c < (t1 - t0) * 3 * N; c += 16) tc::tmem_zero16(trow + c);
+    const uint32_t xbase = tc::smem_u32(smem), gbase = tc::smem_u32(sG);
+    int ring = 0;
+    auto products = [&](int s) {  // issued by one lane
+        const int i0 = max(0, 2 - at.p), i1 = min(3, at.nz + 2 - at.p);
+        const int s0 = (ring + at.p - 2 + i0) % RG;
+        const int n0 = min(i1 - i0, RG - s0), n1 = i1 - i0 - n0;  // planes up to the ring's end, and from its start
+        const uint64_t a0 = tc::smem_desc(xbase + (uint32_t)(s % ST) * PB, kMarchHX * 16, kMarchLbo);
+        const uint64_t b0 = tc::smem_desc(gbase, 128, kWgGroup);
+#pragma unroll 1
+        for (int seg = 0; seg < (n1 > 0 ? 2 : 1); ++seg) {
+            const int n = seg ? n1 : n0, i = seg ? i0 + n0 : i0;
+            const uint32_t id = tc::idesc_bf16_mn(M, N) + ((uint32_t)((n - 1) * (N >> 3)) << 17);
+            const uint64_t bs = b0 + (seg ? 0u : (uint32_t)(s0 * (GB / 16)));
+            uint32_t d = tmem + (uint32_t)(i * N);
+#pragma unroll 1
+            for (int t = t0; t < t1; ++t, d += 3 * N) {
+                const uint64_t as = a0 + (uint32_t)(t % 3 + kMarchHX * (t / 3));
+#pragma unroll
+                for (int k = 0; k < 8; ++k) tc::mma_bf16_acc(d, as + 2 * kMarchHX * k, bs + 16 * k, id);
+            }
+        }
+        tc::mma_commit(&done[s % ST]);
+    };
+    bool ok = true;
+    int s = 0;
+#pragma unroll 1
+    for (;; ++s) {
+        const bool more = at.u < u1;
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(ST - 2) : "memory");  // step s's planes have landed
+        tc::fence_proxy_async();
+        tc::fence_before_sync();
+        ok = __syncthreads_and(ok) != 0;
+        if (!ok) break;  // the whole CTA
+        if (more && warp == 4) {
+            tc::fence_after_sync();
+            if (tc::elect_one()) products(s);
+            __syncwarp();
+        }
+        if (s > 0 && warp < 4) {
+            ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[(s - 1) % ST], ((s - 1) / ST) & 1, kTcWaitIter));
+            if (ok && ld.u < u1) load(s - 1 + ST);  // on a timeout this warp writes no more
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        if (!more) break;
+        const int nz = at.nz;
+        if (at.next(g, u1)) ring = (ring + nz) % RG;
+    }
+    tc::fence_after_sync();
+    if (!__syncthreads_and(ok)) {
+        // a wait ran out: let every copy and product in flight finish (bounded) before the tensor
+        // memory goes back
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        if (tid == 0) {
+            atomicExch(err, 1);
+            for (int q = max(0, s - ST); q < s; ++q) tc::mbar_wait(&done[q % ST], (q / ST) & 1, kTcWaitIter);
+        }
+    } else if (warp < 4) {
+        // row ci is lane ci, of 64 rows lanes 0..15 of each warp; every CTA starts at an offset of its own
+        const int ci = M == 64 ? 16 * warp + lane : 32 * warp + lane;
+        const bool rv = ci < C && (M == 128 || lane < 16);
+        const int nt = t1 - t0;
+#pragma unroll 1
+        for (int q = 0; q < nt * 3; ++q) {
+            const int e = (q + (int)blockIdx.x) % (nt * 3), t = t0 + e / 3, tz = 2 - e % 3;
+#pragma unroll
+            for (int c0 = 0; c0 < N; c0 += 16) {
+                float v[16];
+                tc::tmem_ld16(trow + (uint32_t)(e * N + c0), v);
+                if (rv)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        atomicAdd(&dW[((long long)(c0 + j) * 27 + 9 * tz + t) * C + ci], v[j]);
+            }
+        }
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, 512);
 }
 
 }  // namespace mvr

@@ -131,6 +131,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *out)
     for (int i = 0; i < 16; ++i) out[i] = __uint_as_float(r[i]);
 }
 
+// Zero 16 consecutive FP32 columns of the calling warp's 32 lanes.
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(
+                     taddr),
+                 "r"(0u)
+                 : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 // Byte offset of element (row, k) in the canonical layout of a tile with KT elements
 // along K (16-bit elements).
 __host__ __device__ __forceinline__ uint32_t core_offset(int row, int k, int KT)

@@ -40,9 +40,6 @@ int rsize(long long n) { return (int)std::max<long long>(1, std::min<long long>(
 int gsize(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 152 * 32)); }
 
 // ---- tcgen05 convolution launchers --------------------------------------------------
-template <int N>
-size_t wgrad_smem() { return (size_t)kWgStages * wgrad_stage_bytes<N>(); }
-
 // Forward and data-gradient convolutions (k_conv3d_march): one wave of CTAs, each a run of at least
 // kMarchMin output planes.  A run reads two input planes beyond its own and its weights, so runs of
 // 12 planes were better only on large levels, which have them anyway (32 -> 64 channels on 32^3: runs
@@ -85,20 +82,22 @@ cudaError_t launch_conv_concat(const bf16 *low, const bf16 *skip, const bf16 *w,
     return launch_march<N, C, 0, CU>(low, skip, w, bias, out, g, 1, 1, err, s);
 }
 
-template <int N, int C>
-cudaError_t launch_wgrad(const bf16 *X, const bf16 *G, float *dW, const ConvGeom &g, int *err, cudaStream_t s)
+// Weight gradient (k_wgrad_march): runs as in launch_march, one CTA per SM (it holds all tensor memory)
+template <int N, int C, int CU = 0>
+cudaError_t launch_wgrad(const bf16 *X, const bf16 *G, float *dW, const ConvGeom &g, int *err, cudaStream_t s,
+                         const bf16 *X2 = nullptr)
 {
-    const size_t sm = wgrad_smem<N>();
-    cudaError_t e = cudaFuncSetAttribute(k_wgrad_tc<N, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(X2) | reinterpret_cast<uintptr_t>(G)) & 15)
+        return cudaErrorInvalidValue;
+    const size_t sm = wgrad_march_smem<N, C>();
+    cudaError_t e =
+        cudaFuncSetAttribute(k_wgrad_march<N, C, CU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    const int mt = (27 * C + 127) / 128;
-    // split the voxels so that one wave of CTAs runs (as many per SM as their stages fit shared memory)
-    const int res = (int)std::max<size_t>(1, (227 * 1024) / (sm + 1024));
-    long long splits = std::max<long long>(1, (152LL * res) / mt);
-    long long vpc = (g.nvox + splits - 1) / splits;
-    vpc = ((vpc + 63) / 64) * 64;
-    splits = (g.nvox + vpc - 1) / vpc;
-    k_wgrad_tc<N, C><<<dim3((unsigned)mt, (unsigned)splits), 128, sm, s>>>(X, G, dW, g, vpc, err);
+    const long long planes =
+        (long long)((g.W + kMarchX - 1) / kMarchX) * ((g.H + kMarchY - 1) / kMarchY) * g.B * g.D;
+    constexpr int NG = wgrad_splits<N>();
+    const long long grid = std::min<long long>(152 / NG, (planes + kMarchMin - 1) / kMarchMin);
+    k_wgrad_march<N, C, CU><<<dim3((unsigned)grid, NG), kMarchThreads, sm, s>>>(X, G, dW, g, err, X2);
     return cudaGetLastError();
 }
 
@@ -205,28 +204,6 @@ __global__ void k_pool(const bf16 *in, bf16 *out, ConvGeom lo, int C)
             s += __bfloat162float(in[src * C + c]);
         }
         out[i] = __float2bfloat16(0.125f * s);
-    }
-}
-
-// out[n] = [up(low)[n] (Cu channels), skip[n] (Cs channels)], nearest upsampling x2, in
-// chunks of 8 channels (16 bytes); Cu and Cs are multiples of 8
-__global__ void k_up_concat(const bf16 *low, const bf16 *skip, bf16 *out, ConvGeom hi, int Cu, int Cs)
-{
-    const int Ct = Cu + Cs, K = Ct / 8, Ku = Cu / 8;
-    const long long n = hi.nvox * K;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int c8 = (int)(i % K);
-        const long long v = i / K;
-        uint4 val;
-        if (c8 < Ku) {
-            int x, y, z, b;
-            vox_coords(hi, v, x, y, z, b);
-            const long long lv = (((long long)b * (hi.D / 2) + z / 2) * (hi.H / 2) + y / 2) * (hi.W / 2) + x / 2;
-            val = reinterpret_cast<const uint4 *>(low + lv * Cu)[c8];
-        } else {
-            val = reinterpret_cast<const uint4 *>(skip + v * Cs)[c8 - Ku];
-        }
-        reinterpret_cast<uint4 *>(out + v * Ct)[c8] = val;
     }
 }
 
@@ -488,7 +465,7 @@ public:
     ~UNet();
     int init();
     int set_input(const float *psi, const float *psi_next, const float *psi_target);
-    int forward(float *pred, bool fused = false);
+    int forward(float *pred);
     int train_step(float lr, double *loss);
     int propose(const float *psi, float *out, float cap);
     long long num_params() const { return nparams_; }
@@ -531,7 +508,7 @@ private:
     float *params_ = nullptr, *grads_ = nullptr, *am_ = nullptr, *av_ = nullptr;
     bf16 *wt_[5] = {}, *wtt_[5] = {};
     bf16 *in16_ = nullptr, *e1_ = nullptr, *p1_ = nullptr, *e2_ = nullptr, *p2_ = nullptr, *b3_ = nullptr;
-    bf16 *c2_ = nullptr, *d2_ = nullptr, *c1_ = nullptr, *d1_ = nullptr;
+    bf16 *d2_ = nullptr, *d1_ = nullptr;
     bf16 *G_ = nullptr;  // BF16 gradient scratch (largest: level 1 x 16 or level 2 x 32)
     float *out_ = nullptr, *target_ = nullptr;
     float *gc1_ = nullptr, *gc2_ = nullptr, *gd2_ = nullptr, *gb3_ = nullptr, *gp2_ = nullptr, *gp1_ = nullptr;
@@ -584,7 +561,7 @@ int UNet::init()
     }
     const long long n1 = g1_.nvox, n2 = g2_.nvox, n3 = g3_.nvox;
     A_(in16_, n1 * 16) A_(e1_, n1 * 16) A_(p1_, n2 * 16) A_(e2_, n2 * 32) A_(p2_, n3 * 32) A_(b3_, n3 * 64)
-    A_(c2_, n2 * 96) A_(d2_, n2 * 32) A_(c1_, n1 * 48) A_(d1_, n1 * 16)
+    A_(d2_, n2 * 32) A_(d1_, n1 * 16)
     A_(G_, std::max(n1 * 16, n2 * 32)) A_(out_, n1) A_(target_, n1)
     A_(gc1_, n1 * 48) A_(gc2_, n2 * 96) A_(gd2_, n2 * 32) A_(gb3_, n3 * 64) A_(gp2_, n3 * 32) A_(gp1_, n2 * 16)
     A_(mean_, B_) A_(meanp_, (long long)B_ * kMeanParts) A_(loss_, 1) A_(err_dev_, 1)
@@ -641,7 +618,7 @@ int UNet::set_input(const float *psi, const float *psi_next, const float *psi_ta
     return cuda(cudaGetLastError(), "k_features");
 }
 
-int UNet::forward(float *pred, bool fused)
+int UNet::forward(float *pred)
 {
     cudaSetDevice(dev_);
     int rc = refresh_weights();
@@ -654,15 +631,9 @@ int UNet::forward(float *pred, bool fused)
     C_(conv_any(32, 16, 0, p1_, wt_[1], params_ + boff_[1], e2_, g2_, 1, 1, err_dev_, s_))
     k_pool<<<gsize(g3_.nvox * 32), 256, 0, s_>>>(e2_, p2_, g3_, 32);
     C_(conv_any(64, 32, 0, p2_, wt_[2], params_ + boff_[2], b3_, g3_, 1, 1, err_dev_, s_))
-    if (fused) {  // inference: the decoder convolutions read [up(low), skip] directly
-        C_((launch_conv_concat<32, 96, 64>(b3_, e2_, wt_[3], params_ + boff_[3], d2_, g2_, err_dev_, s_)))
-        C_((launch_conv_concat<16, 48, 32>(d2_, e1_, wt_[4], params_ + boff_[4], d1_, g1_, err_dev_, s_)))
-    } else {  // training: the concatenations are kept for the backward pass
-        k_up_concat<<<gsize(n2 * 12), 256, 0, s_>>>(b3_, e2_, c2_, g2_, 64, 32);
-        C_(conv_any(32, 96, 0, c2_, wt_[3], params_ + boff_[3], d2_, g2_, 1, 1, err_dev_, s_))
-        k_up_concat<<<gsize(n1 * 6), 256, 0, s_>>>(d2_, e1_, c1_, g1_, 32, 16);
-        C_(conv_any(16, 48, 0, c1_, wt_[4], params_ + boff_[4], d1_, g1_, 1, 1, err_dev_, s_))
-    }
+    // the decoder convolutions read [up(low), skip] where they are, here and in the weight gradients
+    C_((launch_conv_concat<32, 96, 64>(b3_, e2_, wt_[3], params_ + boff_[3], d2_, g2_, err_dev_, s_)))
+    C_((launch_conv_concat<16, 48, 32>(d2_, e1_, wt_[4], params_ + boff_[4], d1_, g1_, err_dev_, s_)))
     k_head<<<gsize(n1), 256, 0, s_>>>(d1_, params_ + whoff_, params_ + bhoff_, out_, n1);
     C_(cudaGetLastError())
     if (pred) C_(cudaMemcpyAsync(pred, out_, sizeof(float) * (size_t)n1, cudaMemcpyDeviceToDevice, s_))
@@ -689,13 +660,13 @@ int UNet::train_step(float lr, double *loss)
                                           grads_ + bhoff_, G_, db[4]);
     C_(cudaGetLastError())
     // layer 5: 48 -> 16 on c1 = [up(d2), e1]
-    C_(wgrad_any(16, 48, c1_, G_, dW[4], g1_, err_dev_, s_))
+    C_((launch_wgrad<16, 48, 32>(d2_, G_, dW[4], g1_, err_dev_, s_, e1_)))
     C_(conv_any(48, 16, 1, G_, wtt_[4], nullptr, gc1_, g1_, -1, 0, err_dev_, s_))
     k_up_back<<<gsize(n2 * 32), 256, 0, s_>>>(gc1_, 48, g2_, 32, gd2_);
     k_mask_grad<32><<<rsize(n2 * (32 / 8)), 256, 0, s_>>>(gd2_, 32, 0, nullptr, g2_, d2_, G_, db[3]);
     C_(cudaGetLastError())
     // layer 4: 96 -> 32 on c2 = [up(b3), e2]
-    C_(wgrad_any(32, 96, c2_, G_, dW[3], g2_, err_dev_, s_))
+    C_((launch_wgrad<32, 96, 64>(b3_, G_, dW[3], g2_, err_dev_, s_, e2_)))
     C_(conv_any(96, 32, 1, G_, wtt_[3], nullptr, gc2_, g2_, -1, 0, err_dev_, s_))
     k_up_back<<<gsize(n3 * 64), 256, 0, s_>>>(gc2_, 96, g3_, 64, gb3_);
     k_mask_grad<64><<<rsize(n3 * (64 / 8)), 256, 0, s_>>>(gb3_, 64, 0, nullptr, g3_, b3_, G_, db[2]);
@@ -731,7 +702,7 @@ int UNet::train_step(float lr, double *loss)
 
 int UNet::propose(const float *psi, float *out, float cap)
 {
-    int rc = forward(nullptr, true);
+    int rc = forward(nullptr);
     if (rc != MVR_OK) return rc;
     k_propose<<<gsize(g1_.nvox), 256, 0, s_>>>(psi, out_, out, g1_.nvox, cap);
     if ((rc = cuda(cudaGetLastError(), "k_propose")) != MVR_OK) return rc;
@@ -825,7 +796,7 @@ extern "C" int mvr_unet_set_input(mvr_unet *h, const float *psi, const float *ps
 }
 // inference: the decoder convolutions read [up(low), skip] directly (the training step keeps the
 // concatenations for its backward pass)
-extern "C" int mvr_unet_forward(mvr_unet *h, float *pred) { return h ? h->net->forward(pred, true) : MVR_ERR_ARG; }
+extern "C" int mvr_unet_forward(mvr_unet *h, float *pred) { return h ? h->net->forward(pred) : MVR_ERR_ARG; }
 extern "C" int mvr_unet_train_step(mvr_unet *h, float lr, double *loss)
 {
     return h ? h->net->train_step(lr, loss) : MVR_ERR_ARG;

@@ -149,3 +149,19 @@ def test_conv_columns_and_runs(ci, co, dims):
     # at most 27 * 64 FP32 additions of products that are exact: about sqrt(1728) 2^-24 of the sum's norm
     assert rel(dxd.cpu().numpy(), U.conv_dgrad(g, w)) <= 1e-5
     assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("ci,co", [(16, 16), (48, 16), (16, 32), (96, 32), (32, 64)])
+@pytest.mark.parametrize("dims", [(1, 1, 1, 1), (7, 5, 1, 2), (9, 17, 6, 1), (8, 16, 23, 1), (20, 33, 11, 3)])
+def test_weight_gradient_columns_and_runs(ci, co, dims):
+    X, Y, Z, B = dims
+    rng = np.random.default_rng(1000 * ci + 10 * co + X)
+    x = U.bf16(rng.standard_normal((B, Z, Y, X, ci)))
+    g = U.bf16(rng.standard_normal((B, Z, Y, X, co)))
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    xd, gd = dev_bf16(x), dev_bf16(g)
+    dwd = torch.ones((co, 27, ci), dtype=torch.float32, device="cuda")
+    M.conv3d_tc_wgrad(xd.data_ptr(), ci, gd.data_ptr(), co, dwd.data_ptr(), dims, err.data_ptr())
+    # added to what is there; up to 21780 FP32 additions of exact products: sqrt(21780) 2^-24
+    assert rel(dwd.cpu().numpy(), 1.0 + U.conv_wgrad(x, g)) <= 1e-5
+    assert int(err.item()) == 0
