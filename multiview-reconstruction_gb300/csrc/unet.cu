@@ -161,13 +161,19 @@ __global__ void k_patch_partials(const float *psi, long long per, double *parts)
     if (threadIdx.x == 0) parts[(long long)blockIdx.y * kMeanParts + blockIdx.x] = (double)sh[0] + (double)sl[0];
 }
 
-__global__ void k_patch_mean(const double *parts, long long per, int B, double *mean)
+__global__ void __launch_bounds__(kMeanParts) k_patch_mean(const double *parts, long long per, double *mean)
 {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    double s = 0.0;
-    for (int k = 0; k < kMeanParts; ++k) s += parts[(long long)b * kMeanParts + k];
-    mean[b] = s / (double)per;
+    __shared__ double sw[kMeanParts / 32];
+    double s = parts[(long long)blockIdx.x * kMeanParts + threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s = 0.0;
+        for (int w = 0; w < kMeanParts / 32; ++w) s += sw[w];
+        mean[blockIdx.x] = s / (double)per;
+    }
 }
 
 // features: [log(psi / mean), log(psi_next / psi), 0 x 14] as BF16; target log(psi_m / psi)
@@ -189,21 +195,32 @@ __global__ void k_features(const float *psi, const float *psi_next, const float 
     }
 }
 
-// 2x2x2 average pooling, channels-last BF16
+// 2x2x2 average pooling, channels-last BF16; a thread takes 8 channels (16 bytes) of a voxel, as every
+// channels-last kernel here: one channel per thread read 2 bytes at a time (16 channels on 128^3: 34 us)
 __global__ void k_pool(const bf16 *in, bf16 *out, ConvGeom lo, int C)
 {
-    const long long n = lo.nvox * C;
+    const int K = C / 8;
+    const long long n = lo.nvox * K;
     const int W2 = lo.W * 2, H2 = lo.H * 2, D2 = lo.D * 2;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % C);
+        const int k = (int)(i % K);
         int x, y, z, b;
-        vox_coords(lo, i / C, x, y, z, b);
-        float s = 0.0f;
+        vox_coords(lo, i / K, x, y, z, b);
+        uint4 v[8];
+#pragma unroll
         for (int q = 0; q < 8; ++q) {
             const long long src = (((long long)b * D2 + 2 * z + (q >> 2)) * H2 + 2 * y + ((q >> 1) & 1)) * W2 + 2 * x + (q & 1);
-            s += __bfloat162float(in[src * C + c]);
+            v[q] = __ldg(reinterpret_cast<const uint4 *>(in + src * C) + k);
         }
-        out[i] = __float2bfloat16(0.125f * s);
+        __align__(16) bf16 o[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            float s = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) s += __bfloat162float(reinterpret_cast<const bf16 *>(&v[q])[c]);
+            o[c] = __float2bfloat16(0.125f * s);
+        }
+        reinterpret_cast<uint4 *>(out)[i] = *reinterpret_cast<const uint4 *>(o);
     }
 }
 
@@ -211,9 +228,12 @@ __global__ void k_pool(const bf16 *in, bf16 *out, ConvGeom lo, int C)
 __global__ void k_head(const bf16 *d1, const float *wh, const float *bh, float *out, long long n)
 {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        __align__(16) bf16 d[16];
+        reinterpret_cast<uint4 *>(d)[0] = __ldg(reinterpret_cast<const uint4 *>(d1 + i * 16));
+        reinterpret_cast<uint4 *>(d)[1] = __ldg(reinterpret_cast<const uint4 *>(d1 + i * 16) + 1);
         float s = bh[0];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) s += wh[c] * __bfloat162float(d1[i * 16 + c]);
+        for (int c = 0; c < 16; ++c) s += wh[c] * __bfloat162float(d[c]);
         out[i] = s;
     }
 }
@@ -347,18 +367,24 @@ __global__ void __launch_bounds__(256) k_mask_grad(const float *gsk, int gsk_str
 // of gcat[child][c], c < Cu
 __global__ void k_up_back(const float *gcat, int Ct, ConvGeom lo, int Cu, float *glow)
 {
-    const long long n = lo.nvox * Cu;
+    const int K = Cu / 4;
+    const long long n = lo.nvox * K;
     const int W2 = lo.W * 2, H2 = lo.H * 2, D2 = lo.D * 2;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % Cu);
+        const int k = (int)(i % K);
         int x, y, z, b;
-        vox_coords(lo, i / Cu, x, y, z, b);
-        float s = 0.0f;
+        vox_coords(lo, i / K, x, y, z, b);
+        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
         for (int q = 0; q < 8; ++q) {
             const long long src = (((long long)b * D2 + 2 * z + (q >> 2)) * H2 + 2 * y + ((q >> 1) & 1)) * W2 + 2 * x + (q & 1);
-            s += gcat[src * Ct + c];
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(gcat + src * Ct) + k);
+            s.x += v.x;
+            s.y += v.y;
+            s.z += v.z;
+            s.w += v.w;
         }
-        glow[i] = s;
+        reinterpret_cast<float4 *>(glow)[i] = s;
     }
 }
 
@@ -612,7 +638,7 @@ int UNet::set_input(const float *psi, const float *psi_next, const float *psi_ta
     cudaSetDevice(dev_);
     const long long per = g1_.nvox / B_;
     k_patch_partials<<<dim3(kMeanParts, B_), 256, 0, s_>>>(psi, per, meanp_);
-    k_patch_mean<<<(B_ + 127) / 128, 128, 0, s_>>>(meanp_, per, B_, mean_);
+    k_patch_mean<<<B_, kMeanParts, 0, s_>>>(meanp_, per, mean_);
     k_features<<<gsize(g1_.nvox), 256, 0, s_>>>(psi, psi_next, psi_target, g1_.nvox, per, mean_, in16_,
                                                 psi_target ? target_ : nullptr);
     return cuda(cudaGetLastError(), "k_features");
@@ -627,9 +653,9 @@ int UNet::forward(float *pred)
 #define C_(expr)                                         \
     if ((rc = cuda((expr), #expr)) != MVR_OK) return rc;
     C_(conv_any(16, 16, 0, in16_, wt_[0], params_ + boff_[0], e1_, g1_, 1, 1, err_dev_, s_))
-    k_pool<<<gsize(n2 * 16), 256, 0, s_>>>(e1_, p1_, g2_, 16);
+    k_pool<<<gsize(n2 * 2), 256, 0, s_>>>(e1_, p1_, g2_, 16);
     C_(conv_any(32, 16, 0, p1_, wt_[1], params_ + boff_[1], e2_, g2_, 1, 1, err_dev_, s_))
-    k_pool<<<gsize(g3_.nvox * 32), 256, 0, s_>>>(e2_, p2_, g3_, 32);
+    k_pool<<<gsize(g3_.nvox * 4), 256, 0, s_>>>(e2_, p2_, g3_, 32);
     C_(conv_any(64, 32, 0, p2_, wt_[2], params_ + boff_[2], b3_, g3_, 1, 1, err_dev_, s_))
     // the decoder convolutions read [up(low), skip] where they are, here and in the weight gradients
     C_((launch_conv_concat<32, 96, 64>(b3_, e2_, wt_[3], params_ + boff_[3], d2_, g2_, err_dev_, s_)))
@@ -662,13 +688,13 @@ int UNet::train_step(float lr, double *loss)
     // layer 5: 48 -> 16 on c1 = [up(d2), e1]
     C_((launch_wgrad<16, 48, 32>(d2_, G_, dW[4], g1_, err_dev_, s_, e1_)))
     C_(conv_any(48, 16, 1, G_, wtt_[4], nullptr, gc1_, g1_, -1, 0, err_dev_, s_))
-    k_up_back<<<gsize(n2 * 32), 256, 0, s_>>>(gc1_, 48, g2_, 32, gd2_);
+    k_up_back<<<gsize(n2 * 8), 256, 0, s_>>>(gc1_, 48, g2_, 32, gd2_);
     k_mask_grad<32><<<rsize(n2 * (32 / 8)), 256, 0, s_>>>(gd2_, 32, 0, nullptr, g2_, d2_, G_, db[3]);
     C_(cudaGetLastError())
     // layer 4: 96 -> 32 on c2 = [up(b3), e2]
     C_((launch_wgrad<32, 96, 64>(b3_, G_, dW[3], g2_, err_dev_, s_, e2_)))
     C_(conv_any(96, 32, 1, G_, wtt_[3], nullptr, gc2_, g2_, -1, 0, err_dev_, s_))
-    k_up_back<<<gsize(n3 * 64), 256, 0, s_>>>(gc2_, 96, g3_, 64, gb3_);
+    k_up_back<<<gsize(n3 * 16), 256, 0, s_>>>(gc2_, 96, g3_, 64, gb3_);
     k_mask_grad<64><<<rsize(n3 * (64 / 8)), 256, 0, s_>>>(gb3_, 64, 0, nullptr, g3_, b3_, G_, db[2]);
     C_(cudaGetLastError())
     // layer 3: 32 -> 64 on pool(e2)
