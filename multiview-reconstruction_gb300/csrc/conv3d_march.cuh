@@ -135,19 +135,45 @@ struct MarchPlanes {
     }
 };
 
-// OUT_MODE 0: BF16 output with bias (+ReLU when relu != 0); 1: FP32 output, no bias.
-template <int N, int C, int OUT_MODE, int CU = 0>
+// What becomes of the output.  The 2x2x2 sums and the head are formed from the accumulators: as kernels of
+// their own they read everything back (16 channels on 128^3: averages 14 us and head 13 us, against 8
+// and 5 more here; the 48-channel gradient on 4 x 64^3 written whole and summed after it 126 us, now 53).
+enum MarchOut {
+    MARCH_BF16,   // out: BF16 with bias (+ReLU when relu != 0); out2 (or NULL): its 2x2x2 averages, BF16
+    MARCH_FP32,   // out: FP32, no bias
+    MARCH_HEAD,   // out: FP32, one value per voxel: MARCH_BF16's 16 channels times wh, plus bh[0]
+    MARCH_SPLIT,  // gradient of a concatenation: the first CB channels summed over 2x2x2 voxels into
+                  // out, the others into out2, both FP32
+};
+
+// Sum of 16 channels over the four voxels (x, y) of a quad: lane bits 0 and 3.  Each lane keeps four
+// channels, 8 (bit 0) + 4 (bit 3) onwards, and sends the others.
+__device__ __forceinline__ void quad_sum(const float (&v)[16], float (&r)[4], int lane)
+{
+    const bool ox = lane & 1, oy = lane & 8;
+    float h[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) h[j] = (ox ? v[j + 8] : v[j]) + __shfl_xor_sync(0xffffffffu, ox ? v[j] : v[j + 8], 1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) r[j] = (oy ? h[j + 4] : h[j]) + __shfl_xor_sync(0xffffffffu, oy ? h[j] : h[j + 4], 8);
+}
+
+template <int N, int C, int OUT, int CU = 0, int CB = 0>
 __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloat16 *__restrict__ act,
-                                                      const __nv_bfloat16 *__restrict__ wk,
-                                                      const float *__restrict__ bias, void *out, ConvGeom g, int sign,
-                                                      int relu, int *err,
-                                                      const __nv_bfloat16 *__restrict__ act2 = nullptr)
+                                                                const __nv_bfloat16 *__restrict__ wk,
+                                                                const float *__restrict__ bias, void *out, ConvGeom g,
+                                                                int sign, int relu, int *err,
+                                                                const __nv_bfloat16 *__restrict__ act2, void *out2,
+                                                                const float *__restrict__ wh,
+                                                                const float *__restrict__ bh)
 {
     constexpr int NS = march_ns<N, C>(), ST = kMarchStages, CH = C / 8;
     constexpr uint32_t COLS = march_cols<NS, C>();
     constexpr int R = (int)COLS / NS;  // ring of output planes: three being added to, one being read
     constexpr int PB = CH * kMarchLbo, B_TAP = 3 * NS * C * 2;
     static_assert(N % NS == 0 && NS % 16 == 0 && 3 * NS <= 256 && C % 16 == 0 && R >= 4, "tile shape");
+    static_assert(OUT != MARCH_HEAD || NS == 16, "a thread holds the head's 16 channels");
+    static_assert(CB % 16 == 0 && (OUT == MARCH_SPLIT) == (CB > 0), "channel split of the output");
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *sB = smem + ((ST * PB + 1023) / 1024) * 1024;
     __shared__ __align__(8) uint64_t done[ST];
@@ -160,11 +186,12 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
     }
     const long long planes =
         (long long)((g.W + kMarchX - 1) / kMarchX) * ((g.H + kMarchY - 1) / kMarchY) * g.B * g.D;
-    const long long u1 = planes * (blockIdx.x + 1) / gridDim.x;
+    const int pz = g.D & 1 ? 1 : 2;  // a run begins and ends between pairs of planes (sums over 2x2x2 voxels)
+    const long long u1 = planes / pz * (blockIdx.x + 1) / gridDim.x * pz;
     const int co0 = blockIdx.y * NS;
     // the copies run kMarchStages - 1 steps ahead of the products, past the ends of parts
     MarchAt ld, at;
-    ld.u = at.u = planes * blockIdx.x / gridDim.x;
+    ld.u = at.u = planes / pz * blockIdx.x / gridDim.x * pz;
     ld.start(g, u1);
     at.start(g, u1);
     MarchPlanes<C, CU> in(g, act, act2, tid);
@@ -225,8 +252,12 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
     };
     bool ok = true;
     int s = 0, slot = -1;  // slot of the output plane that step s - 1 completed, or -1
-    long long n = 0;       // this thread's voxel of it
-    bool rv = false;
+    long long n = 0;       // this thread's voxel of it, and the voxel of the half-size volume
+    long long nl = 0;
+    bool rv = false, odd = false;
+    const int lane = tid & 31;
+    const bool pool = OUT == MARCH_BF16 && out2 != nullptr;
+    float pair[NS / 16][4];  // the quad's sums of an even plane
 #pragma unroll 1
     for (;; ++s) {
         const bool more = at.u < u1;
@@ -251,20 +282,50 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
                 for (int c0 = 0; c0 < NS; c0 += 16) {
                     float v[16];
                     tc::tmem_ld16(trow + c0, v);
-                    if (!rv) continue;
-                    if (OUT_MODE == 0) {
+                    if constexpr (OUT == MARCH_BF16 || OUT == MARCH_HEAD) {
                         __align__(16) __nv_bfloat16 w[16];
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
                             float a = v[j] + (bias ? bias[co0 + c0 + j] : 0.0f);
                             if (relu) a = fmaxf(a, 0.0f);
                             w[j] = __float2bfloat16(a);
+                            v[j] = __bfloat162float(w[j]);
                         }
-                        uint4 *op = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(out) + n * N + co0 + c0);
-                        op[0] = reinterpret_cast<const uint4 *>(w)[0];
-                        op[1] = reinterpret_cast<const uint4 *>(w)[1];
-                    } else {
-                        float4 *op = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + n * N + co0 + c0);
+                        if constexpr (OUT == MARCH_HEAD) {
+                            float h = bh[0];
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) h += wh[j] * v[j];
+                            if (rv) static_cast<float *>(out)[n] = h;
+                        } else if (rv) {
+                            uint4 *op = reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(out) + n * N + co0 + c0);
+                            op[0] = reinterpret_cast<const uint4 *>(w)[0];
+                            op[1] = reinterpret_cast<const uint4 *>(w)[1];
+                        }
+                    }
+                    if ((OUT == MARCH_SPLIT && co0 + c0 < CB) || (OUT == MARCH_BF16 && pool)) {
+                        float (&q)[4] = pair[c0 / 16];
+                        float r[4];
+                        quad_sum(v, r, lane);
+                        if (!odd) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) q[j] = r[j];
+                        } else if (rv) {
+                            const int c = co0 + c0 + (lane & 1) * 8 + (lane >> 3 & 1) * 4;
+                            if constexpr (OUT == MARCH_SPLIT) {
+                                *reinterpret_cast<float4 *>(static_cast<float *>(out) + nl * CB + c) =
+                                    make_float4(q[0] + r[0], q[1] + r[1], q[2] + r[2], q[3] + r[3]);
+                            } else {
+                                __align__(8) __nv_bfloat16 w[4];
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) w[j] = __float2bfloat16(0.125f * (q[j] + r[j]));
+                                *reinterpret_cast<uint2 *>(static_cast<__nv_bfloat16 *>(out2) + nl * N + c) =
+                                    *reinterpret_cast<const uint2 *>(w);
+                            }
+                        }
+                    } else if ((OUT == MARCH_SPLIT || OUT == MARCH_FP32) && rv) {
+                        float4 *op = reinterpret_cast<float4 *>(
+                            OUT == MARCH_SPLIT ? static_cast<float *>(out2) + n * (N - CB) + co0 + c0 - CB
+                                               : static_cast<float *>(out) + n * N + co0 + c0);
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
                             op[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
@@ -278,7 +339,10 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
         if (at.p >= 2) {
             const int x = at.x0 + (tid & 7), y = at.y0 + (tid >> 3 & 15);
             slot = (ring + at.p - 2) % R;
-            n = (((long long)at.b * g.D + at.zs + at.p - 2) * g.H + y) * g.W + x;
+            const int z = at.zs + at.p - 2;
+            n = (((long long)at.b * g.D + z) * g.H + y) * g.W + x;
+            nl = (((long long)at.b * (g.D >> 1) + (z >> 1)) * (g.H >> 1) + (y >> 1)) * (g.W >> 1) + (x >> 1);
+            odd = z & 1;
             rv = x < g.W && y < g.H;
         }
         const int nz = at.nz;

@@ -45,41 +45,32 @@ int gsize(long long n) { return (int)std::max<long long>(1, std::min<long long>(
 // 12 planes were better only on large levels, which have them anyway (32 -> 64 channels on 32^3: runs
 // of 3, 6 and 12 planes 14, 19 and 28 us; 16 -> 32 on 64^3 27, 24 and 28 us).
 constexpr int kMarchMin = 4;
-template <int N, int C, int OUT, int CU>
-cudaError_t launch_march(const bf16 *act, const bf16 *act2, const bf16 *w, const float *bias, void *out,
-                         const ConvGeom &g, int sign, int relu, int *err, cudaStream_t s)
+struct MarchArgs {
+    const bf16 *act, *act2 = nullptr;  // act2: the other channels of a concatenation
+    const bf16 *w;
+    const float *bias = nullptr;
+    void *out, *out2 = nullptr;
+    int sign = 1, relu = 0;
+    const float *wh = nullptr, *bh = nullptr;
+};
+template <int N, int C, int OUT, int CU = 0, int CB = 0>
+cudaError_t launch_march(const MarchArgs &a, const ConvGeom &g, int *err, cudaStream_t s)
 {
     constexpr int NS = march_ns<N, C>();
-    if ((reinterpret_cast<uintptr_t>(act) | reinterpret_cast<uintptr_t>(act2) | reinterpret_cast<uintptr_t>(w) |
-         reinterpret_cast<uintptr_t>(out)) & 15)
+    if ((reinterpret_cast<uintptr_t>(a.act) | reinterpret_cast<uintptr_t>(a.act2) | reinterpret_cast<uintptr_t>(a.w) |
+         reinterpret_cast<uintptr_t>(a.out)) & 15)
         return cudaErrorInvalidValue;
     const size_t sm = march_smem<NS, C>();
     cudaError_t e =
-        cudaFuncSetAttribute(k_conv3d_march<N, C, OUT, CU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaFuncSetAttribute(k_conv3d_march<N, C, OUT, CU, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     const long long res = std::max<long long>(1, std::min<long long>((227 * 1024) / (sm + 1024), 512 / march_cols<NS, C>()));
     const long long planes =
         (long long)((g.W + kMarchX - 1) / kMarchX) * ((g.H + kMarchY - 1) / kMarchY) * g.B * g.D;
     const long long grid = std::min(std::max<long long>(152 * res / (N / NS), 1), (planes + kMarchMin - 1) / kMarchMin);
-    k_conv3d_march<N, C, OUT, CU><<<dim3((unsigned)grid, N / NS), kMarchThreads, sm, s>>>(act, w, bias, out, g, sign,
-                                                                                          relu, err, act2);
+    k_conv3d_march<N, C, OUT, CU, CB><<<dim3((unsigned)grid, N / NS), kMarchThreads, sm, s>>>(
+        a.act, a.w, a.bias, a.out, g, a.sign, a.relu, err, a.act2, a.out2, a.wh, a.bh);
     return cudaGetLastError();
-}
-
-template <int N, int C, int OUT>
-cudaError_t launch_conv(const bf16 *act, const bf16 *w, const float *bias, void *out, const ConvGeom &g, int sign,
-                        int relu, int *err, cudaStream_t s)
-{
-    return launch_march<N, C, OUT, 0>(act, nullptr, w, bias, out, g, sign, relu, err, s);
-}
-
-// Decoder convolution (bias, ReLU, BF16 out) on the concatenation [up(low) (CU channels),
-// skip (C - CU channels)] without materialising it.
-template <int N, int C, int CU>
-cudaError_t launch_conv_concat(const bf16 *low, const bf16 *skip, const bf16 *w, const float *bias, void *out,
-                               const ConvGeom &g, int *err, cudaStream_t s)
-{
-    return launch_march<N, C, 0, CU>(low, skip, w, bias, out, g, 1, 1, err, s);
 }
 
 // Weight gradient (k_wgrad_march): runs as in launch_march, one CTA per SM (it holds all tensor memory)
@@ -103,12 +94,13 @@ cudaError_t launch_wgrad(const bf16 *X, const bf16 *G, float *dW, const ConvGeom
 
 // forward (N = Cout, C = Cin) and dgrad (N = Cin, C = Cout) shapes of the five layers
 cudaError_t conv_any(int N, int C, int out_mode, const bf16 *act, const bf16 *w, const float *bias, void *out,
-                     const ConvGeom &g, int sign, int relu, int *err, cudaStream_t s)
+                     const ConvGeom &g, int sign, int relu, int *err, cudaStream_t s, void *pool = nullptr)
 {
+    MarchArgs a;
+    a.act = act, a.w = w, a.bias = bias, a.out = out, a.out2 = pool, a.sign = sign, a.relu = relu;
 #define MVR_CONV_CASE(NN, CC)                                                                              \
     if (N == NN && C == CC)                                                                                \
-        return out_mode == 0 ? launch_conv<NN, CC, 0>(act, w, bias, out, g, sign, relu, err, s)            \
-                             : launch_conv<NN, CC, 1>(act, w, bias, out, g, sign, relu, err, s);
+        return out_mode == 0 ? launch_march<NN, CC, MARCH_BF16>(a, g, err, s) : launch_march<NN, CC, MARCH_FP32>(a, g, err, s);
     MVR_CONV_CASE(16, 16)
     MVR_CONV_CASE(32, 16)
     MVR_CONV_CASE(64, 32)
@@ -192,35 +184,6 @@ __global__ void k_features(const float *psi, const float *psi_next, const float 
         o[0] = reinterpret_cast<const uint4 *>(f)[0];
         o[1] = reinterpret_cast<const uint4 *>(f)[1];
         if (target && psi_m) target[i] = logf(fmaxf(psi_m[i], 1e-12f) / p);
-    }
-}
-
-// 2x2x2 average pooling, channels-last BF16; a thread takes 8 channels (16 bytes) of a voxel, as every
-// channels-last kernel here: one channel per thread read 2 bytes at a time (16 channels on 128^3: 34 us)
-__global__ void k_pool(const bf16 *in, bf16 *out, ConvGeom lo, int C)
-{
-    const int K = C / 8;
-    const long long n = lo.nvox * K;
-    const int W2 = lo.W * 2, H2 = lo.H * 2, D2 = lo.D * 2;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(i % K);
-        int x, y, z, b;
-        vox_coords(lo, i / K, x, y, z, b);
-        uint4 v[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const long long src = (((long long)b * D2 + 2 * z + (q >> 2)) * H2 + 2 * y + ((q >> 1) & 1)) * W2 + 2 * x + (q & 1);
-            v[q] = __ldg(reinterpret_cast<const uint4 *>(in + src * C) + k);
-        }
-        __align__(16) bf16 o[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            float s = 0.0f;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) s += __bfloat162float(reinterpret_cast<const bf16 *>(&v[q])[c]);
-            o[c] = __float2bfloat16(0.125f * s);
-        }
-        reinterpret_cast<uint4 *>(out)[i] = *reinterpret_cast<const uint4 *>(o);
     }
 }
 
@@ -363,31 +326,6 @@ __global__ void __launch_bounds__(256) k_mask_grad(const float *gsk, int gsk_str
     }
 }
 
-// gradient of up(low) inside a concat gradient: glow[lv][c] = sum over the 8 children
-// of gcat[child][c], c < Cu
-__global__ void k_up_back(const float *gcat, int Ct, ConvGeom lo, int Cu, float *glow)
-{
-    const int K = Cu / 4;
-    const long long n = lo.nvox * K;
-    const int W2 = lo.W * 2, H2 = lo.H * 2, D2 = lo.D * 2;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(i % K);
-        int x, y, z, b;
-        vox_coords(lo, i / K, x, y, z, b);
-        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const long long src = (((long long)b * D2 + 2 * z + (q >> 2)) * H2 + 2 * y + ((q >> 1) & 1)) * W2 + 2 * x + (q & 1);
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(gcat + src * Ct) + k);
-            s.x += v.x;
-            s.y += v.y;
-            s.z += v.z;
-            s.w += v.w;
-        }
-        reinterpret_cast<float4 *>(glow)[i] = s;
-    }
-}
-
 // BF16 copies of the FP32 master weights: W[co][t][ci] and its transpose WT[ci][t][co]
 __global__ void k_weights_bf16(const float *w, int Co, int Ci, bf16 *wt, bf16 *wtt)
 {
@@ -491,7 +429,7 @@ public:
     ~UNet();
     int init();
     int set_input(const float *psi, const float *psi_next, const float *psi_target);
-    int forward(float *pred);
+    int forward(float *pred, bool train = false);
     int train_step(float lr, double *loss);
     int propose(const float *psi, float *out, float cap);
     long long num_params() const { return nparams_; }
@@ -537,7 +475,7 @@ private:
     bf16 *d2_ = nullptr, *d1_ = nullptr;
     bf16 *G_ = nullptr;  // BF16 gradient scratch (largest: level 1 x 16 or level 2 x 32)
     float *out_ = nullptr, *target_ = nullptr;
-    float *gc1_ = nullptr, *gc2_ = nullptr, *gd2_ = nullptr, *gb3_ = nullptr, *gp2_ = nullptr, *gp1_ = nullptr;
+    float *gs1_ = nullptr, *gs2_ = nullptr, *gd2_ = nullptr, *gb3_ = nullptr, *gp2_ = nullptr, *gp1_ = nullptr;
     double *mean_ = nullptr, *meanp_ = nullptr, *loss_ = nullptr;
     int *err_dev_ = nullptr;
     int step_ = 0;
@@ -589,7 +527,7 @@ int UNet::init()
     A_(in16_, n1 * 16) A_(e1_, n1 * 16) A_(p1_, n2 * 16) A_(e2_, n2 * 32) A_(p2_, n3 * 32) A_(b3_, n3 * 64)
     A_(d2_, n2 * 32) A_(d1_, n1 * 16)
     A_(G_, std::max(n1 * 16, n2 * 32)) A_(out_, n1) A_(target_, n1)
-    A_(gc1_, n1 * 48) A_(gc2_, n2 * 96) A_(gd2_, n2 * 32) A_(gb3_, n3 * 64) A_(gp2_, n3 * 32) A_(gp1_, n2 * 16)
+    A_(gs1_, n1 * 16) A_(gs2_, n2 * 32) A_(gd2_, n2 * 32) A_(gb3_, n3 * 64) A_(gp2_, n3 * 32) A_(gp1_, n2 * 16)
     A_(mean_, B_) A_(meanp_, (long long)B_ * kMeanParts) A_(loss_, 1) A_(err_dev_, 1)
 #undef A_
     // He initialisation from a seeded generator (host), zero biases
@@ -644,7 +582,7 @@ int UNet::set_input(const float *psi, const float *psi_next, const float *psi_ta
     return cuda(cudaGetLastError(), "k_features");
 }
 
-int UNet::forward(float *pred)
+int UNet::forward(float *pred, bool train)
 {
     cudaSetDevice(dev_);
     int rc = refresh_weights();
@@ -652,15 +590,22 @@ int UNet::forward(float *pred)
     const long long n1 = g1_.nvox, n2 = g2_.nvox;
 #define C_(expr)                                         \
     if ((rc = cuda((expr), #expr)) != MVR_OK) return rc;
-    C_(conv_any(16, 16, 0, in16_, wt_[0], params_ + boff_[0], e1_, g1_, 1, 1, err_dev_, s_))
-    k_pool<<<gsize(n2 * 2), 256, 0, s_>>>(e1_, p1_, g2_, 16);
-    C_(conv_any(32, 16, 0, p1_, wt_[1], params_ + boff_[1], e2_, g2_, 1, 1, err_dev_, s_))
-    k_pool<<<gsize(g3_.nvox * 4), 256, 0, s_>>>(e2_, p2_, g3_, 32);
+    C_(conv_any(16, 16, 0, in16_, wt_[0], params_ + boff_[0], e1_, g1_, 1, 1, err_dev_, s_, p1_))
+    C_(conv_any(32, 16, 0, p1_, wt_[1], params_ + boff_[1], e2_, g2_, 1, 1, err_dev_, s_, p2_))
     C_(conv_any(64, 32, 0, p2_, wt_[2], params_ + boff_[2], b3_, g3_, 1, 1, err_dev_, s_))
     // the decoder convolutions read [up(low), skip] where they are, here and in the weight gradients
-    C_((launch_conv_concat<32, 96, 64>(b3_, e2_, wt_[3], params_ + boff_[3], d2_, g2_, err_dev_, s_)))
-    C_((launch_conv_concat<16, 48, 32>(d2_, e1_, wt_[4], params_ + boff_[4], d1_, g1_, err_dev_, s_)))
-    k_head<<<gsize(n1), 256, 0, s_>>>(d1_, params_ + whoff_, params_ + bhoff_, out_, n1);
+    MarchArgs a;
+    a.act = b3_, a.act2 = e2_, a.w = wt_[3], a.bias = params_ + boff_[3], a.out = d2_, a.relu = 1;
+    C_((launch_march<32, 96, MARCH_BF16, 64>(a, g2_, err_dev_, s_)))
+    a.act = d2_, a.act2 = e1_, a.w = wt_[4], a.bias = params_ + boff_[4];
+    if (train) {
+        a.out = d1_;
+        C_((launch_march<16, 48, MARCH_BF16, 32>(a, g1_, err_dev_, s_)))
+        k_head<<<gsize(n1), 256, 0, s_>>>(d1_, params_ + whoff_, params_ + bhoff_, out_, n1);
+    } else {  // d1 is of use to the backward pass alone
+        a.out = out_, a.wh = params_ + whoff_, a.bh = params_ + bhoff_;
+        C_((launch_march<16, 48, MARCH_HEAD, 32>(a, g1_, err_dev_, s_)))
+    }
     C_(cudaGetLastError())
     if (pred) C_(cudaMemcpyAsync(pred, out_, sizeof(float) * (size_t)n1, cudaMemcpyDeviceToDevice, s_))
 #undef C_
@@ -669,7 +614,7 @@ int UNet::forward(float *pred)
 
 int UNet::train_step(float lr, double *loss)
 {
-    int rc = forward(nullptr);
+    int rc = forward(nullptr, true);
     if (rc != MVR_OK) return rc;
     const long long n1 = g1_.nvox, n2 = g2_.nvox, n3 = g3_.nvox;
 #define C_(expr)                                         \
@@ -687,27 +632,28 @@ int UNet::train_step(float lr, double *loss)
     C_(cudaGetLastError())
     // layer 5: 48 -> 16 on c1 = [up(d2), e1]
     C_((launch_wgrad<16, 48, 32>(d2_, G_, dW[4], g1_, err_dev_, s_, e1_)))
-    C_(conv_any(48, 16, 1, G_, wtt_[4], nullptr, gc1_, g1_, -1, 0, err_dev_, s_))
-    k_up_back<<<gsize(n2 * 8), 256, 0, s_>>>(gc1_, 48, g2_, 32, gd2_);
+    MarchArgs a;
+    a.act = G_, a.w = wtt_[4], a.out = gd2_, a.out2 = gs1_, a.sign = -1;
+    C_((launch_march<48, 16, MARCH_SPLIT, 0, 32>(a, g1_, err_dev_, s_)))
     k_mask_grad<32><<<rsize(n2 * (32 / 8)), 256, 0, s_>>>(gd2_, 32, 0, nullptr, g2_, d2_, G_, db[3]);
     C_(cudaGetLastError())
     // layer 4: 96 -> 32 on c2 = [up(b3), e2]
     C_((launch_wgrad<32, 96, 64>(b3_, G_, dW[3], g2_, err_dev_, s_, e2_)))
-    C_(conv_any(96, 32, 1, G_, wtt_[3], nullptr, gc2_, g2_, -1, 0, err_dev_, s_))
-    k_up_back<<<gsize(n3 * 16), 256, 0, s_>>>(gc2_, 96, g3_, 64, gb3_);
+    a.w = wtt_[3], a.out = gb3_, a.out2 = gs2_;
+    C_((launch_march<96, 32, MARCH_SPLIT, 0, 64>(a, g2_, err_dev_, s_)))
     k_mask_grad<64><<<rsize(n3 * (64 / 8)), 256, 0, s_>>>(gb3_, 64, 0, nullptr, g3_, b3_, G_, db[2]);
     C_(cudaGetLastError())
     // layer 3: 32 -> 64 on pool(e2)
     C_(wgrad_any(64, 32, p2_, G_, dW[2], g3_, err_dev_, s_))
     C_(conv_any(32, 64, 1, G_, wtt_[2], nullptr, gp2_, g3_, -1, 0, err_dev_, s_))
-    // e2: skip gradient (channels 64..95 of c2) + pooled gradient from level 3
-    k_mask_grad<32><<<rsize(n2 * (32 / 8)), 256, 0, s_>>>(gc2_, 96, 64, gp2_, g2_, e2_, G_, db[1]);
+    // e2: skip gradient (channels 64..95 of the concatenation) + pooled gradient from level 3
+    k_mask_grad<32><<<rsize(n2 * (32 / 8)), 256, 0, s_>>>(gs2_, 32, 0, gp2_, g2_, e2_, G_, db[1]);
     C_(cudaGetLastError())
     // layer 2: 16 -> 32 on pool(e1)
     C_(wgrad_any(32, 16, p1_, G_, dW[1], g2_, err_dev_, s_))
     C_(conv_any(16, 32, 1, G_, wtt_[1], nullptr, gp1_, g2_, -1, 0, err_dev_, s_))
-    // e1: skip gradient (channels 32..47 of c1) + pooled gradient from level 2
-    k_mask_grad<16><<<rsize(n1 * (16 / 8)), 256, 0, s_>>>(gc1_, 48, 32, gp1_, g1_, e1_, G_, db[0]);
+    // e1: skip gradient (channels 32..47) + pooled gradient from level 2
+    k_mask_grad<16><<<rsize(n1 * (16 / 8)), 256, 0, s_>>>(gs1_, 16, 0, gp1_, g1_, e1_, G_, db[0]);
     C_(cudaGetLastError())
     // layer 1: 16 -> 16 on the input features
     C_(wgrad_any(16, 16, in16_, G_, dW[0], g1_, err_dev_, s_))

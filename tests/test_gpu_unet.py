@@ -165,3 +165,35 @@ def test_weight_gradient_columns_and_runs(ci, co, dims):
     # added to what is there; up to 21780 FP32 additions of exact products: sqrt(21780) 2^-24
     assert rel(dwd.cpu().numpy(), 1.0 + U.conv_wgrad(x, g)) <= 1e-5
     assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("dims,B", [((4, 4, 4), 3), ((12, 20, 8), 1), ((20, 36, 12), 2)])
+def test_unet_gradients_on_ragged_columns(dims, B):
+    # averages, the head and the split gradient of the concatenations, with columns and runs that end inside
+    # the volume; the tolerances of the 8^3 case above
+    rng = np.random.default_rng(dims[0])
+    shape = (B, dims[2], dims[1], dims[0])
+    psi = rng.uniform(10, 100, shape).astype(np.float32)
+    psi_n = (psi * rng.uniform(0.8, 1.25, shape)).astype(np.float32)
+    psi_t = (psi * rng.uniform(0.7, 1.4, shape)).astype(np.float32)
+    with M.UNet(B, dims, seed=3) as net:
+        pd, rd, td = (torch.from_numpy(a).cuda() for a in (psi, psi_n, psi_t))
+        net.set_input(pd.data_ptr(), rd.data_ptr(), td.data_ptr())
+        params = net.params()
+        loss = net.train_step(0.0)
+        grads = net.grads()
+        pred = torch.empty_like(pd)
+        net.forward(pred.data_ptr())
+    loss_ref, g_ref, _ = U.forward_backward(params, U.features(psi, psi_n), np.log(psi_t / psi).astype(np.float64))
+    assert abs(loss - loss_ref) <= 1e-3 * loss_ref
+    # the forward pass alone forms the same predictions
+    t = torch.log(td / pd)
+    assert abs(float(((pred - t) ** 2).mean()) - loss) <= 1e-3 * loss
+    o = 0
+    for ci, co in U.LAYERS:
+        nw = co * 27 * ci
+        assert rel(grads[o:o + nw], g_ref[o:o + nw]) <= 3e-2, (ci, co)
+        o += nw
+        assert rel(grads[o:o + co], g_ref[o:o + co]) <= 3e-2, (ci, co, "bias")
+        o += co
+    assert rel(grads[o:o + 17], g_ref[o:o + 17]) <= 1e-3
