@@ -52,15 +52,19 @@ bool kernel_host_copy(int dev)
     return cached[dev] == 1;
 }
 
+// CTAs of a copy: 64 of 256 threads already move all that the host link takes (28 MB up at 202 GB/s, down
+// at 184, the same with 152 to 1216), and more of them only take threads from the convolutions they run
+// beside: the 192^3 block takes 710 us with 608, 677 with 152, 653 with 64, 658 with 32 and 690 with 16.
+constexpr int kCopyCtas = 64;
 cudaError_t host_copy(void *dst, const void *src, size_t bytes, cudaMemcpyKind kind, int dev, cudaStream_t s)
 {
     if (!kernel_host_copy(dev)) return cudaMemcpyAsync(dst, src, bytes, kind, s);
     const bool vec = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | bytes) & 15) == 0;
     if (vec)
-        k_copy_words<<<608, 256, 0, s>>>(static_cast<float4 *>(dst), static_cast<const float4 *>(src),
+        k_copy_words<<<kCopyCtas, 256, 0, s>>>(static_cast<float4 *>(dst), static_cast<const float4 *>(src),
                                          (long long)(bytes / 16));
     else
-        k_copy_floats<<<608, 256, 0, s>>>(static_cast<float *>(dst), static_cast<const float *>(src),
+        k_copy_floats<<<kCopyCtas, 256, 0, s>>>(static_cast<float *>(dst), static_cast<const float *>(src),
                                           (long long)(bytes / 4));
     return cudaGetLastError();
 }
@@ -250,8 +254,7 @@ extern "C" int mvr_block_run_seq(mvr_block *h, int view, float *psi, const float
     if (h->seps[view].ready()) {
         // the first convolution needs psi alone and the update alone the weight: the image and the
         // weight come up on a second stream behind psi (all three share the host link) while the
-        // first convolution and the quotient run: 731 -> 712 us at 192^3, the rest of which is the
-        // link's 113 MB and the update between the last upload and psi's way back
+        // first convolution and the quotient run: 731 -> 653 us at 192^3 (the link's 113 MB take 574)
         BLK_CUDA(h, h->copy_stream());
         BLK_CUDA(h, cudaEventRecord(h->ev_psi, s));
         BLK_CUDA(h, cudaStreamWaitEvent(h->copy, h->ev_psi, 0));
