@@ -27,8 +27,9 @@
  * Java thread).  There is no CPU fallback: without a usable GB300 (sm_103a) the
  * create calls fail with MVR_ERR_CUDA.
  *
- * FP32 FFT domains with Px, Py in {128, 192} run on the plane kernels (x and y transforms
- * fused per z-plane); the environment variable MVR_PLANE_KERNELS=0, read when kernels are
+ * Blocks, and iterations without statistics, run on separable transforms (mvr_decon_run says
+ * when).  Where block plans remain, FP32 FFT domains with Px, Py in {128, 192} run on the plane
+ * kernels (x and y transforms fused per z-plane); the environment variable MVR_PLANE_KERNELS=0, read when kernels are
  * set or a deconvolution is prepared, selects the row / column kernels instead (for
  * comparisons; results agree to float rounding).
  */

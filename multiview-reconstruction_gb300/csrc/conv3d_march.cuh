@@ -201,11 +201,7 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
         if (ld.next(g, u1)) in.column(ld);
     };
     // the weights, per offset (dy, dx) 3 NS rows: output plane z - 1 (dz = 1), z, z + 1, each NS channels
-    // (every CTA reads the same ones at the same time: each starts at a place of its own)
-    constexpr int WN = 27 * NS * CH;
-    const int rot = (int)((blockIdx.x * 331u) % WN);
-    for (int s0 = tid; s0 < WN; s0 += kMarchThreads) {
-        const int s = s0 + rot < WN ? s0 + rot : s0 + rot - WN;
+    for (int s = tid; s < 27 * NS * CH; s += kMarchThreads) {
         const int t = s / (3 * NS * CH), rem = s - t * (3 * NS * CH), r = rem / CH, j = rem - r * CH;
         const int i = r / NS, tz = (1 - i) * sign + 1;
         cp_async16(sB + t * B_TAP + tc::core_offset(r, 8 * j, C),
