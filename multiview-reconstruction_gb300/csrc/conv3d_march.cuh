@@ -25,6 +25,7 @@
 // 680 and 115 us, 16 -> 16 193 and 60, 96 -> 32 292 and 70; 16 -> 32 40 and 26, 32 -> 64 (32^3) 20 and 19.
 #pragma once
 #include "conv3d_tc.cuh"
+#include "pdl.cuh"
 
 namespace mvr {
 
@@ -208,14 +209,19 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
                    reinterpret_cast<const uint4 *>(
                        wk + ((long long)(co0 + r - i * NS) * 27 + 9 * tz + (sign > 0 ? t : 8 - t)) * C) + j, true);
     }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    // From here on this CTA has its tensor memory, so a next kernel that starts beside it (launch_pdl)
+    // takes only what is left.  Every CTA of the kernel before has its own for the same reason, and the
+    // weights above are older than that kernel.
+    pdl_trigger();
+    pdl_wait();
 #pragma unroll 1
     for (int s = 0; s < ST; ++s) {
         if (ld.u < u1 && warp < 4) load(s);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
     const uint32_t tmem = __shfl_sync(0xffffffffu, tbase, 0);
     const uint32_t hbase = tc::smem_u32(smem), bbase = tc::smem_u32(sB);
     int ring = 0;  // output planes of the parts before: plane j of a part has the columns of slot (ring + j) % R
@@ -444,14 +450,16 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
             in.column(ld);
         }
     };
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    pdl_trigger();  // behind the allocation, as above
+    pdl_wait();
 #pragma unroll 1
     for (int s = 0; s < ST; ++s) {
         if (ld.u < u1 && warp < 4) load(s);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
     const uint32_t tmem = __shfl_sync(0xffffffffu, tbase, 0);
     const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
     if (warp < 4)

@@ -29,6 +29,7 @@
 #include "conv3d_tc.cuh"
 #include "conv3d_march.cuh"
 #include "fsum.cuh"
+#include "pdl.cuh"
 
 namespace mvr {
 namespace {
@@ -52,6 +53,7 @@ struct MarchArgs {
     void *out, *out2 = nullptr;
     int sign = 1, relu = 0;
     const float *wh = nullptr, *bh = nullptr;
+    bool early = false;  // may start beside the kernel before it, which did not write the weights
 };
 template <int N, int C, int OUT, int CU = 0, int CB = 0>
 cudaError_t launch_march(const MarchArgs &a, const ConvGeom &g, int *err, cudaStream_t s)
@@ -68,9 +70,8 @@ cudaError_t launch_march(const MarchArgs &a, const ConvGeom &g, int *err, cudaSt
     const long long planes =
         (long long)((g.W + kMarchX - 1) / kMarchX) * ((g.H + kMarchY - 1) / kMarchY) * g.B * g.D;
     const long long grid = std::min(std::max<long long>(152 * res / (N / NS), 1), (planes + kMarchMin - 1) / kMarchMin);
-    k_conv3d_march<N, C, OUT, CU, CB><<<dim3((unsigned)grid, N / NS), kMarchThreads, sm, s>>>(
-        a.act, a.w, a.bias, a.out, g, a.sign, a.relu, err, a.act2, a.out2, a.wh, a.bh);
-    return cudaGetLastError();
+    return launch_dep(!a.early, k_conv3d_march<N, C, OUT, CU, CB>, dim3((unsigned)grid, N / NS), kMarchThreads, sm, s,
+                      a.act, a.w, a.bias, a.out, g, a.sign, a.relu, err, a.act2, a.out2, a.wh, a.bh);
 }
 
 // Weight gradient (k_wgrad_march): runs as in launch_march, one CTA per SM (it holds all tensor memory)
@@ -94,9 +95,11 @@ cudaError_t launch_wgrad(const bf16 *X, const bf16 *G, float *dW, const ConvGeom
 
 // forward (N = Cout, C = Cin) and dgrad (N = Cin, C = Cout) shapes of the five layers
 cudaError_t conv_any(int N, int C, int out_mode, const bf16 *act, const bf16 *w, const float *bias, void *out,
-                     const ConvGeom &g, int sign, int relu, int *err, cudaStream_t s, void *pool = nullptr)
+                     const ConvGeom &g, int sign, int relu, int *err, cudaStream_t s, void *pool = nullptr,
+                     bool early = false)
 {
     MarchArgs a;
+    a.early = early;
     a.act = act, a.w = w, a.bias = bias, a.out = out, a.out2 = pool, a.sign = sign, a.relu = relu;
 #define MVR_CONV_CASE(NN, CC)                                                                              \
     if (N == NN && C == CC)                                                                                \
@@ -591,10 +594,11 @@ int UNet::forward(float *pred, bool train)
 #define C_(expr)                                         \
     if ((rc = cuda((expr), #expr)) != MVR_OK) return rc;
     C_(conv_any(16, 16, 0, in16_, wt_[0], params_ + boff_[0], e1_, g1_, 1, 1, err_dev_, s_, p1_))
-    C_(conv_any(32, 16, 0, p1_, wt_[1], params_ + boff_[1], e2_, g2_, 1, 1, err_dev_, s_, p2_))
-    C_(conv_any(64, 32, 0, p2_, wt_[2], params_ + boff_[2], b3_, g3_, 1, 1, err_dev_, s_))
+    C_(conv_any(32, 16, 0, p1_, wt_[1], params_ + boff_[1], e2_, g2_, 1, 1, err_dev_, s_, p2_, true))
+    C_(conv_any(64, 32, 0, p2_, wt_[2], params_ + boff_[2], b3_, g3_, 1, 1, err_dev_, s_, nullptr, true))
     // the decoder convolutions read [up(low), skip] where they are, here and in the weight gradients
     MarchArgs a;
+    a.early = true;
     a.act = b3_, a.act2 = e2_, a.w = wt_[3], a.bias = params_ + boff_[3], a.out = d2_, a.relu = 1;
     C_((launch_march<32, 96, MARCH_BF16, 64>(a, g2_, err_dev_, s_)))
     a.act = d2_, a.act2 = e1_, a.w = wt_[4], a.bias = params_ + boff_[4];
@@ -633,7 +637,7 @@ int UNet::train_step(float lr, double *loss)
     // layer 5: 48 -> 16 on c1 = [up(d2), e1]
     C_((launch_wgrad<16, 48, 32>(d2_, G_, dW[4], g1_, err_dev_, s_, e1_)))
     MarchArgs a;
-    a.act = G_, a.w = wtt_[4], a.out = gd2_, a.out2 = gs1_, a.sign = -1;
+    a.act = G_, a.w = wtt_[4], a.out = gd2_, a.out2 = gs1_, a.sign = -1, a.early = true;
     C_((launch_march<48, 16, MARCH_SPLIT, 0, 32>(a, g1_, err_dev_, s_)))
     k_mask_grad<32><<<rsize(n2 * (32 / 8)), 256, 0, s_>>>(gd2_, 32, 0, nullptr, g2_, d2_, G_, db[3]);
     C_(cudaGetLastError())
@@ -645,13 +649,13 @@ int UNet::train_step(float lr, double *loss)
     C_(cudaGetLastError())
     // layer 3: 32 -> 64 on pool(e2)
     C_(wgrad_any(64, 32, p2_, G_, dW[2], g3_, err_dev_, s_))
-    C_(conv_any(32, 64, 1, G_, wtt_[2], nullptr, gp2_, g3_, -1, 0, err_dev_, s_))
+    C_(conv_any(32, 64, 1, G_, wtt_[2], nullptr, gp2_, g3_, -1, 0, err_dev_, s_, nullptr, true))
     // e2: skip gradient (channels 64..95 of the concatenation) + pooled gradient from level 3
     k_mask_grad<32><<<rsize(n2 * (32 / 8)), 256, 0, s_>>>(gs2_, 32, 0, gp2_, g2_, e2_, G_, db[1]);
     C_(cudaGetLastError())
     // layer 2: 16 -> 32 on pool(e1)
     C_(wgrad_any(32, 16, p1_, G_, dW[1], g2_, err_dev_, s_))
-    C_(conv_any(16, 32, 1, G_, wtt_[1], nullptr, gp1_, g2_, -1, 0, err_dev_, s_))
+    C_(conv_any(16, 32, 1, G_, wtt_[1], nullptr, gp1_, g2_, -1, 0, err_dev_, s_, nullptr, true))
     // e1: skip gradient (channels 32..47) + pooled gradient from level 2
     k_mask_grad<16><<<rsize(n1 * (16 / 8)), 256, 0, s_>>>(gs1_, 16, 0, gp1_, g1_, e1_, G_, db[0]);
     C_(cudaGetLastError())
