@@ -233,7 +233,7 @@ def load_peaks():
 def ncu_traffic():
     """DRAM bytes per launch (read + write) from the committed ncu summary: the lines of
     its ```traffic block, 'kernel-family bytes'."""
-    path = os.path.join(ROOT, "profiles", "plane_kernels_4view_256cubed.md")
+    path = os.path.join(ROOT, "profiles", "separable_4view_256cubed.md")
     out, inside = {}, False
     if os.path.exists(path):
         for line in open(path):
@@ -599,7 +599,8 @@ def run_gb300(args, ws, rank, local):
                 "traffic": traffic, "bytes_per_launch": dbytes / max(1, dlaunch),
                 "path_achieved": path_bytes / (total_ms / 1e3) / 1e9, "kernels": kernels}
     # the whole path against the algorithmic byte model of one view-block, 28 N + 48 Pc
-    # (N block voxels, Pc = (bx / 2 + 1) by bz spectrum values), over the timed steps
+    # (N block voxels, Pc = (bx / 2 + 1) by bz spectrum values), over the timed steps; above 1 where
+    # the library's tiles transform fewer points than the caller's blocks would
     b_it = 0.0
     for v in range(W.views):
         b = W.vblocks[v]
