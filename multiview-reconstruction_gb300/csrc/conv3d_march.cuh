@@ -83,11 +83,13 @@ struct MarchAt {
 };
 
 // The copies of input planes, by 128 threads.  CU > 0: the input is the concatenation [nearest x2
-// upsampling of `act` (CU channels, a volume of half the size), act2 (C - CU channels)].
+// upsampling of `act` (CU channels, a volume of half the size), act2 (C - CU channels)].  kMarchHalf: `act`
+// holds the lower half of the channels, the others are zero (a product takes 16, the network's input has two).
+constexpr int kMarchHalf = -1;
 template <int C, int CU>
 struct MarchPlanes {
-    static constexpr int CH = C / 8, ITEMS = kMarchPlane * CH, LI = (ITEMS + 127) / 128;
-    static_assert(CU % 8 == 0 && (CU == 0 || CU < C), "concatenated channel split");
+    static constexpr int CH = CU == kMarchHalf ? C / 16 : C / 8, ITEMS = kMarchPlane * CH, LI = (ITEMS + 127) / 128;
+    static_assert(CU == kMarchHalf || (CU % 8 == 0 && CU >= 0 && CU < C), "concatenated channel split");
     const ConvGeom &g;
     const uint4 *act, *act2;
     int tid;
@@ -105,11 +107,21 @@ struct MarchPlanes {
             const int k = tid + 128 * i, h = k / CH, j = k - h * CH;
             const int xx = at.x0 - 1 + h % kMarchHX, yy = at.y0 - 1 + h / kMarchHX;
             const bool in = k < ITEMS && xx >= 0 && yy >= 0 && xx < g.W && yy < g.H;
-            if constexpr (CU == 0) off[i] = in ? ((h / kMarchHX) * g.W + h % kMarchHX) * CH + j : -1;
+            if constexpr (CU <= 0) off[i] = in ? ((h / kMarchHX) * g.W + h % kMarchHX) * CH + j : -1;
             else if (j < CU / 8)
                 off[i] = in ? ((h / kMarchHX + 1) / 2 * (g.W >> 1) + (h % kMarchHX + 1) / 2) * (CU / 8) + j : -1;
             else off[i] = in ? ((h / kMarchHX) * g.W + h % kMarchHX) * (CH - CU / 8) + j - CU / 8 : -1;
         }
+    }
+    // the K groups that are not stored, in every buffer, once
+    __device__ __forceinline__ void clear(uint8_t *planes) const
+    {
+        if constexpr (CU == kMarchHalf)
+            for (int k = tid; k < kMarchStages * CH * kMarchPlane; k += kMarchThreads) {
+                const int g8 = k / kMarchPlane, st = g8 / CH;
+                *reinterpret_cast<uint4 *>(planes + (st * 2 * CH + CH + g8 - st * CH) * kMarchLbo +
+                                           16 * (k - g8 * kMarchPlane)) = make_uint4(0, 0, 0, 0);
+            }
     }
     __device__ __forceinline__ void copy(const MarchAt &at, uint8_t *dst) const
     {
@@ -120,7 +132,7 @@ struct MarchPlanes {
         const bool zin = z >= 0 && z < g.D;
         const int zz = zin ? z : 0;
         const uint4 *lo, *hi = nullptr;
-        if constexpr (CU == 0) {
+        if constexpr (CU <= 0) {
             lo = act + corner(zz, g.D, g.H, g.W, at.y0 - 1, at.x0 - 1) * CH;
         } else {
             lo = act + corner(zz >> 1, g.D >> 1, g.H >> 1, g.W >> 1, at.y0 / 2 - 1, at.x0 / 2 - 1) * (CU / 8);
@@ -130,7 +142,7 @@ struct MarchPlanes {
         for (int i = 0; i < LI; ++i) {
             const int k = tid + 128 * i, h = k / CH, j = k - h * CH;
             const bool in = zin && off[i] >= 0;
-            const uint4 *src = CU == 0 || j < CU / 8 ? lo : hi;
+            const uint4 *src = CU <= 0 || j < CU / 8 ? lo : hi;
             if ((i + 1) * 128 <= ITEMS || k < ITEMS) cp_async16(dst + j * kMarchLbo + 16 * h, in ? src + off[i] : act, in);
         }
     }
@@ -197,6 +209,7 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
     at.start(g, u1);
     MarchPlanes<C, CU> in(g, act, act2, tid);
     in.column(ld);
+    in.clear(smem);
     auto load = [&](int s) {  // the next input plane, of step s, into its buffer
         in.copy(ld, smem + (s % ST) * PB);
         if (ld.next(g, u1)) in.column(ld);
@@ -430,6 +443,7 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
     at.start(g, u1);
     MarchPlanes<C, CU> in(g, X, X2, tid);
     in.column(ld);
+    in.clear(smem);
     int lring = 0;  // output planes of the parts before: plane j of a part is in slot (ring + j) % RG
     auto load = [&](int s) {  // the next plane of X, of step s, and of G
         in.copy(ld, smem + (s % ST) * PB);
