@@ -395,15 +395,17 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
 // it, so there a non-finite X reaches the gradient of the outward offsets as well.
 constexpr int kWgRing = 8;  // planes of G: three being multiplied, the others on their way
 constexpr int kWgGroup = 128 * 16 + 16;  // stride of G's channel groups (padding: distinct banks)
-template <int N>
-__host__ __device__ constexpr int wgrad_offsets()  // offsets (dy, dx) of one CTA
+// Up to 16 channels the 64 rows of a product are eight x shifts of one channel group, 16 bytes apart, of which
+// the first three are dx = -1, 0, 1: a product per (dy, channel group) instead of one per (dy, dx).
+template <int C, int CU>
+__host__ __device__ constexpr int wgrad_units()  // products of one K step
 {
-    return 512 / (3 * N) < 9 ? 512 / (3 * N) : 9;
+    return C > 16 ? 9 : 3 * (CU == kMarchHalf ? C / 16 : C / 8);
 }
-template <int N>
-__host__ __device__ constexpr int wgrad_splits()
+template <int N, int C, int CU>
+__host__ __device__ constexpr int wgrad_splits()  // CTAs that share them: 512 columns hold 512 / (3 N)
 {
-    return (9 + wgrad_offsets<N>() - 1) / wgrad_offsets<N>();
+    return (wgrad_units<C, CU>() + 512 / (3 * N) - 1) / (512 / (3 * N));
 }
 template <int N, int C>
 __host__ __device__ constexpr size_t wgrad_march_smem()
@@ -419,6 +421,8 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
 {
     constexpr int ST = kMarchStages, RG = kWgRing, CH = C / 8, PB = CH * kMarchLbo, GB = (N / 8) * kWgGroup;
     constexpr int M = C <= 64 ? 64 : 128;
+    constexpr bool XS = C <= 16;  // x shifts in the rows
+    constexpr int NU = wgrad_units<C, CU>(), NJ = XS ? NU / 3 : 1;
     static_assert(C <= 128 && N % 16 == 0 && 3 * N <= 256, "tile shape");
     // A's rows beyond C end inside the ring of G
     static_assert((M / 8 - CH) * kMarchLbo <= RG * GB, "rows beyond C stay in shared memory");
@@ -436,14 +440,13 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
     const long long planes =
         (long long)((g.W + kMarchX - 1) / kMarchX) * ((g.H + kMarchY - 1) / kMarchY) * g.B * g.D;
     const long long u1 = planes * (blockIdx.x + 1) / gridDim.x;
-    const int t0 = 9 * blockIdx.y / gridDim.y, t1 = 9 * (blockIdx.y + 1) / gridDim.y;
+    const int t0 = NU * blockIdx.y / gridDim.y, t1 = NU * (blockIdx.y + 1) / gridDim.y;
     MarchAt ld, at;
     ld.u = at.u = planes * blockIdx.x / gridDim.x;
     ld.start(g, u1);
     at.start(g, u1);
     MarchPlanes<C, CU> in(g, X, X2, tid);
     in.column(ld);
-    in.clear(smem);
     int lring = 0;  // output planes of the parts before: plane j of a part is in slot (ring + j) % RG
     auto load = [&](int s) {  // the next plane of X, of step s, and of G
         in.copy(ld, smem + (s % ST) * PB);
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
         const int i0 = max(0, 2 - at.p), i1 = min(3, at.nz + 2 - at.p);
         const int s0 = (ring + at.p - 2 + i0) % RG;
         const int n0 = min(i1 - i0, RG - s0), n1 = i1 - i0 - n0;  // planes up to the ring's end, and from its start
-        const uint64_t a0 = tc::smem_desc(xbase + (uint32_t)(s % ST) * PB, kMarchHX * 16, kMarchLbo);
+        const uint64_t a0 = tc::smem_desc(xbase + (uint32_t)(s % ST) * PB, kMarchHX * 16, XS ? 16 : kMarchLbo);
         const uint64_t b0 = tc::smem_desc(gbase, 128, kWgGroup);
 #pragma unroll 1
         for (int seg = 0; seg < (n1 > 0 ? 2 : 1); ++seg) {
@@ -494,7 +497,7 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
             uint32_t d = tmem + (uint32_t)(i * N);
 #pragma unroll 1
             for (int t = t0; t < t1; ++t, d += 3 * N) {
-                const uint64_t as = a0 + (uint32_t)(t % 3 + kMarchHX * (t / 3));
+                const uint64_t as = a0 + (uint32_t)(XS ? kMarchHX * (t / NJ) + t % NJ * (kMarchLbo / 16) : t % 3 + kMarchHX * (t / 3));
 #pragma unroll
                 for (int k = 0; k < 8; ++k) tc::mma_bf16_acc(d, as + 2 * kMarchHX * k, bs + 16 * k, id);
             }
@@ -535,13 +538,14 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
             for (int q = max(0, s - ST); q < s; ++q) tc::mbar_wait(&done[q % ST], (q / ST) & 1, kTcWaitIter);
         }
     } else if (warp < 4) {
-        // row ci is lane ci, of 64 rows lanes 0..15 of each warp; every CTA starts at an offset of its own
-        const int ci = M == 64 ? 16 * warp + lane : 32 * warp + lane;
-        const bool rv = ci < C && (M == 128 || lane < 16);
+        // row r is lane r, of 64 rows lanes 0..15 of each warp; every CTA starts at an offset of its own
+        const int r = M == 64 ? 16 * warp + lane : 32 * warp + lane;
+        const bool rv = r < (XS ? 24 : C) && (M == 128 || lane < 16);
         const int nt = t1 - t0;
 #pragma unroll 1
         for (int q = 0; q < nt * 3; ++q) {
             const int e = (q + (int)blockIdx.x) % (nt * 3), t = t0 + e / 3, tz = 2 - e % 3;
+            const int ci = XS ? 8 * (t % NJ) + r % 8 : r, tap = 9 * tz + (XS ? 3 * (t / NJ) + r / 8 : t);
 #pragma unroll
             for (int c0 = 0; c0 < N; c0 += 16) {
                 float v[16];
@@ -549,7 +553,7 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
                 if (rv)
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        atomicAdd(&dW[((long long)(c0 + j) * 27 + 9 * tz + t) * C + ci], v[j]);
+                        atomicAdd(&dW[((long long)(c0 + j) * 27 + tap) * C + ci], v[j]);
             }
         }
     }

@@ -87,7 +87,7 @@ cudaError_t launch_wgrad(const bf16 *X, const bf16 *G, float *dW, const ConvGeom
     if (e != cudaSuccess) return e;
     const long long planes =
         (long long)((g.W + kMarchX - 1) / kMarchX) * ((g.H + kMarchY - 1) / kMarchY) * g.B * g.D;
-    constexpr int NG = wgrad_splits<N>();
+    constexpr int NG = wgrad_splits<N, C, CU>();
     const long long grid = std::min<long long>(152 / NG, (planes + kMarchMin - 1) / kMarchMin);
     k_wgrad_march<N, C, CU><<<dim3((unsigned)grid, NG), kMarchThreads, sm, s>>>(X, G, dW, g, err, X2);
     return cudaGetLastError();
