@@ -390,13 +390,13 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
 //
 // What bounds it: the operands' way out of shared memory, 2 KB of A (64 rows; 4 KB for more than 64
 // channels) and 1.5 KB of B per product.  48 x 16 channels on
-// 4 x 64^3 voxels: 97 us (0.85 ms with 27 copies of X out of L2, one per offset), 16 x 16: 94 us (0.30),
-// 96 x 32 on 4 x 32^3: 42 us (0.25).  A column's ragged edge multiplies G's zeros with the X beside
+// 4 x 64^3 voxels: 97 us (0.85 ms with 27 copies of X out of L2, one per offset), 16 x 16, 8 of them stored: 34 us
+// (0.30), 96 x 32 on 4 x 32^3: 42 us (0.25), 16 x 32: 21 us (0.048).  A column's ragged edge multiplies G's zeros with the X beside
 // it, so there a non-finite X reaches the gradient of the outward offsets as well.
 constexpr int kWgRing = 8;  // planes of G: three being multiplied, the others on their way
 constexpr int kWgGroup = 128 * 16 + 16;  // stride of G's channel groups (padding: distinct banks)
 // Up to 16 channels the 64 rows of a product are eight x shifts of one channel group, 16 bytes apart, of which
-// the first three are dx = -1, 0, 1: a product per (dy, channel group) instead of one per (dy, dx).
+// the first three are dx = -1, 0, 1: a product per (dy, channel group) instead of one per (dy, dx) (16 x 16: 95 -> 44 us).
 template <int C, int CU>
 __host__ __device__ constexpr int wgrad_units()  // products of one K step
 {
@@ -406,6 +406,13 @@ template <int N, int C, int CU>
 __host__ __device__ constexpr int wgrad_splits()  // CTAs that share them: 512 columns hold 512 / (3 N)
 {
     return (wgrad_units<C, CU>() + 512 / (3 * N) - 1) / (512 / (3 * N));
+}
+// tensor-memory columns of a CTA (a power of two); with few of them two CTAs share an SM (16 x 16: 44 -> 34 us)
+template <int N, int C, int CU>
+__host__ __device__ constexpr int wgrad_cols()
+{
+    constexpr int S = wgrad_splits<N, C, CU>(), n = (wgrad_units<C, CU>() + S - 1) / S * 3 * N;
+    return n <= 128 ? 128 : (n <= 256 ? 256 : 512);
 }
 template <int N, int C>
 __host__ __device__ constexpr size_t wgrad_march_smem()
@@ -422,6 +429,7 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
     constexpr int ST = kMarchStages, RG = kWgRing, CH = C / 8, PB = CH * kMarchLbo, GB = (N / 8) * kWgGroup;
     constexpr int M = C <= 64 ? 64 : 128;
     constexpr bool XS = C <= 16;  // x shifts in the rows
+    constexpr uint32_t COLS = wgrad_cols<N, C, CU>();
     constexpr int NU = wgrad_units<C, CU>(), NJ = XS ? NU / 3 : 1;
     static_assert(C <= 128 && N % 16 == 0 && 3 * N <= 256, "tile shape");
     // A's rows beyond C end inside the ring of G
@@ -432,7 +440,7 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
     __shared__ __align__(8) uint64_t done[ST];
     __shared__ uint32_t tbase;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    if (warp == 0) tc::tmem_alloc(&tbase, 512);
+    if (warp == 0) tc::tmem_alloc(&tbase, COLS);
     if (tid == 0) {
         for (int i = 0; i < ST; ++i) tc::mbar_init(&done[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -559,7 +567,7 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, 512);
+    if (warp == 0) tc::tmem_dealloc(tmem, COLS);
 }
 
 }  // namespace mvr

@@ -74,7 +74,7 @@ cudaError_t launch_march(const MarchArgs &a, const ConvGeom &g, int *err, cudaSt
                       a.act, a.w, a.bias, a.out, g, a.sign, a.relu, err, a.act2, a.out2, a.wh, a.bh);
 }
 
-// Weight gradient (k_wgrad_march): runs as in launch_march, one CTA per SM (it holds all tensor memory)
+// Weight gradient (k_wgrad_march): runs as in launch_march, as many CTAs per SM as share its tensor memory
 template <int N, int C, int CU = 0>
 cudaError_t launch_wgrad(const bf16 *X, const bf16 *G, float *dW, const ConvGeom &g, int *err, cudaStream_t s,
                          const bf16 *X2 = nullptr)
@@ -88,7 +88,8 @@ cudaError_t launch_wgrad(const bf16 *X, const bf16 *G, float *dW, const ConvGeom
     const long long planes =
         (long long)((g.W + kMarchX - 1) / kMarchX) * ((g.H + kMarchY - 1) / kMarchY) * g.B * g.D;
     constexpr int NG = wgrad_splits<N, C, CU>();
-    const long long grid = std::min<long long>(152 / NG, (planes + kMarchMin - 1) / kMarchMin);
+    const long long res = std::max<long long>(1, std::min<long long>((227 * 1024) / (sm + 1024), 512 / wgrad_cols<N, C, CU>()));
+    const long long grid = std::min<long long>(152 * res / NG, (planes + kMarchMin - 1) / kMarchMin);
     k_wgrad_march<N, C, CU><<<dim3((unsigned)grid, NG), kMarchThreads, sm, s>>>(X, G, dW, g, err, X2);
     return cudaGetLastError();
 }
