@@ -63,11 +63,6 @@ __device__ __forceinline__ FPair fp_add(FPair a, FPair b)
     const FPair s = fp_sum(a.h, b.h);
     return fp_quick(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
 }
-__device__ __forceinline__ FPair fp_add(FPair a, float b)
-{
-    const FPair s = fp_sum(a.h, b);
-    return fp_quick(s.h, __fadd_rn(s.l, a.l));
-}
 __device__ __forceinline__ FPair fp_mul(FPair a, float b)
 {
     const float p = __fmul_rn(a.h, b);
