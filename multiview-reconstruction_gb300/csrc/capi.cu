@@ -312,6 +312,7 @@ extern "C" int mvr_block_run_mul(mvr_block *h, float *psi, const float *const *i
         if (!imgs[v] || !ws[v]) return h->fail(MVR_ERR_ARG, "block pointers must not be NULL");
         if (!h->kernels_set(v)) return h->fail(MVR_ERR_STATE, "mvr_block_set_kernels was not called for every view");
     }
+    BLK_CUDA(h, cudaSetDevice(h->eng.device()));
     bool sep = true;
     for (int v = 0; v < h->nviews; ++v) sep = sep && h->seps[v].ready();
     if (!sep)
@@ -324,7 +325,6 @@ extern "C" int mvr_block_run_mul(mvr_block *h, float *psi, const float *const *i
             }
             pls.push_back(&h->plans[v]);
         }
-    BLK_CUDA(h, cudaSetDevice(h->eng.device()));
     cudaStream_t s = h->eng.stream();
     const size_t bytes = sizeof(float) * (size_t)h->nvox;
     const int dev = h->eng.device();

@@ -84,6 +84,7 @@ int Engine<T>::cuda_check(cudaError_t e, const char *what)
 {
     if (e == cudaSuccess) return OK;
     err_ = std::string(what) + ": " + cudaGetErrorString(e);
+    cudaGetLastError();  // reported here: the launch checks of a later call start clean
     return e == cudaErrorMemoryAllocation ? ERR_OOM : ERR_CUDA;
 }
 
@@ -185,7 +186,7 @@ int Engine<T>::cuda_check(cudaError_t e, const char *what)
 
 namespace {
 template <typename V>
-V *dev_twiddles_impl(int n, cudaStream_t s, std::string &err)
+V *dev_twiddles_impl(int n, cudaStream_t s, cudaError_t &e)
 {
     typedef typename Re<V>::t T;
     std::vector<V> h(n);
@@ -196,12 +197,14 @@ V *dev_twiddles_impl(int n, cudaStream_t s, std::string &err)
         h[k].y = (T)std::sin(a);
     }
     V *d = nullptr;
-    cudaError_t e = cudaMalloc(&d, sizeof(V) * (size_t)n);
-    if (e != cudaSuccess) { err = cudaGetErrorString(e); return nullptr; }
+    if (e != cudaSuccess) return nullptr;  // of the table before
+    e = cudaMalloc(&d, sizeof(V) * (size_t)n);
+    if (e != cudaSuccess) return nullptr;
     e = cudaMemcpyAsync(d, h.data(), sizeof(V) * (size_t)n, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) { err = cudaGetErrorString(e); cudaFree(d); return nullptr; }
-    return d;
+    if (e == cudaSuccess) return d;
+    cudaFree(d);
+    return nullptr;
 }
 
 template <typename T, bool B>
@@ -501,6 +504,15 @@ int Engine<T>::make_plan(Plan<T> &pl, const int b[3], const float *k1, const int
             return fail(ERR_ARG, "kernel larger than the block under circular boundary");
     }
     free_plan(pl);
+    const int rc = fill_plan(pl, b, k1, kd1, k2, k_on_device, boundary);
+    if (rc != OK) free_plan(pl);  // a plan with k1h has its spectra
+    return rc;
+}
+
+template <typename T>
+int Engine<T>::fill_plan(Plan<T> &pl, const int b[3], const float *k1, const int kd1[3], const float *k2,
+                         bool k_on_device, int boundary)
+{
     for (int d = 0; d < 3; ++d) {
         pl.b[d] = b[d];
         pl.kd[d] = kd1[d];
@@ -525,11 +537,11 @@ int Engine<T>::make_plan(Plan<T> &pl, const int b[3], const float *k1, const int
     for (const FftDesc *dd : {&pl.dx, &pl.dy, &pl.dz})
         for (int st = 0; st < dd->ns; ++st)
             if (dd->radix[st] == 7 || dd->radix[st] == 11 || dd->radix[st] == 13) pl.big = true;
-    std::string e;
+    cudaError_t e = cudaSuccess;
     pl.twx = dev_twiddles_impl<V>(pl.P[0], stream_, e);
     pl.twy = dev_twiddles_impl<V>(pl.P[1], stream_, e);
     pl.twz = dev_twiddles_impl<V>(pl.P[2], stream_, e);
-    if (!pl.twx || !pl.twy || !pl.twz) return fail(ERR_CUDA, "twiddle upload: " + e);
+    MVR_TRY(cuda_check(e, "twiddle upload"));
     // launch shapes
     const int m = pl.P[0] / 2;
     const size_t per_row = 2 * sizeof(V) * (size_t)(m + 1);
@@ -1338,15 +1350,27 @@ int Engine<T>::sep_make(SepPlan &pl, const int P[3], const float *k1, const floa
     } else {
         if (stream_ == nullptr) return fail(ERR_STATE, "engine not initialised");
         sep_free(pl);
+        const int rc = sep_fill(pl, P, k1, k2, kd, on_device);
+        if (rc != OK) sep_free(pl);  // a plan with k2h has its spectra
+        return rc;
+    }
+}
+
+template <typename T>
+int Engine<T>::sep_fill(SepPlan &pl, const int P[3], const float *k1, const float *k2, const int kd[3], bool on_device)
+{
+    if constexpr (sizeof(T) != sizeof(float)) {
+        return ERR_STATE;
+    } else {
         for (int d = 0; d < 3; ++d) {
             pl.P[d] = P[d];
             pl.kd[d] = kd[d];
         }
-        std::string e;
+        cudaError_t e = cudaSuccess;
         pl.twx = dev_twiddles_impl<float2>(P[0], stream_, e);
         pl.twy = dev_twiddles_impl<float2>(P[1], stream_, e);
         pl.twz = dev_twiddles_impl<float2>(P[2], stream_, e);
-        if (!pl.twx || !pl.twy || !pl.twz) return fail(ERR_CUDA, "twiddle upload: " + e);
+        MVR_TRY(cuda_check(e, "twiddle upload"));
         const long long kn = (long long)kd[0] * kd[1] * kd[2];
         if (!on_device && kn > kcap_) {
             cudaFree(kbuf_);

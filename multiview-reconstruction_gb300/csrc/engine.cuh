@@ -217,6 +217,9 @@ private:
     int launch_update(const Plan<T> &pl, const BlockMaps &bms, int nb, V *S, const UpdateArgs &ua, int epi,
                       double bytes, double *stats_dev);
     BlockMaps block_maps(const Plan<T> &pl, const BlockPlace *bps, int nb) const;
+    int fill_plan(Plan<T> &pl, const int b[3], const float *k1, const int kd1[3], const float *k2, bool k_on_device,
+                  int boundary);
+    int sep_fill(SepPlan &pl, const int P[3], const float *k1, const float *k2, const int kd[3], bool on_device);
     // y forward, z (times K), y inverse of a tile batch, the column blocks in slabs on two streams when
     // the spectra outgrow L2; first: the passes ended in a join of the streams
     int sep_yzy(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, int nt, int map, int out_w, const float2 *K,

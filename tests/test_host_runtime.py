@@ -1,0 +1,89 @@
+"""The library's host code on a stand-in for the CUDA runtime (fake_cudart.c): devices that the calling
+thread is not on, and calls that fail.  No kernel runs; what is checked is which device memory is
+allocated on, whether launches are accepted, and that a call after a failed one starts over."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+import build_lib
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+PRELUDE = """
+import ctypes as C, numpy as np, sys
+sys.path[:0] = [{pkg!r}]
+import mvrgb300 as M
+F = C.CDLL({fake!r})
+F.fake_live.restype = F.fake_launches.restype = C.c_longlong
+F.fake_fail.argtypes = [C.c_int, C.c_longlong]
+MALLOC, LAUNCH = 0, 1
+K = lambda n: np.ones(n[::-1], np.float32) / np.prod(n)
+A = lambda b, n=None: np.ones(b[::-1], np.float32) if n is None else [np.ones(b[::-1], np.float32) for _ in range(n)]
+"""
+
+
+@pytest.fixture(scope="session")
+def fake(tmp_path_factory):
+    build_lib.build()
+    so = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    inc = os.path.join(os.path.dirname(os.path.dirname(build_lib._nvcc())), "include")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", f"-I{inc}", "-o", so, os.path.join(HERE, "fake_cudart.c")], check=True)
+    return so
+
+
+def run(fake, body, devices=2, **env):
+    pre = PRELUDE.format(pkg=build_lib.HERE, fake=fake)
+    e = {k: v for k, v in os.environ.items() if not k.startswith("MVR_")}
+    r = subprocess.run([sys.executable, "-c", pre + body], capture_output=True, text=True, timeout=120,
+                       env=dict(e, LD_PRELOAD=fake, FAKE_DEVICES=str(devices), **env))
+    assert r.returncode == 0, r.stderr[-2000:]
+    return r.stdout
+
+
+# a Mul block with one view off the separable transforms: its plan and the other view's are block plans
+MIXED = """
+b = (40, 8, 24)
+def make():
+    w = M.BlockWorker(b, num_views=2, device=1)
+    for v, k in enumerate(((5, 5, 5), (5, 21, 5))):
+        w.set_kernels(v, K(k), K(k))
+    return w
+def step(w):
+    n = F.fake_launches()
+    w.run_iteration_mul(A(b), A(b, 2), A(b, 2), [1.0, 1.0])
+    return F.fake_launches() - n
+"""
+
+
+def test_mixed_mul_block_on_another_device_than_the_threads(fake):
+    run(fake, MIXED + """
+w = make()
+assert F.cudaSetDevice(0) == 0
+n0 = F.fake_live(0)
+step(w)
+assert F.fake_live(0) == n0, "memory of device 0"
+""")
+
+
+@pytest.mark.parametrize("kind", ["MALLOC", "LAUNCH"])
+def test_mixed_mul_block_after_a_plan_that_failed(fake, kind):
+    # whichever allocation (three tables, two spectra; then the step's own) or launch of the plan fails,
+    # the next call makes it anew
+    run(fake, MIXED + f"""
+w = make()
+first, later = step(w), step(w)
+assert first > later  # the first made the plan
+failed = 0
+for i in range(12 if {kind} == MALLOC else first - later):
+    w = make()
+    F.fake_fail({kind}, i)
+    try:
+        step(w)
+        F.fake_fail({kind}, -1)
+        continue  # fewer allocations than that
+    except M.MvrError:
+        failed += 1
+    assert (step(w), step(w)) == (later if {kind} == MALLOC and i >= 5 else first, later), i
+assert failed >= 4
+""")
