@@ -1,5 +1,6 @@
 // Host side of the block iteration (see engine.cuh).
 #include "engine.cuh"
+#include "per_device.h"
 #include "rows_warp.cuh"
 #include "cols_warp.cuh"
 #include "cols_tile.cuh"
@@ -11,7 +12,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 
 namespace mvr {
 
@@ -275,8 +275,8 @@ template <typename T>
 void set_smem_limits()
 {
     // allow every instantiation to use up to the opt-in maximum; launches size it exactly
-    static std::once_flag once;
-    std::call_once(once, [] {
+    static PerDevice once;
+    once([] {
         const int m = (int)kSmemMax;
         set_smem_limits_big<T, false>(m);
         set_smem_limits_big<T, true>(m);
@@ -292,6 +292,7 @@ void set_smem_limits()
         set_smem_limits_tcols<12>(m);
         set_smem_limits_tcols<16>(m);
         set_smem_limits_tcols<18>(m);
+        return cudaSuccess;
     });
 }
 

@@ -15,6 +15,7 @@
 // algorithmic bytes: forward 38 us (3.8 TB/s), quotient 54 us (4.1 TB/s), update 60 us (4.6 TB/s).
 #pragma once
 #include "pdl.cuh"
+#include "per_device.h"
 #include "rows_warp.cuh"
 #include "sep.cuh"
 #include "sep_dft.cuh"
@@ -584,8 +585,8 @@ struct Sx {
     }
     static cudaError_t ready()
     {
-        static const cudaError_t e = limits();
-        return e;
+        static PerDevice once;
+        return once(limits);
     }
     static cudaError_t fwd(const SepGeom &g, const SepTiles &tl, int nt, int ctas, const SepSrc &src, float2 *S, int vec,
                            const float2 *tw, cudaStream_t s)

@@ -14,6 +14,7 @@
 // columns) and, in the z pass, by the load latency of the data and K^ (4.9 TB/s on 320).
 #pragma once
 #include "pdl.cuh"
+#include "per_device.h"
 #include "sep.cuh"
 #include "sep_dft.cuh"
 
@@ -362,8 +363,8 @@ struct Yz {
     }
     static cudaError_t ready()
     {
-        static const cudaError_t e = limits();
-        return e;
+        static PerDevice once;
+        return once(limits);
     }
     static cudaError_t y_fwd(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int map, int kdy, int kdz, float2 *S,
                              const float2 *tw, cudaStream_t s, int planes)

@@ -1,11 +1,11 @@
 // Launchers of the plane kernels (see xy_plane.cuh).
+#include "per_device.h"
 #include "xy.cuh"
 #include "xy_pair.cuh"
 #include "xy_plane.cuh"
 
 #include <algorithm>
 #include <cstdlib>
-#include <mutex>
 
 namespace mvr {
 
@@ -162,14 +162,15 @@ int pair_clusters()
 
 void set_limits()
 {
-    static std::once_flag once;
-    std::call_once(once, [] {
+    static PerDevice once;
+    once([] {
         set_limits_pair<6, 6>();
         set_limits_pair<8, 8>();
         set_limits_one<4, 8>();
         set_limits_one<4, 12>();
         set_limits_one<6, 8>();
         set_limits_one<6, 12>();
+        return cudaSuccess;
     });
 }
 

@@ -87,3 +87,19 @@ for i in range(12 if {kind} == MALLOC else first - later):
     assert (step(w), step(w)) == (later if {kind} == MALLOC and i >= 5 else first, later), i
 assert failed >= 4
 """)
+
+
+# kernels with more than 48 KB of shared memory: y and z lengths from 360 and x length 576 of the separable
+# transforms, the plane and pair kernels, the row / column kernels
+@pytest.mark.parametrize("block,env", [
+    ((572, 356, 476), {}), ((316, 60, 356), {}), ((188, 188, 60), {"MVR_PLANE_KERNELS": "1"}),
+    ((252, 252, 60), {"MVR_PAIR_KERNELS": "1"}), ((236, 500, 404), {"MVR_PLANE_KERNELS": "0"}),
+])
+def test_every_device_gets_the_shared_memory_of_the_kernels(fake, block, env):
+    run(fake, f"""
+b = {block}
+for dev in (0, 1):
+    w = M.BlockWorker(b, device=dev)
+    w.set_kernels(0, K((5, 5, 5)), K((5, 5, 5)))
+    w.run_iteration(0, A(b), A(b), A(b), 1.0)
+""", **env)
