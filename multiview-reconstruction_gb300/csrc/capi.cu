@@ -215,8 +215,11 @@ extern "C" int mvr_block_set_kernels(mvr_block *h, int view, const float *k1, co
     // plane kernels, 256^3 304 / 467 us, 156 x 156 x 124 with the reference's extensions (domains
     // without plane kernels) 70 / 320 us, 40 x 36 x 44 20 / 34 us
     int P[3];
-    if (!mvr::block_kernels_forced() && mvr::block_tile(h->b, ks, h->eng.boundary(), P, h->tiles[view]))
-        return h->from_engine(h->eng.sep_make(h->seps[view], P, k1, k2, ks, false));
+    if (!mvr::block_kernels_forced() && mvr::block_tile(h->b, ks, h->eng.boundary(), P, h->tiles[view])) {
+        const int rc = h->eng.sep_make(h->seps[view], P, k1, k2, ks, false);
+        if (rc != mvr::ERR_OOM) return h->from_engine(rc);
+        h->eng.drop_scratch();  // no room for that domain: the block plan's is smaller
+    }
     return h->from_engine(h->eng.make_plan(h->plans[view], h->b, k1, ks, k2, ks));
 }
 

@@ -1058,8 +1058,8 @@ int Decon<T>::make_tiles()
         if (!jacobi_[st]) continue;
         const int rc = make_step_tiles(st);
         if (rc == MVR_ERR_OOM) {  // no room for the tiles' spectra: this step stays on its blocks
-            cudaGetLastError();
             for (int v = p_.mul ? 0 : st; v < (p_.mul ? p_.num_views : st + 1); ++v) free_tiles(views_[v]);
+            engine_.drop_scratch();
             continue;
         }
         D_TRY(rc);

@@ -423,6 +423,16 @@ int Engine<T>::reserve(long long Pc, long long nvox_block, long long rows, int n
 }
 
 template <typename T>
+void Engine<T>::drop_scratch()
+{
+    cudaFree(S0_);
+    cudaFree(S1_);
+    S0_ = S1_ = nullptr;
+    Scap_ = 0;
+    ++alloc_epoch_;
+}
+
+template <typename T>
 int Engine<T>::reserve_prod(long long n)
 {
     if (n > prodcap_) {

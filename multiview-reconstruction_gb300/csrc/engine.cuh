@@ -152,6 +152,7 @@ public:
     // Tiles per launch for a domain, and the scratch a launch of nt tiles takes (allocated here).
     int sep_batch(const int P[3]) const;
     int sep_reserve(const int P[3], int nt, bool mul, long long voxels, long long rows);
+    void drop_scratch();  // the spectra buffers given back (reserved again by what needs them)
     // The FFT schedules a plan admits (codes SCHED_*), and the one in use.
     int kernel_spectra(Plan<T> &pl, const float *k1, const float *k2, bool k_on_device);
     std::vector<int> schedule_candidates(const Plan<T> &pl) const;

@@ -103,3 +103,53 @@ for dev in (0, 1):
     w.set_kernels(0, K((5, 5, 5)), K((5, 5, 5)))
     w.run_iteration(0, A(b), A(b), A(b), 1.0)
 """, **env)
+
+
+def test_block_without_room_for_the_separable_transforms(fake):
+    # each of the first allocations fails in turn: the block's kernels are taken all the same (a block plan,
+    # whose domain is the smaller one), with the bytes that a block plan alone would hold
+    run(fake, """
+import os
+b, k = (33, 33, 33), (5, 5, 5)
+def live(fail):
+    w = M.BlockWorker(b, device=1)
+    n0 = F.fake_live(1)
+    F.fake_fail(MALLOC, fail)
+    w.set_kernels(0, K(k), K(k))
+    F.fake_fail(MALLOC, -1)
+    n1 = F.fake_live(1) - n0
+    w.run_iteration(0, A(b), A(b), A(b), 1.0)
+    return n1
+sep = live(-1)
+os.environ["MVR_RATIO_BAND"] = "0"
+plan = live(-1)
+del os.environ["MVR_RATIO_BAND"]
+assert plan < sep
+assert [live(i) for i in (0, 2, 3, 4, 6, 7, 8)] == [plan] * 7
+""")
+
+
+def test_volume_without_room_for_the_tiles(fake):
+    # as above for the tiles of a volume: prepare succeeds, the step stays on its blocks
+    run(fake, """
+D, b, k = (40, 36, 24), (48, 40, 32), (5, 5, 5)
+def prepare(fail, n):
+    with M.Deconvolution(D, n, b, psf_type=M.PSF_INDEPENDENT, filter_blocks=False, device=1) as d:
+        for v in range(n):
+            d.set_view(v, A(D), A(D), K(k))
+        F.fake_fail(MALLOC, fail)
+        try:
+            d.prepare()
+        except M.MvrError:
+            return None
+        finally:
+            F.fake_fail(MALLOC, -1)
+        n0 = F.fake_launches()
+        d.run_iterations(1)
+        return F.fake_launches() - n0
+tiles, n = prepare(-1, 1), 0
+while prepare(n, 1) is None:  # allocations of the block plans
+    n += 1
+rest = [prepare(i, 1) for i in range(n, n + 6)]  # three tables, two spectra; none
+assert len(set(rest[:5])) == 1 and rest[0] not in (None, tiles) and rest[5] == tiles, (tiles, n, rest)
+""")
