@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Z)
         const unsigned k0 = at + T * u * pitch;
         const unsigned long long pol = sep_policy(g.stream);
 #pragma unroll
-        for (int k2 = 0; k2 < T; ++k2) kv[k2] = live ? sep_ld2(kp + (k0 + k2 * pitch), pol) : make_float2(0.0f, 0.0f);
+        for (int k2 = 0; k2 < T; ++k2) kv[k2] = live ? sep_ldk(kp + (k0 + k2 * pitch), pol) : make_float2(0.0f, 0.0f);
     }
     __syncthreads();
     if (u < V) {
