@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -100,6 +102,7 @@ struct FuseView {
     int fblend, dblend;
     int adjust;        // intensity adjustment v -> v m00 + m01 (rounded once to float)
     FPair m00, m01;
+    double m[2];       // the same in double
 };
 
 struct FuseViews {
@@ -162,15 +165,67 @@ __device__ __forceinline__ void fp_gather(FPair &s, float x)
     s.l = __fadd_rn(s.l, t.l);
 }
 
+// One voxel with positions, interpolation and sums in double: for the voxels where a sample or a sum left
+// the range of a float (samples that are infinite or not a number among them: the residuals of the
+// pairs would turn an infinity into NaN).  In a kernel of its own behind k_fuse_group, which marks them:
+// 14 us of 551 (3 views, 256^3); as a call in that kernel 16 registers and 19 us.
+__device__ __forceinline__ void fuse_voxel(const FuseViews &fv, double s0, double s1, double s2, float &image, float &weight)
+{
+    const double s[3] = {s0, s1, s2};
+    double sumI = 0.0, sumW = 0.0, sumD = 0.0;
+    for (int k = 0; k < fv.n; ++k) {
+        const FuseView &v = fv.v[k];
+        double t[3], w[3];
+        apply_affine(v.inv, s, t);
+        long long at = 0;
+        bool in = true;
+        float dw = INFINITY, dd = INFINITY, wf = 1.0f, wd = 1.0f;
+        for (int d = 2; d >= 0; --d) {
+            const float tf = (float)t[d], l2 = __fsub_rn(v.top[d], tf);
+            if (v.fblend) dw = fminf(dw, blend_distance(tf, l2, v.fb[d]));
+            if (v.dblend) dd = fminf(dd, blend_distance(tf, l2, v.db[d]));
+            const double fl = floor(t[d]);
+            w[d] = __dsub_rn(t[d], fl);
+            in = in && t[d] > 0.0 && t[d] < v.dims[d] - 1;
+            at = at * v.dims[d] + (in ? (long long)fl : 0);
+        }
+        if (!(dw > 0.0f)) wf = 0.0f;
+        if (!(dd > 0.0f)) wd = 0.0f;
+        for (int d = 0; d < 3; ++d) {
+            const float tf = (float)t[d], l2 = __fsub_rn(v.top[d], tf);
+            if (wf != 0.0f && v.fblend) wf = blend_factor(wf, blend_distance(tf, l2, v.fb[d]), v.fr[d], v.fri[d]);
+            if (wd != 0.0f && v.dblend) wd = blend_factor(wd, blend_distance(tf, l2, v.db[d]), v.dr[d], v.dri[d]);
+        }
+        sumD += (double)wd;
+        if (wf == 0.0f) continue;
+        float val = 0.0f;  // outsideValueImg
+        if (in) {
+            const float *p = v.img + at;
+            const long long sy = v.dims[0], sz = (long long)v.dims[0] * v.dims[1];
+            val = fmaxf(1.0f, nlinear3(w, [&](int dx, int dy, int dz) {  // minValueImg
+                const float x = __ldg(p + dz * sz + dy * sy + dx);
+                return v.adjust ? __double2float_rn(__dadd_rn(__dmul_rn((double)x, v.m[0]), v.m[1])) : x;
+            }));
+        }
+        sumI += (double)val * (double)wf;
+        sumW += (double)wf;
+    }
+    image = sumW > 0.0 ? (float)(sumI / sumW) : 0.0f;
+    weight = (float)sumD;
+}
+// The last call that left voxels to k_fuse_wide, by its number (calls run on any stream).
+constexpr int kWideCalls = 1024;
+__device__ unsigned long long d_wide[kWideCalls];
+
 // A CTA takes kFuseRows rows of the box: the part of t that is constant along a row is formed in
 // double, once per row, view and axis (apply_affine at the row's first voxel), and t = base + x
 // step on pairs of floats per voxel.  Bound by instruction issue (82 % of the issue slots): 3 views
-// with blending into a 256^3 box 0.50 ms, 12.9 ms in double; 2 or 4 voxels of a thread at a time
-// (a view's constants fetched once for them) 0.54 and 0.94 ms: the branches of the border zones
+// with blending into a 256^3 box 0.54 ms, 13.1 ms in double; 2 or 4 voxels of a thread at a time
+// (a view's constants fetched once for them) 0.58 and 0.98 ms: the branches of the border zones
 // keep them from overlapping.
 __global__ void __launch_bounds__(kFuseThreads)
     k_fuse_group(const __grid_constant__ FuseViews fv, long long bx, long long by, long long bz, int nx, int ny, int nz,
-                 float *__restrict__ out_img, float *__restrict__ out_w)
+                 float *__restrict__ out_img, float *__restrict__ out_w, unsigned long long call)
 {
     __shared__ FPair base[kFuseRows][kFuseMaxViews][3];
     const int y0 = blockIdx.x * kFuseRows, z = blockIdx.y;
@@ -189,6 +244,7 @@ __global__ void __launch_bounds__(kFuseThreads)
         const int row = i / nx, x = i - row * nx;
         const float xf = (float)x;
         FPair sumI = {0.0f, 0.0f}, sumW = {0.0f, 0.0f}, sumD = {0.0f, 0.0f};
+        bool wide = false;  // a sample is not finite
         for (int k = 0; k < fv.n; ++k) {
             const FuseView &v = fv.v[k];
             float f[3], dw[3], dd[3];
@@ -227,7 +283,12 @@ __global__ void __launch_bounds__(kFuseThreads)
                 for (int d = 0; d < 3; ++d) wd = blend_factor(wd, dd[d], v.dr[d], v.dri[d]);
             fp_gather(sumD, wd);
             if (wf == 0.0f) continue;
-            const float val = in ? fmaxf(1.0f, trilinear(v, c, f)) : 0.0f;  // minValueImg, outsideValueImg
+            float val = 0.0f;  // outsideValueImg
+            if (in) {
+                const float q = trilinear(v, c, f);
+                wide = wide || !(fabsf(q) <= FLT_MAX);
+                val = fmaxf(1.0f, q);  // minValueImg
+            }
             const FPair q = fp_prod(val, wf);
             fp_gather(sumI, q.h);
             sumI.l = __fadd_rn(sumI.l, q.l);
@@ -240,8 +301,24 @@ __global__ void __launch_bounds__(kFuseThreads)
             const float r = __fadd_rn(__fmaf_rn(-q, sumW.h, sumI.h), __fmaf_rn(-q, sumW.l, sumI.l));
             im = __fadd_rn(q, __fdividef(r, sumW.h));
         }
-        out_img[o0 + i] = im;
+        wide = wide || !(fabsf(im) <= FLT_MAX);
+        if (wide) d_wide[call % kWideCalls] = call;
+        out_img[o0 + i] = wide ? NAN : im;
         out_w[o0 + i] = __fadd_rn(sumD.h, sumD.l);
+    }
+}
+
+// The voxels that k_fuse_group of this call left as NaN, if it left any.
+__global__ void __launch_bounds__(kFuseThreads)
+    k_fuse_wide(const __grid_constant__ FuseViews fv, long long bx, long long by, long long bz, int nx, int ny, int nz,
+                float *__restrict__ out_img, float *__restrict__ out_w, unsigned long long call)
+{
+    if (d_wide[call % kWideCalls] != call) return;
+    const long long n = (long long)nx * ny * nz;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        if (out_img[i] == out_img[i]) continue;
+        const long long x = i % nx, y = i / nx % ny, z = i / nx / ny;
+        fuse_voxel(fv, (double)(x + bx), (double)(y + by), (double)(z + bz), out_img[i], out_w[i]);
     }
 }
 
@@ -291,6 +368,8 @@ extern "C" MVR_API int mvr_fuse_group(const mvr_fuse_view *views, int num_views,
         v.adjust = s.intensity_adjust ? 1 : 0;
         v.m00 = fp_from(s.intensity[0]);
         v.m01 = fp_from(s.intensity[1]);
+        v.m[0] = s.intensity[0];
+        v.m[1] = s.intensity[1];
         v.img = s.img;
         if (!invert_affine(s.model, v.inv)) return fuse_fail(MVR_ERR_ARG, "mvr_fuse_group: a view model is singular");
         for (int d = 0; d < 3; ++d) v.step[d] = fp_from(v.inv[4 * d]);
@@ -298,6 +377,8 @@ extern "C" MVR_API int mvr_fuse_group(const mvr_fuse_view *views, int num_views,
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) return fuse_fail(MVR_ERR_CUDA, cudaGetErrorString(e));
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    static std::atomic<unsigned long long> calls{0};
+    const unsigned long long call = ++calls;
     const std::vector<FPair> &lut = blending_lut();
     e = cudaMemcpyToSymbolAsync(d_lut, lut.data(), sizeof(FPair) * lut.size(), 0, cudaMemcpyHostToDevice, s);
     // planes beyond the grid's y limit go out in further launches
@@ -306,7 +387,9 @@ extern "C" MVR_API int mvr_fuse_group(const mvr_fuse_view *views, int num_views,
         const long long at = (long long)z0 * bb_dims[0] * bb_dims[1];
         const dim3 grid((unsigned)((bb_dims[1] + kFuseRows - 1) / kFuseRows), (unsigned)nz);
         k_fuse_group<<<grid, kFuseThreads, 0, s>>>(fv, bb_min[0], bb_min[1], bb_min[2] + z0, bb_dims[0], bb_dims[1], nz,
-                                                   image_out + at, weight_out + at);
+                                                   image_out + at, weight_out + at, call);
+        k_fuse_wide<<<152, kFuseThreads, 0, s>>>(fv, bb_min[0], bb_min[1], bb_min[2] + z0, bb_dims[0], bb_dims[1], nz,
+                                                     image_out + at, weight_out + at, call);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

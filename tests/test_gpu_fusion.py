@@ -112,3 +112,43 @@ def test_fuse_group_edges(bb_min, bb_dims, angle, scale, shift, nv, blend):
     assert safe.mean() > (0.8 if nv < 16 else 0.3) or angle == 0.0
     assert np.abs(got_i - ref_img)[safe].max(initial=0.0) <= 1e-5 * max(1.0, float(np.abs(ref_img).max()))
     assert np.abs(got_w - ref_w)[safe].max(initial=0.0) <= 1e-6 * max(1, nv)
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 3.3e38, -3.3e38])
+@pytest.mark.parametrize("nv,intensity", [(1, None), (3, None), (1, (1.5, -2.0)), (2, (-4.0, 0.0))])
+def test_fuse_group_samples_beyond_the_float_range(value, nv, intensity):
+    # samples that are infinite, not a number, or so large that differences and sums leave the float range:
+    # the double sums of the oracle.  Where it says NaN (Inf - Inf, or a NaN sample), max(1, NaN) is 1 here;
+    # that changes a voxel of one view only, so voxels of several are left out there
+    rng = np.random.default_rng(3)
+    views = []
+    for k in range(nv):
+        img = rng.uniform(1, 300, (9, 16, 24)).astype(np.float32)
+        img[3:5, 4:9, 6 + k:12 + k] = value
+        img[5, 10, 7:9] = (value, -value)
+        v = {"img": img, "model": model(21.0 + 9 * k, 1.25, (0.37 + k, -0.71, 0.43))}
+        if intensity:
+            v["intensity"] = intensity
+        v["fusion"] = v["decon"] = ((0.0, 0.0, 0.0), (6.0, 6.0, 3.0))
+        views.append(v)
+    bb_min, bb_dims = (-2, -1, -9), (30, 18, 24)
+    with np.errstate(all="ignore"):
+        ref_img, ref_w = O.fuse_group(views, bb_min, bb_dims)
+    dev = [torch.from_numpy(v["img"]).cuda() for v in views]
+    out = [torch.full((bb_dims[2], bb_dims[1], bb_dims[0]), -1.0, device="cuda") for _ in range(2)]
+    M.fuse_group([dict(v, img_ptr=d.data_ptr(), dims=(24, 16, 9)) for v, d in zip(views, dev)], bb_min, bb_dims,
+                 out[0].data_ptr(), out[1].data_ptr())
+    img, w = (o.cpu().numpy() for o in out)
+    nan = np.isnan(ref_img)
+    if nv == 1:
+        ref_img = np.where(nan, np.float32(1), ref_img)
+        nan[:] = False
+    assert not np.isnan(img).any()
+    odd = np.abs(ref_img) > 1e30
+    assert odd.any() or not value > 0 or intensity == (-4.0, 0.0)
+    same = np.isinf(ref_img) & ~nan
+    assert np.array_equal(img[same], ref_img[same])
+    fin = np.isfinite(ref_img)
+    assert np.abs(img / np.where(fin, ref_img, 1) - 1)[fin & (ref_img != 0)].max() <= 1e-5
+    assert not img[fin & (ref_img == 0)].any()
+    assert np.abs(w - ref_w).max() <= 1e-6 * nv
