@@ -133,8 +133,9 @@ __device__ __forceinline__ float blend_factor(float w, float dist, float range, 
     return __fadd_rn(ph, __fmaf_rn(c.l, w, __fmaf_rn(c.h, w, -ph)));
 }
 
-// Linear interpolation at floor(t) + f in [0, 1)^3 (all eight neighbours exist: t lies strictly
-// inside): differences and fused multiply-adds along x, y, z.  With `adjust` every neighbour goes
+// Linear interpolation at floor(t) + f in [0, 1]^3 (all eight neighbours exist: t lies strictly
+// inside) along x, y, z, with both weights u = 1 - f and f rounded from the pair that t is: a difference
+// form (b - a) f + a keeps f's distance to 1 only to 2^-25, which a bright neighbour multiplies.  With `adjust` every neighbour goes
 // through the intensity adjustment first (IntensityAdjuster.apply,
 // fusion/intensityadjust/IntensityAdjuster.java: v m00 + m01, stored as float).
 __device__ __forceinline__ float fuse_value(const FuseView &v, float x)
@@ -143,8 +144,8 @@ __device__ __forceinline__ float fuse_value(const FuseView &v, float x)
     const FPair q = fp_add(fp_mul(v.m00, x), v.m01);
     return __fadd_rn(q.h, q.l);
 }
-__device__ __forceinline__ float lerp(float a, float b, float f) { return __fmaf_rn(f, __fsub_rn(b, a), a); }
-__device__ __forceinline__ float trilinear(const FuseView &v, const int *i, const float *f)
+__device__ __forceinline__ float lerp(float a, float b, float u, float f) { return __fmaf_rn(f, b, __fmul_rn(u, a)); }
+__device__ __forceinline__ float trilinear(const FuseView &v, const int *i, const float *u, const float *f)
 {
     const long long sy = v.dims[0], sz = (long long)v.dims[0] * v.dims[1];
     const float *p = v.img + ((long long)i[2] * v.dims[1] + i[1]) * sy + i[0];
@@ -153,8 +154,9 @@ __device__ __forceinline__ float trilinear(const FuseView &v, const int *i, cons
     for (int k = 0; k < 8; ++k) c[k] = __ldg(p + (k & 1) + (k & 2 ? sy : 0) + (k & 4 ? sz : 0));
 #pragma unroll
     for (int k = 0; k < 8; ++k) c[k] = fuse_value(v, c[k]);
-    return lerp(lerp(lerp(c[0], c[1], f[0]), lerp(c[2], c[3], f[0]), f[1]),
-                lerp(lerp(c[4], c[5], f[0]), lerp(c[6], c[7], f[0]), f[1]), f[2]);
+    const float y0 = lerp(lerp(c[0], c[1], u[0], f[0]), lerp(c[2], c[3], u[0], f[0]), u[1], f[1]);
+    const float y1 = lerp(lerp(c[4], c[5], u[0], f[0]), lerp(c[6], c[7], u[0], f[0]), u[1], f[1]);
+    return lerp(y0, y1, u[2], f[2]);
 }
 
 // hi + lo += x, the rounding errors of the high part gathered in the low one
@@ -220,10 +222,10 @@ __device__ unsigned long long d_wide[kWideCalls];
 // A CTA takes kFuseRows rows of the box: the part of t that is constant along a row is formed in
 // double, once per row, view and axis (apply_affine at the row's first voxel), and t = base + x
 // step on pairs of floats per voxel.  Bound by instruction issue (82 % of the issue slots): 3 views
-// with blending into a 256^3 box 0.54 ms, 13.1 ms in double; 2 or 4 voxels of a thread at a time
+// with blending into a 256^3 box 0.55 ms, 13.1 ms in double; 2 or 4 voxels of a thread at a time
 // (a view's constants fetched once for them) 0.58 and 0.98 ms: the branches of the border zones
-// keep them from overlapping.
-__global__ void __launch_bounds__(kFuseThreads)
+// keep them from overlapping.  Six CTAs per SM: 554 us, five 571.
+__global__ void __launch_bounds__(kFuseThreads, 6)
     k_fuse_group(const __grid_constant__ FuseViews fv, long long bx, long long by, long long bz, int nx, int ny, int nz,
                  float *__restrict__ out_img, float *__restrict__ out_w, unsigned long long call)
 {
@@ -247,7 +249,7 @@ __global__ void __launch_bounds__(kFuseThreads)
         bool wide = false;  // a sample is not finite
         for (int k = 0; k < fv.n; ++k) {
             const FuseView &v = fv.v[k];
-            float f[3], dw[3], dd[3];
+            float f[3], u[3], dw[3], dd[3];
             int c[3];
             bool in = true;
 #pragma unroll
@@ -261,12 +263,13 @@ __global__ void __launch_bounds__(kFuseThreads)
                     const double s[3] = {(double)(x + bx), (double)(y0 + row + by), (double)(z + bz)};
                     t = fp_from(apply_affine_row(v.inv + 4 * d, s));
                 }
-                float fl = floorf(t.h);
-                f[d] = __fadd_rn(__fsub_rn(t.h, fl), t.l);
-                if (f[d] < 0.0f) {  // t just below an integer
+                float fl = floorf(t.h), r = __fsub_rn(t.h, fl);
+                if (r < -t.l) {  // t just below an integer
                     fl -= 1.0f;
-                    f[d] += 1.0f;
+                    r = 1.0f;
                 }
+                f[d] = __fadd_rn(r, t.l);
+                u[d] = __fsub_rn(__fsub_rn(1.0f, r), t.l);
                 c[d] = (int)fl;
                 in = in && t.h > 0.0f && fl < v.top[d];
                 const float l2 = __fsub_rn(v.top[d], t.h);
@@ -285,7 +288,7 @@ __global__ void __launch_bounds__(kFuseThreads)
             if (wf == 0.0f) continue;
             float val = 0.0f;  // outsideValueImg
             if (in) {
-                const float q = trilinear(v, c, f);
+                const float q = trilinear(v, c, u, f);
                 wide = wide || !(fabsf(q) <= FLT_MAX);
                 val = fmaxf(1.0f, q);  // minValueImg
             }

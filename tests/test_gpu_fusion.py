@@ -152,3 +152,21 @@ def test_fuse_group_samples_beyond_the_float_range(value, nv, intensity):
     assert np.abs(img / np.where(fin, ref_img, 1) - 1)[fin & (ref_img != 0)].max() <= 1e-5
     assert not img[fin & (ref_img == 0)].any()
     assert np.abs(w - ref_w).max() <= 1e-6 * nv
+
+
+def test_fuse_group_next_to_bright_samples():
+    # a dim sample whose bright neighbour has a weight of 2e-5 to 3e-4: the weights' relative error counts,
+    # not their distance to 1.  Three interpolations of two rounded weights, a product and a sum each, and
+    # the oracle's eight rounded terms: 1.1e-6
+    rng = np.random.default_rng(11)
+    for frac in (2e-5, 3e-4, 1 - 1e-4):
+        img = np.where(rng.random((10, 14, 30)) < 0.3, rng.uniform(1e6, 4e6, (10, 14, 30)), rng.uniform(1, 3, (10, 14, 30)))
+        img = img.astype(np.float32)
+        v = {"img": img, "model": model(0.0, 1.0, (-frac, frac - 1.0, -frac))}
+        bb_min, bb_dims = (1, 1, 1), (26, 10, 7)
+        ref, _ = O.fuse_group([v], bb_min, bb_dims)
+        d = torch.from_numpy(img).cuda()
+        out = [torch.full((bb_dims[2], bb_dims[1], bb_dims[0]), -1.0, device="cuda") for _ in range(2)]
+        M.fuse_group([dict(v, img_ptr=d.data_ptr(), dims=(30, 14, 10))], bb_min, bb_dims, out[0].data_ptr(), out[1].data_ptr())
+        assert (ref > 0).all()
+        assert np.abs(out[0].cpu().numpy() / ref - 1).max() <= 2e-6
