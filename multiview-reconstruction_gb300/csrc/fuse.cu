@@ -34,6 +34,7 @@ namespace {
 constexpr int kFuseMaxViews = 16;
 constexpr int kFuseRows = 8;        // rows of one plane a CTA takes at a time
 constexpr int kFuseThreads = 256;
+constexpr int kFuseLong = 1 << 24;  // a row's x is a float up to here
 
 // ---- pairs of floats (hi + lo, about 48 bits) ------------------------------------------------
 // The GPU's double rate is a small fraction of its float rate: one fused voxel in double (affine
@@ -230,8 +231,9 @@ __global__ void __launch_bounds__(kFuseThreads, 6)
                  float *__restrict__ out_img, float *__restrict__ out_w, unsigned long long call)
 {
     __shared__ FPair base[kFuseRows][kFuseMaxViews][3];
-    const int y0 = blockIdx.x * kFuseRows, z = blockIdx.y;
-    const int rows = min(kFuseRows, ny - y0);
+    const int per = nx > kFuseLong ? 1 : kFuseRows;
+    const int y0 = blockIdx.x * per, z = blockIdx.y;
+    const int rows = min(per, ny - y0);
     for (int i = threadIdx.x; i < rows * fv.n; i += kFuseThreads) {
         const int k = i / rows, r = i - k * rows;
         const double s[3] = {(double)bx, (double)(y0 + r + by), (double)(z + bz)};
@@ -240,13 +242,13 @@ __global__ void __launch_bounds__(kFuseThreads, 6)
         for (int d = 0; d < 3; ++d) base[r][k][d] = fp_from(t[d]);
     }
     __syncthreads();
-    const int total = rows * nx;
+    const unsigned total = (unsigned)rows * nx;
     const long long o0 = ((long long)z * ny + y0) * nx;
-    for (int i = threadIdx.x; i < total; i += kFuseThreads) {
+    for (unsigned i = threadIdx.x; i < total; i += kFuseThreads) {
         const int row = i / nx, x = i - row * nx;
         const float xf = (float)x;
         FPair sumI = {0.0f, 0.0f}, sumW = {0.0f, 0.0f}, sumD = {0.0f, 0.0f};
-        bool wide = false;  // a sample is not finite
+        bool wide = x >= kFuseLong;  // or a sample is not finite
         for (int k = 0; k < fv.n; ++k) {
             const FuseView &v = fv.v[k];
             float f[3], u[3], dw[3], dd[3];
@@ -388,7 +390,8 @@ extern "C" MVR_API int mvr_fuse_group(const mvr_fuse_view *views, int num_views,
     for (int z0 = 0; z0 < bb_dims[2] && e == cudaSuccess; z0 += 65535) {
         const int nz = std::min(65535, bb_dims[2] - z0);
         const long long at = (long long)z0 * bb_dims[0] * bb_dims[1];
-        const dim3 grid((unsigned)((bb_dims[1] + kFuseRows - 1) / kFuseRows), (unsigned)nz);
+        const int per = bb_dims[0] > kFuseLong ? 1 : kFuseRows;
+        const dim3 grid((unsigned)((bb_dims[1] + per - 1) / per), (unsigned)nz);
         k_fuse_group<<<grid, kFuseThreads, 0, s>>>(fv, bb_min[0], bb_min[1], bb_min[2] + z0, bb_dims[0], bb_dims[1], nz,
                                                    image_out + at, weight_out + at, call);
         k_fuse_wide<<<152, kFuseThreads, 0, s>>>(fv, bb_min[0], bb_min[1], bb_min[2] + z0, bb_dims[0], bb_dims[1], nz,

@@ -170,3 +170,20 @@ def test_fuse_group_next_to_bright_samples():
         M.fuse_group([dict(v, img_ptr=d.data_ptr(), dims=(30, 14, 10))], bb_min, bb_dims, out[0].data_ptr(), out[1].data_ptr())
         assert (ref > 0).all()
         assert np.abs(out[0].cpu().numpy() / ref - 1).max() <= 2e-6
+
+
+def test_fuse_group_rows_beyond_the_float_integers():
+    # a box of one row of 2^24 + 60 voxels: the end of the row, where x is no float any more, equals a small
+    # box there (the oracle's)
+    rng = np.random.default_rng(2)
+    n = 1 << 24
+    img = rng.uniform(1, 300, (6, 9, 50)).astype(np.float32)
+    v = {"img": img, "model": model(0.0, 1.0, (n + 3.37, -2.21, -1.63)), "fusion": ((0, 0, 0), (5, 5, 5)),
+         "decon": ((0, 0, 0), (4, 4, 4))}
+    ref = O.fuse_group([v], (n, 0, 0), (60, 1, 1))
+    d = torch.from_numpy(img).cuda()
+    out = [torch.full((n + 60,), -1.0, device="cuda") for _ in range(2)]
+    M.fuse_group([dict(v, img_ptr=d.data_ptr(), dims=(50, 9, 6))], (0, 0, 0), (n + 60, 1, 1), out[0].data_ptr(), out[1].data_ptr())
+    for a, b in zip(out, ref):
+        assert np.abs(a[n:].cpu().numpy() - b.reshape(-1)).max() <= 1e-5 * b.max()
+        assert not a[:n].any()
