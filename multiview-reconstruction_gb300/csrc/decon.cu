@@ -310,6 +310,34 @@ __global__ void k_block_content(const float *__restrict__ w, long long D0, long 
     }
 }
 
+// Tiles of several launches: the marks (BadMap) of one launch's psi and quotients concern voxels of others,
+// so they are completed and applied behind the last launch.  Both kernels end at once where nothing is
+// marked.  First the quotients of blocks that read a psi that is not finite:
+__global__ void k_bad_quotients(BadMap *bad, ImgPtrs ip, int nv, long long D0, long long D1, long long n)
+{
+    if (!bad->any[BAD_PSI]) return;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        bool data = false;
+        for (int v = 0; v < nv; ++v) data = data || ip.img[v][i] > 0.0f;
+        if (data) bad_mark(bad, BAD_QUOTIENT, (int)(i % D0), (int)(i / D0 % D1), (int)(i / D0 / D1), true);
+    }
+}
+// then the voxels of marked blocks: the second convolution is NaN, next_value takes minI.
+template <typename T>
+__global__ void k_bad_values(BadMap *bad, const T *__restrict__ psi, T *__restrict__ dst, FusePtrs ws, int nv, int mul,
+                             T minI, long long D0, long long D1, long long n)
+{
+    if (!bad->any[BAD_QUOTIENT]) return;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        if (!bad_voxel(bad, (int)(i % D0), (int)(i / D0 % D1), (int)(i / D0 / D1))) continue;
+        T w = (T)0;
+        for (int v = 0; v < nv; ++v) w += (T)ws.w[v][i];
+        if (mul) w = w < (T)1 ? w : (T)1;
+        const T last = psi[i];
+        dst[i] = last + (minI - last) * w;
+    }
+}
+
 int grid_for(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 152 * 16)); }
 
 }  // namespace
@@ -484,6 +512,7 @@ private:
     {
         if (e == cudaSuccess) return MVR_OK;
         err_ = std::string(what) + ": " + cudaGetErrorString(e);
+        cudaGetLastError();  // reported here
         return e == cudaErrorMemoryAllocation ? MVR_ERR_OOM : MVR_ERR_CUDA;
     }
     int eng(int rc)
@@ -500,6 +529,11 @@ private:
     int make_step_tiles(int st);
     void free_tiles(View &vw);
     int run_tiles(int st);
+    int run_tile_batches(int st);
+    int make_marks(int st);
+    int clear_marks(int st);
+    void free_marks();
+    int overlap(const View &vw, int d) const;
     int run_iteration(double *stats_base, size_t stats_stride);
     int init_psi(int method, double sigma, double *avg_out);
     int autotune();
@@ -565,6 +599,8 @@ private:
     std::vector<int> sort_dim_;
     std::vector<int> jacobi_;
     std::vector<std::vector<SepTile>> tiles_;  // per step: the library's own tiles of the volume (may be empty)
+    std::vector<BadMap *> bad_;                // per step: the marks of its blocks
+    std::vector<size_t> bad_bytes_;            // of the marks
     std::vector<float> max_;
     double *d_scratch_ = nullptr;  // reductions
     int *d_perm_ = nullptr;
@@ -604,6 +640,7 @@ Decon<T>::~Decon()
         engine_.free_plan(v.plan);
         free_tiles(v);
     }
+    free_marks();
     cudaFree(psi_);
     cudaFree(stage_);
     cudaFree(d_scratch_);
@@ -787,6 +824,13 @@ bool sched_env_forced()
 }
 }  // namespace
 
+// The block grid's overlap: the doubled kernel 2k-1, or block - effective + 1 with an effective size.
+template <typename T>
+int Decon<T>::overlap(const View &vw, int d) const
+{
+    return vw.eff[0] > 0 ? vw.bsize(p_.block_size)[d] - vw.eff[d] + 1 : 2 * vw.kd[d] - 1;
+}
+
 // DeconViewPSF.init 119-254 for all views in order.
 template <typename T>
 int Decon<T>::psf_init()
@@ -922,12 +966,9 @@ int Decon<T>::prepare()
         // effective block size is set (at least the doubled kernel)
         int kk[3];
         for (int d = 0; d < 3; ++d) {
-            kk[d] = 2 * vw.kd[d] - 1;
-            if (vw.eff[0] > 0) {
-                if (bs[d] - vw.eff[d] + 1 < kk[d])
-                    return fail(MVR_ERR_ARG, "effective block leaves less overlap than the doubled kernel (2k-1)");
-                kk[d] = bs[d] - vw.eff[d] + 1;
-            }
+            kk[d] = overlap(vw, d);
+            if (kk[d] < 2 * vw.kd[d] - 1)
+                return fail(MVR_ERR_ARG, "effective block leaves less overlap than the doubled kernel (2k-1)");
         }
         if (!divide_blocks(D, kk, bs, all, sort_dim_[st]))
             return fail(MVR_ERR_ARG, "block size smaller than the doubled kernel (2k-1)");
@@ -1006,6 +1047,43 @@ void Decon<T>::free_tiles(View &vw)
 }
 
 template <typename T>
+int Decon<T>::clear_marks(int st)
+{
+    unsigned *any = bad_[st]->any;  // (an address; the marks follow)
+    const size_t at = (char *)any - (char *)bad_[st];
+    D_CUDA(cudaMemsetAsync(any, 0, bad_bytes_[st] - at, engine_.stream()));
+    return MVR_OK;
+}
+
+// The marks of a step's blocks (BadMap), all clear.
+template <typename T>
+int Decon<T>::make_marks(int st)
+{
+    const View &vw = views_[st];
+    BadMap m{};
+    m.n = 1;
+    for (int d = 0; d < 3; ++d) {
+        m.bs[d] = vw.bsize(p_.block_size)[d];
+        const int kk = overlap(vw, d);
+        m.eff[d] = m.bs[d] - kk + 1;
+        m.half[d] = kk / 2;
+        m.nb[d] = (p_.dims[d] + m.eff[d] - 1) / m.eff[d];
+        m.n *= m.nb[d];
+    }
+    D_CUDA(cudaMalloc(&bad_[st], m.bytes()));
+    bad_bytes_[st] = m.bytes();
+    D_CUDA(cudaMemcpyAsync(bad_[st], &m, sizeof(m), cudaMemcpyHostToDevice, engine_.stream()));
+    return clear_marks(st);
+}
+template <typename T>
+void Decon<T>::free_marks()
+{
+    for (BadMap *m : bad_) cudaFree(m);
+    bad_.assign(num_steps(), nullptr);
+    bad_bytes_.assign(num_steps(), 0);
+}
+
+template <typename T>
 int Decon<T>::make_step_tiles(int st)
 {
     const int nv = p_.num_views, v0 = p_.mul ? 0 : st, v1 = p_.mul ? nv : st + 1;
@@ -1044,6 +1122,7 @@ int Decon<T>::make_step_tiles(int st)
     }
     if constexpr (sizeof(T) == sizeof(float))
         D_TRY(eng(engine_.sep_reserve(P, std::min((int)tiles.size(), engine_.sep_batch(P)), p_.mul && nv > 1, n_, rows)));
+    D_TRY(make_marks(st));
     tiles_[st] = std::move(tiles);
     return MVR_OK;
 }
@@ -1053,6 +1132,7 @@ int Decon<T>::make_tiles()
 {
     tiles_.assign(num_steps(), {});
     for (auto &vw : views_) free_tiles(vw);
+    free_marks();
     if (force_sched_ >= 0 || block_kernels_forced()) return MVR_OK;
     for (int st = 0; st < num_steps(); ++st) {
         if (!jacobi_[st]) continue;
@@ -1067,9 +1147,44 @@ int Decon<T>::make_tiles()
     return MVR_OK;
 }
 
-// One view-step (Seq) or iteration (Mul) on the step's tiles: psi read, the staging volume written.
+// One view-step (Seq) or iteration (Mul) on the step's tiles: psi read, the staging volume written.  The
+// update of one launch for all tiles applies the marks of this step itself (FP32); otherwise they are
+// cleared before and applied behind the launches.
 template <typename T>
 int Decon<T>::run_tiles(int st)
+{
+    const std::vector<SepTile> &tiles = tiles_[st];
+    BadMap *bad = bad_[st];
+    const bool inside = sizeof(T) == sizeof(float) && (long long)tiles.size() <= engine_.sep_batch(views_[st].sep.P);
+    cudaStream_t s = engine_.stream();
+    if (!inside) D_TRY(clear_marks(st));
+    engine_.marks(bad, inside ? 3 : 0);
+    const int rc = run_tile_batches(st);
+    engine_.marks(nullptr, 0);
+    D_TRY(rc);
+    if (!inside) {
+        ImgPtrs ip{};
+        FusePtrs ws{};
+        const int v0 = p_.mul ? 0 : st, nv = p_.mul ? p_.num_views : 1;
+        for (int v = 0; v < nv; ++v) {
+            ip.img[v] = views_[v0 + v].img;
+            ws.w[v] = views_[v0 + v].w;
+        }
+        const long long D0 = p_.dims[0], D1 = p_.dims[1];
+        const int grid = std::min(grid_for(n_), 152 * 4);
+        if (tiles.size() > 1) {
+            k_bad_quotients<<<grid, 256, 0, s>>>(bad, ip, nv, D0, D1, n_);
+            D_CUDA(cudaGetLastError());
+        }
+        k_bad_values<T><<<grid, 256, 0, s>>>(bad, psi_, stage_, ws, nv, p_.mul, (T)p_.min_value, D0, D1, n_);
+        D_CUDA(cudaGetLastError());
+    }
+    std::swap(psi_, stage_);
+    return MVR_OK;
+}
+
+template <typename T>
+int Decon<T>::run_tile_batches(int st)
 {
     const std::vector<SepTile> &tiles = tiles_[st];
     std::vector<const float *> imgs, ws;
@@ -1111,7 +1226,6 @@ int Decon<T>::run_tiles(int st)
                 D_TRY(eng(engine_.run_seq(views_[st].tplan, &bp, 1, views_[st].img, views_[st].w, max_[st], nullptr)));
         }
     }
-    std::swap(psi_, stage_);
     return MVR_OK;
 }
 

@@ -788,6 +788,7 @@ BlockMaps Engine<T>::block_maps(const Plan<T> &pl, const BlockPlace *bps, int nb
         }
         bm.fast_x = block_fast_x(bm);
     }
+    bms.bad = bad_;
     return bms;
 }
 
@@ -1552,7 +1553,9 @@ int Engine<T>::sep_seq(const SepPlan &pl, const SepTile *tiles, int nt, const fl
         MVR_TRY(sep_reserve(pl.P, nt, false, 0, max_rows(tiles, nt)));
         int planes;
         const SepTiles tl = sep_tiles(tiles, nt, planes);
-        const SepGeom g = sep_batch_geom(pl.P, tiles, nt, planes, device_);
+        SepGeom g = sep_batch_geom(pl.P, tiles, nt, planes, device_);
+        g.bad = bad_;
+        g.clear = bad_clear_;
         MVR_TRY(sep_conv1(pl, g, tl, nt, psi_src, img, S0_, S0_, true, img_ready));
         SepUpd u{};
         u.psi = psi_src;
@@ -1592,7 +1595,9 @@ int Engine<T>::sep_mul(const std::vector<const SepPlan *> &pls, const SepTile *c
         for (int v = 0; v < nv; ++v) {
             int planes;
             const SepTiles tl = sep_tiles(tiles[v], nt, planes);
-            const SepGeom g = sep_batch_geom(pls[v]->P, tiles[v], nt, planes, device_);
+            SepGeom g = sep_batch_geom(pls[v]->P, tiles[v], nt, planes, device_);
+            g.bad = bad_;
+            g.clear = bad_clear_ & ((v == 0 ? 1 : 0) | (v == nv - 1 ? 2 : 0));
             const bool same = v > 0 && std::memcmp(pls[v]->P, pls[v - 1]->P, sizeof(pls[v]->P)) == 0 &&
                               std::memcmp(tiles[v], tiles[v - 1], sizeof(SepTile) * (size_t)nt) == 0;
             MVR_TRY(sep_conv1(*pls[v], g, tl, nt, psi_src, imgs[v], S0_, S1_, !same));

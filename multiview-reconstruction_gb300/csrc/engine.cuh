@@ -152,6 +152,13 @@ public:
     // Tiles per launch for a domain, and the scratch a launch of nt tiles takes (allocated here).
     int sep_batch(const int P[3]) const;
     int sep_reserve(const int P[3], int nt, bool mul, long long voxels, long long rows);
+    // Marks of the blocks that read values that are not finite, for the tile launches that follow (NULL: none);
+    // clear: SepGeom's
+    void marks(BadMap *bad, int clear)
+    {
+        bad_ = bad;
+        bad_clear_ = clear;
+    }
     void drop_scratch();  // the spectra buffers given back (reserved again by what needs them)
     // The FFT schedules a plan admits (codes SCHED_*), and the one in use.
     int kernel_spectra(Plan<T> &pl, const float *k1, const float *k2, bool k_on_device);
@@ -235,6 +242,8 @@ private:
     double lambda_ = 0.0;
     float min_value_ = 1e-4f;
     cudaStream_t stream_ = nullptr;
+    BadMap *bad_ = nullptr;
+    int bad_clear_ = 0;
     cudaStream_t side_ = nullptr;                       // every other slab of sep_yzy
     cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
     V *S0_ = nullptr, *S1_ = nullptr;

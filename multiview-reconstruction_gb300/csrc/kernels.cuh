@@ -40,11 +40,62 @@ struct BlockMap {
     int fast_x;          // 1: domain x == block x and the block row lies inside the volume
 };
 
+// ---- values that are not finite -------------------------------------------------------
+// The reference's blocks are FFT domains of their own: a voxel of psi or a quotient that is not finite
+// reaches every voxel of the blocks that read it, through their transforms, and no other.  In a domain
+// around the whole volume it would reach every voxel.  Where tiles replace the caller's blocks such a
+// value enters the transform as 1, the blocks that read it are marked here, and the update takes their
+// second convolution as NaN.  The grid of blocks is regular: block i covers [i eff - half, i eff - half
+// + bs) along an axis and writes [i eff, (i + 1) eff).
+struct BadMap {  // in device memory, the marks behind it: n for quotients, n for psi
+    int n;       // blocks
+    int nb[3], eff[3], half[3], bs[3];
+    unsigned any[2];  // some block is marked: [BAD_QUOTIENT], [BAD_PSI]
+    __host__ __device__ size_t bytes() const { return sizeof(BadMap) + 2 * sizeof(unsigned) * (size_t)n; }
+    __device__ __forceinline__ unsigned *marks(int kind) { return reinterpret_cast<unsigned *>(this + 1) + kind * n; }
+};
+enum { BAD_QUOTIENT = 0, BAD_PSI = 1 };
+// Marks the blocks that read voxel (x, y, z); after_psi: those among them whose psi is marked.
+__device__ __forceinline__ void bad_mark(BadMap *b, int kind, int x, int y, int z, bool after_psi = false)
+{
+    const int v[3] = {x, y, z};
+    int lo[3], hi[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int t = v[d] + b->half[d];
+        hi[d] = min(b->nb[d] - 1, t / b->eff[d]);
+        lo[d] = t < b->bs[d] ? 0 : (t - b->bs[d]) / b->eff[d] + 1;
+    }
+#pragma unroll 1
+    for (int k = lo[2]; k <= hi[2]; ++k)
+#pragma unroll 1
+        for (int j = lo[1]; j <= hi[1]; ++j)
+#pragma unroll 1
+            for (int i = lo[0]; i <= hi[0]; ++i) {
+                const int at = (k * b->nb[1] + j) * b->nb[0] + i;
+                if (after_psi && !b->marks(BAD_PSI)[at]) continue;
+                b->marks(kind)[at] = 1;
+                b->any[kind] = 1;
+            }
+}
+// Is voxel (x, y, z) written by a block with a quotient that is not finite?
+__device__ __forceinline__ bool bad_voxel(BadMap *b, int x, int y, int z)
+{
+    return b->marks(BAD_QUOTIENT)[(z / b->eff[2] * b->nb[1] + y / b->eff[1]) * b->nb[0] + x / b->eff[0]] != 0;
+}
+__device__ __forceinline__ void bad_clear(BadMap *b, int kind)
+{
+    if (!b->any[kind]) return;
+    for (int i = 0; i < b->n; ++i) b->marks(kind)[i] = 0;
+    b->any[kind] = 0;
+}
+
 // The blocks of one batched launch: blockIdx.y (rows) / blockIdx.z (columns) picks
 // the block; block i's spectrum starts at i * Pc.
 constexpr int kMaxBatch = 16;
 struct BlockMaps {
     BlockMap m[kMaxBatch];
+    BadMap *bad;  // FP64 tiles; NULL elsewhere
 };
 
 // 1 when every domain x maps to volume x = off + x without extension or mirroring.
@@ -111,10 +162,21 @@ struct SrcMirror {  // psi (or any volume) under the block's mirror mapping
     __device__ __forceinline__ Row row(const BlockMap &m, int y, int z) const { return mirror_row(m, y, z); }
     template <typename T>
     __device__ __forceinline__ T at(const Row &r, const BlockMap &m, int x) const { return (T)vol[r.base + mirror_x(m, x)]; }
+    static constexpr bool kMarks = true;
+    // v, or 1 where it is not finite, its blocks marked
+    template <typename T>
+    __device__ __forceinline__ T finite(T v, const Row &r, const BlockMap &m, int x, BadMap *b) const
+    {
+        if (isfinite(v)) return v;
+        const long long row = r.base / m.D[0];
+        bad_mark(b, BAD_PSI, (int)mirror_x(m, x), (int)(row % m.D[1]), (int)(row / m.D[1]));
+        return (T)1;
+    }
 };
 
 template <typename TS>
 struct SrcZero {  // a block buffer [b] with zero outside it (FFTConvolution with extendZero)
+    static constexpr bool kMarks = false;
     const TS *blk;
     struct Row { long long base; };
     __device__ __forceinline__ Row row(const BlockMap &m, int y, int z) const
@@ -134,6 +196,7 @@ struct SrcZero {  // a block buffer [b] with zero outside it (FFTConvolution wit
 };
 
 struct SrcKernel {  // kernel placed with its centre (k/2) at the origin, wrapped, scaled
+    static constexpr bool kMarks = false;
     const float *k;
     int kd[3];
     double scale;
@@ -253,6 +316,12 @@ __global__ void __launch_bounds__(256) k_rows_fwd(Src src, typename Cx<T>::t *__
 #pragma unroll
             for (int u = 0; u < kRowBatch; ++u) {
                 const int q = c0 + lane + 32 * u;
+                if constexpr (sizeof(T) == sizeof(double) && Src::kMarks) {
+                    if (bms.bad && q < m) {
+                        v0[u] = src.finite(v0[u], R, bm, 2 * q, bms.bad);
+                        v1[u] = src.finite(v1[u], R, bm, 2 * q + 1, bms.bad);
+                    }
+                }
                 if (q < m) A[r * ps + q] = cx<V>(v0[u], v1[u]);
             }
         }
@@ -457,8 +526,18 @@ __global__ void __launch_bounds__(256) k_rows_ratio(typename Cx<T>::t *__restric
                 const V c = zz[q];  // conv1 at x = 2q, 2q+1 (kernel spectrum carries 1/(Px Py Pz))
                 T out[2] = {c.x, c.y};
 #pragma unroll
-                for (int h = 0; h < 2; ++h)  // -1 marks the value-1 extension outside the block
+                for (int h = 0; h < 2; ++h) {  // -1 marks the value-1 extension outside the block
                     out[h] = im[u][h] < 0.0f ? (T)1 : (T)quotient(im[u][h], out[h]);
+                    if constexpr (sizeof(T) == sizeof(double)) {
+                        // (a tile: no extension, ex and the row's coordinates are domain indices)
+                        if (bms.bad && im[u][h] > 0.0f && (!isfinite(out[h]) || bms.bad->any[BAD_PSI])) {
+                            const int x = (int)bm.off[0] + 2 * q + h, yy = (int)bm.off[1] + y, zz = (int)bm.off[2] + z;
+                            if (bms.bad->any[BAD_PSI]) bad_mark(bms.bad, BAD_QUOTIENT, x, yy, zz, true);
+                            if (!isfinite(out[h])) bad_mark(bms.bad, BAD_QUOTIENT, x, yy, zz);
+                        }
+                        if (bms.bad && !isfinite(out[h])) out[h] = (T)1;
+                    }
+                }
                 zz[q] = cx<V>(out[0], out[1]);
             }
         }

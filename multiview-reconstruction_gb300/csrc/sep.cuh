@@ -45,6 +45,8 @@ struct SepGeom {
     int Zs;            // planes a tile's spectrum buffer holds
     long long stride;  // complex values per tile: nxb Zs Py 16 + Zs Py
     int stream;        // 1: volumes and K^ pass through L2 with the evict-first priority
+    BadMap *bad;       // marks of the blocks that read values that are not finite (NULL: a block of its own)
+    int clear;         // 1: the forward pass clears the quotients' marks, 2: the update psi's
 };
 inline SepGeom sep_geom(const int P[3], int planes)
 {
@@ -54,6 +56,8 @@ inline SepGeom sep_geom(const int P[3], int planes)
     g.Zs = planes;
     g.stride = ((long long)g.nxb * 16 + 1) * planes * P[1];
     g.stream = 0;
+    g.bad = nullptr;
+    g.clear = 0;
     return g;
 }
 

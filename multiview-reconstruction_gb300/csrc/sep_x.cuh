@@ -48,6 +48,7 @@ struct SxShape {
 template <int V>
 struct SxRows {
     long long a[SxShape<V>::R], b[SxShape<V>::R];  // row bases in the volume (-1: no row) and in the spectrum
+    unsigned flag;                                 // blocks are marked (BadMap)
 };
 
 // x phase 2 with the packed-real split (forward) or merge (inverse), one unit per warp and round.
@@ -249,6 +250,86 @@ __device__ __forceinline__ void sx_rows(SxRows<V> &sr, const SepTile &t, int r0,
     }
 }
 
+// ---- values that are not finite (BadMap) ----------------------------------------------------
+// A row item whose phase-1 transform shows one (its zero frequency is the sum of the inputs) is done
+// again by the thread that had it, with 1 in the value's place, as plain sums: the ordinary path pays two
+// comparisons per item and one register.  (No local arrays and no calls: with either, the kernel has a stack,
+// and 2 views of 128 x 128 x 64 take 4 % longer; so 1.5 %, 4 views of 256^3 0.8 %.)
+__device__ __forceinline__ bool sx_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+__device__ __forceinline__ bool sx_finite(float2 v) { return sx_finite(v.x) && sx_finite(v.y); }
+
+// The word at m (or 0) into shared memory, its way there behind the loads that f starts and waits for.
+template <class F>
+__device__ __forceinline__ void sx_flag(unsigned &flag, const unsigned *m, F f)
+{
+    const unsigned v = threadIdx.x == 0 && m ? *m : 0;
+    f();
+    if (threadIdx.x == 0) flag = v;
+}
+
+template <int V>
+__device__ __forceinline__ float2 sx_root(const float2 *tw, int j)  // W_V^j, j < V^2
+{
+    const int f = 32 * (j % V), m = SxShape<V>::m;
+    return f < m ? tw[f] : make_float2(-tw[f - m].x, -tw[f - m].y);
+}
+// Phase 1 of x(v), v < V, into the item's line elements p[k1 BS].
+template <int V, class X>
+__device__ __forceinline__ void sx_p1_sums(float2 *p, const float2 *tw, int t, X x)
+{
+#pragma unroll 1
+    for (int k1 = 0; k1 < V; ++k1) {
+        float2 s = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+        for (int v = 0; v < V; ++v) s = cadd(s, cmul(x(v), sx_root<V>(tw, v * k1)));
+        p[k1 * SxShape<V>::BS] = cmul(s, tw[SxShape<V>::m + 16 * k1 + t]);
+    }
+}
+// psi: the item at x = g0 + 32 v + {0, 1} of the row at (y, z)
+template <int V>
+__device__ __forceinline__ void sx_fwd_again(BadMap *b, const float *row, float2 *p, const float2 *tw, int t, int g0, int N, int y,
+                                             int z)
+{
+    sx_p1_sums<V>(p, tw, t, [&](int v) {
+        float c[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = abs(g0 + 32 * v + h), j = min(max(min(i, 2 * N - 2 - i), 0), N - 1);
+            c[h] = row[j];
+            if (sx_finite(c[h])) continue;
+            bad_mark(b, BAD_PSI, j, y, z);
+            c[h] = 1.0f;
+        }
+        return make_float2(c[0], c[1]);
+    });
+}
+// The quotient, conv1's phase-1 values still in p; s[v stride]: the item's elements of the spectrum lines,
+// which the CTA has read and not yet written.
+template <int V>
+__device__ __forceinline__ void sx_ratio_again(BadMap *b, const float *row, float2 *p, float2 *s, long long stride,
+                                               const float2 *tw, int t, int g0, int N, int y, int z)
+{
+#pragma unroll 1
+    for (int v = 0; v < V; ++v) {
+        float2 q = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+        for (int k1 = 0; k1 < V; ++k1)
+            q = cadd(q, cmul(p[k1 * SxShape<V>::BS], cconj(cmul(tw[SxShape<V>::m + 16 * k1 + t], sx_root<V>(tw, v * k1)))));
+        float c[2] = {q.x, q.y};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = g0 + 32 * v + h;
+            const bool in = i >= 0 && i < N;
+            c[h] = quotient_fast(in ? row[i] : 0.0f, c[h]);
+            if (sx_finite(c[h])) continue;
+            if (in) bad_mark(b, BAD_QUOTIENT, i, y, z);
+            c[h] = 1.0f;
+        }
+        s[v * stride] = make_float2(c[0], c[1]);
+    }
+    sx_p1_sums<V>(p, tw, t, [&](int v) { return s[v * stride]; });
+}
+
 // ---- forward ------------------------------------------------------------------------------
 template <int V>
 __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_FWD)
@@ -270,7 +351,9 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_FWD)
     __syncthreads();
     const unsigned long long pol = sep_policy(g.stream);
     const bool pairs = sx_pairs(vec, t.a[0], 0, t.a[0].N);
+    unsigned again = 0;  // bit k: the thread's k-th item
     pdl_wait();
+    if ((g.clear & 1) && blockIdx.x + blockIdx.y + threadIdx.x == 0) bad_clear(g.bad, BAD_QUOTIENT);
     for (int it = threadIdx.x; it < SH::R * 16; it += SH::NT) {
         const int q = it & 15, row = it >> 4;
         const long long base = sr.a[row];
@@ -298,9 +381,18 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_FWD)
             }
         }
         sx_p1<V, false>(a, tw, q);
+        if (!sx_finite(a[0])) again |= 1u << it / SH::NT;
 #pragma unroll
         for (int k1 = 0; k1 < V; ++k1) A[k1 * SH::BS + row * kSepRS + q] = a[k1];
     }
+    if (again && g.bad)
+#pragma unroll 1
+        for (int it = threadIdx.x; it < SH::R * 16; it += SH::NT) {
+            if (!(again >> it / SH::NT & 1)) continue;
+            const int q = it & 15, row = it >> 4, r = r0 + row;
+            sx_fwd_again<V>(g.bad, src.vol + sr.a[row], A + row * kSepRS + q, tw, q, t.a[0].lo + 2 * q, t.a[0].N,
+                            t.a[1].v0 + r % ny, t.a[2].v0 + r / ny);
+        }
     __syncthreads();
     sx_p2<V, false>(A, tw);
     __syncthreads();
@@ -331,7 +423,8 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_RATIO)
     const long long bstride = (long long)g.Zs * g.P[1] * 16;
     const unsigned long long pol = sep_policy(g.stream);
     const bool pairs = sx_pairs(vec, t.a[0], 0, t.a[0].N);
-    sx_load_lines<V>(A, base, bstride, sr.b);
+    unsigned again = 0;
+    sx_flag(sr.flag, g.bad ? &g.bad->any[BAD_PSI] : nullptr, [&] { sx_load_lines<V>(A, base, bstride, sr.b); });
     __syncthreads();
     sx_p2<V, true>(A, tw);
     __syncthreads();
@@ -356,8 +449,30 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_RATIO)
 #pragma unroll
         for (int v = 0; v < V; ++v) a[v] = make_float2(quotient_fast(im[v].x, a[v].x), quotient_fast(im[v].y, a[v].y));
         sx_p1<V, false>(a, tw, q);
+        if (g.bad && !sx_finite(a[0])) {
+            again |= 1u << it / SH::NT;
+            continue;
+        }
 #pragma unroll
         for (int k1 = 0; k1 < V; ++k1) p[k1 * SH::BS] = a[k1];
+    }
+    if (again)
+#pragma unroll 1
+        for (int it = threadIdx.x; it < SH::R * 16; it += SH::NT) {
+            if (!(again >> it / SH::NT & 1)) continue;
+            const int q = it & 15, row = it >> 4, r = r0 + row;
+            if (sr.a[row] < 0) continue;
+            sx_ratio_again<V>(g.bad, img + sr.a[row], A + row * kSepRS + q, base + sr.b[row] + q, bstride, tw, q,
+                              t.a[0].lo + 2 * q, t.a[0].N, t.a[1].q0 + r % t.a[1].nq, t.a[2].q0 + r / t.a[1].nq);
+        }
+    if (sr.flag) {  // the quotients of a block that reads it, where the image is positive
+        const int N = t.a[0].N;
+#pragma unroll 1
+        for (int i = threadIdx.x; i < SH::R * N; i += SH::NT) {
+            const int row = i / N, x = i - row * N, r = r0 + row;
+            if (sr.a[row] >= 0 && img[sr.a[row] + x] > 0.0f)
+                bad_mark(g.bad, BAD_QUOTIENT, x, t.a[1].q0 + r % t.a[1].nq, t.a[2].q0 + r / t.a[1].nq, true);
+        }
     }
     __syncthreads();
     sx_p2<V, false>(A, tw);
@@ -493,6 +608,16 @@ __device__ __forceinline__ void sx_mul_rows(const float2 *A, const SepUpd &u, in
     }
 }
 
+// psi of voxel `at` in a block whose second convolution is NaN: next_value takes minI.
+__device__ __forceinline__ void sx_bad_value(const SepUpd &u, bool mul, long long at)
+{
+    float w = 0.0f;
+    for (int v = 0; v < u.nviews; ++v) w += u.weight[v][at];
+    if (mul) w = w < 1.0f ? w : 1.0f;
+    const float last = u.psi[at];
+    u.dst[at] = __fadd_rn(last, __fmul_rn(__fsub_rn(u.c.minI, last), w));
+}
+
 // The written voxels alone: Seq (DeconvolutionMethods.java:103-182, 320-358) or the running product
 // and final value of Mul (:370-419); with ST the change statistics over them.
 template <int V, bool MUL, bool ST>
@@ -522,7 +647,9 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_UPD)
     sx_rows<V>(sr, t, r0, t.a[1].w0, t.a[1].nw, t.a[2].w0, t.a[2].nw, g.P[1]);
     __syncthreads();
     pdl_wait();
-    sx_load_lines<V>(A, S + (long long)blockIdx.y * g.stride, (long long)g.Zs * g.P[1] * 16, sr.b);
+    if ((g.clear & 2) && blockIdx.x + blockIdx.y + threadIdx.x == 0) bad_clear(g.bad, BAD_PSI);
+    sx_flag(sr.flag, g.bad && epi != EPI_MUL_FIRST && epi != EPI_MUL_ACC ? &g.bad->any[BAD_QUOTIENT] : nullptr,
+            [&] { sx_load_lines<V>(A, S + (long long)blockIdx.y * g.stride, (long long)g.Zs * g.P[1] * 16, sr.b); });
     __syncthreads();
     sx_p2<V, true>(A, tw);
     __syncthreads();
@@ -551,6 +678,15 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_UPD)
     if constexpr (MUL) {
         __syncthreads();
         sx_mul_rows<V, ST>(A, u, epi, t, sr.a, ksum, kcomp, kmax, pol);
+    }
+    if (!ST && sr.flag) {
+        __syncthreads();  // behind the rows' stores
+#pragma unroll 1
+        for (int i = threadIdx.x; i < SH::R * nx; i += SH::NT) {
+            const int row = i / nx, x = x0 + i - row * nx, r = r0 + row;
+            if (sr.a[row] >= 0 && bad_voxel(g.bad, x, t.a[1].w0 + r % t.a[1].nw, t.a[2].w0 + r / t.a[1].nw))
+                sx_bad_value(u, MUL, sr.a[row] + x);
+        }
     }
     if (ST) stats_to_partials(ksum, kcomp, kmax, red_s, red_m, u.partials, slot);
 }
