@@ -1211,6 +1211,24 @@ const std::vector<int> &sep_lengths(int axis)
     return axis == 0 ? x : yz;
 }
 
+namespace {
+// The tile that writes [e0, e1), psi's rows up to `reach` voxels beyond.
+SepAxis axis_tile(int N, int r, int e0, int e1, int P, bool even_lo, int reach)
+{
+    SepAxis a;
+    a.lo = std::max(e0 - 2 * r, -r);
+    if (even_lo && (a.lo & 1)) --a.lo;
+    a.N = N;
+    a.v0 = std::max(a.lo, 0);
+    a.nv = std::min({N, a.lo + P, e1 + reach}) - a.v0;
+    a.q0 = std::max(e0 - r, 0);
+    a.nq = std::min(e1 + r, N) - a.q0;
+    a.w0 = e0;
+    a.nw = e1 - e0;
+    return a;
+}
+}  // namespace
+
 bool split_axis(int N, int k, const std::vector<int> &lens, bool even_lo, AxisTiles &out)
 {
     const int r = k / 2, slack = even_lo ? 1 : 0;
@@ -1241,19 +1259,22 @@ bool split_axis(int N, int k, const std::vector<int> &lens, bool even_lo, AxisTi
     for (int i = 0; i < n; ++i) {
         const int cap = (P - (i == 0 || i == n - 1 ? 3 : 4) * r - slack) & ~slack;
         const int e1 = i == n - 1 ? N : std::min(N, e0 + cap);
-        SepAxis a;
-        a.lo = std::max(e0 - 2 * r, -r);
-        if (even_lo && (a.lo & 1)) --a.lo;
-        a.N = N;
-        a.v0 = std::max(a.lo, 0);
-        a.nv = std::min(N, a.lo + P) - a.v0;
-        a.q0 = std::max(e0 - r, 0);
-        a.nq = std::min(e1 + r, N) - a.q0;
-        a.w0 = e0;
-        a.nw = e1 - e0;
+        const SepAxis a = axis_tile(N, r, e0, e1, P, even_lo, P);
         if (a.nw > 0) out.tiles.push_back(a);
         e0 = e1;
     }
+    return true;
+}
+
+bool grid_axis(int N, int k, int eff, const std::vector<int> &lens, bool even_lo, AxisTiles &out)
+{
+    const int r = k / 2, n = std::min(eff, N), slack = even_lo ? 1 : 0;
+    if (r + (even_lo && (r & 1) ? 1 : 0) > N - 1) return false;
+    const auto fit = std::lower_bound(lens.begin(), lens.end(), n + 4 * r + slack);
+    if (fit == lens.end()) return false;
+    out.P = *fit;
+    out.tiles.clear();
+    for (int e0 = 0; e0 < N; e0 += eff) out.tiles.push_back(axis_tile(N, r, e0, std::min(N, e0 + eff), out.P, even_lo, 2 * r));
     return true;
 }
 

@@ -99,6 +99,9 @@ struct AxisTiles {
 // false when there is none, or when the mirror extension would reflect twice (reach >= N).
 // even_lo: tiles start at even coordinates (8-byte loads of pairs along x).
 bool split_axis(int N, int k, const std::vector<int> &lens, bool even_lo, AxisTiles &out);
+// The tiles of a block grid: [i eff, (i + 1) eff), each in a domain of the smallest length that holds it and
+// psi on twice the reach either side, like the block it stands for.
+bool grid_axis(int N, int k, int eff, const std::vector<int> &lens, bool even_lo, AxisTiles &out);
 // The one tile of a block under the engine's boundary rule: the mirror-single / value-1 extension
 // around the block, or the block itself as a periodic domain.  false: no separable transforms.
 bool block_tile(const int b[3], const int kd[3], int boundary, int P[3], SepTile &tile);

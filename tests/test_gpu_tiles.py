@@ -227,3 +227,38 @@ def test_queued_iterations_in_place_on_odd_rows(b, kd):
     for _ in range(3):
         ref, _ = O.block_seq(ref, img, w, k1, k2, 0.006, 1e-4, 300.0)
     assert rel(d[0].cpu().numpy(), ref) <= 3e-5  # 1e-5 an iteration, as above
+
+
+@pytest.mark.parametrize("mul", [False, True])
+def test_dim_blocks_far_from_bright_ones(mul):
+    # beads of 2e4 in the first 180 columns, 1e-3 to 2e-3 elsewhere: blocks from column 344 on hold no bead, and
+    # their voxels (from 352 on) keep the rounding of their own transforms, voxel by voxel; the second view's
+    # step reads the first one's 8 columns beyond, so from 360 on.  Tolerance: the FP32 bound of one iteration,
+    # here relative to each voxel
+    fft = pytest.importorskip("scipy.signal")
+    dims, kd, block, nv = (560, 48, 48), (9, 9, 9), (192, 64, 64), 2
+    rng = np.random.default_rng(31)
+    shape = dims[::-1]
+    psi = rng.uniform(1e-3, 2e-3, shape).astype(np.float32)
+    psi[rng.integers(0, 48, 30), rng.integers(0, 48, 30), rng.integers(0, 180, 30)] = 2e4
+    psfs = [synthetic.make_psf(kd, 1.0, 1.5, 40.0 * v) for v in range(nv)]
+    imgs = [np.maximum(fft.fftconvolve(psi[:, :, :200].astype(np.float64), p.astype(np.float64), "same"), 1e-3) for p in psfs]
+    imgs = [np.concatenate([i, fft.fftconvolve(psi[:, :, 200:].astype(np.float64), p.astype(np.float64), "same")], 2)
+            for i, p in zip(imgs, psfs)]
+    imgs = [(i * rng.uniform(0.7, 1.4, shape)).astype(np.float32) for i in imgs]
+    ws = [rng.uniform(0.2, 0.5, shape).astype(np.float32) for _ in range(nv)]
+    with M.Deconvolution(dims, nv, block, mul=mul, psf_type=M.PSF_INDEPENDENT, lam=0.006) as d:
+        for v in range(nv):
+            d.set_view(v, imgs[v], ws[v], psfs[v])
+        d.prepare()
+        d.set_psi(psi)
+        ks = [d.kernels(v, psfs[v].shape) for v in range(nv)]
+        mx = d.max_intensities()
+        d.run_iterations(1)
+        out = d.get_psi()
+    ref, _ = O.decon_run(psi, imgs, ws, [k[0] for k in ks], [k[1] for k in ks], block, 1, mul=mul, lam=0.006,
+                         max_intensities=mx, fp64=True)
+    assert rel(out, ref) <= 1e-5
+    dark = np.s_[:, :, 360:]
+    assert ref[dark].max() < 0.1
+    assert np.abs(out[dark] / ref[dark] - 1).max() <= 1e-5

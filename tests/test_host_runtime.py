@@ -150,6 +150,6 @@ def prepare(fail, n):
 tiles, n = prepare(-1, 1), 0
 while prepare(n, 1) is None:  # allocations of the block plans
     n += 1
-rest = [prepare(i, 1) for i in range(n, n + 8)]  # three tables, two spectra, the blocks' marks; none
-assert len(set(rest[:6])) == 1 and rest[0] not in (None, tiles) and rest[6:] == [tiles] * 2, (tiles, n, rest)
+rest = [prepare(i, 1) for i in range(n, n + 10)]  # two for the blocks' levels, three tables, two spectra, marks
+assert len(set(rest[:8])) == 1 and rest[0] not in (None, tiles) and rest[8:] == [tiles] * 2, (tiles, n, rest)
 """)
