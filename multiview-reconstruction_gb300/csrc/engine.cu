@@ -1424,7 +1424,8 @@ int Engine<T>::sep_fill(SepPlan &pl, const int P[3], const float *k1, const floa
                 MVR_CUDA(cudaMemcpyAsync(kbuf_, k, sizeof(float) * (size_t)kn, cudaMemcpyHostToDevice, stream_));
                 k = kbuf_;
             }
-            SepSrc src{k, 1, {kd[0], kd[1], kd[2]}, 1.0 / ((double)P[0] * P[1] * P[2])};
+            // (K1^: a quarter, see sx_quotient)
+            SepSrc src{k, 1, {kd[0], kd[1], kd[2]}, (which ? 1.0 : 0.25) / ((double)P[0] * P[1] * P[2])};
             launches_ += 3;
             MVR_CUDA(sep_x_fwd(g, tl, 1, src, S0_, pl.twx, stream_));
             const SepSlab all{0, g.nxb, false};

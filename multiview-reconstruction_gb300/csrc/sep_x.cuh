@@ -250,6 +250,16 @@ __device__ __forceinline__ void sx_rows(SxRows<V> &sr, const SepTile &t, int r0,
     }
 }
 
+// The quotient by a quarter of conv1 (K1^ carries the factor): the approximate division takes divisors up to
+// 2^126 and returns 0 beyond.  Its two ulp are not seen behind the transforms' rounding: with IEEE divisions
+// and roots here and in the update the errors against 64 bits stay where they are (156 x 156 x 124 block
+// 1.1e-7 and 1.2e-7, 2 views of 128 x 128 x 64 6.5e-7 and 6.6e-7, 256^3 1.3e-7 both) and 4 views of 256^3 take 2 to
+// 8 % longer.
+__device__ __forceinline__ float sx_quotient(float img, float quarter)
+{
+    return img > 0.0f ? __fdividef(0.25f * img, quarter) : 1.0f;
+}
+
 // ---- values that are not finite (BadMap) ----------------------------------------------------
 // A row item whose phase-1 transform shows one (its zero frequency is the sum of the inputs) is done
 // again by the thread that had it, with 1 in the value's place, as plain sums: the ordinary path pays two
@@ -320,7 +330,7 @@ __device__ __forceinline__ void sx_ratio_again(BadMap *b, const float *row, floa
         for (int h = 0; h < 2; ++h) {
             const int i = g0 + 32 * v + h;
             const bool in = i >= 0 && i < N;
-            c[h] = quotient_fast(in ? row[i] : 0.0f, c[h]);
+            c[h] = sx_quotient(in ? row[i] : 0.0f, c[h]);
             if (sx_finite(c[h])) continue;
             if (in) bad_mark(b, BAD_QUOTIENT, i, y, z);
             c[h] = 1.0f;
@@ -447,7 +457,7 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_RATIO)
             else sx_load_zero<V, false>(im, img + ib, t.a[0].lo + 2 * q, 0, n, pol);
         }
 #pragma unroll
-        for (int v = 0; v < V; ++v) a[v] = make_float2(quotient_fast(im[v].x, a[v].x), quotient_fast(im[v].y, a[v].y));
+        for (int v = 0; v < V; ++v) a[v] = make_float2(sx_quotient(im[v].x, a[v].x), sx_quotient(im[v].y, a[v].y));
         sx_p1<V, false>(a, tw, q);
         if (g.bad && !sx_finite(a[0])) {
             again |= 1u << it / SH::NT;

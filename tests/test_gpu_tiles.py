@@ -262,3 +262,19 @@ def test_dim_blocks_far_from_bright_ones(mul):
     dark = np.s_[:, :, 360:]
     assert ref[dark].max() < 0.1
     assert np.abs(out[dark] / ref[dark] - 1).max() <= 1e-5
+
+
+def test_quotient_by_a_value_above_2_to_126():
+    # a hot voxel of 1.2e38, a kernel of one voxel: the quotient 1e38 / 1.2e38 (the approximate division alone
+    # returns 0 there), psi becomes 1e38.  A periodic domain: an extended one can hold mirror images of the
+    # voxel, and the transform's sum of those leaves the float range
+    b = (64, 32, 32)
+    psi = np.ones(b[::-1], np.float32)
+    img = np.zeros(b[::-1], np.float32)  # quotient 1
+    psi[9, 10, 20], img[9, 10, 20] = 1.2e38, 1e38
+    w = np.ones_like(psi)
+    one = np.ones((1, 1, 1), np.float32)
+    with M.BlockWorker(b, 1e-4, 0.0, 1, M.BOUNDARY_CIRCULAR) as wk:
+        wk.set_kernels(0, one, one)
+        wk.run_iteration(0, psi, img, w, 1e38)
+    assert abs(psi[9, 10, 20] / 1e38 - 1) <= 1e-5
