@@ -414,7 +414,9 @@ MVR_API int mvr_unet_propose(mvr_unet *h, const float *psi, float *psi_out, floa
 /* One 3x3x3 convolution layer on the tensor cores (device BF16 [B][z][y][x][C] volumes,
  * dims {x, y, z, B}): transposed == 0 is the forward pass (weights [n_out][27][c_act],
  * bias, ReLU, BF16 output), transposed == 1 the data gradient (weights transposed
- * [n_out][27][c_act], FP32 output).  err_dev: device int, set on a tensor-core timeout. */
+ * [n_out][27][c_act], FP32 output).  err_dev: device int, set on a tensor-core timeout.
+ * Volumes and weights start on 16-byte boundaries; channel pairs that the U-Net has not, and
+ * pointers elsewhere, are refused with MVR_ERR_UNSUPPORTED. */
 MVR_API int mvr_conv3d_tc(const void *act, int c_act, const void *weights, int n_out, const float *bias, int relu,
                           int transposed, void *out, const int dims[4], int *err_dev, void *stream);
 /* Weight gradient dw[c_out][27][c_in] += sum_n g[n][c_out] x[n + off][c_in] (FP32). */

@@ -712,6 +712,13 @@ int UNet::set_params(const float *host)
 // ---- layer-level entry points (used by the gradient checks) ----------------------------
 namespace {
 thread_local std::string g_tc_error;
+// 16-byte copies: true, or the call's error says so
+bool tc_aligned(const void *a, const void *b, const void *c)
+{
+    if (!((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15)) return true;
+    g_tc_error = "volumes and weights must start on 16-byte boundaries";
+    return false;
+}
 int tc_status(cudaError_t e, int *err_dev, cudaStream_t s)
 {
     if (e != cudaSuccess) {
@@ -788,6 +795,7 @@ extern "C" int mvr_conv3d_tc(const void *act, int c_act, const void *weights, in
                              int transposed, void *out, const int dims[4], int *err_dev, void *stream)
 {
     if (!act || !weights || !out || !dims || !err_dev) return MVR_ERR_ARG;
+    if (!mvr::tc_aligned(act, weights, out)) return MVR_ERR_UNSUPPORTED;
     mvr::ConvGeom g{dims[3], dims[2], dims[1], dims[0], (long long)dims[0] * dims[1] * dims[2] * dims[3]};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const cudaError_t e =
@@ -804,6 +812,7 @@ extern "C" int mvr_conv3d_tc_wgrad(const void *x, int c_in, const void *g, int c
                                    int *err_dev, void *stream)
 {
     if (!x || !g || !dw || !dims || !err_dev) return MVR_ERR_ARG;
+    if (!mvr::tc_aligned(x, g, nullptr)) return MVR_ERR_UNSUPPORTED;
     mvr::ConvGeom gg{dims[3], dims[2], dims[1], dims[0], (long long)dims[0] * dims[1] * dims[2] * dims[3]};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const cudaError_t e = mvr::wgrad_any(c_out, c_in, static_cast<const __nv_bfloat16 *>(x),

@@ -129,3 +129,19 @@ def test_block_grid_matches_oracle(lib, dims, k, b):
         assert sd == O.sort_dim(nb, mr)
     with pytest.raises(M.MvrError):
         M.block_grid(dims, (b[0], 3, 3), b)  # block smaller than the doubled kernel
+
+
+def test_convolution_layers_say_what_they_refuse(lib):
+    # before any device work: a pointer that is not on 16 bytes is not called a channel pair
+    args = dict(act_ptr=4096, c_act=16, w_ptr=4096, n_out=16, bias_ptr=0, relu=0, transposed=0, out_ptr=4096,
+                dims_xyzb=(8, 16, 4, 1), err_ptr=4096)
+    for key in ("act_ptr", "w_ptr", "out_ptr"):
+        with pytest.raises(M.MvrError, match="16-byte") as e:
+            M.conv3d_tc(**dict(args, **{key: 4098}))
+        assert e.value.code == M.ERR_UNSUPPORTED
+    with pytest.raises(M.MvrError, match="channel pair"):
+        M.conv3d_tc(**dict(args, c_act=17))
+    for x, g in ((4098, 4096), (4096, 4104)):
+        with pytest.raises(M.MvrError, match="16-byte") as e:
+            M.conv3d_tc_wgrad(x, 16, g, 16, 4096, (8, 16, 4, 1), 4096)
+        assert e.value.code == M.ERR_UNSUPPORTED
