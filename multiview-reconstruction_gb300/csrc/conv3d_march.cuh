@@ -392,7 +392,8 @@ __global__ void __launch_bounds__(kMarchThreads) k_conv3d_march(const __nv_bfloa
 // channels) and 1.5 KB of B per product.  48 x 16 channels on
 // 4 x 64^3 voxels: 97 us (0.85 ms with 27 copies of X out of L2, one per offset), 16 x 16, 8 of them stored: 34 us
 // (0.30), 96 x 32 on 4 x 32^3: 42 us (0.25), 16 x 32: 21 us (0.048).  A column's ragged edge multiplies G's zeros with the X beside
-// it, so there a non-finite X reaches the gradient of the outward offsets as well.
+// it: an X that is not finite reaches the outward offsets there, and what is not finite at the end of a run with
+// ragged columns is summed again without the tensor cores (wgrad_again).
 constexpr int kWgRing = 8;  // planes of G: three being multiplied, the others on their way
 constexpr int kWgGroup = 128 * 16 + 16;  // stride of G's channel groups (padding: distinct banks)
 // Up to 16 channels the 64 rows of a product are eight x shifts of one channel group, 16 bytes apart, of which
@@ -418,6 +419,37 @@ template <int N, int C>
 __host__ __device__ constexpr size_t wgrad_march_smem()
 {
     return (size_t)kMarchStages * (C / 8) * kMarchLbo + (size_t)kWgRing * (N / 8) * kWgGroup;
+}
+
+// Element (tap, ci, co) of the run's share, plain sums over the voxels of the volume.
+template <int N, int C, int CU>
+__device__ __forceinline__ float wgrad_again(const __nv_bfloat16 *X, const __nv_bfloat16 *X2, const __nv_bfloat16 *G,
+                                             const ConvGeom &g, long long u0, long long u1, int tap, int ci, int co)
+{
+    const int dz = tap / 9 - 1, dy = tap / 3 % 3 - 1, dx = tap % 3 - 1;
+    float s = 0.0f;
+    MarchAt at;
+#pragma unroll 1
+    for (long long u = u0; u < u1; ++u) {
+        at.u = u;
+        at.start(g, u1);
+        const int z = at.zs + dz;
+        if (z < 0 || z >= g.D) continue;
+#pragma unroll 1
+        for (int v = 0; v < 128; ++v) {
+            const int x = at.x0 + (v & 7), y = at.y0 + (v >> 3), xx = x + dx, yy = y + dy;
+            if (x >= g.W || y >= g.H || xx < 0 || yy < 0 || xx >= g.W || yy >= g.H) continue;
+            const long long n = (((long long)at.b * g.D + z) * g.H + yy) * g.W + xx;
+            __nv_bfloat16 a;
+            if constexpr (CU == kMarchHalf) a = ci < C / 2 ? X[n * (C / 2) + ci] : __float2bfloat16(0.0f);
+            else if constexpr (CU == 0) a = X[n * C + ci];
+            else if (ci >= CU) a = X2[n * (C - CU) + ci - CU];
+            else
+                a = X[((((long long)at.b * (g.D >> 1) + (z >> 1)) * (g.H >> 1) + (yy >> 1)) * (g.W >> 1) + (xx >> 1)) * CU + ci];
+            s += __bfloat162float(G[((((long long)at.b * g.D + at.zs) * g.H + y) * g.W + x) * N + co]) * __bfloat162float(a);
+        }
+    }
+    return s;
 }
 
 template <int N, int C, int CU = 0>
@@ -550,6 +582,7 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
         const int r = M == 64 ? 16 * warp + lane : 32 * warp + lane;
         const bool rv = r < (XS ? 24 : C) && (M == 128 || lane < 16);
         const int nt = t1 - t0;
+        const bool ragged = g.W % kMarchX || g.H % kMarchY;
 #pragma unroll 1
         for (int q = 0; q < nt * 3; ++q) {
             const int e = (q + (int)blockIdx.x) % (nt * 3), t = t0 + e / 3, tz = 2 - e % 3;
@@ -558,10 +591,24 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
             for (int c0 = 0; c0 < N; c0 += 16) {
                 float v[16];
                 tc::tmem_ld16(trow + (uint32_t)(e * N + c0), v);
-                if (rv)
+                if (!ragged) {
+                    if (rv)
 #pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        atomicAdd(&dW[((long long)(c0 + j) * 27 + tap) * C + ci], v[j]);
+                        for (int j = 0; j < 16; ++j)
+                            atomicAdd(&dW[((long long)(c0 + j) * 27 + tap) * C + ci], v[j]);
+                    continue;
+                }
+#pragma unroll 1
+                for (int j = 0; j < 16; ++j) {
+                    float a = v[0];
+#pragma unroll
+                    for (int i = 1; i < 16; ++i) a = i == j ? v[i] : a;
+                    if (!rv) continue;
+                    if (!(fabsf(a) <= 3.402823466e38f))
+                        a = wgrad_again<N, C, CU>(X, X2, G, g, planes * blockIdx.x / gridDim.x, u1, tap, ci, c0 + j);
+                    atomicAdd(&dW[((long long)(c0 + j) * 27 + tap) * C + ci], a);
+                }
+                __syncwarp();
             }
         }
     }

@@ -197,3 +197,32 @@ def test_unet_gradients_on_ragged_columns(dims, B):
         assert rel(grads[o:o + co], g_ref[o:o + co]) <= 3e-2, (ci, co, "bias")
         o += co
     assert rel(grads[o:o + 17], g_ref[o:o + 17]) <= 1e-3
+
+
+@pytest.mark.parametrize("ci,co", U.LAYERS)
+def test_weight_gradient_of_an_infinite_voxel_at_a_ragged_edge(ci, co):
+    # x = 11 and y = 17 are the last of the volume and inside the last column of voxels: the offsets that reach
+    # them from outside stay finite, the others are what the sums over the volume give
+    rng = np.random.default_rng(ci + co)
+    B, X, Y, Z = 1, 12, 18, 4
+    x = U.bf16(rng.standard_normal((B, Z, Y, X, ci)))
+    g = U.bf16(rng.uniform(0.1, 1.0, (B, Z, Y, X, co)))
+    x[0, 1, 5, 11, 1], x[0, 2, 17, 3, 0] = np.inf, -np.inf
+    with np.errstate(all="ignore"):
+        ref = np.zeros((co, 27, ci))
+        for t in range(27):
+            dz, dy, dx = t // 9 - 1, t // 3 % 3 - 1, t % 3 - 1
+            n = tuple(slice(max(0, -d), s - max(0, d)) for d, s in zip((dz, dy, dx), (Z, Y, X)))
+            m = tuple(slice(max(0, d), s - max(0, -d)) for d, s in zip((dz, dy, dx), (Z, Y, X)))
+            gs, xs = g[(0, *n)].reshape(-1, co).astype(np.float64), x[(0, *m)].reshape(-1, ci).astype(np.float64)
+            for c in range(ci):
+                ref[:, t, c] = (gs * xs[:, c:c + 1]).sum(0)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    xd, gd = dev_bf16(x), dev_bf16(g)
+    dw = torch.zeros((co, 27, ci), dtype=torch.float32, device="cuda")
+    M.conv3d_tc_wgrad(xd.data_ptr(), ci, gd.data_ptr(), co, dw.data_ptr(), (X, Y, Z, B), err.data_ptr())
+    dw = dw.cpu().numpy()
+    fin = np.isfinite(ref)
+    assert 0 < (~fin).sum() < 2 * 27 * co - 9 * co  # both voxels, without the offsets that point outward
+    assert np.array_equal(np.isfinite(dw), fin) and np.array_equal(dw[~fin], ref[~fin])
+    assert rel(dw[fin], ref[fin]) <= 1e-5
