@@ -1273,9 +1273,11 @@ int Decon<T>::run_tiles(int st)
         const int grid = std::min(grid_for(n_), 152 * 4);
         if (tiles.size() > 1) {
             k_bad_quotients<<<grid, 256, 0, s>>>(bad, ip, nv, D0, D1, n_);
+            engine_.count_launches(1);
             D_CUDA(cudaGetLastError());
         }
         k_bad_values<T><<<grid, 256, 0, s>>>(bad, psi_, stage_, ws, nv, p_.mul, (T)p_.min_value, D0, D1, n_);
+        engine_.count_launches(1);
         D_CUDA(cudaGetLastError());
     }
     std::swap(psi_, stage_);
@@ -1667,7 +1669,7 @@ int Decon<T>::run_iteration(double *stats_base, size_t stats_stride)
         D_CUDA(cudaGraphLaunch(g.exec, s));
         psi_ = g.psi_end;
         stage_ = g.stage_end;
-        engine_.count_replayed(g.launches);
+        engine_.count_launches(g.launches);
         return MVR_OK;
     }
     bool seen = false;

@@ -1485,7 +1485,7 @@ int Engine<T>::sep_yzy(const SepPlan &pl, const SepGeom &g, const SepTiles &tl, 
         MVR_CUDA(sep_z(gs, sl, tl, nt, map, out_w, nullptr, S0, S1, K, pl.twz, s));
         sl.first = false;
         MVR_CUDA(sep_y_inv(gs, sl, tl, nt, out_w, S1, pl.twy, s));
-        launches_ += 3;
+        launches_ += fwd ? 3 : 2;
     }
     MVR_CUDA(cudaEventRecord(ev_join_, side_));
     MVR_CUDA(cudaStreamWaitEvent(stream_, ev_join_, 0));

@@ -190,8 +190,8 @@ public:
     // launch accounting: every kernel launch of the engine (and of its owner through
     // count_launch) is counted; with profiling on, each is bracketed by CUDA events
     long long launches() const { return launches_; }
-    // adds launches replayed from a captured graph to the count
-    void count_replayed(long long n) { launches_ += n; }
+    // adds launches replayed from a captured graph, or of kernels of the owner, to the count
+    void count_launches(long long n) { launches_ += n; }
     // changes whenever the engine's scratch buffers are reallocated (captured graphs
     // that use them are then stale)
     long long alloc_epoch() const { return alloc_epoch_; }

@@ -153,3 +153,26 @@ while prepare(n, 1) is None:  # allocations of the block plans
 rest = [prepare(i, 1) for i in range(n, n + 10)]  # two for the blocks' levels, three tables, two spectra, marks
 assert len(set(rest[:8])) == 1 and rest[0] not in (None, tiles) and rest[8:] == [tiles] * 2, (tiles, n, rest)
 """)
+
+
+@pytest.mark.parametrize("dims,block,views,mul,fp64", [
+    ((40, 36, 24), (48, 40, 32), 2, False, False), ((40, 36, 24), (48, 40, 32), 3, True, False),
+    ((40, 36, 24), (48, 40, 32), 2, False, True), ((40, 36, 24), (48, 40, 32), 2, True, True),
+    ((280, 280, 280), (300, 300, 300), 2, False, False), ((280, 280, 280), (300, 300, 300), 3, True, False),  # slabs
+    ((1180, 40, 36), (120, 60, 60), 2, True, True),  # several FP64 tiles
+])
+def test_launch_count(fake, dims, block, views, mul, fp64):
+    # what the handle reports is what the runtime was asked for
+    run(fake, f"""
+D, b, n = {dims}, {block}, {views}
+with M.Deconvolution(D, n, b, mul={mul}, psf_type=M.PSF_INDEPENDENT, filter_blocks=False,
+                     precision=M.PRECISION_FP64 if {fp64} else M.PRECISION_FP32) as d:
+    for v in range(n):
+        d.set_view(v, A(D), A(D), K((5, 5, 5)))
+    d.prepare()
+    d.set_graphs(False)
+    for _ in range(2):
+        f0, c0 = F.fake_launches(), d.launch_count()
+        d.run_iterations(1)
+        assert F.fake_launches() - f0 == d.launch_count() - c0, (F.fake_launches() - f0, d.launch_count() - c0)
+""")
