@@ -29,9 +29,11 @@
  *
  * Blocks, and iterations without statistics, run on separable transforms (mvr_decon_run says
  * when).  Where block plans remain, FP32 FFT domains with Px, Py in {128, 192} run on the plane
- * kernels (x and y transforms fused per z-plane); the environment variable MVR_PLANE_KERNELS=0, read when kernels are
- * set or a deconvolution is prepared, selects the row / column kernels instead (for
- * comparisons; results agree to float rounding).
+ * kernels (x and y transforms fused per z-plane).  For comparisons (results agree to float
+ * rounding), environment variables read when kernels are set or a deconvolution is prepared:
+ * MVR_PLANE_KERNELS=0 selects the row / column kernels instead, and MVR_PLANE_KERNELS,
+ * MVR_XY_PERSIST, MVR_COLS_PIPE or MVR_PAIR_KERNELS set to anything, or MVR_RATIO_BAND=0, keep
+ * every step on block plans.
  */
 #ifndef MVR_GB300_H
 #define MVR_GB300_H
@@ -205,7 +207,12 @@ MVR_API int mvr_block_grid(const long long dims[3], const int kernel_size[3], co
  * the block voxels outside the regions written back to psi (which the reference computes
  * and discards) are not computed, and a view-step whose blocks all read psi before the step
  * runs in FFT domains of the library's choice instead of the blocks' (odd kernel sizes, no
- * dropped block, no forced schedule); psi is the same either way up to float rounding. */
+ * dropped block, no forced schedule); psi is the same either way up to float rounding.  That
+ * rounding is relative to the magnitudes in the domain: where prepare finds a block whose
+ * images lie more than 16 times below the volume's root mean square, the domains are the
+ * blocks' own, so that dim regions keep the blocks' precision (call prepare again for images
+ * of another kind).  A psi or quotient that is not finite affects the blocks that read it and
+ * no other, as with statistics. */
 MVR_API int mvr_decon_run(mvr_decon *h, int iterations, double *stats);
 /* runIterations with the inputs on the host (no reference counterpart as one call: the
  * reference driver holds images, weights and psi in host memory and copies blocks per call):

@@ -1114,9 +1114,9 @@ int Decon<T>::dim_blocks(int st, double &ratio)
 // the fewest transformed voxels, which one domain around the volume usually is (a tile next to
 // a face of the volume needs the kernel's reach beyond it once, a block of the grid twice on
 // every side).  256^3 with 31 x 31 x 61 kernels: one 288 x 288 x 320 domain (1.6 voxels per volume
-// voxel) instead of 16 blocks of 192^3 (6.8): 4.93 -> 1.78 ms per iteration; 6 views of 512 x 512 x
-// 256 32.2 -> 13.4 ms, 3 views of 211 x 187 x 143 (Mul, mixed-radix block sizes) 14.0 -> 0.56 ms, 2
-// views of 96 x 88 x 72 in FP64 2.09 -> 1.16 ms.  Kernels of even sizes stay on the blocks: two of
+// voxel) instead of 16 blocks of 192^3 (6.8): 4.92 -> 1.26 ms per iteration; 6 views of 512 x 512 x
+// 256 32.2 -> 8.1 ms, 3 views of 211 x 187 x 143 (Mul, mixed-radix block sizes) 14.0 -> 0.43 ms, 2
+// views of 96 x 88 x 72 in FP64 2.09 -> 1.17 ms.  Kernels of even sizes stay on the blocks: two of
 // them reach one voxel further to one side than the grid's overlap of k - 1, so what they leave
 // at a block's edge belongs to the grid.  A forced schedule, or one of the environment
 // switches of the block kernels, keeps the steps on the blocks.

@@ -12,7 +12,7 @@
 //
 // Three or more CTAs per SM, so that one CTA's loads overlap another's transforms: the passes are
 // bound by instruction issue and HBM traffic together.  65536 rows of 288 reals (one view of 256^3),
-// algorithmic bytes: forward 38 us (3.8 TB/s), quotient 54 us (4.1 TB/s), update 60 us (4.6 TB/s).
+// algorithmic bytes: forward 37 us (3.9 TB/s), quotient 56 us (3.9 TB/s), update 61 us (4.5 TB/s).
 #pragma once
 #include "pdl.cuh"
 #include "per_device.h"

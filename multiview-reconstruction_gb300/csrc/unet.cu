@@ -779,8 +779,7 @@ extern "C" int mvr_unet_set_input(mvr_unet *h, const float *psi, const float *ps
 {
     return h ? h->net->set_input(psi, psi_next, psi_target) : MVR_ERR_ARG;
 }
-// inference: the decoder convolutions read [up(low), skip] directly (the training step keeps the
-// concatenations for its backward pass)
+// inference: the head is formed in the last convolution's epilogue (the training step keeps its input)
 extern "C" int mvr_unet_forward(mvr_unet *h, float *pred) { return h ? h->net->forward(pred) : MVR_ERR_ARG; }
 extern "C" int mvr_unet_train_step(mvr_unet *h, float lr, double *loss)
 {
