@@ -393,6 +393,7 @@ int Engine<T>::init(int device, int boundary, double lambda, float min_value)
     MVR_CUDA(cudaSetDevice(device));
     MVR_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     set_smem_limits<T>();
+    if (sizeof(T) == sizeof(float)) xy_limits();
     return OK;
 }
 
@@ -1400,6 +1401,7 @@ int Engine<T>::sep_fill(SepPlan &pl, const int P[3], const float *k1, const floa
             pl.kd[d] = kd[d];
         }
         cudaError_t e = cudaSuccess;
+        MVR_CUDA(sep_ready(P));
         pl.twx = dev_twiddles_impl<float2>(P[0], stream_, e);
         pl.twy = dev_twiddles_impl<float2>(P[1], stream_, e);
         pl.twz = dev_twiddles_impl<float2>(P[2], stream_, e);

@@ -66,6 +66,16 @@ int sep_row_ctas(int Px, int rows)
     return o ? (rows + o->rows - 1) / o->rows : 0;
 }
 
+cudaError_t sep_ready(const int P[3])
+{
+    const SxOps *x = sx_ops(P[0]);
+    const YzOps *y = yz_ops(P[1]), *z = yz_ops(P[2]);
+    if (!x || !y || !z) return cudaErrorInvalidValue;
+    cudaError_t e = x->ready();
+    if (e == cudaSuccess) e = y->ready();
+    return e == cudaSuccess ? z->ready() : e;
+}
+
 cudaError_t sep_x_fwd(const SepGeom &g, const SepTiles &tl, int nt, const SepSrc &src, float2 *S, const float2 *twx,
                       cudaStream_t s)
 {

@@ -89,6 +89,10 @@ struct SepUpd {
     double *partials;     // {sum, max} per CTA, or NULL: no statistics
 };
 
+// Shared-memory opt-ins of the passes of a domain, on the current device: made with the plan, not asked for
+// by each launch.
+cudaError_t sep_ready(const int P[3]);
+
 // x passes.  CTAs per tile of a pass over `rows` rows, and slots of its partials.
 int sep_row_ctas(int Px, int rows);
 cudaError_t sep_x_fwd(const SepGeom &g, const SepTiles &tl, int nt, const SepSrc &src, float2 *S, const float2 *twx,

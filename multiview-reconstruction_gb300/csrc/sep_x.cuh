@@ -703,6 +703,7 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_UPD)
 
 struct SxOps {
     int rows;  // per CTA
+    cudaError_t (*ready)();  // on the current device, before the first launch there
     cudaError_t (*fwd)(const SepGeom &, const SepTiles &, int, int, const SepSrc &, float2 *, int, const float2 *,
                        cudaStream_t);
     cudaError_t (*ratio)(const SepGeom &, const SepTiles &, int, int, const float *, float2 *, int, const float2 *,
@@ -737,22 +738,16 @@ struct Sx {
     static cudaError_t fwd(const SepGeom &g, const SepTiles &tl, int nt, int ctas, const SepSrc &src, float2 *S, int vec,
                            const float2 *tw, cudaStream_t s)
     {
-        const cudaError_t e = ready();
-        if (e != cudaSuccess) return e;
         return launch_pdl(k_sep_x_fwd<V>, dim3(ctas, nt), SH::NT, SH::smem, s, src, S, tl, g, vec, tw);
     }
     static cudaError_t ratio(const SepGeom &g, const SepTiles &tl, int nt, int ctas, const float *img, float2 *S,
                              int vec, const float2 *tw, cudaStream_t s, bool first)
     {
-        const cudaError_t e = ready();
-        if (e != cudaSuccess) return e;
         return launch_dep(first, k_sep_x_ratio<V>, dim3(ctas, nt), SH::NT, SH::smem, s, S, img, tl, g, vec, tw);
     }
     static cudaError_t update(const SepGeom &g, const SepTiles &tl, int nt, int ctas, int epi, const SepUpd &u,
                               const float2 *S, int vec, const float2 *tw, cudaStream_t s, bool first)
     {
-        const cudaError_t e = ready();
-        if (e != cudaSuccess) return e;
         const dim3 grid(ctas, nt);
         const bool st = u.partials && (epi == EPI_SEQ || epi == EPI_MUL_FINAL);
 #define SX_UPD(M, ST) launch_dep(first, k_sep_x_update<V, M, ST>, grid, SH::NT, SH::smem, s, S, u, epi, tl, g, vec, tw)
@@ -762,7 +757,7 @@ struct Sx {
     }
     static const SxOps *ops()
     {
-        static const SxOps o = {SH::R, &fwd, &ratio, &update};
+        static const SxOps o = {SH::R, &ready, &fwd, &ratio, &update};
         return &o;
     }
 };

@@ -341,6 +341,7 @@ __global__ void __launch_bounds__(YzShape<T, V>::NT, YzShape<T, V>::MINB_Z)
 
 // The launches of one length.
 struct YzOps {
+    cudaError_t (*ready)();  // on the current device, before the first launch there
     cudaError_t (*y_fwd)(const SepGeom &, const SepSlab &, const SepTiles &, int, int, int, int, float2 *, const float2 *,
                          cudaStream_t, int);
     cudaError_t (*y_inv)(const SepGeom &, const SepSlab &, const SepTiles &, int, int, float2 *, const float2 *,
@@ -369,22 +370,16 @@ struct Yz {
     static cudaError_t y_fwd(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int map, int kdy, int kdz, float2 *S,
                              const float2 *tw, cudaStream_t s, int planes)
     {
-        const cudaError_t e = ready();
-        if (e != cudaSuccess) return e;
         return launch_dep(sl.first, k_sep_y_fwd<T, V>, dim3(sl.n, planes, nt), SH::NT, SH::smem, s, S, tl, g, sl, map, kdy, kdz, tw);
     }
     static cudaError_t y_inv(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int out_w, float2 *S, const float2 *tw,
                              cudaStream_t s, int planes)
     {
-        const cudaError_t e = ready();
-        if (e != cudaSuccess) return e;
         return launch_dep(sl.first, k_sep_y_inv<T, V>, dim3(planes, sl.n, nt), SH::NT, SH::smem, s, S, tl, g, sl, out_w, tw);
     }
     static cudaError_t z(const SepGeom &g, const SepSlab &sl, const SepTiles &tl, int nt, int map, int out_w, int kdz, const float2 *src,
                          float2 *dst, const float2 *K, const float2 *tw, cudaStream_t s)
     {
-        const cudaError_t e = ready();
-        if (e != cudaSuccess) return e;
         const dim3 grid(sl.n * g.P[1] + (sl.x0 == 0 ? (g.P[1] + 15) / 16 : 0), nt);
         if (K)
             return launch_dep(sl.first, k_sep_z<T, V, true>, grid, SH::NT, SH::smem, s, src, dst, K, tl, g, sl, map, out_w, kdz, tw);
@@ -392,7 +387,7 @@ struct Yz {
     }
     static const YzOps *ops()
     {
-        static const YzOps o = {&y_fwd, &y_inv, &z};
+        static const YzOps o = {&ready, &y_fwd, &y_inv, &z};
         return &o;
     }
 };

@@ -160,25 +160,10 @@ int pair_clusters()
     return n;
 }
 
-void set_limits()
-{
-    static PerDevice once;
-    once([] {
-        set_limits_pair<6, 6>();
-        set_limits_pair<8, 8>();
-        set_limits_one<4, 8>();
-        set_limits_one<4, 12>();
-        set_limits_one<6, 8>();
-        set_limits_one<6, 12>();
-        return cudaSuccess;
-    });
-}
-
 template <class Src>
 cudaError_t fwd(int combo, const Src &src, float2 *S, const BlockMaps &bms, int nb, int Pz, long long Pc,
                 const float2 *twx, const float2 *twy, cudaStream_t s, bool persist)
 {
-    set_limits();
     const int nitems = Pz * nb;
     if (combo >= 10000) {
         PAIR_DISPATCH(combo, return launch_pair(k_xy2_fwd<VX_, VH_, Src>,
@@ -194,6 +179,21 @@ cudaError_t fwd(int combo, const Src &src, float2 *S, const BlockMaps &bms, int 
 }
 
 }  // namespace
+
+// Shared-memory opt-ins on the current device, once for each.
+void xy_limits()
+{
+    static PerDevice once;
+    once([] {
+        set_limits_pair<6, 6>();
+        set_limits_pair<8, 8>();
+        set_limits_one<4, 8>();
+        set_limits_one<4, 12>();
+        set_limits_one<6, 8>();
+        set_limits_one<6, 12>();
+        return cudaSuccess;
+    });
+}
 
 cudaError_t xy_fwd_mirror(int combo, const float *psi, float2 *S, const BlockMaps &bms, int nb, int Pz, long long Pc,
                           const float2 *twx, const float2 *twy, cudaStream_t s, bool persist)
@@ -216,7 +216,6 @@ cudaError_t xy_fwd_kernel(int combo, const SrcKernel &src, float2 *S, const Bloc
 cudaError_t xy_ratio(int combo, float2 *S, const float *img, const BlockMaps &bms, int nb, int z0, int nzb,
                      long long Pc, const float2 *twx, const float2 *twy, cudaStream_t s, bool persist)
 {
-    set_limits();
     const int nitems = nzb * nb;
     if (combo >= 10000) {
         PAIR_DISPATCH(combo, return launch_pair(k_xy2_ratio<VX_, VH_>,
@@ -234,7 +233,6 @@ cudaError_t xy_ratio(int combo, float2 *S, const float *img, const BlockMaps &bm
 cudaError_t xy_update(int combo, int epi, float2 *S, const UpdateArgs &ua, const BlockMaps &bms, int nb, int Pz,
                       long long Pc, const float2 *twx, const float2 *twy, cudaStream_t s)
 {
-    set_limits();
     int planes = Pz;
     if (ua.prune) {
         if (epi == EPI_STORE) return cudaErrorInvalidValue;

@@ -7,6 +7,8 @@
 
 namespace mvr {
 
+// The kernels' shared-memory opt-ins on the current device, before the first launch there.
+void xy_limits();
 // The plane-kernel shape for an FP32 FFT domain P (x, y), or 0 when none exists.
 int xy_combo(const int P[3]);
 // The pair-kernel shape (two CTAs per plane, a thread-block cluster) for P, or 0.  Shape codes
