@@ -75,22 +75,24 @@ cudaError_t launch_march(const MarchArgs &a, const ConvGeom &g, int *err, cudaSt
 }
 
 // Weight gradient (k_wgrad_march): runs as in launch_march, as many CTAs per SM as share its tensor memory
-template <int N, int C, int CU = 0>
+template <int N, int C, int CU = 0, bool RAGGED = false>
 cudaError_t launch_wgrad(const bf16 *X, const bf16 *G, float *dW, const ConvGeom &g, int *err, cudaStream_t s,
                          const bf16 *X2 = nullptr)
 {
+    if constexpr (!RAGGED)
+        if (g.W % kMarchX || g.H % kMarchY) return launch_wgrad<N, C, CU, true>(X, G, dW, g, err, s, X2);
     if ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(X2) | reinterpret_cast<uintptr_t>(G)) & 15)
         return cudaErrorInvalidValue;
     const size_t sm = wgrad_march_smem<N, C>();
     cudaError_t e =
-        cudaFuncSetAttribute(k_wgrad_march<N, C, CU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaFuncSetAttribute(k_wgrad_march<N, C, CU, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     const long long planes =
         (long long)((g.W + kMarchX - 1) / kMarchX) * ((g.H + kMarchY - 1) / kMarchY) * g.B * g.D;
     constexpr int NG = wgrad_splits<N, C, CU>();
     const long long res = std::max<long long>(1, std::min<long long>((227 * 1024) / (sm + 1024), 512 / wgrad_cols<N, C, CU>()));
     const long long grid = std::min<long long>(152 * res / NG, (planes + kMarchMin - 1) / kMarchMin);
-    k_wgrad_march<N, C, CU><<<dim3((unsigned)grid, NG), kMarchThreads, sm, s>>>(X, G, dW, g, err, X2);
+    k_wgrad_march<N, C, CU, RAGGED><<<dim3((unsigned)grid, NG), kMarchThreads, sm, s>>>(X, G, dW, g, err, X2);
     return cudaGetLastError();
 }
 
