@@ -213,7 +213,7 @@ extern "C" int mvr_block_set_kernels(mvr_block *h, int view, const float *k1, co
     }
     // separable transforms wherever the block has them: 192^3 circular 127 us against 163 us of the
     // plane kernels, 256^3 304 / 467 us, 156 x 156 x 124 with the reference's extensions (domains
-    // without plane kernels) 70 / 320 us, 40 x 36 x 44 20 / 34 us
+    // without plane kernels) 62 / 320 us, 40 x 36 x 44 20 / 34 us; padded the most, 2.5 to 5 times faster (sep.cu)
     int P[3];
     if (!mvr::block_kernels_forced() && mvr::block_tile(h->b, ks, h->eng.boundary(), P, h->tiles[view])) {
         const int rc = h->eng.sep_make(h->seps[view], P, k1, k2, ks, false);
