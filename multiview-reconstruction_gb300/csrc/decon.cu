@@ -311,11 +311,11 @@ __global__ void k_block_content(const float *__restrict__ w, long long D0, long 
 }
 
 // Energy, voxels with data and voxels of each block's box inside the volume, the box as in k_block_content:
-// out[3 b .. 3 b + 2], zeroed before.  A warp takes a row of the box.
+// out[3 b .. 3 b + 2], zeroed before.  A warp takes a row of the box.  Block blockIdx.x (there may be more than 65535).
 __global__ void __launch_bounds__(256) k_block_level(const float *__restrict__ img, int D0, int D1, int D2,
                                                      const long long *__restrict__ offs, int bx, int by, int bz, double *out)
 {
-    const int blk = blockIdx.y;
+    const int blk = blockIdx.x;
     int lo[3], n[3];
     const int D[3] = {D0, D1, D2}, b[3] = {bx, by, bz};
     for (int d = 0; d < 3; ++d) {
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(256) k_block_level(const float *__restrict__ i
     }
     float e = 0.0f, data = 0.0f;  // a thread's: below 2^24 voxels
     const int rows = n[1] * n[2];
-    for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8) {
+    for (int r = blockIdx.y * 8 + (threadIdx.x >> 5); r < rows; r += gridDim.y * 8) {
         const int z = r / n[1], y = r - z * n[1];
         const float *p = img + ((long long)(lo[2] + z) * D1 + lo[1] + y) * D0 + lo[0];
         for (int x = threadIdx.x & 31; x < n[0]; x += 32) {
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(256) k_block_level(const float *__restrict__ i
     if (threadIdx.x & 31) return;
     atomicAdd(out + 3 * blk, (double)e);
     atomicAdd(out + 3 * blk + 1, (double)data);
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[3 * blk + 2] = (double)n[0] * rows;
+    if (blockIdx.y == 0 && threadIdx.x == 0) out[3 * blk + 2] = (double)n[0] * rows;
 }
 
 // Tiles of several launches: the marks (BadMap) of one launch's psi and quotients concern voxels of others,
@@ -1088,7 +1088,7 @@ int Decon<T>::dim_blocks(int st, double &ratio)
     for (int v = p_.mul ? 0 : st; e == cudaSuccess && v < (p_.mul ? p_.num_views : st + 1); ++v) {
         e = cudaMemsetAsync(d_out, 0, sizeof(double) * h.size(), s);
         if (e != cudaSuccess) break;
-        k_block_level<<<dim3(64, (unsigned)bl.size()), 256, 0, s>>>(
+        k_block_level<<<dim3((unsigned)bl.size(), 64), 256, 0, s>>>(
             views_[v].img, p_.dims[0], p_.dims[1], p_.dims[2], d_offs, cs[0], cs[1], cs[2], d_out);
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), d_out, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, s);

@@ -2,7 +2,7 @@
  * code (test_host_runtime.py): FAKE_DEVICES devices whose memory is host memory, kernels that do
  * nothing, and the checks of the real runtime that depend on the calling thread's device: a launch
  * goes to a stream of the current device, and needs the opt-in of that device for more than 48 KB of
- * dynamic shared memory.  fake_fail() makes a later call fail; fake_live() counts what is allocated. */
+ * dynamic shared memory.  Grids are checked too: at most 65535 blocks along y and z.  fake_fail() makes a later call fail; fake_live() counts what is allocated. */
 #define _GNU_SOURCE
 #include <stddef.h>
 #include <stdlib.h>
@@ -213,9 +213,10 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const
     *n = 1;
     return cudaSuccess;
 }
-static cudaError_t launch(const void *f, size_t smem, cudaStream_t s)
+static cudaError_t launch(const void *f, Dim g, size_t smem, cudaStream_t s)
 {
     ++launches;
+    if (!g.x || !g.y || !g.z || g.x > 2147483647u || g.y > 65535 || g.z > 65535) return ret(cudaErrorInvalidConfiguration);
     if (fails(1)) return ret(cudaErrorLaunchFailure);
     if (s && ((struct stream *)s)->dev != cur) return ret(cudaErrorInvalidResourceHandle);
     if (smem > 48 * 1024 && smem > (size_t)funcs[func_at(f)].bytes[cur]) return ret(cudaErrorInvalidValue);
@@ -224,7 +225,7 @@ static cudaError_t launch(const void *f, size_t smem, cudaStream_t s)
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **args)
 {
     (void)args;
-    return launch(f, c->dynamicSmemBytes, c->stream);
+    return launch(f, (Dim){c->gridDim.x, c->gridDim.y, c->gridDim.z}, c->dynamicSmemBytes, c->stream);
 }
 
 static struct {
@@ -255,8 +256,8 @@ cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *f)
 }
 cudaError_t __cudaLaunchKernel(cudaKernel_t k, Dim g, Dim b, void **args, size_t smem, cudaStream_t s)
 {
-    (void)g, (void)b, (void)args;
-    return launch((const void *)k, smem, s);
+    (void)b, (void)args;
+    return launch((const void *)k, g, smem, s);
 }
 void **__cudaRegisterFatBinary(void *f)
 {

@@ -176,3 +176,14 @@ with M.Deconvolution(D, n, b, mul={mul}, psf_type=M.PSF_INDEPENDENT, filter_bloc
         d.run_iterations(1)
         assert F.fake_launches() - f0 == d.launch_count() - c0, (F.fake_launches() - f0, d.launch_count() - c0)
 """)
+
+
+def test_more_blocks_than_a_grid_has_rows(fake):
+    # 70000 blocks of 16 voxels, 12 apart: prepare looks at their levels in one launch
+    run(fake, """
+D = (840000, 3, 3)
+with M.Deconvolution(D, 1, (16, 16, 16), psf_type=M.PSF_INDEPENDENT, filter_blocks=False) as d:
+    d.set_view(0, A(D), A(D), K((3, 3, 3)))
+    d.prepare()
+    d.run_iterations(1)
+""")
