@@ -212,9 +212,10 @@ __device__ __forceinline__ void sx_load_zero(float2 (&a)[V], const float *row, i
         }
     }
 }
-// The same under the mirror-single extension of [0, N).
+// The same under the mirror-single extension of [0, N), no voxel beyond `last` (the last one that the tile
+// takes from psi: a domain that is longer would hold the magnitudes of others).
 template <int V, bool PAIRS>
-__device__ __forceinline__ void sx_load_mirror(float2 (&a)[V], const float *row, int g0, int N,
+__device__ __forceinline__ void sx_load_mirror(float2 (&a)[V], const float *row, int g0, int N, int last,
                                                unsigned long long pol)
 {
     const float *p = row + g0;
@@ -222,12 +223,12 @@ __device__ __forceinline__ void sx_load_mirror(float2 (&a)[V], const float *row,
 #pragma unroll
     for (int v = 0; v < V; ++v) {
         const int g = g0 + 32 * v;
-        if (PAIRS && (unsigned)g < (unsigned)N) {
+        if (PAIRS && (unsigned)g < (unsigned)last) {
             a[v] = sep_ld2(p + 32 * v, pol);
         } else {
             const int i = abs(g), j = abs(g + 1);
-            a[v].x = sep_ld(row + min(max(min(i, top - i), 0), N - 1), pol);
-            a[v].y = sep_ld(row + min(max(min(j, top - j), 0), N - 1), pol);
+            a[v].x = sep_ld(row + min(max(min(i, top - i), 0), last), pol);
+            a[v].y = sep_ld(row + min(max(min(j, top - j), 0), last), pol);
         }
     }
 }
@@ -297,14 +298,14 @@ __device__ __forceinline__ void sx_p1_sums(float2 *p, const float2 *tw, int t, X
 }
 // psi: the item at x = g0 + 32 v + {0, 1} of the row at (y, z)
 template <int V>
-__device__ __forceinline__ void sx_fwd_again(BadMap *b, const float *row, float2 *p, const float2 *tw, int t, int g0, int N, int y,
-                                             int z)
+__device__ __forceinline__ void sx_fwd_again(BadMap *b, const float *row, float2 *p, const float2 *tw, int t, int g0, int N,
+                                             int last, int y, int z)
 {
     sx_p1_sums<V>(p, tw, t, [&](int v) {
         float c[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int i = abs(g0 + 32 * v + h), j = min(max(min(i, 2 * N - 2 - i), 0), N - 1);
+            const int i = abs(g0 + 32 * v + h), j = min(max(min(i, 2 * N - 2 - i), 0), last);
             c[h] = row[j];
             if (sx_finite(c[h])) continue;
             bad_mark(b, BAD_PSI, j, y, z);
@@ -373,8 +374,9 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_FWD)
             for (int v = 0; v < V; ++v) a[v] = make_float2(0.0f, 0.0f);
         } else if (!src.kernel) {
             const float *p = src.vol + base;
-            if (pairs) sx_load_mirror<V, true>(a, p, t.a[0].lo + 2 * q, t.a[0].N, pol);
-            else sx_load_mirror<V, false>(a, p, t.a[0].lo + 2 * q, t.a[0].N, pol);
+            const int last = t.a[0].v0 + t.a[0].nv - 1;
+            if (pairs) sx_load_mirror<V, true>(a, p, t.a[0].lo + 2 * q, t.a[0].N, last, pol);
+            else sx_load_mirror<V, false>(a, p, t.a[0].lo + 2 * q, t.a[0].N, last, pol);
         } else {  // taps wrapped around the origin, scaled
             const int r = r0 + row, z = r / ny, y = r - z * ny;
             const float *p = src.vol + ((long long)z * src.kd[1] + y) * src.kd[0];
@@ -401,7 +403,7 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_FWD)
             if (!(again >> it / SH::NT & 1)) continue;
             const int q = it & 15, row = it >> 4, r = r0 + row;
             sx_fwd_again<V>(g.bad, src.vol + sr.a[row], A + row * kSepRS + q, tw, q, t.a[0].lo + 2 * q, t.a[0].N,
-                            t.a[1].v0 + r % ny, t.a[2].v0 + r / ny);
+                            t.a[0].v0 + t.a[0].nv - 1, t.a[1].v0 + r % ny, t.a[2].v0 + r / ny);
         }
     __syncthreads();
     sx_p2<V, false>(A, tw);
@@ -432,7 +434,8 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_RATIO)
     float2 *base = S + (long long)blockIdx.y * g.stride;
     const long long bstride = (long long)g.Zs * g.P[1] * 16;
     const unsigned long long pol = sep_policy(g.stream);
-    const bool pairs = sx_pairs(vec, t.a[0], 0, t.a[0].N);
+    const int end = t.a[0].v0 + t.a[0].nv;  // no image beyond the tile's psi: N, or the end of a dim block
+    const bool pairs = sx_pairs(vec, t.a[0], 0, end);
     unsigned again = 0;
     sx_flag(sr.flag, g.bad ? &g.bad->any[BAD_PSI] : nullptr, [&] { sx_load_lines<V>(A, base, bstride, sr.b); });
     __syncthreads();
@@ -443,7 +446,7 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_RATIO)
         const long long ib = sr.a[row];
         constexpr bool EARLY = V < 12;  // the image ahead of the transform, as the registers allow
         float2 im[V], a[V];
-        const int n = ib < 0 ? 0 : t.a[0].N;  // no row: no voxel
+        const int n = ib < 0 ? 0 : end;  // no row: no voxel
         if (EARLY) {
             if (pairs) sx_load_zero<V, true>(im, img + ib, t.a[0].lo + 2 * q, 0, n, pol);
             else sx_load_zero<V, false>(im, img + ib, t.a[0].lo + 2 * q, 0, n, pol);
@@ -473,7 +476,7 @@ __global__ void __launch_bounds__(SxShape<V>::NT, SxShape<V>::MINB_RATIO)
             const int q = it & 15, row = it >> 4, r = r0 + row;
             if (sr.a[row] < 0) continue;
             sx_ratio_again<V>(g.bad, img + sr.a[row], A + row * kSepRS + q, base + sr.b[row] + q, bstride, tw, q,
-                              t.a[0].lo + 2 * q, t.a[0].N, t.a[1].q0 + r % t.a[1].nq, t.a[2].q0 + r / t.a[1].nq);
+                              t.a[0].lo + 2 * q, end, t.a[1].q0 + r % t.a[1].nq, t.a[2].q0 + r / t.a[1].nq);
         }
     if (sr.flag) {  // the quotients of a block that reads it, where the image is positive
         const int N = t.a[0].N;

@@ -264,6 +264,37 @@ def test_dim_blocks_far_from_bright_ones(mul):
     assert np.abs(out[dark] / ref[dark] - 1).max() <= 1e-5
 
 
+@pytest.mark.parametrize("mul", [False, True])
+def test_dim_block_beside_bright_voxels_it_does_not_read(mul):
+    # beads of 2e4 in columns 364 to 387 alone: the block of [176, 352) reads [168, 360), its domain of 224 would
+    # reach to column 392.  Voxels below 344 (the second view's step reads the first one's 8 columns beyond) keep
+    # the rounding of their own transforms.  Tolerance as above
+    fft = pytest.importorskip("scipy.signal")
+    dims, kd, block, nv = (560, 48, 48), (9, 9, 9), (192, 64, 64), 2
+    rng = np.random.default_rng(37)
+    shape = dims[::-1]
+    psi = rng.uniform(1e-3, 2e-3, shape).astype(np.float32)
+    psi[rng.integers(0, 48, 30), rng.integers(0, 48, 30), rng.integers(364, 388, 30)] = 2e4
+    psfs = [synthetic.make_psf(kd, 1.0, 1.5, 40.0 * v) for v in range(nv)]
+    imgs = [np.maximum(fft.fftconvolve(psi.astype(np.float64), p.astype(np.float64), "same"), 1e-3) for p in psfs]
+    imgs = [(i * rng.uniform(0.7, 1.4, shape)).astype(np.float32) for i in imgs]
+    ws = [rng.uniform(0.2, 0.5, shape).astype(np.float32) for _ in range(nv)]
+    with M.Deconvolution(dims, nv, block, mul=mul, psf_type=M.PSF_INDEPENDENT, lam=0.006) as d:
+        for v in range(nv):
+            d.set_view(v, imgs[v], ws[v], psfs[v])
+        d.prepare()
+        d.set_psi(psi)
+        ks = [d.kernels(v, psfs[v].shape) for v in range(nv)]
+        mx = d.max_intensities()
+        d.run_iterations(1)
+        out = d.get_psi()
+    ref, _ = O.decon_run(psi, imgs, ws, [k[0] for k in ks], [k[1] for k in ks], block, 1, mul=mul, lam=0.006,
+                         max_intensities=mx, fp64=True)
+    assert rel(out, ref) <= 1e-5
+    assert ref[:, :, :344].max() < 0.1
+    assert np.abs(out[:, :, :344] / ref[:, :, :344] - 1).max() <= 1e-5
+
+
 def test_quotient_by_a_value_above_2_to_126():
     # a hot voxel of 1.2e38, a kernel of one voxel: the quotient 1e38 / 1.2e38 (the approximate division alone
     # returns 0 there), psi becomes 1e38.  A periodic domain: an extended one can hold mirror images of the
