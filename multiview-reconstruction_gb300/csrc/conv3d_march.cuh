@@ -452,7 +452,8 @@ __device__ __forceinline__ float wgrad_again(const __nv_bfloat16 *X, const __nv_
     return s;
 }
 
-// RAGGED: a kernel of its own, whose registers cost the other 1 to 5 %.
+// RAGGED: a kernel of its own, whose registers cost the other 1 to 5 %.  One check per 16 sums, behind which they are
+// added as without it: a training step on 60 x 36 x 40 takes 347 us, 339 unchecked, 558 with every sum picked out and checked.
 template <int N, int C, int CU, bool RAGGED>
 __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat16 *__restrict__ X,
                                                                const __nv_bfloat16 *__restrict__ G, float *dW,
@@ -591,22 +592,25 @@ __global__ void __launch_bounds__(kMarchThreads) k_wgrad_march(const __nv_bfloat
             for (int c0 = 0; c0 < N; c0 += 16) {
                 float v[16];
                 tc::tmem_ld16(trow + (uint32_t)(e * N + c0), v);
-                if constexpr (!RAGGED) {
-                    if (rv)
+                bool finite = true;
+                if constexpr (RAGGED)
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            atomicAdd(&dW[((long long)(c0 + j) * 27 + tap) * C + ci], v[j]);
-                } else {
+                    for (int j = 0; j < 16; ++j) finite = finite && fabsf(v[j]) <= 3.402823466e38f;
+                if (rv && finite)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        atomicAdd(&dW[((long long)(c0 + j) * 27 + tap) * C + ci], v[j]);
+                if constexpr (RAGGED) {
+                    if (rv && !finite)
 #pragma unroll 1
-                    for (int j = 0; j < 16; ++j) {
-                        float a = v[0];
+                        for (int j = 0; j < 16; ++j) {
+                            float a = v[0];
 #pragma unroll
-                        for (int i = 1; i < 16; ++i) a = i == j ? v[i] : a;
-                        if (!rv) continue;
-                        if (!(fabsf(a) <= 3.402823466e38f))
-                            a = wgrad_again<N, C, CU>(X, X2, G, g, planes * blockIdx.x / gridDim.x, u1, tap, ci, c0 + j);
-                        atomicAdd(&dW[((long long)(c0 + j) * 27 + tap) * C + ci], a);
-                    }
+                            for (int i = 1; i < 16; ++i) a = i == j ? v[i] : a;
+                            if (!(fabsf(a) <= 3.402823466e38f))
+                                a = wgrad_again<N, C, CU>(X, X2, G, g, planes * blockIdx.x / gridDim.x, u1, tap, ci, c0 + j);
+                            atomicAdd(&dW[((long long)(c0 + j) * 27 + tap) * C + ci], a);
+                        }
                     __syncwarp();
                 }
             }
